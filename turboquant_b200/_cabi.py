@@ -37,6 +37,7 @@ EXPORTS = (
 )
 
 _lib = None
+_native = None
 
 
 class TurboQuantError(RuntimeError):
@@ -56,6 +57,22 @@ def lib() -> ctypes.CDLL:
         L.tq_decode_workspace_bytes.restype = ctypes.c_size_t
         _lib = L
     return _lib
+
+
+def native():
+    """The native call path (csrc/tq_torch.cpp) bound to the library's entry points: calls whose tensors need no
+    conversion skip the Python checks and the ctypes boxing below."""
+    global _native
+    if _native is None:
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise TurboQuantError(f"turboquant_b200._native is missing or does not load ({e}): build it with "
+                                  "`python -m turboquant_b200.build`") from None
+        L = lib()
+        module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in EXPORTS}, TurboQuantError)
+        _native = module
+    return _native
 
 
 def _check(rc: int) -> None:
@@ -170,6 +187,9 @@ def write_kv_cache(kv_cache: torch.Tensor, key: torch.Tensor, value: torch.Tenso
 
 
 def quantize_flat(x: torch.Tensor, signs: torch.Tensor, bits: int, cache_order: bool = False):
+    done = native().quantize_flat(x, signs, bits, cache_order)
+    if done is not None:
+        return done
     _cuda(x, "x")
     _cuda(signs, "signs")
     x = x.contiguous()
@@ -189,6 +209,9 @@ def quantize_flat(x: torch.Tensor, signs: torch.Tensor, bits: int, cache_order: 
 
 def dequantize_flat(packed: torch.Tensor, norms: torch.Tensor, signs: torch.Tensor, dim: int,
                     bits: int, cache_order: bool = False) -> torch.Tensor:
+    done = native().dequantize_flat(packed, norms, signs, dim, bits, cache_order)
+    if done is not None:
+        return done
     _cuda(packed, "packed")
     _cuda(norms, "norms")
     packed = packed.contiguous()

@@ -1,13 +1,15 @@
-"""Builds libturboquant_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libturboquant_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and the native call path of the
+Python layer (_native.so, the one file that sees torch's headers) with g++.
 
     python -m turboquant_b200.build [--force]
 
 The cache-write, flat-quantizer and bulk-dequantizer translation units are compiled with -fmad=false: their
 arithmetic must round every product and sum separately to stay bit-identical to the torch
-quantizer.  No torch headers are involved; the library exports plain C symbols only.
+quantizer.  The library itself involves no torch headers and exports plain C symbols only.
 """
 from __future__ import annotations
 
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -17,6 +19,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libturboquant_b200.so"
+NATIVE = PKG / "_native.so"
+NATIVE_SRC = CSRC / "tq_torch.cpp"
 HEADER = PKG.parent / "include" / "turboquant_b200.h"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -41,6 +45,17 @@ def _stale(target: Path, sources) -> bool:
     return any(Path(s).stat().st_mtime > t for s in sources)
 
 
+def _native_command() -> list[str]:
+    import sysconfig
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-isystem", str(root / "include"), "-isystem", str(root / "include/torch/csrc/api/include"),
+            "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"], str(NATIVE_SRC), "-o", str(NATIVE),
+            "-L", str(root / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = PKG / "build"
@@ -58,8 +73,13 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             subprocess.check_call(cmd)
         return obj
 
-    with ThreadPoolExecutor(max_workers=4) as ex:
+    with ThreadPoolExecutor(max_workers=5) as ex:
+        native = None
+        if force or _stale(NATIVE, [NATIVE_SRC, HEADER, Path(__file__)]):
+            native = ex.submit(subprocess.check_call, _native_command())
         objs = list(ex.map(compile_one, UNITS.items()))
+        if native:
+            native.result()
     if force or _stale(LIB, objs):
         subprocess.check_call(["nvcc", *ARCH, "-shared", "-o", str(LIB), *map(str, objs)])
     return LIB

@@ -944,6 +944,40 @@ int write_guard_stats(unsigned long long* out2) {
     return TQ_OK;
 }
 
+// The code search's table, as the kernels' float operations bin the boundaries; `problem` names a codebook it cannot serve.
+struct BinTable {
+    float2 entry[kBins];
+    const char* problem;
+};
+static BinTable make_bin_table() {
+    BinTable t{};
+    float cen[16], bnd[15];
+    host_codebook(kD, 4, cen, bnd);
+    int bin_of[15];
+    for (int i = 0; i < 15; i++) {
+        volatile float kf = fmaf(bnd[i], 64.0f, kBinMagic);
+        float kff = kf;
+        uint32_t bits;
+        memcpy(&bits, &kff, 4);
+        bin_of[i] = (int)(bits - 0x4B000000u);
+        if (bin_of[i] < 0 || bin_of[i] >= kBins || (i > 0 && bin_of[i] <= bin_of[i - 1])) t.problem = "boundaries too close for the bin table";
+        // the guarded kernel may look a value next to a bin edge up in either neighbour: no
+        // boundary may sit that close to an edge (edges are at (k +- 1/2) / 64)
+        const double pos = (double)bnd[i] * 64.0 - std::floor((double)bnd[i] * 64.0 + 0.5);
+        if (std::fabs(std::fabs(pos) - 0.5) * (1.0 / 64.0) <= 1.0 / 8192.0) t.problem = "a boundary lies next to a bin edge";
+    }
+    for (int k = 0; k < kBins; k++) {
+        int below = 0;
+        float inside = INFINITY;  // no boundary in this bin: the comparison is never true
+        for (int i = 0; i < 15; i++) {
+            if (bin_of[i] < k) below++;
+            if (bin_of[i] == k) inside = bnd[i];
+        }
+        t.entry[k] = make_float2(inside, (float)below);
+    }
+    return t;
+}
+
 int device_sm_count(int* out);
 int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv_heads, int slot_bytes, const void* key,
                   const void* value, int in_dtype, int64_t num_tokens, int64_t k_token_stride, int64_t v_token_stride,
@@ -1012,34 +1046,10 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
     p.slot_is_i64 = slot_dtype == TQ_I64;
     p.zero_pad = (flags & TQ_WRITE_ZERO_PAD) != 0;
     p.signs = signs;
-    float cen[16], bnd[15];
-    host_codebook(kD, 4, cen, bnd);
-    {   // bins of y (same float operations as the kernel's code_f)
-        int bin_of[15];
-        for (int i = 0; i < 15; i++) {
-            volatile float kf = fmaf(bnd[i], 64.0f, kBinMagic);
-            float kff = kf;
-            uint32_t bits;
-            memcpy(&bits, &kff, 4);
-            bin_of[i] = (int)(bits - 0x4B000000u);
-            TQ_REQUIRE(bin_of[i] >= 0 && bin_of[i] < kBins && (i == 0 || bin_of[i] > bin_of[i - 1]), TQ_ERR_UNSUPPORTED,
-                       "boundaries too close for the bin table");
-            // the guarded kernel may look a value next to a bin edge up in either neighbour: no
-            // boundary may sit that close to an edge (edges are at (k +- 1/2) / 64)
-            const double pos = (double)bnd[i] * 64.0 - std::floor((double)bnd[i] * 64.0 + 0.5);
-            TQ_REQUIRE(std::fabs(std::fabs(pos) - 0.5) * (1.0 / 64.0) > 1.0 / 8192.0, TQ_ERR_UNSUPPORTED,
-                       "a boundary lies next to a bin edge");
-        }
-        for (int k = 0; k < kBins; k++) {
-            int below = 0;
-            float inside = INFINITY;  // no boundary in this bin: the comparison is never true
-            for (int i = 0; i < 15; i++) {
-                if (bin_of[i] < k) below++;
-                if (bin_of[i] == k) inside = bnd[i];
-            }
-            p.bin_table[k] = make_float2(inside, (float)below);
-        }
-    }
+    // built once: the search for every bin cost more host time than the launch of a decode step's few rows
+    static const BinTable table = make_bin_table();
+    TQ_REQUIRE(!table.problem, TQ_ERR_UNSUPPORTED, "%s", table.problem);
+    memcpy(p.bin_table, table.entry, sizeof(p.bin_table));
     p.fwht_scale = (float)(1.0 / sqrt((double)kD));
     int sms = 0;
     int rc = device_sm_count(&sms);

@@ -56,6 +56,16 @@ class TurboQuantPagedAttention:
         self.num_ctas = num_ctas
         self._signs: dict[torch.device, torch.Tensor] = {}
         self._workspaces: dict[tuple, torch.Tensor] = {}
+        self._layer = None
+
+    @property
+    def _calls(self):
+        """This geometry's native call path.  It takes the calls whose tensors need no conversion once the signs and the
+        workspace of the call exist; it answers None to any other, which the methods below then convert, allocate for or
+        refuse.  (Created on first use: it needs the built library.)"""
+        if self._layer is None:
+            self._layer = _cabi.native().Layer(self.num_heads, self.head_size, self.num_kv_heads, self.scale, self.num_ctas)
+        return self._layer
 
     def signs(self, device) -> torch.Tensor:
         device = torch.device(device)
@@ -63,6 +73,7 @@ class TurboQuantPagedAttention:
         if s is None:
             s = make_signs(self.padded_dim, self.seed).to(device)
             self._signs[device] = s
+            self._calls.set_signs(s)
         return s
 
     def workspace(self, batch: int, device, queries: int = 1) -> torch.Tensor:
@@ -76,6 +87,7 @@ class TurboQuantPagedAttention:
                                                   self.head_size, self.num_ctas)
             ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)  # zeroed once: the status word is sticky
             self._workspaces[key] = ws
+            self._calls.set_workspace(batch, queries, ws)
         return ws
 
     @staticmethod
@@ -84,6 +96,8 @@ class TurboQuantPagedAttention:
 
     def write(self, key: torch.Tensor, value: torch.Tensor, kv_cache: torch.Tensor,
               slot_mapping: torch.Tensor, zero_pad: bool = False) -> None:
+        if self._calls.write(key, value, kv_cache, slot_mapping, zero_pad):
+            return
         n = slot_mapping.shape[0]
         if n == 0:
             return
@@ -96,6 +110,9 @@ class TurboQuantPagedAttention:
     def decode(self, query: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor,
                seq_lens: torch.Tensor, output: torch.Tensor | None = None,
                out_lse: torch.Tensor | None = None) -> torch.Tensor:
+        done = self._calls.decode(query, kv_cache, block_table, seq_lens, output, out_lse, False)
+        if done is not None:
+            return done
         if query.dim() == 4:
             return self.decode_shared(query, kv_cache, block_table, seq_lens, output, out_lse)
         if query.dim() == 2:
@@ -121,6 +138,9 @@ class TurboQuantPagedAttention:
         csrc/src/decode_v5_tc_binding.cu:783-785) and stream the KV once per repeat; here the KV
         is streamed once.  queries x (heads / kv_heads) must not exceed 32 (8 for head sizes other than
         128 / 96 and for KV-head counts other than 2, 4, 8, 16: ``_cabi.decode_max_queries_per_seq``)."""
+        done = self._calls.decode(query, kv_cache, block_table, seq_lens, output, out_lse, False) if query.dim() == 4 else None
+        if done is not None:
+            return done
         B, NQ = query.shape[0], query.shape[1]
         if output is None:
             output = torch.empty_like(query)
@@ -143,6 +163,9 @@ class TurboQuantPagedAttention:
         queries x (heads / kv_heads) <= 32 query columns: a chunk of a continuing prefill, or the
         verification step of speculative decoding.  The reference's prefill ignores the cache
         (turboquant/vllm_backend_fused.py:336-369)."""
+        done = self._calls.decode(query, kv_cache, block_table, seq_lens, output, out_lse, True) if query.dim() == 4 else None
+        if done is not None:
+            return done
         B, NQ = query.shape[0], query.shape[1]
         if output is None:
             output = torch.empty_like(query)
@@ -163,6 +186,9 @@ class TurboQuantPagedAttention:
         with the chunk's fresh K / V and run a varlen attention kernel on the result.  The reference's
         prefill ignores the cache (vllm_backend_fused.py:336-369); this is the missing piece for
         chunked prefill over a quantized cache.  ``total_tokens`` is passed by the caller (no sync)."""
+        done = self._calls.dequant(kv_cache, block_table, seq_lens, cu_seqlens, total_tokens, dtype)
+        if done is not None:
+            return done
         dev = kv_cache.device
         k = torch.empty((total_tokens, self.num_kv_heads, self.head_size), dtype=dtype, device=dev)
         v = torch.empty_like(k)
