@@ -31,6 +31,7 @@ UNITS = {
     "tq_flat.cu": ["-fmad=false"],
     "tq_decode.cu": [],
     "tq_decode_mq.cu": [],
+    "tq_decode_split.cu": [],
     "tq_dequant.cu": ["-fmad=false"],
     "tq_pages.cu": [],
     "tq_generic.cu": ["-fmad=false"],

@@ -40,6 +40,7 @@
 // would add a 2-byte-per-element shared-memory round trip to a kernel whose limiters are the
 // shared-memory lookups and instruction issue, not MMA throughput (the tensor pipe is 22% busy).
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "tq_decode_common.cuh"
@@ -846,6 +847,11 @@ int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_hea
                    const float* signs, float sm_scale, void* workspace, size_t workspace_bytes, void* out, int out_dtype,
                    float* out_lse, int emit_rotated, int num_ctas, void* stream);
 
+int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim, int padded,
+                 const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
+                 int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
+                 void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
+                 int all_or_nothing, int ctas, cudaStream_t s);
 bool mq_applicable(int num_kv_heads, int cols);
 int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks, int grid, int causal, cudaStream_t stream);
 
@@ -974,6 +980,11 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
     TQ_REQUIRE(workspace_bytes >= w.total, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, w.total);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
+    static const long long split_max = getenv("TQ_SPLIT_MAX") ? atoll(getenv("TQ_SPLIT_MAX")) : 4096;
+    if (!wide && !x && num_ctas == 0 && (page_indptr ? 0 : (long long)batch * max_pages * num_kv_heads) <= split_max)
+        return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes, page_indices,
+                            page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes, out, out_dtype,
+                            out_lse, emit_rotated, 1, ctas, s);
 
     DecodeParams p{};
     p.q = q;

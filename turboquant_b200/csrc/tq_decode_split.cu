@@ -1,0 +1,908 @@
+// Paged decode attention split over (sequence, KV head, page range): every padded head size (64, 128, 256).
+//
+// The streaming kernel of tq_decode.cu gives a block all KV heads of a page range, which is what a long context of
+// 128-wide heads wants (whole page halves in a few bulk copies) and what a short one does not: 1024 cached tokens are
+// eight blocks of four pages per warp, and the merge reads one partial per block, head and page lane.  Here a group of
+// warps takes ONE head of a page range.  Work that fits the chip in one page per warp is spread that wide; anything larger is cut into
+// equal ranges whatever the batch looks like, with the heads of a range side by side in one block.
+//
+//   * One block per SM = kGroups groups of kGroupWarps warps around one lookup table.  A group works alone (its own
+//     named barrier); the table, the longest part of a block's prologue, is filled before the dependency wait.
+//   * Plan on the device, by every warp for itself from seq_lens (no barrier): see SplitPlan.
+//   * A warp takes whole pages of its head: 16-byte asynchronous copies into its own ring of stages, codes looked up straight
+//     into mma.sync.m16n8k16 fragments (the scheme of tq_decode.cu: K bytes are A fragments of S = K^ Q^T, V nibbles of
+//     two tokens zipped into bytes are A fragments of O^T += V^^T P).
+//   * The group's warps combine in shared memory.  A head whose whole sequence the group covered is finished there
+//     (inverse rotation, cast, store); only a head that was cut leaves partials for the merge kernel, which replans
+//     while the decode kernel runs (it is launched when every decode block is past its own wait) and has two dependent
+//     round trips to memory left after its wait.
+#include <cmath>
+#include <cstring>
+
+#include "tq_decode_common.cuh"
+
+namespace tq {
+
+constexpr int kSplitMaxGroup = 8;    // query columns per KV head
+
+template <int PD>
+struct SplitShape {
+    static constexpr int kE = PD / 32;                       // elements per lane of a row
+    static constexpr int kKBytes = PD / 8, kVBytes = PD / 16;  // code bytes per lane and token, K and V
+    static constexpr int kRow = ((PD / 2 + 2 * (PD / 64)) + 15) & ~15;   // staged bytes of a slot: 48 / 80 / 144
+    // Pitches of the staged rows and the token of an MMA row, chosen so that the K loads (16 bytes a lane: two
+    // rows at a time; 8 bytes at head 64) and the V loads (four rows, 32 bytes each) meet no bank twice.  128: rows 2i, 2i + 1 are
+    // tokens i, i + 4 (80-byte K rows 64 bytes apart mod 128; 96-byte V rows of tokens 0 ... 3 in four quarters).
+    // 256: 144-byte rows do it as they are.  64: the V loads do, two K loads take three wavefronts for two.
+    static constexpr int kKPitch = kRow, kVPitch = PD == 128 ? 96 : kRow;
+    static constexpr int kStageBytes = 16 * (kKPitch + kVPitch);
+    static constexpr int kStages = PD == 256 ? 2 : 3;
+    static constexpr int kRingBytes = kStages * kStageBytes;
+    // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
+    // (128), 64 + 32 at 256 (168)
+    static constexpr int kGroups = 4, kGroupWarps = PD == 64 ? 6 : PD == 128 ? 4 : 3;
+    static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
+    static constexpr int kRingsBelow = PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
+    static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)(kWarps - kRingsBelow) * kRingBytes;   // from offset 0: ample
+    static_assert(kRingBytes >= kSplitMaxGroup * PD * 4, "a warp's partial output goes through its ring");
+    // A page's copies, 16 bytes a lane: rounds of kRoundTokens tokens' code bytes (kPieces lanes a token) for K, the same for V, and one
+    // round for the 16 + 16 pieces with the norms.  Rounds lie a fixed distance apart, so a lane keeps two source pointers.
+    static constexpr int kPieces = PD / 32, kRoundTokens = 32 / kPieces, kRounds = 16 / kRoundTokens;
+    static __device__ __forceinline__ int token(int r) { return PD == 128 ? (r & 8) + ((r & 1) << 2) + ((r & 7) >> 1) : r; }
+};
+
+struct SplitParams {
+    const void* q;
+    const uint8_t* kv_cache;
+    const int32_t* page_indices;
+    const int32_t* page_indptr;
+    const int32_t* seq_lens;
+    const float* signs;
+    int32_t* header;        // workspace word 0: sticky status
+    float* partial_lse;     // [2 x groups of the grid][group columns], base 2
+    float* partial_o;       // [2 x groups of the grid][group columns][PD], normalized, rotated domain
+    void* out;
+    float* out_lse;
+    int64_t slab_bytes, num_blocks, kv_begin, kv_end, tok_stride;
+    int batch, kv_heads, group, max_pages, q_dtype, out_dtype, emit_rotated;
+    int nq, real_heads, real_group, head_dim, slot_bytes;
+    int grid, head_set, head_sets;   // blocks of the decode launch; heads side by side in a block when the work is cut evenly, and kv_heads / head_set
+    float inv_warps;        // 1 / warps of the grid
+    int all_or_nothing;     // a sequence longer than its table empties the whole batch (128-wide heads), or only itself
+    float k_scale, v_scale, scale;
+    uint16_t centroid_h[16];
+};
+
+// ---------------------------------------------------------------------------------------------
+// The plan: which (sequence, head, page range) a worker takes, and which workers a head's partials come from.  Both kernels
+// compute it from seq_lens, every warp for itself: a lane holds one sequence of a batch of 32.
+//   pieces: every head is cut into equal pieces of at most kGroupWarps x `tiles` pages, with the smallest number of tiles (pages per
+//           warp) for which all pieces fit the groups of the grid; a worker is a group and takes one piece.  One start and one combine per
+//           group, and a head that fits a piece is not cut at all; but the pieces of a ragged batch are of many sizes.
+//   even:   the list of all pages (sequence, head set, page) is cut into equal ranges, one per worker, with kSplitItemCost virtual
+//           pages in front of every item for what starting it costs (queries to rotate, a combine).  The head_set groups of a worker
+//           take neighbouring heads of the same pages, so that the slots they read share their DRAM lines.
+// Pieces are taken when their tiles exceed the even share by at most kSplitSlackTiles (about what a second start costs a group).
+// ---------------------------------------------------------------------------------------------
+constexpr int kSplitItemCost = 6, kSplitSlackTiles = 3;
+
+// n / d for 0 <= n < 2^24, d > 0: a reciprocal, then the quotient put right.  (The plan is repeated by every warp, and the compiler's
+// division is three times as long.)
+__device__ __forceinline__ int split_div(int n, int d) {
+    int q = (int)((float)n * __frcp_rn((float)d));
+    const int r = n - q * d;
+    q += r >= d ? 1 : r < 0 ? -1 : 0;
+    return q;
+}
+// ceil(n / d), as above
+__device__ __forceinline__ int split_div_up(int n, int d) { return split_div(n + d - 1, d); }
+
+// the list position where worker c's range begins: c total / workers
+__device__ __forceinline__ int split_cut(int c, int total, int workers) {
+    if (total < (1 << 20) && workers < (1 << 12)) return (int)((uint32_t)c * (uint32_t)total / (uint32_t)workers);
+    return (int)((int64_t)c * total / workers);
+}
+
+struct SplitPlan {
+    int lane, base;          // this batch of 32 starts at sequence `base`
+    int np, len;             // the lane's sequence: pages inside the window, tokens up to the window's end
+    int vstart, vend;        // its span in the list, in units of pieces or of virtual pages (even)
+    int run;                 // end of the span of the last sequence before this batch
+    int total, workers, head_set;
+    int piece;               // pages of a piece at most, 0: the even cut
+    bool too_long;           // some sequence is longer than its page table
+    bool void_batch;         // ... and that empties the batch
+};
+
+__device__ __forceinline__ int split_pages(const SplitParams& p, int b, int& len_out, bool& too_long) {
+    int64_t len = p.seq_lens[b];
+    if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
+    const int first = (int)(p.kv_begin / kPageTokens);
+    const int64_t last = (len + kPageTokens - 1) / kPageTokens;
+    len_out = (int)len;
+    int np = last > first ? (int)(last - first) : 0;
+    const int have = p.page_indptr ? p.page_indptr[b + 1] - p.page_indptr[b] : p.max_pages;
+    if (np > 0 && first + np > have) {
+        too_long = true;
+        np = 0;
+    }
+    return np;
+}
+
+__device__ __forceinline__ void split_load(const SplitParams& p, SplitPlan& s, int base, int run, bool keep) {
+    bool dummy = false;
+    if (!keep) {
+        s.np = 0;
+        if (base + s.lane < p.batch && !s.void_batch) s.np = split_pages(p, base + s.lane, s.len, dummy);
+    }
+    s.base = base;
+    s.run = run;
+    int v = 0;
+    if (s.np > 0) v = s.piece ? p.kv_heads * split_div_up(s.np, s.piece) : p.head_sets * (s.np + kSplitItemCost);
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (s.lane >= o) incl += t;
+    }
+    s.vstart = run + incl - v;
+    s.vend = run + incl;
+}
+
+template <int GW, int NG>
+__device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, int lane) {
+    s.lane = lane;
+    s.too_long = s.void_batch = false;
+    s.len = 0;
+    int pages = 0, nonempty = 0, np_first = 0, len_first = 0;
+    for (int base = 0; base < p.batch; base += 32) {
+        int np = 0, len = 0;
+        if (base + lane < p.batch) np = split_pages(p, base + lane, len, s.too_long);
+        if (base == 0) { np_first = np; len_first = len; }
+        nonempty += __popc(__ballot_sync(0xffffffffu, np > 0));
+        pages += __reduce_add_sync(0xffffffffu, np);
+    }
+    s.too_long = __any_sync(0xffffffffu, s.too_long);
+    s.void_batch = s.too_long && p.all_or_nothing;
+    if (s.void_batch) pages = nonempty = np_first = 0;
+    s.np = np_first;
+    s.len = len_first;
+    // the smallest number of tiles whose pieces fit, from the even share on
+    const int groups = p.grid * NG;
+    const float even = (float)pages * (float)p.kv_heads * p.inv_warps;     // pages per warp (rounding it either way is fine)
+    const int share = (int)even + (even > (float)(int)even ? 1 : 0);
+    s.piece = 0;
+    int pieces = 0;
+    for (int t = share < 1 ? 1 : share; t <= share + kSplitSlackTiles && p.batch <= 256; t++) {
+        const int size = t * GW;
+        pieces = __reduce_add_sync(0xffffffffu, split_div_up(np_first, size));
+        for (int base = 32; base < p.batch && !s.void_batch; base += 32) {
+            int len;
+            bool dummy;
+            const int np = base + lane < p.batch ? split_pages(p, base + lane, len, dummy) : 0;
+            pieces += __reduce_add_sync(0xffffffffu, split_div_up(np, size));
+        }
+        if (pieces * p.kv_heads <= groups) {
+            s.piece = size;
+            break;
+        }
+    }
+    s.head_set = s.piece ? 1 : p.head_set;
+    s.workers = p.grid * (s.head_set == 1 ? NG : s.head_set == 2 ? NG / 2 : NG / 4);
+    s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * kSplitItemCost);
+    split_load(p, s, 0, 0, true);
+}
+
+__device__ __forceinline__ void split_cp_async16_if(bool on, uint32_t dst, const void* src) {   // predicated: no branch in the loop
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(dst), "l"(src), "r"((uint32_t)on) : "memory");
+}
+// A value the compiler cannot work out again: a lane's constants stay in registers through the page loop instead of being recomputed
+// from the thread index in every iteration.
+__device__ __forceinline__ uint32_t split_keep(uint32_t v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+__device__ __forceinline__ void split_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void split_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// BYTES (4, 8, 16 or 32) of a staged code row into words
+template <int BYTES>
+__device__ __forceinline__ void split_lds(uint32_t addr, uint32_t (&w)[BYTES / 4]) {
+    if constexpr (BYTES == 4) {
+        w[0] = lds32(addr);
+    } else if constexpr (BYTES == 8) {
+        const uint2 v = lds64(addr);
+        w[0] = v.x; w[1] = v.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < BYTES / 16; i++) {
+            const uint4 v = lds128(addr + 16 * i);
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+    }
+}
+
+// Hadamard butterflies of a row over a warp: lane l holds elements E l ... E l + E - 1.
+template <int E>
+__device__ __forceinline__ void split_fwht(float (&v)[E], int lane) {
+#pragma unroll
+    for (int h = 1; h < E; h <<= 1) {
+#pragma unroll
+        for (int i = 0; i < E; i++) {
+            if ((i & h) == 0) {
+                const float a = v[i], b = v[i + h];
+                v[i] = a + b;
+                v[i + h] = a - b;
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+#pragma unroll
+        for (int i = 0; i < E; i++) {
+            const float o = __shfl_xor_sync(0xffffffffu, v[i], m);
+            v[i] = (lane & m) ? o - v[i] : v[i] + o;
+        }
+    }
+}
+
+// E consecutive elements of a 16- or 32-bit row as fp32; `at` is the element index of the first one, rows hold `dim` elements
+template <int E>
+__device__ __forceinline__ void split_load_row(const void* base, int dtype, int64_t row, int dim, int d0, float (&v)[E]) {
+    const int64_t at = row * dim + d0;
+    if (dtype != TQ_F32 && dim % E == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0) {   // E 16-bit elements: 4, 8 or 16 bytes
+        if (d0 >= dim) {
+#pragma unroll
+            for (int i = 0; i < E; i++) v[i] = 0.0f;
+            return;
+        }
+        uint32_t w[E / 2];
+        const uint16_t* src = reinterpret_cast<const uint16_t*>(base) + at;
+        if constexpr (E == 2) w[0] = *reinterpret_cast<const uint32_t*>(src);
+        else if constexpr (E == 4) { const uint2 t = *reinterpret_cast<const uint2*>(src); w[0] = t.x; w[1] = t.y; }
+        else { const uint4 t = *reinterpret_cast<const uint4*>(src); w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w; }
+#pragma unroll
+        for (int i = 0; i < E / 2; i++) {
+            if (dtype == TQ_BF16) {
+                v[2 * i] = __uint_as_float(w[i] << 16);
+                v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            } else {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                v[2 * i] = f.x;
+                v[2 * i + 1] = f.y;
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < E; i++) v[i] = d0 + i < dim ? load_q(base, dtype, at + i) : 0.0f;
+}
+
+// A finished row (normalized, rotated domain): back through the rotation and out, or out as it is.
+template <int PD>
+__device__ __forceinline__ void split_finish(const SplitParams& p, const float* signs, int b, int head, int col, float (&o)[PD / 32], float lse2, int lane) {
+    constexpr int E = PD / 32;
+    const int qi = col / p.real_group, hh = col - qi * p.real_group;
+    const int64_t orow = ((int64_t)b * p.nq + qi) * p.real_heads + head * p.real_group + hh;
+    const int d0 = lane * E;
+    if (p.emit_rotated) {
+        float* dst = reinterpret_cast<float*>(p.out) + orow * PD + d0;
+#pragma unroll
+        for (int i = 0; i < E; i++) dst[i] = o[i];
+        if (p.out_lse && lane == 0) p.out_lse[orow] = lse2;
+        return;
+    }
+    split_fwht<E>(o, lane);
+    const int dim = p.head_dim;
+#pragma unroll
+    for (int i = 0; i < E; i++) o[i] *= p.scale * signs[d0 + i];
+    const int64_t at = orow * dim + d0;
+    if (p.out_dtype != TQ_F32 && dim % E == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
+        if (d0 < dim) {
+            uint32_t w[E / 2];
+#pragma unroll
+            for (int i = 0; i < E / 2; i++) {
+                if (p.out_dtype == TQ_BF16) {
+                    const __nv_bfloat162 t = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
+                    w[i] = *reinterpret_cast<const uint32_t*>(&t);
+                } else {
+                    w[i] = pack_half2(o[2 * i], o[2 * i + 1]);
+                }
+            }
+            uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + at;
+            if constexpr (E == 2) *reinterpret_cast<uint32_t*>(dst) = w[0];
+            else if constexpr (E == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < E; i++) {
+            if (d0 + i >= dim) continue;
+            if (p.out_dtype == TQ_BF16) reinterpret_cast<__nv_bfloat16*>(p.out)[at + i] = __float2bfloat16_rn(o[i]);
+            else if (p.out_dtype == TQ_F16) reinterpret_cast<__half*>(p.out)[at + i] = __float2half_rn(o[i]);
+            else reinterpret_cast<float*>(p.out)[at + i] = o[i];
+        }
+    }
+    if (p.out_lse && lane == 0) p.out_lse[orow] = lse2 * 0.6931471805599453f;
+}
+
+template <int PD>
+__global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kernel(const __grid_constant__ SplitParams p) {
+    using F = SplitShape<PD>;
+    constexpr int E = F::kE, NG = F::kGroups, GW = F::kGroupWarps;
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ float m_s[NG][GW][kSplitMaxGroup], l_s[NG][GW][kSplitMaxGroup];
+    __shared__ float sign_s[PD];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
+    const int g = lane >> 2, tg = lane & 3;
+    const uint32_t smem_base = smem_u32(smem);
+    const int G = p.group;
+    if (smem_base + F::kRingsBelow * F::kRingBytes > kLutAddr) {   // the map does not fit
+        grid_dependency_wait();
+        if (tid == 0) atomicExch(&p.header[0], 3);
+        return;
+    }
+    uint8_t* const ring = smem + (warp < F::kRingsBelow ? (uint32_t)warp * F::kRingBytes
+                                                       : kLutAddr + kLutSpan - smem_base + (uint32_t)(warp - F::kRingsBelow) * F::kRingBytes);
+    const uint32_t ring_at = smem_u32(ring);
+    uint8_t* const lut = smem + (kLutAddr - smem_base);
+    // byte `off` of row r of the group's rotated queries (PD fp16), in the unused upper halves of the table's 256-byte rows
+    auto q_ptr = [&](int r, uint32_t off) -> uint8_t* {
+        const uint32_t at = (uint32_t)(gg * kSplitMaxGroup + r) * (PD * 2) + off;
+        return lut + ((at >> 7) << 8) + 128u + (at & 127u);
+    };
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + gg), "r"(GW * 32) : "memory"); };
+
+    // lookup table: entry v, column c = {centroid(v & 15), centroid(v >> 4)}; a warp writes whole rows
+    {
+        // a warp's store covers four rows, 16 bytes a lane
+        const uint32_t mine = p.centroid_h[lane & 15];
+        for (int v = 4 * warp + (lane >> 3); v < 256; v += 4 * F::kWarps) {
+            const uint32_t e = __shfl_sync(0xffffffffu, mine, v & 15) | (__shfl_sync(0xffffffffu, mine, v >> 4) << 16);
+            *reinterpret_cast<uint4*>(lut + v * 256 + 16 * (lane & 7)) = make_uint4(e, e, e, e);
+        }
+    }
+    // the signs are a constant of the context (as in the cache write): read ahead of the wait
+    for (int i = tid; i < PD; i += F::kThreads) sign_s[i] = p.signs[i];
+    // The small inputs into L2 while the kernel before this one drains: a whole KV stream may have passed since they were last
+    // touched, and a prefetch hands no value over.
+    if (blockIdx.x == 0 && tid * 32 < p.batch) prefetch_l2(p.seq_lens + tid * 32);
+    if (!p.page_indptr)
+        for (int64_t i = ((int64_t)blockIdx.x * F::kThreads + tid) * 32; i < (int64_t)p.batch * p.max_pages && i < (2 << 20); i += (int64_t)gridDim.x * F::kThreads * 32)
+            prefetch_l2(p.page_indices + i);
+    __syncthreads();
+    grid_dependency_wait();      // seq_lens, the page table, Q, the cache and the workspace belong to earlier kernels
+    grid_launch_dependents();    // the merge may now be scheduled: it reads seq_lens ahead of its own wait
+
+    SplitPlan s;
+    split_plan<GW, NG>(p, s, lane);
+    if (s.too_long && blockIdx.x == 0 && tid == 0) atomicExch(&p.header[0], kStatusSeqTooLong);
+    const int hs = s.head_set;
+    const int sub = hs == 1 ? gg : hs == 2 ? gg >> 1 : gg >> 2, hsub = gg - sub * hs;
+    const int worker = sub * p.grid + (int)blockIdx.x;   // neighbouring workers sit on different SMs
+    int pos, hi;
+    if (s.piece) {
+        pos = worker;
+        hi = worker < s.total ? worker + 1 : worker;
+    } else {
+        pos = split_cut(worker, s.total, s.workers);
+        hi = split_cut(worker + 1, s.total, s.workers);
+    }
+    // the lane's sequence of the plan waits in shared memory while pages are worked on (registers are what the loop is short of)
+    auto plan_at = [&]() -> uint8_t* {
+        const uint32_t at = (uint32_t)(NG * kSplitMaxGroup * PD * 2) + (uint32_t)warp * 512u + (uint32_t)lane * 16u;
+        return lut + ((at >> 7) << 8) + 128u + (at & 127u);
+    };
+    *reinterpret_cast<int4*>(plan_at()) = make_int4(s.np, s.len, s.vstart, s.vend);
+    const int piece = s.piece;
+    int base = 0;
+    const uint32_t lut_lane = split_keep(smem_u32(lut) + 4u * lane);
+    const int fp = (int)(p.kv_begin / kPageTokens);
+    // this lane's places in a stage: code pieces, norm pieces; fragment rows
+    const int c_tok = lane / F::kPieces, c_piece = lane % F::kPieces;
+    const uint32_t dst_k = split_keep(ring_at + c_tok * F::kKPitch + 16 * c_piece);
+    const uint32_t dst_v = F::kKPitch == F::kVPitch ? dst_k + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + c_tok * F::kVPitch + 16 * c_piece);
+    const uint32_t dst_n = split_keep(ring_at + (lane < 16 ? lane * F::kKPitch : 16 * F::kKPitch + (lane - 16) * F::kVPitch) + PD / 2);
+    const int ta = F::token(g), tb = ta + 8;
+    const uint32_t k_at = split_keep(ring_at + ta * F::kKPitch + tg * F::kKBytes), kn_at = split_keep(ring_at + ta * F::kKPitch + PD / 2);
+    const uint32_t v_at = split_keep(ring_at + 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + g * F::kVBytes);
+    const uint32_t vn_at = F::kKPitch == F::kVPitch ? kn_at + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + ta * F::kVPitch + PD / 2);
+    constexpr int kVNext = (PD == 128 ? 4 : 1) * F::kVPitch;      // from token(2 tg) to token(2 tg + 1)
+    const uint32_t page_bytes = (uint32_t)(kPageTokens * p.tok_stride), round_bytes = (uint32_t)(F::kRoundTokens * p.tok_stride);
+    bool bad_page = false;
+
+    while (pos < hi) {
+        // ---- the next segment: a page range of one head -------------------------------------------------
+        int4 e = *reinterpret_cast<const int4*>(plan_at());
+        int run_end = __shfl_sync(0xffffffffu, e.w, 31);
+        while (pos >= run_end && base + 32 < p.batch) {
+            base += 32;
+            s.piece = piece;
+            s.head_set = hs;
+            split_load(p, s, base, run_end, false);
+            e = make_int4(s.np, s.len, s.vstart, s.vend);
+            *reinterpret_cast<int4*>(plan_at()) = e;
+            run_end = __shfl_sync(0xffffffffu, e.w, 31);
+        }
+        const uint32_t ahead = __ballot_sync(0xffffffffu, e.w > pos);
+        if (ahead == 0) break;
+        const int bl = __ffs(ahead) - 1, b = base + bl;
+        const int np = __shfl_sync(0xffffffffu, e.x, bl), rel = pos - __shfl_sync(0xffffffffu, e.z, bl);
+        const int len = __shfl_sync(0xffffffffu, e.y, bl);
+        int hset, p0, p1;
+        if (piece) {
+            const int pieces = split_div_up(np, piece);
+            hset = split_div(rel, pieces);
+            const int j = rel - hset * pieces, size = split_div(np, pieces), more = np - size * pieces;
+            p0 = j * size + (j < more ? j : more);           // the first `more` pieces take a page more
+            p1 = p0 + size + (j < more ? 1 : 0);
+            pos = hi;
+        } else {
+            const int item = np + kSplitItemCost;
+            hset = split_div(rel, item);
+            const int off = rel - hset * item;
+            const int left = hi - pos, rest = item - off;      // up to the end of the range or of the item
+            const int take = left < rest ? left : rest;
+            p0 = off > kSplitItemCost ? off - kSplitItemCost : 0;
+            p1 = off + take - kSplitItemCost;
+            pos += take;
+            if (p1 <= p0) continue;
+        }
+        const int head = hset * hs + hsub;
+
+        // ---- page ids, the first stages' copies, the queries ------------------------------------------------
+        const int n = p1 - p0 > wg ? (p1 - p0 - wg + GW - 1) / GW : 0;      // this warp's pages: p0 + wg + GW i
+        const int32_t* ids = p.page_indices + (p.page_indptr ? (int64_t)p.page_indptr[b] : (int64_t)b * p.max_pages) + fp + p0 + wg;
+        auto fetch_ids = [&](int i) -> int {
+            int id = 0;
+            if (i + lane < n) {
+                id = ids[(i + lane) * GW];
+                if ((uint64_t)(int64_t)id >= (uint64_t)p.num_blocks) {       // no address is formed from it: page 0 in its place
+                    id = 0;
+                    bad_page = true;
+                }
+            }
+            return id;
+        };
+        int id_now = fetch_ids(0), id_next = n > 32 ? fetch_ids(32) : 0;
+        float qv[2][E];     // this warp's query rows wg and wg + GW (up to 8 rows a group; a third one at head 256 below)
+        const float* sign = sign_s + lane * E;
+        auto q_row = [&](int r) -> int64_t {
+            const int qi = r / p.real_group, hh = r - qi * p.real_group;
+            return ((int64_t)b * p.nq + qi) * p.real_heads + head * p.real_group + hh;
+        };
+        if (wg < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg), p.head_dim, lane * E, qv[0]);
+        if (wg + GW < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg + GW), p.head_dim, lane * E, qv[1]);
+        const uint8_t* const src_k = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)(c_tok * p.tok_stride) + 16 * c_piece;
+        const uint8_t* const src_n = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)((lane & 15) * p.tok_stride) + PD / 2 + (lane < 16 ? 0 : p.slab_bytes);
+        auto issue = [&](int i, uint32_t stage_off) {
+            const uint32_t id = (uint32_t)__shfl_sync(0xffffffffu, id_now, i & 31);
+            const bool on = i < n;
+            const uint8_t* const k = src_k + (uint64_t)id * page_bytes;
+            const uint8_t* const v = k + p.slab_bytes;
+#pragma unroll
+            for (int r = 0; r < F::kRounds; r++) {
+                split_cp_async16_if(on, dst_k + stage_off + r * F::kRoundTokens * F::kKPitch, k + r * round_bytes);
+                split_cp_async16_if(on, dst_v + stage_off + r * F::kRoundTokens * F::kVPitch, v + r * round_bytes);
+            }
+            split_cp_async16_if(on, dst_n + stage_off, src_n + (uint64_t)id * page_bytes);
+            split_cp_async_commit();
+        };
+#pragma unroll
+        for (int i = 0; i < F::kStages - 1; i++) issue(i, i * F::kStageBytes);
+        auto put_q = [&](int r, float (&v)[E]) {
+#pragma unroll
+            for (int i = 0; i < E; i++) v[i] *= sign[i];
+            split_fwht<E>(v, lane);
+            // each (even, odd) pair swapped: a code byte dequantizes to {low half: odd dim, high half: even dim}
+#pragma unroll
+            for (int i = 0; i < E / 2; i++)
+                *reinterpret_cast<uint32_t*>(q_ptr(r, (uint32_t)(lane * E + 2 * i) * 2u)) = pack_half2(v[2 * i + 1] * p.scale, v[2 * i] * p.scale);
+        };
+        if (wg < G) put_q(wg, qv[0]);
+        if (wg + GW < G) put_q(wg + GW, qv[1]);
+        for (int r = wg + 2 * GW; r < G; r += GW) {
+            split_load_row<E>(p.q, p.q_dtype, q_row(r), p.head_dim, lane * E, qv[0]);
+            put_q(r, qv[0]);
+        }
+        group_sync();
+        uint32_t qf[PD / 8];       // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column g
+#pragma unroll
+        for (int i = 0; i < PD / 32; i++) {
+            const uint4 t = g < G ? *reinterpret_cast<const uint4*>(q_ptr(g, (uint32_t)(tg * (PD / 4)) * 2u + 16u * i)) : make_uint4(0u, 0u, 0u, 0u);
+            qf[4 * i] = t.x; qf[4 * i + 1] = t.y; qf[4 * i + 2] = t.z; qf[4 * i + 3] = t.w;
+        }
+
+        // ---- pages -----------------------------------------------------------------------------------------
+        float o_acc[PD / 16][4];
+#pragma unroll
+        for (int i = 0; i < PD / 16; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) o_acc[i][j] = 0.0f;
+        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
+        uint32_t st = 0, st_issue = (F::kStages - 1) * F::kStageBytes;      // stage offsets
+        int left = len - (fp + p0 + wg) * kPageTokens;                       // tokens from this warp's page on
+        for (int it = 0; it < n; it++, left -= GW * kPageTokens) {
+            const int ahead_i = it + F::kStages - 1;
+            if ((ahead_i & 31) == 0) {          // the ids of the next 32 pages, and the load of those after them
+                id_now = id_next;
+                id_next = ahead_i + 32 < n ? fetch_ids(ahead_i + 32) : 0;
+            }
+            issue(ahead_i, st_issue);
+            split_cp_async_wait<F::kStages - 1>();
+            __syncwarp();
+            {
+                // ---- S = K^ Q^T -----------------------------------------------------------------------------
+                uint32_t ka[F::kKBytes / 4], kb[F::kKBytes / 4];
+                split_lds<F::kKBytes>(k_at + st, ka);
+                split_lds<F::kKBytes>(k_at + st + 8 * F::kKPitch, kb);
+                // the V codes too, ahead of the vote below
+                uint32_t v0[F::kVBytes / 4], v1[F::kVBytes / 4], v2[F::kVBytes / 4], v3[F::kVBytes / 4];
+                split_lds<F::kVBytes>(v_at + st, v0);
+                split_lds<F::kVBytes>(v_at + st + kVNext, v1);
+                split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch, v2);
+                split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch + kVNext, v3);
+                float s_acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int w = 0; w < F::kKBytes / 4; w++) {
+                    uint32_t ra[4], rb[4];
+                    dequant8(ka[w], lut_lane, ra);
+                    dequant8(kb[w], lut_lane, rb);
+                    mma16816(s_acc, ra[0], rb[0], ra[1], rb[1], qf[4 * w], qf[4 * w + 1]);
+                    mma16816(s_acc2, ra[2], rb[2], ra[3], rb[3], qf[4 * w + 2], qf[4 * w + 3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) s_acc[i] += s_acc2[i];
+                // ---- online softmax (base 2): rows g, g + 8 are tokens ta, tb; columns 2tg, 2tg + 1 query heads.  Only the
+                // last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
+                // slots contain) and their scores biased to -inf.  Row 0 of every page is inside.
+                float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kKPitch) * p.k_scale;
+                float vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kVPitch) * p.v_scale;
+                float bias_a = 0.0f, bias_b = 0.0f;
+                if (left < kPageTokens) {
+                    if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
+                    if (tb >= left) { kfb = 0.0f; vfb = 0.0f; bias_b = -INFINITY; }
+                }
+                const float x0 = fmaf(s_acc[0], kfa, bias_a), x1 = fmaf(s_acc[1], kfa, bias_a);
+                const float x2 = fmaf(s_acc[2], kfb, bias_b), x3 = fmaf(s_acc[3], kfb, bias_b);
+                float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
+                if (__any_sync(0xffffffffu, mx0 > m0 + kRaiseThreshold || mx1 > m1 + kRaiseThreshold)) {
+#pragma unroll
+                    for (int o = 4; o < 32; o <<= 1) {
+                        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+                    }
+                    const bool raise0 = mx0 > m0 + kRaiseThreshold, raise1 = mx1 > m1 + kRaiseThreshold;
+                    const float c0 = raise0 ? fast_exp2(m0 - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1 - mx1) : 1.0f;
+                    if (raise0) m0 = mx0;
+                    if (raise1) m1 = mx1;
+                    l0 *= c0;
+                    l1 *= c1;
+#pragma unroll
+                    for (int i = 0; i < PD / 16; i++) {
+                        o_acc[i][0] *= c0; o_acc[i][1] *= c1; o_acc[i][2] *= c0; o_acc[i][3] *= c1;
+                    }
+                }
+                const float e0 = fast_exp2(x0 - m0), e1 = fast_exp2(x1 - m1), e2 = fast_exp2(x2 - m0), e3 = fast_exp2(x3 - m1);
+                l0 += e0 + e2;
+                l1 += e1 + e3;
+                const uint32_t pb0 = movmatrix_trans(pack_half2(e0 * vfa, e1 * vfa));
+                const uint32_t pb1 = movmatrix_trans(pack_half2(e2 * vfb, e3 * vfb));
+                // ---- O^T += V^^T P ----------------------------------------------------------------------------
+#pragma unroll
+                for (int w = 0; w < F::kVBytes / 4; w++) {
+                    const uint32_t lo01 = (v0[w] & 0x0F0F0F0Fu) | ((v1[w] << 4) & 0xF0F0F0F0u);      // odd dims
+                    const uint32_t hi01 = ((v0[w] >> 4) & 0x0F0F0F0Fu) | (v1[w] & 0xF0F0F0F0u);      // even dims
+                    const uint32_t lo23 = (v2[w] & 0x0F0F0F0Fu) | ((v3[w] << 4) & 0xF0F0F0F0u);
+                    const uint32_t hi23 = ((v2[w] >> 4) & 0x0F0F0F0Fu) | (v3[w] & 0xF0F0F0F0u);
+                    uint32_t a_lo01[4], a_hi01[4], a_lo23[4], a_hi23[4];
+                    dequant8(lo01, lut_lane, a_lo01);
+                    dequant8(hi01, lut_lane, a_hi01);
+                    dequant8(lo23, lut_lane, a_lo23);
+                    dequant8(hi23, lut_lane, a_hi23);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)     // rows: g <- odd dim, g + 8 <- even dim of code byte 4 w + j
+                        mma16816(o_acc[4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0, pb1);
+                }
+            }
+            __syncwarp();      // every lane has read the stage before a later iteration copies into it
+            st_issue = st;
+            st = st + F::kStageBytes == F::kRingBytes ? 0 : st + F::kStageBytes;
+        }
+        split_cp_async_wait<0>();
+
+        // ---- combine the group's warps ------------------------------------------------------------------------
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+        }
+        if (g == 0) {
+            m_s[gg][wg][2 * tg] = m0;      // columns past the group are zero queries: nobody reads them
+            m_s[gg][wg][2 * tg + 1] = m1;
+            l_s[gg][wg][2 * tg] = l0;
+            l_s[gg][wg][2 * tg + 1] = l1;
+        }
+        // The warp's accumulators as rows of PD floats in its own ring (the copies have landed and been read).  The 16-byte pieces of
+        // a row are swapped by the column, which keeps the four columns a quarter warp stores at a time in different banks.
+        __syncwarp();
+        float* const mine = reinterpret_cast<float*>(ring);
+        if (n > 0) {
+#pragma unroll
+            for (int w = 0; w < F::kVBytes / 2; w++) {      // bytes 2 w, 2 w + 1 of this lane: dims d ... d + 3
+                const int piece = (g * F::kVBytes + 2 * w) / 2;
+                if (2 * tg < G)
+                    *reinterpret_cast<float4*>(mine + (2 * tg) * PD + 4 * (piece ^ tg)) =
+                        make_float4(o_acc[2 * w][2], o_acc[2 * w][0], o_acc[2 * w + 1][2], o_acc[2 * w + 1][0]);
+                if (2 * tg + 1 < G)
+                    *reinterpret_cast<float4*>(mine + (2 * tg + 1) * PD + 4 * (piece ^ tg)) =
+                        make_float4(o_acc[2 * w][3], o_acc[2 * w][1], o_acc[2 * w + 1][3], o_acc[2 * w + 1][1]);
+            }
+        }
+        group_sync();
+        const bool whole = p0 == 0 && p1 == np;
+        const int slot = (worker * 2 + (p0 == 0 ? 1 : 0)) * hs + hsub;
+        for (int r = wg; r < G; r += GW) {
+            float mm = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < GW; w++) mm = fmaxf(mm, m_s[gg][w][r]);
+            float o[E], ll = 0.0f;
+#pragma unroll
+            for (int i = 0; i < E; i++) o[i] = 0.0f;
+#pragma unroll
+            for (int w = 0; w < GW; w++) {
+                const float mw = m_s[gg][w][r];
+                if (mw > -INFINITY) {            // a warp without a page has stored nothing
+                    const float c = fast_exp2(mw - mm);
+                    ll += c * l_s[gg][w][r];
+                    const int other = gg * GW + w;
+                    const float* row = reinterpret_cast<const float*>(
+                                           smem + (other < F::kRingsBelow ? (uint32_t)other * F::kRingBytes
+                                                                         : kLutAddr + kLutSpan - smem_base + (uint32_t)(other - F::kRingsBelow) * F::kRingBytes)) + r * PD;
+                    if constexpr (E == 2) {
+                        const float2 t = *reinterpret_cast<const float2*>(row + 4 * ((lane >> 1) ^ (r >> 1)) + 2 * (lane & 1));
+                        o[0] += c * t.x; o[1] += c * t.y;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < E / 4; i++) {
+                            const float4 t = *reinterpret_cast<const float4*>(row + 4 * ((lane * (E / 4) + i) ^ (r >> 1)));
+                            o[4 * i] += c * t.x; o[4 * i + 1] += c * t.y; o[4 * i + 2] += c * t.z; o[4 * i + 3] += c * t.w;
+                        }
+                    }
+                }
+            }
+            const float inv = ll > 0.0f ? 1.0f / ll : 0.0f, lse2 = ll > 0.0f ? mm + log2f(ll) : -INFINITY;
+#pragma unroll
+            for (int i = 0; i < E; i++) o[i] *= inv;
+            if (whole) {
+                split_finish<PD>(p, sign_s, b, head, r, o, lse2, lane);
+            } else {
+                const int64_t at = (int64_t)slot * G + r;
+                float* dst = p.partial_o + at * PD + lane * E;
+                if constexpr (E == 2) {
+                    *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < E / 4; i++)
+                        *reinterpret_cast<float4*>(dst + 4 * i) = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                }
+                if (lane == 0) p.partial_lse[at] = lse2;
+            }
+        }
+        if (pos < hi) group_sync();    // rings and query rows are free again
+    }
+    if (bad_page) atomicExch(&p.header[0], kStatusBadPage);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Merge of the heads that were cut: RW warps per row (sequence, KV head, column) share its parts.  The plan is made ahead of
+// the wait.  An empty sequence's rows become zeros here; a head that one group covered is finished already.
+// ---------------------------------------------------------------------------------------------
+
+template <int PD, int RW>
+__global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const __grid_constant__ SplitParams p) {
+    using F = SplitShape<PD>;
+    constexpr int E = F::kE, GW = F::kGroupWarps, NG = F::kGroups, kRows = RW == 1 ? 4 : 1;      // rows of the block
+    __shared__ float acc_s[RW][PD], m_s[RW], w_s[RW], sign_s[PD];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int part_warp = RW == 1 ? 0 : warp;
+    const int G = p.group;
+    grid_launch_dependents();
+    const int row = blockIdx.x * kRows + (RW == 1 ? warp : 0);
+    const int bh = row / G, r = row - bh * G, b = bh / p.kv_heads, head = bh - b * p.kv_heads;
+    for (int i = threadIdx.x; i < PD; i += RW == 16 ? 512 : 128) sign_s[i] = p.signs[i];
+    if (RW == 1) __syncthreads();
+    SplitPlan s;
+    split_plan<GW, NG>(p, s, lane);     // every decode block is past its wait: the lengths are final
+    while (s.base + 32 <= b && b < p.batch) split_load(p, s, s.base + 32, __shfl_sync(0xffffffffu, s.vend, 31), false);
+    const int np = __shfl_sync(0xffffffffu, s.np, (b - s.base) & 31), vstart = __shfl_sync(0xffffffffu, s.vstart, (b - s.base) & 31);
+    const int hs = s.head_set, hset = head / hs, hsub = head - hset * hs;
+    int first = 0, count = 0;           // workers of this head's parts
+    if (np > 0) {
+        if (s.piece) {
+            count = split_div_up(np, s.piece);
+            first = vstart + hset * count;
+        } else {
+            const int64_t at = vstart + (int64_t)hset * (np + kSplitItemCost) + kSplitItemCost, end = at + np;   // its pages in the list
+            first = (int)(((at + 1) * s.workers + s.total - 1) / s.total) - 1;
+            count = (int)((end * s.workers + s.total - 1) / s.total) - first;
+        }
+    }
+    grid_dependency_wait();
+    if (count == 1 || b >= p.batch) return;
+    // part i: worker first + i; the first part starts its sequence (odd slot of the worker), the others continue it
+    auto slot_row = [&](int i) -> int64_t { return ((int64_t)((first + i) * 2 + (i == 0 ? 1 : 0)) * hs + hsub) * G + r; };
+    float m = -INFINITY, wsum = 0.0f, acc[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) acc[e] = 0.0f;
+    for (int i0 = part_warp; i0 < count; i0 += 8 * RW) {        // parts i0, i0 + RW, ...: eight payloads and their LSEs in flight together
+        float o[8][E], lse[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int i = i0 + RW * j;
+            lse[j] = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < E; e++) o[j][e] = 0.0f;
+            if (i < count) {
+                const int64_t at = slot_row(i);
+                lse[j] = p.partial_lse[at];
+                const float* src = p.partial_o + at * PD + lane * E;
+                if constexpr (E == 2) {
+                    const float2 t = *reinterpret_cast<const float2*>(src);
+                    o[j][0] = t.x; o[j][1] = t.y;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < E / 4; e++) {
+                        const float4 t = *reinterpret_cast<const float4*>(src + 4 * e);
+                        o[j][4 * e] = t.x; o[j][4 * e + 1] = t.y; o[j][4 * e + 2] = t.z; o[j][4 * e + 3] = t.w;
+                    }
+                }
+            }
+        }
+        float mx = m;
+#pragma unroll
+        for (int j = 0; j < 8; j++) mx = fmaxf(mx, lse[j]);
+        if (mx == -INFINITY) continue;
+        const float c = fast_exp2(m - mx);
+        wsum *= c;
+#pragma unroll
+        for (int e = 0; e < E; e++) acc[e] *= c;
+        m = mx;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float w = fast_exp2(lse[j] - mx);
+            if (w > 0.0f) {      // an empty part's payload is never trusted
+                wsum += w;
+#pragma unroll
+                for (int e = 0; e < E; e++) acc[e] = fmaf(w, o[j][e], acc[e]);
+            }
+        }
+    }
+    float o[E], mm = m, wtot = wsum;
+#pragma unroll
+    for (int e = 0; e < E; e++) o[e] = acc[e];
+    if constexpr (RW > 1) {
+#pragma unroll
+        for (int e = 0; e < E; e++) acc_s[warp][lane * E + e] = acc[e];
+        if (lane == 0) { m_s[warp] = m; w_s[warp] = wsum; }
+        __syncthreads();
+        if (warp != 0) return;
+#pragma unroll
+        for (int w = 1; w < RW; w++) mm = fmaxf(mm, m_s[w]);
+        wtot = 0.0f;
+#pragma unroll
+        for (int e = 0; e < E; e++) o[e] = 0.0f;
+        if (mm > -INFINITY) {
+#pragma unroll
+            for (int w = 0; w < RW; w++) {
+                const float c = fast_exp2(m_s[w] - mm);
+                if (c > 0.0f) {
+                    wtot += c * w_s[w];
+#pragma unroll
+                    for (int e = 0; e < E; e++) o[e] = fmaf(c, acc_s[w][lane * E + e], o[e]);
+                }
+            }
+        }
+    }
+    const float inv = wtot > 0.0f ? 1.0f / wtot : 0.0f;
+#pragma unroll
+    for (int e = 0; e < E; e++) o[e] *= inv;
+    split_finish<PD>(p, sign_s, b, head, r, o, wtot > 0.0f ? mm + log2f(wtot) : -INFINITY, lane);
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+int device_sm_count(int* out);
+
+static size_t split_up(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// partial slots: two per group of the grid, each with the columns of one KV head
+size_t split_workspace_bytes(int columns, int padded, int ctas) {
+    const size_t rows = (size_t)2 * ctas * 4 * columns;
+    return 256 + split_up(rows * sizeof(float)) + split_up(rows * padded * sizeof(float));
+}
+
+template <int PD>
+static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
+    using F = SplitShape<PD>;
+    static_assert(F::kGroups == 4, "split_workspace_bytes counts four groups a block");
+    static bool configured[64] = {};
+    int dev = 0;
+    TQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        TQ_CUDA(cudaFuncSetAttribute(decode_split_kernel<PD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::kSmem));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    p.grid = ctas;
+    p.head_set = p.kv_heads % 4 == 0 ? 4 : p.kv_heads % 2 == 0 ? 2 : 1;
+    p.head_sets = p.kv_heads / p.head_set;
+    p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
+    TQ_CUDA(launch_serialized(decode_split_kernel<PD>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
+    // A head has about groups / (sequences x heads) parts at most: a warp fetches eight at a time, so up to eight go to one warp
+    // (a block takes four rows), more to four or sixteen warps.
+    const int rows = p.batch * p.kv_heads * p.group, parts = p.grid * F::kGroups / (p.batch * p.kv_heads);
+    if (parts > 32) TQ_CUDA(launch_serialized(merge_split_kernel<PD, 16>, dim3((unsigned)rows), dim3(512), 0, s, p));
+    else if (parts > 8) TQ_CUDA(launch_serialized(merge_split_kernel<PD, 4>, dim3((unsigned)rows), dim3(128), 0, s, p));
+    else TQ_CUDA(launch_serialized(merge_split_kernel<PD, 1>, dim3((unsigned)(rows + 3) / 4), dim3(128), 0, s, p));
+    return TQ_OK;
+}
+
+// The caller has checked pointers, types and geometry: 16-byte slots, padded head size 64 / 128 / 256, up to 8 query
+// columns per KV head.
+int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim, int padded,
+                 const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
+                 int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
+                 void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
+                 int all_or_nothing, int ctas, cudaStream_t s) {
+    SplitParams p{};
+    p.group = nq * (real_q_heads / num_kv_heads);
+    const size_t need = split_workspace_bytes(p.group, padded, ctas);
+    TQ_REQUIRE(workspace_bytes >= need, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
+    TQ_REQUIRE((int64_t)batch * num_kv_heads * p.group < (int64_t)1 << 31, TQ_ERR_UNSUPPORTED, "too many rows for one launch");
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    p.q = q;
+    p.kv_cache = static_cast<const uint8_t*>(kv_cache);
+    p.page_indices = page_indices;
+    p.page_indptr = page_indptr;
+    p.seq_lens = seq_lens;
+    p.signs = signs;
+    p.header = reinterpret_cast<int32_t*>(ws);
+    p.partial_lse = reinterpret_cast<float*>(ws + 256);
+    p.partial_o = reinterpret_cast<float*>(ws + 256 + split_up((size_t)2 * ctas * 4 * p.group * sizeof(float)));
+    p.out = out;
+    p.out_lse = out_lse;
+    p.tok_stride = (int64_t)num_kv_heads * slot_bytes;
+    p.slab_bytes = num_blocks * kPageTokens * p.tok_stride;
+    p.num_blocks = num_blocks;
+    p.kv_begin = kv_begin;
+    p.kv_end = kv_end;
+    p.batch = batch;
+    p.kv_heads = num_kv_heads;
+    p.max_pages = max_pages;
+    p.q_dtype = q_dtype;
+    p.out_dtype = out_dtype;
+    p.emit_rotated = emit_rotated;
+    p.nq = nq;
+    p.real_heads = real_q_heads;
+    p.real_group = real_q_heads / num_kv_heads;
+    p.head_dim = head_dim;
+    p.slot_bytes = slot_bytes;
+    p.all_or_nothing = all_or_nothing;
+    const double inv = 1.0 / std::sqrt((double)padded);
+    p.scale = p.v_scale = (float)inv;
+    p.k_scale = (float)(inv * (double)sm_scale * 1.4426950408889634);
+    for (int k = 0; k < 16; k++) {
+        const __half h = __float2half_rn((float)kCentroidsN01_4bit[k]);
+        memcpy(&p.centroid_h[k], &h, 2);
+    }
+    switch (padded) {
+        case 64: return launch_split<64>(p, ctas, s);
+        case 128: return launch_split<128>(p, ctas, s);
+        default: return launch_split<256>(p, ctas, s);
+    }
+}
+
+}  // namespace tq

@@ -489,339 +489,6 @@ __global__ void __launch_bounds__(kGenWarps * 32, 4) decode_generic_kernel(const
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// decode on the tensor cores for the same head sizes: a warp takes whole pages, stages their slots in
-// shared memory with 16-byte asynchronous copies (its own ring of stages, no block-wide barrier in the
-// loop) and dequantizes the codes straight into mma.sync.m16n8k16 fragments.
-//   S = K^ Q^T (16 tokens x 8 query columns): lane (g, tg) reads bytes tg PD/8 ... of the code rows
-//   of tokens g and g + 8; a code byte looked up in a table of fp16 centroid pairs IS one A-fragment
-//   register (two neighbouring contraction slots of one token), so the contraction runs over the dims
-//   in the order the bytes come, and the Q^T fragments are built in that order once per block.
-//   O^T += V^^T P (PD dims x 8 columns): the contraction runs over tokens, so a fragment register
-//   pairs two tokens' values of one dim: lane (g, tg) reads bytes g PD/16 ... of tokens 2tg, 2tg + 1,
-//   2tg + 8, 2tg + 9 and zips the nibbles of a token pair into bytes before the lookup (low nibbles
-//   = odd dims -> accumulator row g, high nibbles = even dims -> row g + 8).
-// The table entry of byte v is {low half: centroid of the low nibble, high half: of the high nibble},
-// one copy per lane side by side (32 KB).  Online softmax in base 2 per page; the
-// K norm is folded into the scores, the V norm into P (moved into place with movmatrix).  Same grid,
-// workspace and merge as the plain kernel above, which stays as the fallback for caches that are not
-// 16-byte aligned.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t gen_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void gen_mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                             uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t gen_movmatrix_trans(uint32_t a) {
-    uint32_t d;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
-    return d;
-}
-__device__ __forceinline__ uint32_t gen_pack_half2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-// table entry of byte j of word w (the table's column of this lane is folded into lut_lane; COLS copies per byte value)
-template <int COLS>
-__device__ __forceinline__ uint32_t gen_lookup(uint32_t w, int j, uint32_t lut_lane) {
-    uint32_t r;
-    uint32_t v;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(v) : "r"(w), "r"(0x4440u | (uint32_t)j));   // byte j of w
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(v * (4u * COLS) + lut_lane));
-    return r;
-}
-// BYTES (4, 8, 16 or 32) of a staged code row into words
-template <int BYTES>
-__device__ __forceinline__ void gen_lds_words(uint32_t addr, uint32_t (&w)[BYTES / 4]) {
-    if constexpr (BYTES == 4) {
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[0]) : "r"(addr));
-    } else if constexpr (BYTES == 8) {
-        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(addr));
-    } else {
-#pragma unroll
-        for (int i = 0; i < BYTES / 16; i++)
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(w[4 * i]), "=r"(w[4 * i + 1]), "=r"(w[4 * i + 2]), "=r"(w[4 * i + 3]) : "r"(addr + 16 * i));
-    }
-}
-__device__ __forceinline__ float gen_lds_half(uint32_t addr) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return __half2float(__ushort_as_half(v));
-}
-__device__ __forceinline__ void gen_cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void gen_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void gen_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <int PD>
-struct FragShape {
-    static constexpr int kKBytes = PD / 8, kVBytes = PD / 16;   // code bytes per lane and token, K and V
-    static constexpr int kVWords = kVBytes / 4;
-    static constexpr int kRow = ((PD / 2 + 2 * (PD / 64)) + 15) & ~15;   // staged bytes of a slot: codes + norms, 48 / 80 / 144
-    static constexpr int kChunks = 2 * 16 * kRow / 16;          // 16-byte copies per page and head (K and V): 96 / 160 / 288
-    static constexpr int kStageBytes = 2 * 16 * kRow;
-    static constexpr int kStages = PD == 256 ? 2 : 3;
-    static constexpr int kLutCols = 32;   // copies of the lookup table side by side: one per lane, no two lanes of a lookup share a bank
-    static constexpr size_t kRing = (size_t)kGenWarps * kStages * kStageBytes;
-    static constexpr size_t kCombine = (size_t)kGenWarps * kGenMaxGroup * PD * 4;   // also covers the rotated queries
-    static constexpr size_t kSmem = kRing > kCombine ? kRing : kCombine;
-    static_assert(kChunks % 32 == 0, "a page's copies divide evenly over the lanes");
-};
-
-template <int PD>
-__global__ void __launch_bounds__(kGenWarps * 32, PD == 64 ? 4 : PD == 128 ? 4 : 3) decode_frags_kernel(const __grid_constant__ GenDecodeParams p) {
-    using F = FragShape<PD>;
-    extern __shared__ __align__(16) uint8_t tsm[];
-    __shared__ float m_s[kGenWarps][kGenMaxGroup], l_s[kGenWarps][kGenMaxGroup];
-    __shared__ float cent_s[16];
-    __shared__ __align__(16) uint32_t lut_s[256 * F::kLutCols];
-    constexpr int pd = PD;
-    const int G = p.group;
-    float* q_s = reinterpret_cast<float*>(tsm);   // [G][pd] rotated queries, before the loop
-    float* o_s = reinterpret_cast<float*>(tsm);   // [warps][G][pd], after the loop
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, tg = lane & 3;
-    const int split = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
-    if (tid < 16) cent_s[tid] = p.centroids[tid];
-
-    // window of this split, in pages
-    int64_t len = p.seq_lens[b];
-    if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
-    const int64_t begin = p.kv_begin > 0 ? p.kv_begin : 0;
-    const int first_page = (int)(begin / kGenPage);
-    const int last_page = (int)((len + kGenPage - 1) / kGenPage);
-    int npages = last_page > first_page ? last_page - first_page : 0;
-    const int64_t tbl = p.page_indptr ? (int64_t)p.page_indptr[b] : (int64_t)b * p.max_pages;
-    const int have = p.page_indptr ? p.page_indptr[b + 1] - p.page_indptr[b] : p.max_pages;
-    if (npages > 0 && first_page + npages > have) {  // the table cannot back this length: read nothing
-        if (tid == 0) atomicExch(&p.header[0], kGenStatusSeqTooLong);
-        npages = 0;
-    }
-    const int per = (npages + p.splits - 1) / p.splits;
-    const int pg0 = first_page + split * per;
-    const int pg1 = min(first_page + npages, pg0 + per);
-
-    // rotate the group's queries: signs, butterflies, 1/sqrt(pd)
-    for (int i = tid; i < G * pd; i += blockDim.x) {
-        const int gg = i / pd, d = i - gg * pd;
-        q_s[i] = d < p.g.head_dim
-                     ? gen_load(p.q, p.q_dtype, gen_q_row(p, b, h, gg) * p.g.head_dim + d) * p.signs[d]
-                     : 0.0f;
-    }
-    __syncthreads();
-    for (int v = tid; v < 256; v += blockDim.x) {   // a row of copies per byte value
-        const uint32_t e = gen_pack_half2(cent_s[v & 15], cent_s[v >> 4]);
-        uint4* row = reinterpret_cast<uint4*>(lut_s + v * F::kLutCols);
-#pragma unroll
-        for (int i = 0; i < F::kLutCols / 4; i++) row[i] = make_uint4(e, e, e, e);
-    }
-    for (int hh = 1; hh < pd; hh <<= 1) {
-        for (int i = tid; i < G * pd / 2; i += blockDim.x) {
-            const int gg = i / (pd / 2), idx = i - gg * (pd / 2);
-            const int j = (idx / hh) * 2 * hh + (idx % hh);
-            float* row = q_s + gg * pd;
-            const float a = row[j], c = row[j + hh];
-            row[j] = a + c;
-            row[j + hh] = a - c;
-        }
-        __syncthreads();
-    }
-    // B fragments of Q^T: column g of the query tile (zero beyond the group).  Step s contracts over the dims of
-    // this lane's code bytes 2s and 2s + 1 (dims 4 (tg PD/16 + s) ...), each byte's odd dim in the lower slot.
-    uint32_t qf[PD / 8];
-#pragma unroll
-    for (int s = 0; s < PD / 16; s++) {
-        const float* row = q_s + g * pd + tg * (PD / 4) + 4 * s;
-        const bool on = g < G;
-        qf[2 * s] = on ? gen_pack_half2(row[1] * p.scale, row[0] * p.scale) : 0u;
-        qf[2 * s + 1] = on ? gen_pack_half2(row[3] * p.scale, row[2] * p.scale) : 0u;
-    }
-    __syncthreads();   // the queries are in registers: their shared memory becomes the warps' stage rings
-
-    float o_acc[PD / 16][4];
-#pragma unroll
-    for (int i = 0; i < PD / 16; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) o_acc[i][j] = 0.0f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
-    const uint32_t lut_lane = gen_smem_u32(lut_s) + 4u * (lane & (F::kLutCols - 1));
-    const uint32_t ring = gen_smem_u32(tsm) + (uint32_t)warp * F::kStages * F::kStageBytes;
-    const size_t tok_stride = (size_t)p.num_kv_heads * p.g.slot_bytes;
-    const int my_pages = pg1 > pg0 + warp ? (pg1 - pg0 - warp + kGenWarps - 1) / kGenWarps : 0;
-    auto page_at = [&](int i) -> int64_t { return i < my_pages ? (int64_t)p.page_indices[tbl + pg0 + warp + i * kGenWarps] : -1; };
-    uint32_t staged = 0;   // bit s: stage s holds a page (its id was inside the cache)
-    // copies of one page into a stage: the 16-byte pieces of the 16 K rows, then of the 16 V rows, dealt over
-    // the lanes; source and destination offsets of this lane's pieces are fixed
-    constexpr int kPieces = 16 * F::kRow / 16, kRounds = (kPieces + 31) / 32;
-    uint32_t src_off[kRounds], dst_off[kRounds];
-#pragma unroll
-    for (int i = 0; i < kRounds; i++) {
-        const int c = lane + 32 * i, tok = c / (F::kRow / 16), piece = c % (F::kRow / 16);
-        src_off[i] = (uint32_t)(tok * tok_stride) + piece * 16;
-        dst_off[i] = tok * F::kRow + piece * 16;
-    }
-    auto issue = [&](int stage, int64_t page) {
-        if ((uint64_t)page < (uint64_t)p.num_blocks) {
-            const uint8_t* base_k = p.kv_cache + (size_t)(page * kGenPage) * tok_stride + (size_t)h * p.g.slot_bytes;
-            const uint8_t* base_v = base_k + p.slab_bytes;
-            const uint32_t dst_k = ring + stage * F::kStageBytes, dst_v = dst_k + 16 * F::kRow;
-#pragma unroll
-            for (int i = 0; i < kRounds; i++) {
-                if (kPieces % 32 == 0 || i + 1 < kRounds || lane + 32 * i < kPieces) {
-                    gen_cp_async16(dst_k + dst_off[i], base_k + src_off[i]);
-                    gen_cp_async16(dst_v + dst_off[i], base_v + src_off[i]);
-                }
-            }
-            staged |= 1u << stage;
-        } else {
-            staged &= ~(1u << stage);
-        }
-        gen_cp_async_commit();
-    };
-#pragma unroll
-    for (int i = 0; i < F::kStages - 1; i++) issue(i, page_at(i));
-    int64_t page_issue = page_at(F::kStages - 1);
-    int st = 0, st_issue = F::kStages - 1;
-    bool bad_page = false;
-    for (int it = 0; it < my_pages; it++) {
-        const int64_t page_after = page_at(it + F::kStages);   // its id arrives while this page is worked on
-        issue(st_issue, page_issue);                            // into the stage the previous iteration has left
-        gen_cp_async_wait<F::kStages - 1>();
-        __syncwarp();
-        if (!((staged >> st) & 1u)) {
-            bad_page = true;   // no address was formed from the id
-        } else {
-            const uint32_t sk = ring + st * F::kStageBytes, sv = sk + 16 * F::kRow;
-            // ---- S = K^ Q^T -------------------------------------------------------------------------------
-            uint32_t ka[F::kKBytes / 4], kb[F::kKBytes / 4];
-            gen_lds_words<F::kKBytes>(sk + g * F::kRow + tg * F::kKBytes, ka);
-            gen_lds_words<F::kKBytes>(sk + (g + 8) * F::kRow + tg * F::kKBytes, kb);
-            float s_acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int s = 0; s < PD / 16; s++) {
-                const uint32_t wa = ka[s >> 1], wb = kb[s >> 1];
-                const int j = 2 * (s & 1);
-                const uint32_t a0 = gen_lookup<F::kLutCols>(wa, j, lut_lane), a2 = gen_lookup<F::kLutCols>(wa, j + 1, lut_lane);
-                const uint32_t a1 = gen_lookup<F::kLutCols>(wb, j, lut_lane), a3 = gen_lookup<F::kLutCols>(wb, j + 1, lut_lane);
-                gen_mma16816((s & 1) ? s_acc2 : s_acc, a0, a1, a2, a3, qf[2 * s], qf[2 * s + 1]);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) s_acc[i] += s_acc2[i];
-            // ---- online softmax (base 2); rows g and g + 8 are tokens, columns 2tg and 2tg + 1 query heads --
-            // The window starts on a page boundary, so only the last page of a sequence can hold tokens outside it:
-            // their norms are zeroed (whatever the unwritten slots contain) and their scores biased to -inf.  Row 0 of
-            // every page is inside, so every column's maximum is finite from the first page on.
-            float kfa = gen_lds_half(sk + g * F::kRow + PD / 2) * p.score_scale, kfb = gen_lds_half(sk + (g + 8) * F::kRow + PD / 2) * p.score_scale;
-            float vfa = gen_lds_half(sv + g * F::kRow + PD / 2), vfb = gen_lds_half(sv + (g + 8) * F::kRow + PD / 2);
-            float bias_a = 0.0f, bias_b = 0.0f;
-            const int64_t t0 = (int64_t)(pg0 + warp + it * kGenWarps) * kGenPage;
-            if (t0 + kGenPage > len) {
-                if (t0 + g >= len) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
-                if (t0 + g + 8 >= len) { kfb = 0.0f; vfb = 0.0f; bias_b = -INFINITY; }
-            }
-            const float x0 = __fmaf_rn(s_acc[0], kfa, bias_a), x1 = __fmaf_rn(s_acc[1], kfa, bias_a);
-            const float x2 = __fmaf_rn(s_acc[2], kfb, bias_b), x3 = __fmaf_rn(s_acc[3], kfb, bias_b);
-            // The running maximum of a column is raised only when a score of the page exceeds it by more than 2^6
-            // (the weights stay within fp16): one vote decides, and only then is the page's maximum reduced across
-            // the lanes and the accumulators rescaled.
-            float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
-            if (__any_sync(0xffffffffu, mx0 > m0 + 6.0f || mx1 > m1 + 6.0f)) {
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-                }
-                const bool r0 = mx0 > m0 + 6.0f, r1 = mx1 > m1 + 6.0f;
-                const float c0 = r0 ? gen_exp2(m0 - mx0) : 1.0f, c1 = r1 ? gen_exp2(m1 - mx1) : 1.0f;
-                if (r0) m0 = mx0;
-                if (r1) m1 = mx1;
-                l0 *= c0;
-                l1 *= c1;
-#pragma unroll
-                for (int mt = 0; mt < PD / 16; mt++) {
-                    o_acc[mt][0] *= c0; o_acc[mt][1] *= c1; o_acc[mt][2] *= c0; o_acc[mt][3] *= c1;
-                }
-            }
-            const float e0 = gen_exp2(x0 - m0), e1 = gen_exp2(x1 - m1), e2 = gen_exp2(x2 - m0), e3 = gen_exp2(x3 - m1);
-            l0 += e0 + e2;
-            l1 += e1 + e3;
-            const uint32_t pb0 = gen_movmatrix_trans(gen_pack_half2(e0 * vfa, e1 * vfa));
-            const uint32_t pb1 = gen_movmatrix_trans(gen_pack_half2(e2 * vfb, e3 * vfb));
-            // ---- O^T += V^^T P: zip the nibbles of a token pair into bytes, look the pairs up ----------------
-            uint32_t v0[F::kVWords], v1[F::kVWords], v2[F::kVWords], v3[F::kVWords];
-            const uint32_t vrow = sv + (2 * tg) * F::kRow + g * F::kVBytes;
-            gen_lds_words<F::kVBytes>(vrow, v0);
-            gen_lds_words<F::kVBytes>(vrow + F::kRow, v1);
-            gen_lds_words<F::kVBytes>(vrow + 8 * F::kRow, v2);
-            gen_lds_words<F::kVBytes>(vrow + 9 * F::kRow, v3);
-#pragma unroll
-            for (int w = 0; w < F::kVWords; w++) {
-                const uint32_t lo01 = (v0[w] & 0x0F0F0F0Fu) | ((v1[w] << 4) & 0xF0F0F0F0u);
-                const uint32_t hi01 = ((v0[w] >> 4) & 0x0F0F0F0Fu) | (v1[w] & 0xF0F0F0F0u);
-                const uint32_t lo23 = (v2[w] & 0x0F0F0F0Fu) | ((v3[w] << 4) & 0xF0F0F0F0u);
-                const uint32_t hi23 = ((v2[w] >> 4) & 0x0F0F0F0Fu) | (v3[w] & 0xF0F0F0F0u);
-#pragma unroll
-                for (int j = 0; j < 4; j++)   // rows: g <- odd dim, g + 8 <- even dim of this lane's code byte 4w + j
-                    gen_mma16816(o_acc[4 * w + j], gen_lookup<F::kLutCols>(lo01, j, lut_lane), gen_lookup<F::kLutCols>(hi01, j, lut_lane),
-                                 gen_lookup<F::kLutCols>(lo23, j, lut_lane), gen_lookup<F::kLutCols>(hi23, j, lut_lane), pb0, pb1);
-            }
-        }
-        __syncwarp();   // every lane has read the stage before the next iteration copies into it
-        page_issue = page_after;
-        st_issue = st;
-        st = st + 1 == F::kStages ? 0 : st + 1;
-    }
-    gen_cp_async_wait<0>();
-    if (bad_page && lane == 0) atomicExch(&p.header[0], kGenStatusBadPage);
-    // this warp's sums over its token lanes, then everything to shared memory for the block's combine
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-        l0 += __shfl_xor_sync(0xffffffffu, l0, o);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-    }
-    __syncthreads();   // every warp has left its ring: the region becomes o_s
-    if (g == 0) {
-        if (2 * tg < G) { m_s[warp][2 * tg] = m0; l_s[warp][2 * tg] = l0; }
-        if (2 * tg + 1 < G) { m_s[warp][2 * tg + 1] = m1; l_s[warp][2 * tg + 1] = l1; }
-    }
-#pragma unroll
-    for (int mt = 0; mt < PD / 16; mt++) {
-        const int d_even = 2 * (g * (PD / 16) + mt);   // accumulator rows g / g + 8 hold the odd / even dim of byte g PD/16 + mt
-        if (2 * tg < G) {
-            o_s[(warp * G + 2 * tg) * pd + d_even + 1] = o_acc[mt][0];
-            o_s[(warp * G + 2 * tg) * pd + d_even] = o_acc[mt][2];
-        }
-        if (2 * tg + 1 < G) {
-            o_s[(warp * G + 2 * tg + 1) * pd + d_even + 1] = o_acc[mt][1];
-            o_s[(warp * G + 2 * tg + 1) * pd + d_even] = o_acc[mt][3];
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < G * pd; i += blockDim.x) {
-        const int gg = i / pd, d = i - gg * pd;
-        float mm = -INFINITY;
-        for (int w = 0; w < kGenWarps; w++) mm = fmaxf(mm, m_s[w][gg]);
-        float ll = 0.0f, acc = 0.0f;
-        if (mm > -INFINITY) {
-            for (int w = 0; w < kGenWarps; w++) {
-                const float sc = gen_exp2(m_s[w][gg] - mm);
-                if (sc > 0.0f) {
-                    ll += sc * l_s[w][gg];
-                    acc += sc * o_s[(w * G + gg) * pd + d];
-                }
-            }
-        }
-        const int64_t row = ((int64_t)b * p.splits + split) * p.num_q_heads + h * G + gg;
-        p.partial_o[row * pd + d] = ll > 0.0f ? acc / ll : 0.0f;
-        if (d == 0) p.partial_lse[row] = ll > 0.0f ? mm + log2f(ll) : -INFINITY;
-    }
-}
-
 struct GenMergeParams {
     const float* partial_o;
     const float* partial_lse;
@@ -1139,23 +806,32 @@ int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv
     return TQ_OK;
 }
 
-// blocks per SM the decode grid is sized to: one wave of resident blocks for head sizes up to 128 (four fit beside
-// their 32 KB tables; more, smaller blocks cost more prologues than they balance), two waves for 256 (three fit;
-// 221 us against 229 for batch 8 x 32768)
-static int generic_blocks_per_sm(int padded) { return padded == 64 ? 4 : padded == 128 ? 4 : 6; }
-
-static int generic_splits(int batch, int num_kv_heads, int num_ctas, int padded) {
-    int ctas = num_ctas;
-    if (ctas <= 0 && device_sm_count(&ctas) != TQ_OK) ctas = 148;
-    int s = (generic_blocks_per_sm(padded) * ctas) / (batch * num_kv_heads > 0 ? batch * num_kv_heads : 1);
+// The plain decode kernel cuts every sequence into the same number of pieces, four blocks per SM in all.
+static int generic_splits(int batch, int num_kv_heads, int ctas) {
+    const int s = (4 * ctas) / (batch * num_kv_heads > 0 ? batch * num_kv_heads : 1);
     return s < 1 ? 1 : (s > 64 ? 64 : s);
 }
 
+size_t split_workspace_bytes(int columns, int padded, int ctas);
+int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim, int padded,
+                 const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
+                 int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
+                 void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
+                 int all_or_nothing, int ctas, cudaStream_t s);
+
+static int generic_ctas(int num_ctas) {
+    int ctas = num_ctas;
+    if (ctas <= 0 && device_sm_count(&ctas) != TQ_OK) ctas = 148;
+    return ctas;
+}
+
 size_t generic_workspace_bytes(int batch, int num_q_heads, int num_kv_heads, int head_dim, int num_ctas) {
-    const int pd = make_geom(head_dim, 0).padded;
-    const size_t rows = (size_t)batch * generic_splits(batch, num_kv_heads, num_ctas, pd) * num_q_heads;
+    const int pd = make_geom(head_dim, 0).padded, ctas = generic_ctas(num_ctas);
+    const size_t rows = (size_t)batch * generic_splits(batch, num_kv_heads, ctas) * num_q_heads;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    return 256 + up(rows * sizeof(float)) + up(rows * pd * sizeof(float));
+    const size_t plain = 256 + up(rows * sizeof(float)) + up(rows * pd * sizeof(float));
+    const size_t split = split_workspace_bytes(num_q_heads / num_kv_heads, pd, ctas);
+    return plain > split ? plain : split;
 }
 
 int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim,
@@ -1180,9 +856,15 @@ int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_hea
     TQ_REQUIRE(workspace_bytes >= generic_workspace_bytes(batch, num_q_heads, num_kv_heads, head_dim, num_ctas), TQ_ERR_WORKSPACE,
                "workspace too small: %zu < %zu", workspace_bytes,
                generic_workspace_bytes(batch, num_q_heads, num_kv_heads, head_dim, num_ctas));
+    const int ctas = generic_ctas(num_ctas);
+    // slots that 16-byte copies can take go to the split kernel on the tensor cores; anything else keeps the plain one
+    if (slot_bytes % 16 == 0 && ((uintptr_t)kv_cache % 16) == 0)
+        return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, make_geom(head_dim, 0).padded, kv_cache, num_blocks,
+                            slot_bytes, page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace,
+                            workspace_bytes, out, out_dtype, out_lse, emit_rotated, 0, ctas, static_cast<cudaStream_t>(stream));
     GenDecodeParams p{};
     p.g = make_geom(head_dim, slot_bytes);
-    p.splits = generic_splits(batch, num_kv_heads, num_ctas, p.g.padded);
+    p.splits = generic_splits(batch, num_kv_heads, ctas);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     const size_t rows = (size_t)batch * p.splits * num_q_heads;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -1224,27 +906,10 @@ int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_hea
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     const dim3 grid((unsigned)p.splits, (unsigned)batch, (unsigned)num_kv_heads);
-    // the tensor-core kernel reads the codes with 16-byte loads; anything else keeps the plain one
-    const bool aligned = slot_bytes % 16 == 0 && ((uintptr_t)kv_cache % 16) == 0 && p.slab_bytes % 16 == 0;
-    if (aligned) {
-        static bool frags_configured[64] = {};
-        if (dev < 0 || dev >= 64 || !frags_configured[dev]) {
-            TQ_CUDA(cudaFuncSetAttribute(decode_frags_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FragShape<64>::kSmem));
-            TQ_CUDA(cudaFuncSetAttribute(decode_frags_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FragShape<128>::kSmem));
-            TQ_CUDA(cudaFuncSetAttribute(decode_frags_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FragShape<256>::kSmem));
-            if (dev >= 0 && dev < 64) frags_configured[dev] = true;
-        }
-        switch (p.g.padded) {
-            case 64: decode_frags_kernel<64><<<grid, kGenWarps * 32, FragShape<64>::kSmem, s>>>(p); break;
-            case 128: decode_frags_kernel<128><<<grid, kGenWarps * 32, FragShape<128>::kSmem, s>>>(p); break;
-            default: decode_frags_kernel<256><<<grid, kGenWarps * 32, FragShape<256>::kSmem, s>>>(p); break;
-        }
-    } else {
-        switch (p.g.qbytes / 32) {
-            case 1: decode_generic_kernel<1><<<grid, kGenWarps * 32, smem, s>>>(p); break;
-            case 2: decode_generic_kernel<2><<<grid, kGenWarps * 32, smem, s>>>(p); break;
-            default: decode_generic_kernel<4><<<grid, kGenWarps * 32, smem, s>>>(p); break;
-        }
+    switch (p.g.qbytes / 32) {
+        case 1: decode_generic_kernel<1><<<grid, kGenWarps * 32, smem, s>>>(p); break;
+        case 2: decode_generic_kernel<2><<<grid, kGenWarps * 32, smem, s>>>(p); break;
+        default: decode_generic_kernel<4><<<grid, kGenWarps * 32, smem, s>>>(p); break;
     }
     TQ_CUDA(cudaGetLastError());
     GenMergeParams m{};
