@@ -1,0 +1,42 @@
+"""The four-lane row kernels of the flat quantizer: every padded size, bit width, element type and pack order, row counts around
+the eight rows of a warp pass, rows on the exceptional paths.  Codes, norms and dequantized values equal the oracle's bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+from turboquant_b200 import _cabi, synthetic
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rows(n, dim, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(n, dim, generator=g)
+    x[:, 1 % dim] *= 20.0                                  # an outlier channel
+    for i, v in enumerate((0.0, 1e-30, 3e-5, 6e4)):        # zero, tiny and large rows
+        if n > 8 + i:
+            x[8 + i] = v
+    if n > 16:
+        x[13, 3], x[14, 5], x[15] = float("inf"), float("nan"), 0.0
+        x[15, 7] = 1.0                                     # one-hot: ties of the transform's outputs
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim,n", [(128, 1), (128, 7), (128, 65), (64, 8), (64, 1000), (96, 66), (72, 9), (256, 33), (192, 300)])
+def test_rows_match_the_oracle(oracle, dim, n, dtype):
+    signs = synthetic.make_signs(1 << (dim - 1).bit_length(), 42)
+    x = _rows(n, dim, dtype, 3 + dim + n)
+    for bits in (1, 2, 3, 4):
+        per = 8 // bits
+        want_p, want_n = oracle.quantize_flat(x.float().numpy(), signs.numpy(), bits)
+        codes = (want_p[:, :, None] >> (bits * np.arange(per, dtype=np.uint8))) & ((1 << bits) - 1)
+        want_c = (codes << (bits * np.arange(per - 1, -1, -1, dtype=np.uint8))).sum(axis=2).astype(np.uint8)
+        for cache_order, want in ((False, want_p), (True, want_c)):
+            p, norms = _cabi.quantize_flat(x.to(DEV), signs.to(DEV), bits, cache_order=cache_order)
+            np.testing.assert_array_equal(p.cpu().numpy(), want, err_msg=f"bits {bits} cache order {cache_order}")
+            # bit for bit, except that a NaN is the canonical one here and carries its input's payload in the oracle
+            np.testing.assert_array_equal(norms.cpu().numpy(), want_n)
+            out = _cabi.dequantize_flat(p, norms, signs.to(DEV), dim, bits, cache_order=cache_order)
+            np.testing.assert_array_equal(out.cpu().numpy(), oracle.dequantize_flat(want_p, want_n, signs.numpy(), dim, bits))

@@ -61,25 +61,6 @@ struct WriteParams {
     alignas(64) CUtensorMap tmap[2];
 };
 
-// Two fp32 values in one 64-bit register and the packed arithmetic of sm_100 (add/sub/mul/fma
-// .f32x2): each lane of a pair is rounded to nearest exactly like the scalar instruction, at half
-// the instruction count.  A lane's elements (8j + 2m, 8j + 2m + 1) form the natural pairs.
-struct P2 { unsigned long long v; };
-__device__ __forceinline__ P2 pk(float lo, float hi) {
-    P2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void up(P2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
-__device__ __forceinline__ P2 add2(P2 a, P2 b) { P2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ P2 sub2(P2 a, P2 b) { P2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ P2 mul2(P2 a, P2 b) { P2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c) {
-    P2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-
 // Code of y among the 15 boundaries: the number of boundaries strictly below y (torch.bucketize,
 // right = False), as a float.  The boundaries are at least 1/64 apart, so the bin
 // k = round(64 y) + kBinZero holds at most one of them; the binning is monotone in y, hence every

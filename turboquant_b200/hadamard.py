@@ -12,7 +12,6 @@ def next_power_of_2(n: int) -> int:
     return 1 if n <= 1 else 1 << (n - 1).bit_length()
 
 
-@torch.no_grad()
 def fwht(x: torch.Tensor) -> torch.Tensor:
     """Normalized FWHT along the last dimension (a power of two up to 256): (1/sqrt(d)) H x."""
     d = x.shape[-1]
@@ -29,10 +28,8 @@ class RandomHadamardRotation:
         self.padded_dim = next_power_of_2(dim)
         self.signs = make_signs(self.padded_dim, seed).to(device)
 
-    @torch.no_grad()
     def rotate(self, x: torch.Tensor) -> torch.Tensor:
         return _cabi.fwht(x, self.padded_dim, self.padded_dim, pre_signs=self.signs).to(x.dtype)
 
-    @torch.no_grad()
     def inverse_rotate(self, y: torch.Tensor) -> torch.Tensor:
         return _cabi.fwht(y, self.padded_dim, self.orig_dim, post_signs=self.signs).to(y.dtype)

@@ -20,17 +20,14 @@ class TurboQuantMSE:
         self.rotation = RandomHadamardRotation(dim, device=device, seed=seed)
         self.codebook = Codebook(self.rotation.padded_dim, bit_width, device=device)
 
-    @torch.no_grad()
     def quantize(self, x: torch.Tensor):
         """x [..., d] -> (packed uint8 [..., padded*bits/8] in the low-first order of the
         reference's ``_pack_bits``, norms fp32 [...])."""
         return _cabi.quantize_flat(x, self.rotation.signs, self.bit_width, cache_order=False)
 
-    @torch.no_grad()
     def quantize_cache_order(self, x: torch.Tensor):
         """Same codes packed the way the paged cache stores them (even dim in the high nibble)."""
         return _cabi.quantize_flat(x, self.rotation.signs, self.bit_width, cache_order=True)
 
-    @torch.no_grad()
     def dequantize(self, packed: torch.Tensor, norms: torch.Tensor) -> torch.Tensor:
         return _cabi.dequantize_flat(packed, norms, self.rotation.signs, self.dim, self.bit_width)
