@@ -100,6 +100,10 @@ struct GenWriteParams {
 
 static __device__ int32_t g_gen_write_dropped = 0;
 
+// Rows (tokens x heads x 2) up to which a warp per row is the faster write, by padded head size: its time is flat until the grid
+// no longer fits the chip at once and then grows 1.4 (64, 128) to 2.7 times (256) as fast as that of the kernels with more rows per warp.
+constexpr int64_t row_warp_rows(int padded) { return padded == 64 ? 4096 : padded == 128 ? 2048 : 8192; }
+
 // Eight lanes own one row and a warp works on four rows at a time.  Lane q of a row holds elements
 // q, q + 8, q + 16, ... (E = padded / 8 registers), which is the torch evaluation order of the norm laid out
 // across lanes: accumulator k of the eight interleaved ones is lane k's running sum over its registers.  Butterfly
@@ -120,6 +124,7 @@ __global__ void __launch_bounds__(kGenWarps * 32, 8) write_rows8_kernel(const __
     __shared__ float bnd_s[16];
     __shared__ __align__(16) uint8_t code_s[kGenWarps][4][G::kRowStride];
     __shared__ float sg_s[G::kPd];
+    grid_launch_dependents();
     if (threadIdx.x < 15) bnd_s[threadIdx.x] = p.boundaries[threadIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = lane & 7, rg = lane >> 3;
@@ -130,6 +135,7 @@ __global__ void __launch_bounds__(kGenWarps * 32, 8) write_rows8_kernel(const __
 
     // signs in shared memory (1 for the padding, which stays +0): E registers less than holding them
     for (int j = threadIdx.x; j < G::kPd; j += kGenWarps * 32) sg_s[j] = j < hd ? p.signs[j] : 1.0f;
+    grid_dependency_wait();   // K, V, the slots and the cache belong to earlier kernels; the signs are a constant of the context
     __syncthreads();
     const float* sg = sg_s + q;
 
@@ -271,15 +277,158 @@ __global__ void __launch_bounds__(kGenWarps * 32, 8) write_rows8_kernel(const __
     }
 }
 
+// A warp per row: the write of a decode step's few new tokens, where nothing counts but the length of the dependent chain.
+// Lane 8 q + k holds elements 8 (JL q + i) + k, i < JL = padded / 32: norm accumulator k passes through the four quarters of the
+// warp in order, butterfly stages 1, 2, 4 are shuffles, then log2(JL) stages between registers, then two shuffles.  The
+// kernel for large writes gives two lanes a row and needs a table in shared memory, which is a chain of 64 elements and the codes of
+// a row one after the other: 8 tokens x 8 heads of 128 take 3.2 us there and 1.6 us here (head 64: 3.0 and 1.5, head 256: 6.6 and 2.0).
+template <typename T, int JL>
+__global__ void __launch_bounds__(128) write_row_warp_kernel(const __grid_constant__ GenWriteParams p) {
+    constexpr int kPd = 32 * JL;
+    __shared__ float bnd_s[16];
+    const int lane = threadIdx.x & 31, k = lane & 7, q4 = lane >> 3;
+    const int H = p.num_kv_heads, hd = p.g.head_dim;
+    grid_launch_dependents();
+    if (threadIdx.x < 15) bnd_s[threadIdx.x] = p.boundaries[threadIdx.x];
+    float sg[JL];      // the signs are a constant of the context: read ahead of the wait
+#pragma unroll
+    for (int i = 0; i < JL; i++) sg[i] = 8 * (JL * q4 + i) + k < hd ? p.signs[8 * (JL * q4 + i) + k] : 1.0f;
+    __syncthreads();
+    const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);      // (token, head, K or V)
+    const int which = (int)(r & 1);
+    const int64_t th = r >> 1;
+    const int64_t t = th < 0x7fffffff ? (int64_t)((uint32_t)th / (uint32_t)H) : th / H;
+    const int h = (int)(th - t * H);
+    grid_dependency_wait();      // K, V, the slots and the cache belong to earlier kernels
+    if (t >= p.num_tokens) return;
+    int64_t slot = p.slot_is_i64 ? reinterpret_cast<const int64_t*>(p.slot_mapping)[t] : (int64_t) reinterpret_cast<const int32_t*>(p.slot_mapping)[t];
+    const T* row = reinterpret_cast<const T*>(p.src[which]) + t * p.token_stride[which] + (int64_t)h * hd;
+    float x[JL];
+#pragma unroll
+    for (int i = 0; i < JL; i++) {
+        const int e = 8 * (JL * q4 + i) + k;
+        x[i] = e < hd ? to_f32(row[e]) : 0.0f;
+    }
+    // norm in the reference order: accumulator k over j = JL q + i, then the accumulators left to right, then the elements past the last
+    // multiple of eight (zeros of the padding add nothing to either)
+    const int full = hd & ~7, ntail = hd - full;
+    float acc = 0.0f, minsq = 3.0e38f, tail_sq = 0.0f, sq[JL];
+#pragma unroll
+    for (int i = 0; i < JL; i++) {
+        const int e0 = 8 * (JL * q4 + i);
+        sq[i] = __fmul_rn(x[i], x[i]);
+        if (e0 + k < hd) minsq = fminf(minsq, sq[i]);
+        if (e0 == full) tail_sq = sq[i];
+        if (e0 >= full) sq[i] = 0.0f;
+    }
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        const float before = s ? __shfl_sync(0xffffffffu, acc, 8 * (s - 1) + k) : 0.0f;
+        if (q4 == s) {
+            acc = before;
+#pragma unroll
+            for (int i = 0; i < JL; i++) acc = __fadd_rn(acc, sq[i]);
+        }
+    }
+    float s = __shfl_sync(0xffffffffu, acc, 24);
+#pragma unroll
+    for (int a = 1; a < 8; a++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, acc, 24 + a));
+    for (int a = 0; a < ntail; a++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, tail_sq, 8 * (full / (8 * JL)) + a));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) minsq = fminf(minsq, __shfl_xor_sync(0xffffffffu, minsq, o));
+    float norm = __fsqrt_rn(s);
+    if (!(norm >= 1e-8f)) norm = (norm != norm) ? __uint_as_float(0x7fc00000u) : 1e-8f;
+    const bool fast = minsq >= 1.1754944e-38f && norm >= 9.0949470e-13f && norm <= 1.0995116e12f &&
+                      (__float_as_uint(norm) & 0x7fffffu) != 0x7fffffu;
+    if (fast) {
+        const float rcp = __frcp_rn(norm);
+#pragma unroll
+        for (int i = 0; i < JL; i++) {
+            const float qv = __fmul_rn(x[i], rcp);
+            x[i] = __fmul_rn(__fmaf_rn(__fmaf_rn(qv, -norm, x[i]), rcp, qv), sg[i]);      // x - q norm is exact
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < JL; i++) x[i] = 8 * (JL * q4 + i) + k < hd ? __fmul_rn(__fdiv_rn(x[i], norm), sg[i]) : 0.0f;
+    }
+    // butterflies in stage order
+    auto across = [&](int m) {
+#pragma unroll
+        for (int i = 0; i < JL; i++) {
+            const float o = __shfl_xor_sync(0xffffffffu, x[i], m);
+            x[i] = (lane & m) ? __fsub_rn(o, x[i]) : __fadd_rn(x[i], o);
+        }
+    };
+    across(1);
+    across(2);
+    across(4);
+#pragma unroll
+    for (int hr = 1; hr < JL; hr <<= 1) {
+#pragma unroll
+        for (int i = 0; i < JL; i++) {
+            if ((i & hr) == 0) {
+                const float a = x[i], b = x[i + hr];
+                x[i] = __fadd_rn(a, b);
+                x[i + hr] = __fsub_rn(a, b);
+            }
+        }
+    }
+    across(8);
+    across(16);
+    // codes: byte k / 2 of word JL q + i; every lane of a quarter ends up with the quarter's words, lane k stores word k
+    uint32_t mine = 0;
+#pragma unroll
+    for (int i = 0; i < JL; i++) {
+        const float y = __fmul_rn(x[i], p.scale);
+        int c = (bnd_s[7] < y) ? 8 : 0;      // boundaries strictly below y
+        c += (bnd_s[c + 3] < y) ? 4 : 0;
+        c += (bnd_s[c + 1] < y) ? 2 : 0;
+        c += (bnd_s[c] < y) ? 1 : 0;
+        if (y != y) c = 15;
+        uint32_t w = (uint32_t)c << (8 * (k >> 1) + ((k & 1) ? 0 : 4));
+#pragma unroll
+        for (int m = 1; m < 8; m <<= 1) w |= __shfl_xor_sync(0xffffffffu, w, m);
+        if (k == i) mine = w;
+    }
+    if (slot >= p.total_slots) {
+        if (lane == 0 && h == 0 && which == 0) atomicAdd(&g_gen_write_dropped, 1);
+        slot = -1;
+    }
+    if (slot < 0) return;
+    uint8_t* dst = p.kv_cache + (size_t)which * p.slab_bytes + ((size_t)slot * H + h) * p.g.slot_bytes;
+    if (k < JL) {
+        uint8_t* at = dst + 4 * (JL * q4 + k);
+        if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+            *reinterpret_cast<uint32_t*>(at) = mine;
+        } else {
+#pragma unroll
+            for (int b = 0; b < 4; b++) at[b] = (uint8_t)(mine >> (8 * b));
+        }
+    }
+    if (lane < kPd / 64)
+        reinterpret_cast<uint16_t*>(dst + kPd / 2)[lane] = (norm != norm) ? (uint16_t)0x7e00u : __half_as_ushort(__float2half_rn(norm));
+    if (p.zero_pad)
+        for (int b = kPd / 2 + 2 * (kPd / 64) + lane; b < p.g.slot_bytes; b += 32) dst[b] = 0;
+}
+
 template <typename T>
-static void launch_write_rows8(const GenWriteParams& p, unsigned grid, cudaStream_t s) {
+static cudaError_t launch_write_row_warp(const GenWriteParams& p, cudaStream_t s) {
+    const dim3 grid((unsigned)((2 * p.num_tokens * p.num_kv_heads + 3) / 4));
+    switch (p.g.padded) {
+        case 64: return launch_serialized(write_row_warp_kernel<T, 2>, grid, dim3(128), 0, s, p);
+        case 128: return launch_serialized(write_row_warp_kernel<T, 4>, grid, dim3(128), 0, s, p);
+        default: return launch_serialized(write_row_warp_kernel<T, 8>, grid, dim3(128), 0, s, p);
+    }
+}
+
+template <typename T>
+static cudaError_t launch_write_rows8(const GenWriteParams& p, unsigned grid, cudaStream_t s) {
+    const dim3 g(grid), b(kGenWarps * 32);
     switch (p.g.padded) {
         case 64:
-            if (p.walk > 1) write_rows8_kernel<T, 8, true><<<grid, kGenWarps * 32, 0, s>>>(p);
-            else write_rows8_kernel<T, 8, false><<<grid, kGenWarps * 32, 0, s>>>(p);
-            break;
-        case 128: write_rows8_kernel<T, 16, false><<<grid, kGenWarps * 32, 0, s>>>(p); break;
-        default: write_rows8_kernel<T, 32, false><<<grid, kGenWarps * 32, 0, s>>>(p); break;
+            return p.walk > 1 ? launch_serialized(write_rows8_kernel<T, 8, true>, g, b, 0, s, p) : launch_serialized(write_rows8_kernel<T, 8, false>, g, b, 0, s, p);
+        case 128: return launch_serialized(write_rows8_kernel<T, 16, false>, g, b, 0, s, p);
+        default: return launch_serialized(write_rows8_kernel<T, 32, false>, g, b, 0, s, p);
     }
 }
 
@@ -789,6 +938,12 @@ int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv
     p.scale = (float)(1.0 / std::sqrt((double)p.g.padded));
     float cen[16];
     host_codebook(p.g.padded, 4, cen, p.boundaries);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (2 * num_tokens * num_kv_heads <= row_warp_rows(p.g.padded)) {
+        TQ_CUDA(in_dtype == TQ_F32 ? launch_write_row_warp<float>(p, s) : in_dtype == TQ_F16 ? launch_write_row_warp<__half>(p, s)
+                                                                                            : launch_write_row_warp<__nv_bfloat16>(p, s));
+        return TQ_OK;
+    }
     // large jobs of the smallest head: a lane group walks all rows of its token (96 us against 101 for 32768 tokens x
     // 8 heads); small jobs (a decode step's new tokens) and the larger heads, where the index arithmetic is a smaller
     // share and fewer groups in flight cost more than it saves (347 us against 337 at head 256): a row per group
@@ -796,13 +951,8 @@ int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv
     const int64_t items = num_tokens * (2 * num_kv_heads / p.walk);
     const int64_t blocks = (items + 4 * kGenWarps - 1) / (4 * kGenWarps);   // four lane groups per warp and pass
     const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (in_dtype) {
-        case TQ_F32: launch_write_rows8<float>(p, grid, s); break;
-        case TQ_F16: launch_write_rows8<__half>(p, grid, s); break;
-        default: launch_write_rows8<__nv_bfloat16>(p, grid, s); break;
-    }
-    TQ_CUDA(cudaGetLastError());
+    TQ_CUDA(in_dtype == TQ_F32 ? launch_write_rows8<float>(p, grid, s) : in_dtype == TQ_F16 ? launch_write_rows8<__half>(p, grid, s)
+                                                                                      : launch_write_rows8<__nv_bfloat16>(p, grid, s));
     return TQ_OK;
 }
 
