@@ -1,0 +1,60 @@
+"""The decode kernel that splits by KV head (short contexts, head sizes 64 / 256): every way its plan can cut a batch, against the
+oracle, several times over the same workspace."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from turboquant_b200 import TurboQuantPagedAttention, synthetic
+from turboquant_b200.paged_attention import kv_cache_shape
+
+from tests.gpu_util import assert_attention_close
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+# (query heads, KV heads, head size, lengths)
+CASES = {
+    "one_page": (32, 8, 128, [1]),
+    "one_head_many_parts": (8, 1, 128, [2000]),                        # more parts than one merge warp takes
+    "cut_heads": (32, 8, 128, [1024, 1000]),
+    "whole_heads_and_empty_rows": (16, 8, 128, [256, 17, 0, 16, 15] * 3),
+    "one_piece_each": (32, 8, 128, [500] * 30),
+    "long_pieces": (40, 8, 128, [500] * 60),
+    "long_pieces_cut": (56, 8, 128, [300] * 33),
+    "ragged_even_cut": (8, 4, 128, [3000, 1, 40, 2500, 700, 16, 33, 129]),
+    "odd_heads": (12, 6, 128, [700, 80, 5]),                            # head sets of two (padded head size 128 of another slot is below)
+    "three_heads": (6, 3, 64, [700, 80, 5]),
+    "many_heads": (32, 32, 128, [333, 90]),
+    "many_sequences": (8, 4, 128, [20] * 300),                          # beyond what the piece search looks at
+    "head_96": (32, 8, 96, [100, 777]),
+    "head_64": (16, 8, 64, [1500, 31, 0, 640]),
+    "head_64_even": (16, 8, 64, [4000, 100, 100, 2000] * 8),
+    "head_80": (8, 2, 80, [400, 65]),
+    "head_256": (16, 8, 256, [900, 31, 0, 200]),
+    "head_256_eight_columns": (32, 4, 256, [300, 47]),
+}
+
+
+@pytest.mark.parametrize("name", [n for n in CASES if n != "odd_heads"] + ["odd_heads"])
+def test_every_cut_matches_the_oracle(oracle, name):
+    hq, hkv, d, lens = CASES[name]
+    if name == "odd_heads":
+        d = 80                                                          # 128-wide heads come in 1, 2, 4, 8, 16 or multiples of 4
+    attn = TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv)
+    case = synthetic.decode_case(seed=len(name), seq_lens=lens, dtype=torch.float16, heads=(hq, hkv), head_dim=d)
+    cache = torch.zeros(kv_cache_shape(max(case.num_blocks, 1), 16, hkv, d), dtype=torch.uint8, device=DEV)
+    attn.write(case.k.to(DEV), case.v.to(DEV), cache, case.slot_mapping.to(DEV))
+    want = oracle.decode_paged(case.q.float().numpy(), cache.cpu().numpy(), case.block_table.numpy(), case.seq_lens.numpy(),
+                               attn.signs(DEV).cpu().numpy(), attn.scale)
+    q, bt, sl = case.q.to(DEV), case.block_table.to(DEV), case.seq_lens.to(DEV)
+    for _ in range(3):
+        out = torch.full_like(q, float("nan"))
+        lse = torch.full(q.shape[:2], float("nan"), dtype=torch.float32, device=DEV)
+        attn.decode(q, cache, bt, sl, out, lse)
+        assert attn.status(len(lens), DEV) == 0
+        assert_attention_close(out.float().cpu().numpy(), want, name)
+        empty = np.array(lens) == 0
+        assert (out.cpu().numpy()[empty] == 0).all() and np.isneginf(lse.cpu().numpy()[empty]).all()
+        assert torch.isfinite(lse[torch.from_numpy(~empty)]).all()

@@ -40,7 +40,6 @@
 // would add a 2-byte-per-element shared-memory round trip to a kernel whose limiters are the
 // shared-memory lookups and instruction issue, not MMA throughput (the tensor pipe is 22% busy).
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
 
 #include "tq_decode_common.cuh"
@@ -847,6 +846,7 @@ int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_hea
                    const float* signs, float sm_scale, void* workspace, size_t workspace_bytes, void* out, int out_dtype,
                    float* out_lse, int emit_rotated, int num_ctas, void* stream);
 
+size_t split_workspace_bytes(int columns, int padded, int ctas);
 int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim, int padded,
                  const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
                  int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
@@ -856,6 +856,7 @@ bool mq_applicable(int num_kv_heads, int cols);
 int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks, int grid, int causal, cudaStream_t stream);
 
 static thread_local cudaEvent_t g_events[3] = {nullptr, nullptr, nullptr};
+cudaEvent_t decode_event(int i) { return g_events[i]; }   // of the calling thread, may be null
 static int g_exchange_spin_limit = kExchangeSpinLimit;
 
 struct WorkspaceLayout {
@@ -911,11 +912,52 @@ static bool single_launch(int num_kv_heads) {
 static int chunk_heads(int remaining) { return remaining >= 16 ? 16 : remaining >= 8 ? 8 : 4; }
 static int largest_chunk(int num_kv_heads) { return single_launch(num_kv_heads) ? num_kv_heads : chunk_heads(num_kv_heads); }
 
+// Page-heads (pages x KV heads; the host knows their bound, batch x table width) up to which the kernel that splits by head is
+// the faster one.  It starts sooner and spreads further, the streaming kernel above moves a page in fewer copies.  Measured on uniform
+// batches, split against streaming, us: 32 query / 8 KV heads, 8192 page-heads 15 / 16 - 22, 32768: 32 - 34 / 27 - 37, 65536: 53 - 58 / 43 - 51; eight
+// query heads per KV head (more rows to rotate and merge per block) or four KV heads (four page lanes, four partials) cross at 65536;
+// more than 16 KV heads take several launches of the streaming kernel on strided rows: 163 against 179 at 262144.  A ragged batch
+// holds fewer pages than its bound and crosses later.
+static int64_t split_limit(int num_kv_heads, int columns) {
+    if (!single_launch(num_kv_heads)) return 262144;
+    return columns > 4 || num_kv_heads <= 4 ? 81920 : 40960;
+}
+
 struct ExchangeArgs {
     int rank, world;
     void* const* bufs;  // host array [world]: every rank's exchange buffer as mapped in this process
     size_t bytes;       // size of each buffer
 };
+
+// Exchange of rotated partials: pass 1 (set_exchange on a merge's parameters) pushes this rank's rows to every rank ...
+static void set_exchange(MergeParams& m, const ExchangeArgs& x, int64_t rows) {
+    m.xmode = 1;
+    m.xrank = x.rank;
+    m.xworld = x.world;
+    m.xrows = rows;
+    m.xspin = g_exchange_spin_limit;
+    for (int w = 0; w < x.world; w++) m.xbuf[w] = static_cast<unsigned char*>(x.bufs[w]);
+}
+// ... and pass 2 waits for every rank's partial in this rank's buffer, merges and rotates back
+static int launch_exchange_wait(const MergeParams& m, cudaStream_t s) {
+    MergeParams f = m;
+    f.xmode = 2;
+    f.header = nullptr;
+    f.page_prefix = nullptr;
+    f.rows = m.xrows;
+    f.num_q_heads = 1;
+    f.nq = 1;
+    f.num_parts = m.xworld;
+    f.emit_rotated = 0;
+    TQ_CUDA(launch_serialized(merge_kernel<4>, dim3((unsigned)m.xrows, 1), dim3(128), 0, s, f));
+    return TQ_OK;
+}
+// both passes over finished rows (one part each)
+static int launch_exchange(MergeParams& m, const ExchangeArgs& x, int64_t rows, cudaStream_t s) {
+    set_exchange(m, x, rows);
+    TQ_CUDA(launch_serialized(merge_kernel<4>, dim3((unsigned)rows, 1), dim3(128), 0, s, m));
+    return launch_exchange_wait(m, s);
+}
 
 static int decode_common(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads,
                          int head_dim, const void* kv_cache, int64_t num_blocks, int block_size,
@@ -980,11 +1022,38 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
     TQ_REQUIRE(workspace_bytes >= w.total, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, w.total);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    static const long long split_max = getenv("TQ_SPLIT_MAX") ? atoll(getenv("TQ_SPLIT_MAX")) : 4096;
-    if (!wide && !x && num_ctas == 0 && (page_indptr ? 0 : (long long)batch * max_pages * num_kv_heads) <= split_max)
-        return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes, page_indices,
-                            page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes, out, out_dtype,
-                            out_lse, emit_rotated, 1, ctas, s);
+    if (!wide && num_ctas == 0 && !page_indptr && (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, nq * real_group)) {
+        auto split = [&](void* o, int o_dtype, float* lse, int rotated) {
+            return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes,
+                                page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes,
+                                o, o_dtype, lse, rotated, 1, ctas, s);
+        };
+        if (!x) {
+            if (g_events[0]) TQ_CUDA(cudaEventRecord(g_events[0], s));
+            rc = split(out, out_dtype, out_lse, emit_rotated);
+            if (rc == TQ_OK && g_events[2]) TQ_CUDA(cudaEventRecord(g_events[2], s));
+            return rc;
+        }
+        // for an exchange: finished rotated rows behind the kernel's own scratch (the streaming layout holds both), pushed from there
+        const size_t scratch = split_workspace_bytes(nq * real_group, kHeadDim, ctas);
+        const size_t rows = (size_t)batch * nq * real_q_heads, lse_bytes = (rows * sizeof(float) + 255) & ~(size_t)255;
+        TQ_REQUIRE(workspace_bytes >= scratch + lse_bytes + rows * kHeadDim * sizeof(float), TQ_ERR_WORKSPACE, "workspace too small");
+        float* const lse = reinterpret_cast<float*>(ws + scratch);
+        float* const o = reinterpret_cast<float*>(ws + scratch + lse_bytes);
+        rc = split(o, TQ_F32, lse, 1);
+        if (rc != TQ_OK) return rc;
+        MergeParams m{};
+        m.partial_o = o;
+        m.partial_lse = lse;
+        m.signs = signs;
+        m.out = out;
+        m.out_lse = out_lse;
+        m.rows = (int64_t)rows;
+        m.num_q_heads = m.nq = m.num_parts = 1;
+        m.head_dim = head_dim;
+        m.out_dtype = out_dtype;
+        return launch_exchange(m, *x, (int64_t)rows, s);
+    }
 
     DecodeParams p{};
     p.q = q;
@@ -1067,31 +1136,15 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
         m.grid_ctas = ctas;
         m.out_dtype = out_dtype;
         m.emit_rotated = emit_rotated;
-        if (x) {
-            m.xmode = 1;
-            m.xrank = x->rank;
-            m.xworld = x->world;
-            m.xrows = (int64_t)batch * nq * real_q_heads;
-            m.xspin = g_exchange_spin_limit;
-            for (int w = 0; w < x->world; w++) m.xbuf[w] = static_cast<unsigned char*>(x->bufs[w]);
-        }
+        if (x) set_exchange(m, *x, (int64_t)batch * nq * real_q_heads);
         // parts per sequence: about (blocks x page lanes) / batch; many of them -> the wide merge
         if ((int64_t)ctas * m.pps > (int64_t)64 * batch)
             TQ_CUDA(launch_serialized(merge_kernel<16>, dim3((unsigned)batch, (unsigned)vheads), dim3(512), 0, s, m));
         else
             TQ_CUDA(launch_serialized(merge_kernel<4>, dim3((unsigned)batch, (unsigned)vheads), dim3(128), 0, s, m));
         if (x) {
-            // second pass: wait for every rank's partial in this rank's buffer, merge, rotate back
-            MergeParams f = m;
-            f.xmode = 2;
-            f.header = nullptr;
-            f.page_prefix = nullptr;
-            f.rows = m.xrows;
-            f.num_q_heads = 1;
-            f.nq = 1;
-            f.num_parts = x->world;
-            f.emit_rotated = 0;
-            TQ_CUDA(launch_serialized(merge_kernel<4>, dim3((unsigned)m.xrows, 1), dim3(128), 0, s, f));
+            rc = launch_exchange_wait(m, s);
+            if (rc != TQ_OK) return rc;
         }
         kv0 += hk;
     }

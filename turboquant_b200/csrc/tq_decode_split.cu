@@ -40,7 +40,7 @@ struct SplitShape {
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
-    static constexpr int kGroups = 4, kGroupWarps = PD == 64 ? 6 : PD == 128 ? 4 : 3;
+    static constexpr int kGroups = 4, kGroupWarps = PD == 64 ? 5 : PD == 128 ? 4 : 3;
     static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
     static constexpr int kRingsBelow = PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
     static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)(kWarps - kRingsBelow) * kRingBytes;   // from offset 0: ample
@@ -816,6 +816,7 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
 // host side
 // ---------------------------------------------------------------------------------------------
 int device_sm_count(int* out);
+cudaEvent_t decode_event(int i);
 
 static size_t split_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -841,6 +842,7 @@ static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
     p.head_sets = p.kv_heads / p.head_set;
     p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
     TQ_CUDA(launch_serialized(decode_split_kernel<PD>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
+    if (cudaEvent_t mid = decode_event(1)) TQ_CUDA(cudaEventRecord(mid, s));
     // A head has about groups / (sequences x heads) parts at most: a warp fetches eight at a time, so up to eight go to one warp
     // (a block takes four rows), more to four or sixteen warps.
     const int rows = p.batch * p.kv_heads * p.group, parts = p.grid * F::kGroups / (p.batch * p.kv_heads);
