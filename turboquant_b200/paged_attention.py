@@ -43,6 +43,8 @@ class TurboQuantPagedAttention:
     does) and never synchronise.
     """
 
+    _layer = None      # the native call path (``_calls``)
+
     def __init__(self, num_heads: int, head_size: int, scale: float, num_kv_heads: int,
                  seed: int = 42, num_ctas: int = 0):
         if not 32 < head_size <= 256:
@@ -56,7 +58,6 @@ class TurboQuantPagedAttention:
         self.num_ctas = num_ctas
         self._signs: dict[torch.device, torch.Tensor] = {}
         self._workspaces: dict[tuple, torch.Tensor] = {}
-        self._layer = None
 
     @property
     def _calls(self):
@@ -65,7 +66,20 @@ class TurboQuantPagedAttention:
         refuse.  (Created on first use: it needs the built library.)"""
         if self._layer is None:
             self._layer = _cabi.native().Layer(self.num_heads, self.head_size, self.num_kv_heads, self.scale, self.num_ctas)
+            for s in self._signs.values():
+                self._layer.set_signs(s)
+            for (_, batch, queries), ws in self._workspaces.items():
+                self._layer.set_workspace(batch, queries, ws)
         return self._layer
+
+    def __setattr__(self, name, value):
+        """The native path holds the geometry: an attribute set later takes effect from the next call on."""
+        object.__setattr__(self, name, value)
+        if name in ("num_heads", "head_size", "num_kv_heads", "scale", "num_ctas"):
+            self._layer = None
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_layer"}      # a copy (pickle, deepcopy) binds its own on first use
 
     def signs(self, device) -> torch.Tensor:
         device = torch.device(device)
