@@ -851,7 +851,7 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
                  const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
                  int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
                  void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
-                 int all_or_nothing, int ctas, cudaStream_t s);
+                 int all_or_nothing, int causal, int ctas, cudaStream_t s);
 bool mq_applicable(int num_kv_heads, int cols);
 int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks, int grid, int causal, cudaStream_t stream);
 
@@ -1022,11 +1022,11 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
     TQ_REQUIRE(workspace_bytes >= w.total, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, w.total);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    if (!wide && num_ctas == 0 && !page_indptr && (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, nq * real_group)) {
+    if (num_ctas == 0 && !page_indptr && (wide || (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, nq * real_group))) {
         auto split = [&](void* o, int o_dtype, float* lse, int rotated) {
             return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes,
                                 page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes,
-                                o, o_dtype, lse, rotated, 1, ctas, s);
+                                o, o_dtype, lse, rotated, 1, causal, ctas, s);
         };
         if (!x) {
             if (g_events[0]) TQ_CUDA(cudaEventRecord(g_events[0], s));

@@ -23,10 +23,13 @@
 
 namespace tq {
 
-constexpr int kSplitMaxGroup = 8;    // query columns per KV head
+constexpr int kSplitMaxGroup = 8;     // query columns per KV head, and with the wide tiles of 128-wide heads
+constexpr int kSplitMaxWide = 32;
 
-template <int PD>
+// NT: tiles of eight query columns (MMA columns) a warp carries through one dequantization of its page.
+template <int PD, int NT>
 struct SplitShape {
+    static constexpr int kCols = 8 * NT;
     static constexpr int kE = PD / 32;                       // elements per lane of a row
     static constexpr int kKBytes = PD / 8, kVBytes = PD / 16;  // code bytes per lane and token, K and V
     static constexpr int kRow = ((PD / 2 + 2 * (PD / 64)) + 15) & ~15;   // staged bytes of a slot: 48 / 80 / 144
@@ -36,15 +39,23 @@ struct SplitShape {
     // 256: 144-byte rows do it as they are.  64: the V loads do, two K loads take three wavefronts for two.
     static constexpr int kKPitch = kRow, kVPitch = PD == 128 ? 96 : kRow;
     static constexpr int kStageBytes = 16 * (kKPitch + kVPitch);
-    static constexpr int kStages = PD == 256 ? 2 : 3;
+    static constexpr int kStages = NT > 2 ? 6 : NT == 2 ? 4 : PD == 256 ? 2 : 3;
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
-    static constexpr int kGroups = 4, kGroupWarps = PD == 64 ? 5 : PD == 128 ? 4 : 3;
+    // Wide tiles: 32 accumulators and 16 query registers a tile, so 12 warps of 168 registers with two tiles, 8 of 255 with three or
+    // four.  Four tiles' queries do not fit: the fragments of the last two are read from shared memory on every page (32 wavefronts
+    // beside the page's 64 lookups; all of them in registers spills).
+    static constexpr int kGroups = NT > 2 ? 2 : 4, kGroupWarps = NT == 2 ? 3 : NT > 2 ? 4 : PD == 64 ? 5 : PD == 128 ? 4 : 3;
+    static constexpr int kRegTiles = NT == 4 ? 2 : NT, kSmemTiles = NT - kRegTiles;
     static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
-    static constexpr int kRingsBelow = PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
+    static constexpr int kRingsBelow = NT > 2 ? 3 : NT == 2 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
     static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)(kWarps - kRingsBelow) * kRingBytes;   // from offset 0: ample
-    static_assert(kRingBytes >= kSplitMaxGroup * PD * 4, "a warp's partial output goes through its ring");
+    static_assert(kRingBytes >= kCols * PD * 4, "a warp's partial output goes through its ring");
+    // in the unused upper halves of the table's rows: rotated queries, the warps' plans, query fragments
+    static constexpr uint32_t kPlanAt = kGroups * kCols * PD * 2, kFragAt = kPlanAt + kWarps * 512;
+    static_assert(kFragAt + kGroups * kSmemTiles * 2048 <= kLutSpan / 2, "the upper halves hold 32 KB");
+    static_assert(NT == 1 || PD == 128, "wide tiles are for 128-wide heads");
     // A page's copies, 16 bytes a lane: rounds of kRoundTokens tokens' code bytes (kPieces lanes a token) for K, the same for V, and one
     // round for the 16 + 16 pieces with the norms.  Rounds lie a fixed distance apart, so a lane keeps two source pointers.
     static constexpr int kPieces = PD / 32, kRoundTokens = 32 / kPieces, kRounds = 16 / kRoundTokens;
@@ -66,6 +77,7 @@ struct SplitParams {
     int64_t slab_bytes, num_blocks, kv_begin, kv_end, tok_stride;
     int batch, kv_heads, group, max_pages, q_dtype, out_dtype, emit_rotated;
     int nq, real_heads, real_group, head_dim, slot_bytes;
+    int causal;             // query i of nq sees the first len - (nq - 1 - i) tokens
     int grid, head_set, head_sets;   // blocks of the decode launch; heads side by side in a block when the work is cut evenly, and kv_heads / head_set
     float inv_warps;        // 1 / warps of the grid
     int all_or_nothing;     // a sequence longer than its table empties the whole batch (128-wide heads), or only itself
@@ -85,6 +97,8 @@ struct SplitParams {
 // Pieces are taken when their tiles exceed the even share by at most kSplitSlackTiles (about what a second start costs a group).
 // ---------------------------------------------------------------------------------------------
 constexpr int kSplitItemCost = 6, kSplitSlackTiles = 3;
+// The running maximum before any score: finite, so that a column whose tokens are all masked so far has exp2(-inf - m) = 0.
+constexpr float kNoMax = -3.402823466e38f;
 
 // n / d for 0 <= n < 2^24, d > 0: a reciprocal, then the quotient put right.  (The plan is repeated by every warp, and the compiler's
 // division is three times as long.)
@@ -327,12 +341,12 @@ __device__ __forceinline__ void split_finish(const SplitParams& p, const float* 
     if (p.out_lse && lane == 0) p.out_lse[orow] = lse2 * 0.6931471805599453f;
 }
 
-template <int PD>
-__global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kernel(const __grid_constant__ SplitParams p) {
-    using F = SplitShape<PD>;
+template <int PD, int NT>
+__global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_kernel(const __grid_constant__ SplitParams p) {
+    using F = SplitShape<PD, NT>;
     constexpr int E = F::kE, NG = F::kGroups, GW = F::kGroupWarps;
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ float m_s[NG][GW][kSplitMaxGroup], l_s[NG][GW][kSplitMaxGroup];
+    __shared__ float m_s[NG][GW][F::kCols], l_s[NG][GW][F::kCols];
     __shared__ float sign_s[PD];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
@@ -350,7 +364,7 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
     uint8_t* const lut = smem + (kLutAddr - smem_base);
     // byte `off` of row r of the group's rotated queries (PD fp16), in the unused upper halves of the table's 256-byte rows
     auto q_ptr = [&](int r, uint32_t off) -> uint8_t* {
-        const uint32_t at = (uint32_t)(gg * kSplitMaxGroup + r) * (PD * 2) + off;
+        const uint32_t at = (uint32_t)(gg * F::kCols + r) * (PD * 2) + off;
         return lut + ((at >> 7) << 8) + 128u + (at & 127u);
     };
     auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + gg), "r"(GW * 32) : "memory"); };
@@ -392,7 +406,7 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
     }
     // the lane's sequence of the plan waits in shared memory while pages are worked on (registers are what the loop is short of)
     auto plan_at = [&]() -> uint8_t* {
-        const uint32_t at = (uint32_t)(NG * kSplitMaxGroup * PD * 2) + (uint32_t)warp * 512u + (uint32_t)lane * 16u;
+        const uint32_t at = F::kPlanAt + (uint32_t)warp * 512u + (uint32_t)lane * 16u;
         return lut + ((at >> 7) << 8) + 128u + (at & 127u);
     };
     *reinterpret_cast<int4*>(plan_at()) = make_int4(s.np, s.len, s.vstart, s.vend);
@@ -409,6 +423,8 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
     const uint32_t k_at = split_keep(ring_at + ta * F::kKPitch + tg * F::kKBytes), kn_at = split_keep(ring_at + ta * F::kKPitch + PD / 2);
     const uint32_t v_at = split_keep(ring_at + 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + g * F::kVBytes);
     const uint32_t vn_at = F::kKPitch == F::kVPitch ? kn_at + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + ta * F::kVPitch + PD / 2);
+    // the lane's 16 bytes of fragment piece 0 (dims 16 i ... of tile j are piece 4 j + i, 512 bytes or four table rows each)
+    const uint32_t frag_at = split_keep(smem_u32(lut) + ((F::kFragAt + gg * F::kSmemTiles * 2048) << 1) + 128u + ((uint32_t)(lane >> 3) << 8) + 16u * (lane & 7));
     constexpr int kVNext = (PD == 128 ? 4 : 1) * F::kVPitch;      // from token(2 tg) to token(2 tg + 1)
     const uint32_t page_bytes = (uint32_t)(kPageTokens * p.tok_stride), round_bytes = (uint32_t)(F::kRoundTokens * p.tok_stride);
     bool bad_page = false;
@@ -467,14 +483,17 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
             return id;
         };
         int id_now = fetch_ids(0), id_next = n > 32 ? fetch_ids(32) : 0;
-        float qv[2][E];     // this warp's query rows wg and wg + GW (up to 8 rows a group; a third one at head 256 below)
+        // this warp's query rows wg, wg + GW, ... (a third one at head 256 below)
+        constexpr int kQRows = NT == 1 ? 2 : (F::kCols + GW - 1) / GW;
+        float qv[kQRows][E];
         const float* sign = sign_s + lane * E;
         auto q_row = [&](int r) -> int64_t {
             const int qi = r / p.real_group, hh = r - qi * p.real_group;
             return ((int64_t)b * p.nq + qi) * p.real_heads + head * p.real_group + hh;
         };
-        if (wg < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg), p.head_dim, lane * E, qv[0]);
-        if (wg + GW < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg + GW), p.head_dim, lane * E, qv[1]);
+#pragma unroll
+        for (int i = 0; i < kQRows; i++)
+            if (wg + i * GW < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg + i * GW), p.head_dim, lane * E, qv[i]);
         const uint8_t* const src_k = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)(c_tok * p.tok_stride) + 16 * c_piece;
         const uint8_t* const src_n = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)((lane & 15) * p.tok_stride) + PD / 2 + (lane < 16 ? 0 : p.slab_bytes);
         auto issue = [&](int i, uint32_t stage_off) {
@@ -501,27 +520,45 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
             for (int i = 0; i < E / 2; i++)
                 *reinterpret_cast<uint32_t*>(q_ptr(r, (uint32_t)(lane * E + 2 * i) * 2u)) = pack_half2(v[2 * i + 1] * p.scale, v[2 * i] * p.scale);
         };
-        if (wg < G) put_q(wg, qv[0]);
-        if (wg + GW < G) put_q(wg + GW, qv[1]);
-        for (int r = wg + 2 * GW; r < G; r += GW) {
+#pragma unroll
+        for (int i = 0; i < kQRows; i++)
+            if (wg + i * GW < G) put_q(wg + i * GW, qv[i]);
+        for (int r = wg + kQRows * GW; r < G; r += GW) {
             split_load_row<E>(p.q, p.q_dtype, q_row(r), p.head_dim, lane * E, qv[0]);
             put_q(r, qv[0]);
         }
         group_sync();
-        uint32_t qf[PD / 8];       // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column g
+        // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column 8 j + g
+        auto q_frag = [&](int j, int i) -> uint4 {
+            return 8 * j + g < G ? *reinterpret_cast<const uint4*>(q_ptr(8 * j + g, (uint32_t)(tg * (PD / 4)) * 2u + 16u * i)) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        uint32_t qf[F::kRegTiles][PD / 8];
 #pragma unroll
-        for (int i = 0; i < PD / 32; i++) {
-            const uint4 t = g < G ? *reinterpret_cast<const uint4*>(q_ptr(g, (uint32_t)(tg * (PD / 4)) * 2u + 16u * i)) : make_uint4(0u, 0u, 0u, 0u);
-            qf[4 * i] = t.x; qf[4 * i + 1] = t.y; qf[4 * i + 2] = t.z; qf[4 * i + 3] = t.w;
+        for (int j = 0; j < F::kRegTiles; j++)
+#pragma unroll
+            for (int i = 0; i < PD / 32; i++) {
+                const uint4 t = q_frag(j, i);
+                qf[j][4 * i] = t.x; qf[j][4 * i + 1] = t.y; qf[j][4 * i + 2] = t.z; qf[j][4 * i + 3] = t.w;
+            }
+        if constexpr (F::kSmemTiles > 0) {
+            for (int k = wg; k < F::kSmemTiles * (PD / 32); k += GW) {
+                const uint4 t = q_frag(F::kRegTiles + k / (PD / 32), k % (PD / 32));
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(frag_at + 1024u * k), "r"(t.x), "r"(t.y), "r"(t.z), "r"(t.w) : "memory");
+            }
+            group_sync();
         }
 
         // ---- pages -----------------------------------------------------------------------------------------
-        float o_acc[PD / 16][4];
+        float o_acc[NT][PD / 16][4], m0[NT], m1[NT], l0[NT], l1[NT];
 #pragma unroll
-        for (int i = 0; i < PD / 16; i++)
+        for (int t = 0; t < NT; t++) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) o_acc[i][j] = 0.0f;
-        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
+            for (int i = 0; i < PD / 16; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) o_acc[t][i][j] = 0.0f;
+            m0[t] = m1[t] = kNoMax;
+            l0[t] = l1[t] = 0.0f;
+        }
         uint32_t st = 0, st_issue = (F::kStages - 1) * F::kStageBytes;      // stage offsets
         int left = len - (fp + p0 + wg) * kPageTokens;                       // tokens from this warp's page on
         for (int it = 0; it < n; it++, left -= GW * kPageTokens) {
@@ -544,17 +581,41 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
                 split_lds<F::kVBytes>(v_at + st + kVNext, v1);
                 split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch, v2);
                 split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch + kVNext, v3);
-                float s_acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                float s_acc[NT][4], s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int t = 0; t < NT; t++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s_acc[t][i] = 0.0f;
 #pragma unroll
                 for (int w = 0; w < F::kKBytes / 4; w++) {
                     uint32_t ra[4], rb[4];
                     dequant8(ka[w], lut_lane, ra);
                     dequant8(kb[w], lut_lane, rb);
-                    mma16816(s_acc, ra[0], rb[0], ra[1], rb[1], qf[4 * w], qf[4 * w + 1]);
-                    mma16816(s_acc2, ra[2], rb[2], ra[3], rb[3], qf[4 * w + 2], qf[4 * w + 3]);
-                }
+                    if constexpr (NT == 1) {       // two chains
+                        mma16816(s_acc[0], ra[0], rb[0], ra[1], rb[1], qf[0][4 * w], qf[0][4 * w + 1]);
+                        mma16816(s_acc2, ra[2], rb[2], ra[3], rb[3], qf[0][4 * w + 2], qf[0][4 * w + 3]);
+                    } else {
+                        uint32_t qs[NT][4];
 #pragma unroll
-                for (int i = 0; i < 4; i++) s_acc[i] += s_acc2[i];
+                        for (int t = 0; t < NT; t++) {
+                            if (t < F::kRegTiles) {
+#pragma unroll
+                                for (int i = 0; i < 4; i++) qs[t][i] = qf[t][4 * w + i];
+                            } else {
+                                const uint4 v = lds128(frag_at + 1024u * ((t - F::kRegTiles) * (PD / 32) + w));
+                                qs[t][0] = v.x; qs[t][1] = v.y; qs[t][2] = v.z; qs[t][3] = v.w;
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[0], rb[0], ra[1], rb[1], qs[t][0], qs[t][1]);
+#pragma unroll
+                        for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[2], rb[2], ra[3], rb[3], qs[t][2], qs[t][3]);
+                    }
+                }
+                if constexpr (NT == 1) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s_acc[0][i] += s_acc2[i];
+                }
                 // ---- online softmax (base 2): rows g, g + 8 are tokens ta, tb; columns 2tg, 2tg + 1 query heads.  Only the
                 // last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
                 // slots contain) and their scores biased to -inf.  Row 0 of every page is inside.
@@ -565,31 +626,59 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
                     if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
                     if (tb >= left) { kfb = 0.0f; vfb = 0.0f; bias_b = -INFINITY; }
                 }
-                const float x0 = fmaf(s_acc[0], kfa, bias_a), x1 = fmaf(s_acc[1], kfa, bias_a);
-                const float x2 = fmaf(s_acc[2], kfb, bias_b), x3 = fmaf(s_acc[3], kfb, bias_b);
-                float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
-                if (__any_sync(0xffffffffu, mx0 > m0 + kRaiseThreshold || mx1 > m1 + kRaiseThreshold)) {
+                bool raise = false;
 #pragma unroll
-                    for (int o = 4; o < 32; o <<= 1) {
-                        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-                        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-                    }
-                    const bool raise0 = mx0 > m0 + kRaiseThreshold, raise1 = mx1 > m1 + kRaiseThreshold;
-                    const float c0 = raise0 ? fast_exp2(m0 - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1 - mx1) : 1.0f;
-                    if (raise0) m0 = mx0;
-                    if (raise1) m1 = mx1;
-                    l0 *= c0;
-                    l1 *= c1;
+                for (int t = 0; t < NT; t++) {
+                    float (&x)[4] = s_acc[t];
+                    x[0] = fmaf(x[0], kfa, bias_a);
+                    x[1] = fmaf(x[1], kfa, bias_a);
+                    x[2] = fmaf(x[2], kfb, bias_b);
+                    x[3] = fmaf(x[3], kfb, bias_b);
+                }
+                if (p.causal && left < kPageTokens + p.nq - 1) {       // a page that some query sees in part, or not at all
 #pragma unroll
-                    for (int i = 0; i < PD / 16; i++) {
-                        o_acc[i][0] *= c0; o_acc[i][1] *= c1; o_acc[i][2] *= c0; o_acc[i][3] *= c1;
+                    for (int t = 0; t < NT; t++) {
+                        const int s0 = left + 1 - p.nq + (8 * t + 2 * tg) / p.real_group, s1 = left + 1 - p.nq + (8 * t + 2 * tg + 1) / p.real_group;
+                        if (ta >= s0) s_acc[t][0] = -INFINITY;
+                        if (ta >= s1) s_acc[t][1] = -INFINITY;
+                        if (tb >= s0) s_acc[t][2] = -INFINITY;
+                        if (tb >= s1) s_acc[t][3] = -INFINITY;
                     }
                 }
-                const float e0 = fast_exp2(x0 - m0), e1 = fast_exp2(x1 - m1), e2 = fast_exp2(x2 - m0), e3 = fast_exp2(x3 - m1);
-                l0 += e0 + e2;
-                l1 += e1 + e3;
-                const uint32_t pb0 = movmatrix_trans(pack_half2(e0 * vfa, e1 * vfa));
-                const uint32_t pb1 = movmatrix_trans(pack_half2(e2 * vfb, e3 * vfb));
+#pragma unroll
+                for (int t = 0; t < NT; t++)
+                    raise |= fmaxf(s_acc[t][0], s_acc[t][2]) > m0[t] + kRaiseThreshold || fmaxf(s_acc[t][1], s_acc[t][3]) > m1[t] + kRaiseThreshold;
+                if (__any_sync(0xffffffffu, raise)) {
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        float mx0 = fmaxf(s_acc[t][0], s_acc[t][2]), mx1 = fmaxf(s_acc[t][1], s_acc[t][3]);
+#pragma unroll
+                        for (int o = 4; o < 32; o <<= 1) {
+                            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+                        }
+                        const bool raise0 = mx0 > m0[t] + kRaiseThreshold, raise1 = mx1 > m1[t] + kRaiseThreshold;
+                        const float c0 = raise0 ? fast_exp2(m0[t] - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1[t] - mx1) : 1.0f;
+                        if (raise0) m0[t] = mx0;
+                        if (raise1) m1[t] = mx1;
+                        l0[t] *= c0;
+                        l1[t] *= c1;
+#pragma unroll
+                        for (int i = 0; i < PD / 16; i++) {
+                            o_acc[t][i][0] *= c0; o_acc[t][i][1] *= c1; o_acc[t][i][2] *= c0; o_acc[t][i][3] *= c1;
+                        }
+                    }
+                }
+                uint32_t pb0[NT], pb1[NT];
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    const float e0 = fast_exp2(s_acc[t][0] - m0[t]), e1 = fast_exp2(s_acc[t][1] - m1[t]);
+                    const float e2 = fast_exp2(s_acc[t][2] - m0[t]), e3 = fast_exp2(s_acc[t][3] - m1[t]);
+                    l0[t] += e0 + e2;
+                    l1[t] += e1 + e3;
+                    pb0[t] = movmatrix_trans(pack_half2(e0 * vfa, e1 * vfa));
+                    pb1[t] = movmatrix_trans(pack_half2(e2 * vfb, e3 * vfb));
+                }
                 // ---- O^T += V^^T P ----------------------------------------------------------------------------
 #pragma unroll
                 for (int w = 0; w < F::kVBytes / 4; w++) {
@@ -604,7 +693,8 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
                     dequant8(hi23, lut_lane, a_hi23);
 #pragma unroll
                     for (int j = 0; j < 4; j++)     // rows: g <- odd dim, g + 8 <- even dim of code byte 4 w + j
-                        mma16816(o_acc[4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0, pb1);
+#pragma unroll
+                        for (int t = 0; t < NT; t++) mma16816(o_acc[t][4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0[t], pb1[t]);
                 }
             }
             __syncwarp();      // every lane has read the stage before a later iteration copies into it
@@ -615,15 +705,18 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
 
         // ---- combine the group's warps ------------------------------------------------------------------------
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-            l0 += __shfl_xor_sync(0xffffffffu, l0, o);
-            l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-        }
-        if (g == 0) {
-            m_s[gg][wg][2 * tg] = m0;      // columns past the group are zero queries: nobody reads them
-            m_s[gg][wg][2 * tg + 1] = m1;
-            l_s[gg][wg][2 * tg] = l0;
-            l_s[gg][wg][2 * tg + 1] = l1;
+        for (int t = 0; t < NT; t++) {
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                l0[t] += __shfl_xor_sync(0xffffffffu, l0[t], o);
+                l1[t] += __shfl_xor_sync(0xffffffffu, l1[t], o);
+            }
+            if (g == 0) {
+                m_s[gg][wg][8 * t + 2 * tg] = m0[t];      // columns past the group are zero queries: nobody reads them
+                m_s[gg][wg][8 * t + 2 * tg + 1] = m1[t];
+                l_s[gg][wg][8 * t + 2 * tg] = l0[t];
+                l_s[gg][wg][8 * t + 2 * tg + 1] = l1[t];
+            }
         }
         // The warp's accumulators as rows of PD floats in its own ring (the copies have landed and been read).  The 16-byte pieces of
         // a row are swapped by the column, which keeps the four columns a quarter warp stores at a time in different banks.
@@ -633,12 +726,13 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
 #pragma unroll
             for (int w = 0; w < F::kVBytes / 2; w++) {      // bytes 2 w, 2 w + 1 of this lane: dims d ... d + 3
                 const int piece = (g * F::kVBytes + 2 * w) / 2;
-                if (2 * tg < G)
-                    *reinterpret_cast<float4*>(mine + (2 * tg) * PD + 4 * (piece ^ tg)) =
-                        make_float4(o_acc[2 * w][2], o_acc[2 * w][0], o_acc[2 * w + 1][2], o_acc[2 * w + 1][0]);
-                if (2 * tg + 1 < G)
-                    *reinterpret_cast<float4*>(mine + (2 * tg + 1) * PD + 4 * (piece ^ tg)) =
-                        make_float4(o_acc[2 * w][3], o_acc[2 * w][1], o_acc[2 * w + 1][3], o_acc[2 * w + 1][1]);
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    const int c = 8 * t + 2 * tg;
+                    const float(&a)[4] = o_acc[t][2 * w], (&b4)[4] = o_acc[t][2 * w + 1];
+                    if (c < G) *reinterpret_cast<float4*>(mine + c * PD + 4 * (piece ^ tg)) = make_float4(a[2], a[0], b4[2], b4[0]);
+                    if (c + 1 < G) *reinterpret_cast<float4*>(mine + (c + 1) * PD + 4 * (piece ^ tg)) = make_float4(a[3], a[1], b4[3], b4[1]);
+                }
             }
         }
         group_sync();
@@ -654,7 +748,7 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
 #pragma unroll
             for (int w = 0; w < GW; w++) {
                 const float mw = m_s[gg][w][r];
-                if (mw > -INFINITY) {            // a warp without a page has stored nothing
+                if (mw > kNoMax) {            // a warp without a page has stored nothing
                     const float c = fast_exp2(mw - mm);
                     ll += c * l_s[gg][w][r];
                     const int other = gg * GW + w;
@@ -662,12 +756,12 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
                                            smem + (other < F::kRingsBelow ? (uint32_t)other * F::kRingBytes
                                                                          : kLutAddr + kLutSpan - smem_base + (uint32_t)(other - F::kRingsBelow) * F::kRingBytes)) + r * PD;
                     if constexpr (E == 2) {
-                        const float2 t = *reinterpret_cast<const float2*>(row + 4 * ((lane >> 1) ^ (r >> 1)) + 2 * (lane & 1));
+                        const float2 t = *reinterpret_cast<const float2*>(row + 4 * ((lane >> 1) ^ ((r & 7) >> 1)) + 2 * (lane & 1));
                         o[0] += c * t.x; o[1] += c * t.y;
                     } else {
 #pragma unroll
                         for (int i = 0; i < E / 4; i++) {
-                            const float4 t = *reinterpret_cast<const float4*>(row + 4 * ((lane * (E / 4) + i) ^ (r >> 1)));
+                            const float4 t = *reinterpret_cast<const float4*>(row + 4 * ((lane * (E / 4) + i) ^ ((r & 7) >> 1)));
                             o[4 * i] += c * t.x; o[4 * i + 1] += c * t.y; o[4 * i + 2] += c * t.z; o[4 * i + 3] += c * t.w;
                         }
                     }
@@ -701,9 +795,9 @@ __global__ void __launch_bounds__(SplitShape<PD>::kThreads, 1) decode_split_kern
 // the wait.  An empty sequence's rows become zeros here; a head that one group covered is finished already.
 // ---------------------------------------------------------------------------------------------
 
-template <int PD, int RW>
+template <int PD, int NT, int RW>
 __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const __grid_constant__ SplitParams p) {
-    using F = SplitShape<PD>;
+    using F = SplitShape<PD, NT>;
     constexpr int E = F::kE, GW = F::kGroupWarps, NG = F::kGroups, kRows = RW == 1 ? 4 : 1;      // rows of the block
     __shared__ float acc_s[RW][PD], m_s[RW], w_s[RW], sign_s[PD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -826,29 +920,29 @@ size_t split_workspace_bytes(int columns, int padded, int ctas) {
     return 256 + split_up(rows * sizeof(float)) + split_up(rows * padded * sizeof(float));
 }
 
-template <int PD>
+template <int PD, int NT>
 static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
-    using F = SplitShape<PD>;
-    static_assert(F::kGroups == 4, "split_workspace_bytes counts four groups a block");
+    using F = SplitShape<PD, NT>;
+    static_assert(F::kGroups <= 4, "split_workspace_bytes counts four groups a block");
     static bool configured[64] = {};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(decode_split_kernel<PD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::kSmem));
+        TQ_CUDA(cudaFuncSetAttribute(decode_split_kernel<PD, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::kSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     p.grid = ctas;
-    p.head_set = p.kv_heads % 4 == 0 ? 4 : p.kv_heads % 2 == 0 ? 2 : 1;
+    p.head_set = F::kGroups == 4 && p.kv_heads % 4 == 0 ? 4 : p.kv_heads % 2 == 0 ? 2 : 1;
     p.head_sets = p.kv_heads / p.head_set;
     p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
-    TQ_CUDA(launch_serialized(decode_split_kernel<PD>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
+    TQ_CUDA(launch_serialized(decode_split_kernel<PD, NT>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
     if (cudaEvent_t mid = decode_event(1)) TQ_CUDA(cudaEventRecord(mid, s));
     // A head has about groups / (sequences x heads) parts at most: a warp fetches eight at a time, so up to eight go to one warp
     // (a block takes four rows), more to four or sixteen warps.
     const int rows = p.batch * p.kv_heads * p.group, parts = p.grid * F::kGroups / (p.batch * p.kv_heads);
-    if (parts > 32) TQ_CUDA(launch_serialized(merge_split_kernel<PD, 16>, dim3((unsigned)rows), dim3(512), 0, s, p));
-    else if (parts > 8) TQ_CUDA(launch_serialized(merge_split_kernel<PD, 4>, dim3((unsigned)rows), dim3(128), 0, s, p));
-    else TQ_CUDA(launch_serialized(merge_split_kernel<PD, 1>, dim3((unsigned)(rows + 3) / 4), dim3(128), 0, s, p));
+    if (parts > 32) TQ_CUDA(launch_serialized(merge_split_kernel<PD, NT, 16>, dim3((unsigned)rows), dim3(512), 0, s, p));
+    else if (parts > 8) TQ_CUDA(launch_serialized(merge_split_kernel<PD, NT, 4>, dim3((unsigned)rows), dim3(128), 0, s, p));
+    else TQ_CUDA(launch_serialized(merge_split_kernel<PD, NT, 1>, dim3((unsigned)(rows + 3) / 4), dim3(128), 0, s, p));
     return TQ_OK;
 }
 
@@ -858,9 +952,10 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
                  const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
                  int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
                  void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
-                 int all_or_nothing, int ctas, cudaStream_t s) {
+                 int all_or_nothing, int causal, int ctas, cudaStream_t s) {
     SplitParams p{};
     p.group = nq * (real_q_heads / num_kv_heads);
+    TQ_REQUIRE(p.group <= (padded == 128 ? kSplitMaxWide : kSplitMaxGroup), TQ_ERR_UNSUPPORTED, "too many query columns: %d", p.group);
     const size_t need = split_workspace_bytes(p.group, padded, ctas);
     TQ_REQUIRE(workspace_bytes >= need, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
     TQ_REQUIRE((int64_t)batch * num_kv_heads * p.group < (int64_t)1 << 31, TQ_ERR_UNSUPPORTED, "too many rows for one launch");
@@ -893,6 +988,7 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
     p.head_dim = head_dim;
     p.slot_bytes = slot_bytes;
     p.all_or_nothing = all_or_nothing;
+    p.causal = causal;
     const double inv = 1.0 / std::sqrt((double)padded);
     p.scale = p.v_scale = (float)inv;
     p.k_scale = (float)(inv * (double)sm_scale * 1.4426950408889634);
@@ -901,9 +997,15 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
         memcpy(&p.centroid_h[k], &h, 2);
     }
     switch (padded) {
-        case 64: return launch_split<64>(p, ctas, s);
-        case 128: return launch_split<128>(p, ctas, s);
-        default: return launch_split<256>(p, ctas, s);
+        case 64: return launch_split<64, 1>(p, ctas, s);
+        case 128:
+            switch ((p.group + 7) / 8) {
+                case 1: return launch_split<128, 1>(p, ctas, s);
+                case 2: return launch_split<128, 2>(p, ctas, s);
+                case 3: return launch_split<128, 3>(p, ctas, s);
+                default: return launch_split<128, 4>(p, ctas, s);
+            }
+        default: return launch_split<256, 1>(p, ctas, s);
     }
 }
 

@@ -967,7 +967,7 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
                  const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
                  int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,
                  void* workspace, size_t workspace_bytes, void* out, int out_dtype, float* out_lse, int emit_rotated,
-                 int all_or_nothing, int ctas, cudaStream_t s);
+                 int all_or_nothing, int causal, int ctas, cudaStream_t s);
 
 static int generic_ctas(int num_ctas) {
     int ctas = num_ctas;
@@ -1011,7 +1011,7 @@ int generic_decode(const void* q, int q_dtype, int batch, int nq, int real_q_hea
     if (slot_bytes % 16 == 0 && ((uintptr_t)kv_cache % 16) == 0)
         return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, make_geom(head_dim, 0).padded, kv_cache, num_blocks,
                             slot_bytes, page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace,
-                            workspace_bytes, out, out_dtype, out_lse, emit_rotated, 0, ctas, static_cast<cudaStream_t>(stream));
+                            workspace_bytes, out, out_dtype, out_lse, emit_rotated, 0, 0, ctas, static_cast<cudaStream_t>(stream));
     GenDecodeParams p{};
     p.g = make_geom(head_dim, slot_bytes);
     p.splits = generic_splits(batch, num_kv_heads, ctas);
