@@ -918,7 +918,12 @@ static int largest_chunk(int num_kv_heads) { return single_launch(num_kv_heads) 
 // query heads per KV head (more rows to rotate and merge per block) or four KV heads (four page lanes, four partials) cross at 65536;
 // more than 16 KV heads take several launches of the streaming kernel on strided rows: 163 against 179 at 262144.  A ragged batch
 // holds fewer pages than its bound and crosses later.
+// More than eight columns, against the tcgen05 kernel: up to 24 the split kernel is faster or equal at every size (8 x 32768 tokens, 8
+// KV heads, 12 / 16 / 24 columns: 124 / 124 / 159 against 163 / 165 / 171; 32 ragged sequences: 38 / 40 / 56 against 69 / 73 / 85).
+// With 32 columns it is up to 65536 (71 against 93 at 32 ragged sequences, 103 against 107 at 8 x 32768 and 4 KV heads), not at 131072
+// (181 against 173).
 static int64_t split_limit(int num_kv_heads, int columns) {
+    if (columns > 8) return columns <= 24 ? INT64_MAX : 81920;
     if (!single_launch(num_kv_heads)) return 262144;
     return columns > 4 || num_kv_heads <= 4 ? 81920 : 40960;
 }
@@ -1022,7 +1027,7 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
     TQ_REQUIRE(workspace_bytes >= w.total, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, w.total);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    if (num_ctas == 0 && !page_indptr && (wide || (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, nq * real_group))) {
+    if (num_ctas == 0 && !page_indptr && ((wide && cols <= 8) || (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, cols))) {
         auto split = [&](void* o, int o_dtype, float* lse, int rotated) {
             return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes,
                                 page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes,

@@ -39,22 +39,28 @@ struct SplitShape {
     // 256: 144-byte rows do it as they are.  64: the V loads do, two K loads take three wavefronts for two.
     static constexpr int kKPitch = kRow, kVPitch = PD == 128 ? 96 : kRow;
     static constexpr int kStageBytes = 16 * (kKPitch + kVPitch);
-    static constexpr int kStages = NT > 2 ? 6 : NT == 2 ? 4 : PD == 256 ? 2 : 3;
+    // Wide tiles (128-wide heads): 32 accumulators a thread and tile.  Two tiles: 12 warps of 168 registers.  Three or four tiles would
+    // leave 8 warps of 255, so two warps go as a pair: each works out the probabilities of its own page and accumulates half of the
+    // dims of both (12 warps again).  Batch 8 x 32768 causal, 32 query / 8 KV heads: 8 queries a row 194 -> 181 us, 6: 171 -> 159 us,
+    // 32 ragged sequences x 4096, 8 queries: 87 -> 71 us; as a pair two tiles are slower (124 -> 140 us).
+    static constexpr bool kPair = NT >= 3;
+    static constexpr int kStages = NT == 2 && !kPair ? 4 : PD == 256 ? 2 : 3;
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
-    // Wide tiles: 32 accumulators and 16 query registers a tile, so 12 warps of 168 registers with two tiles, 8 of 255 with three or
-    // four.  Four tiles' queries do not fit: the fragments of the last two are read from shared memory on every page (32 wavefronts
-    // beside the page's 64 lookups; all of them in registers spills).
-    static constexpr int kGroups = NT > 2 ? 2 : 4, kGroupWarps = NT == 2 ? 3 : NT > 2 ? 4 : PD == 64 ? 5 : PD == 128 ? 4 : 3;
-    static constexpr int kRegTiles = NT == 4 ? 2 : NT, kSmemTiles = NT - kRegTiles;
+    static constexpr int kGroups = kPair ? (NT == 2 ? 4 : 2) : 4, kGroupWarps = kPair ? (NT == 2 ? 4 : 6) : NT == 2 ? 3 : PD == 64 ? 5 : PD == 128 ? 4 : 3;
+    // query fragments kept in registers; the other tiles' are read from shared memory on every page (16 wavefronts a tile beside the
+    // page's 64 lookups; in registers they spill: 8 queries 181 -> 185 us with one tile, 234 with two)
+    static constexpr int kRegTiles = NT == 4 ? 0 : NT == 3 ? 2 : NT;
     static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
-    static constexpr int kRingsBelow = NT > 2 ? 3 : NT == 2 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
-    static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)(kWarps - kRingsBelow) * kRingBytes;   // from offset 0: ample
-    static_assert(kRingBytes >= kCols * PD * 4, "a warp's partial output goes through its ring");
-    // in the unused upper halves of the table's rows: rotated queries, the warps' plans, query fragments
-    static constexpr uint32_t kPlanAt = kGroups * kCols * PD * 2, kFragAt = kPlanAt + kWarps * 512;
-    static_assert(kFragAt + kGroups * kSmemTiles * 2048 <= kLutSpan / 2, "the upper halves hold 32 KB");
+    static constexpr int kRingsBelow = kPair ? (NT == 2 ? 7 : 6) : NT == 2 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
+    // What the warps of a pair hand each other: the probabilities of a page as fragments, two pages' worth in turn.
+    static constexpr int kHandBytes = kPair ? (NT + 1) / 2 * 512 : 0, kHandAt = (kWarps - kRingsBelow) * kRingBytes;
+    static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)kHandAt + 2 * kWarps * kHandBytes;   // from offset 0: ample
+    static_assert(kRingBytes >= kCols * PD * (kPair ? 2 : 4), "a warp's partial output goes through its ring");
+    // in the unused upper halves of the table's rows: rotated queries, the warps' plans
+    static constexpr uint32_t kPlanAt = kGroups * kCols * PD * 2;
+    static_assert(kPlanAt + kWarps * 512 <= kLutSpan / 2, "the upper halves hold 32 KB");
     static_assert(NT == 1 || PD == 128, "wide tiles are for 128-wide heads");
     // A page's copies, 16 bytes a lane: rounds of kRoundTokens tokens' code bytes (kPieces lanes a token) for K, the same for V, and one
     // round for the 16 + 16 pieces with the norms.  Rounds lie a fixed distance apart, so a lane keeps two source pointers.
@@ -348,6 +354,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float m_s[NG][GW][F::kCols], l_s[NG][GW][F::kCols];
     __shared__ float sign_s[PD];
+    __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols];      // a pair's maxima of a page that raises them, and whether it does
+    __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -362,9 +370,11 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                                                        : kLutAddr + kLutSpan - smem_base + (uint32_t)(warp - F::kRingsBelow) * F::kRingBytes);
     const uint32_t ring_at = smem_u32(ring);
     uint8_t* const lut = smem + (kLutAddr - smem_base);
-    // byte `off` of row r of the group's rotated queries (PD fp16), in the unused upper halves of the table's 256-byte rows
+    // byte `off` of row r of the group's rotated queries (PD fp16), in the unused upper halves of the table's 256-byte rows, in the
+    // order of B fragments: piece (tile j = r / 8, i) of 512 bytes holds, 16 bytes a lane (g = r % 8, tg), bytes 16 i ... of quarter tg
     auto q_ptr = [&](int r, uint32_t off) -> uint8_t* {
-        const uint32_t at = (uint32_t)(gg * F::kCols + r) * (PD * 2) + off;
+        const uint32_t tg = off / (PD / 2), i = off % (PD / 2) / 16;
+        const uint32_t at = (uint32_t)gg * F::kCols * (PD * 2) + ((r >> 3) * (PD / 32) + i) * 512u + ((r & 7) * 4 + tg) * 16u + off % 16;
         return lut + ((at >> 7) << 8) + 128u + (at & 127u);
     };
     auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + gg), "r"(GW * 32) : "memory"); };
@@ -423,8 +433,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     const uint32_t k_at = split_keep(ring_at + ta * F::kKPitch + tg * F::kKBytes), kn_at = split_keep(ring_at + ta * F::kKPitch + PD / 2);
     const uint32_t v_at = split_keep(ring_at + 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + g * F::kVBytes);
     const uint32_t vn_at = F::kKPitch == F::kVPitch ? kn_at + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + ta * F::kVPitch + PD / 2);
-    // the lane's 16 bytes of fragment piece 0 (dims 16 i ... of tile j are piece 4 j + i, 512 bytes or four table rows each)
-    const uint32_t frag_at = split_keep(smem_u32(lut) + ((F::kFragAt + gg * F::kSmemTiles * 2048) << 1) + 128u + ((uint32_t)(lane >> 3) << 8) + 16u * (lane & 7));
+    const uint32_t frag_at = split_keep(smem_u32(lut) + ((uint32_t)gg * F::kCols * PD * 4) + 128u + ((uint32_t)(lane >> 3) << 8) + 16u * (lane & 7));
     constexpr int kVNext = (PD == 128 ? 4 : 1) * F::kVPitch;      // from token(2 tg) to token(2 tg + 1)
     const uint32_t page_bytes = (uint32_t)(kPageTokens * p.tok_stride), round_bytes = (uint32_t)(F::kRoundTokens * p.tok_stride);
     bool bad_page = false;
@@ -493,7 +502,12 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
         };
 #pragma unroll
         for (int i = 0; i < kQRows; i++)
-            if (wg + i * GW < G) split_load_row<E>(p.q, p.q_dtype, q_row(wg + i * GW), p.head_dim, lane * E, qv[i]);
+            if (wg + i * GW < G) {
+                split_load_row<E>(p.q, p.q_dtype, q_row(wg + i * GW), p.head_dim, lane * E, qv[i]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; e++) qv[i][e] = 0.0f;
+            }
         const uint8_t* const src_k = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)(c_tok * p.tok_stride) + 16 * c_piece;
         const uint8_t* const src_n = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)((lane & 15) * p.tok_stride) + PD / 2 + (lane < 16 ? 0 : p.slab_bytes);
         auto issue = [&](int i, uint32_t stage_off) {
@@ -522,186 +536,276 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
         };
 #pragma unroll
         for (int i = 0; i < kQRows; i++)
-            if (wg + i * GW < G) put_q(wg + i * GW, qv[i]);
+            if (wg + i * GW < F::kCols) put_q(wg + i * GW, qv[i]);
         for (int r = wg + kQRows * GW; r < G; r += GW) {
             split_load_row<E>(p.q, p.q_dtype, q_row(r), p.head_dim, lane * E, qv[0]);
             put_q(r, qv[0]);
         }
         group_sync();
-        // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column 8 j + g
-        auto q_frag = [&](int j, int i) -> uint4 {
-            return 8 * j + g < G ? *reinterpret_cast<const uint4*>(q_ptr(8 * j + g, (uint32_t)(tg * (PD / 4)) * 2u + 16u * i)) : make_uint4(0u, 0u, 0u, 0u);
-        };
-        uint32_t qf[F::kRegTiles][PD / 8];
+        uint32_t qf[F::kRegTiles > 0 ? F::kRegTiles : 1][PD / 8];    // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column 8 j + g
 #pragma unroll
         for (int j = 0; j < F::kRegTiles; j++)
 #pragma unroll
             for (int i = 0; i < PD / 32; i++) {
-                const uint4 t = q_frag(j, i);
+                const uint4 t = 8 * j + g < G ? lds128(frag_at + 1024u * (j * (PD / 32) + i)) : make_uint4(0u, 0u, 0u, 0u);
                 qf[j][4 * i] = t.x; qf[j][4 * i + 1] = t.y; qf[j][4 * i + 2] = t.z; qf[j][4 * i + 3] = t.w;
             }
-        if constexpr (F::kSmemTiles > 0) {
-            for (int k = wg; k < F::kSmemTiles * (PD / 32); k += GW) {
-                const uint4 t = q_frag(F::kRegTiles + k / (PD / 32), k % (PD / 32));
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(frag_at + 1024u * k), "r"(t.x), "r"(t.y), "r"(t.z), "r"(t.w) : "memory");
-            }
-            group_sync();
-        }
 
         // ---- pages -----------------------------------------------------------------------------------------
-        float o_acc[NT][PD / 16][4], m0[NT], m1[NT], l0[NT], l1[NT];
+        constexpr int kAccTiles = F::kPair ? PD / 32 : PD / 16;       // a warp of a pair keeps half of the dims
+        float o_acc[NT][kAccTiles][4], m0[NT], m1[NT], l0[NT], l1[NT];
 #pragma unroll
         for (int t = 0; t < NT; t++) {
 #pragma unroll
-            for (int i = 0; i < PD / 16; i++)
+            for (int i = 0; i < kAccTiles; i++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) o_acc[t][i][j] = 0.0f;
             m0[t] = m1[t] = kNoMax;
             l0[t] = l1[t] = 0.0f;
         }
+        // S = K^ Q^T of the page in stage `st`: rows g, g + 8 are tokens ta, tb, columns 8 t + 2 tg, + 1 query heads; and the V norms
+        auto scores = [&](uint32_t st, int left, float (&s_acc)[NT][4], float& vfa, float& vfb) {
+            uint32_t ka[F::kKBytes / 4], kb[F::kKBytes / 4];
+            split_lds<F::kKBytes>(k_at + st, ka);
+            split_lds<F::kKBytes>(k_at + st + 8 * F::kKPitch, kb);
+            float s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) s_acc[t][i] = 0.0f;
+#pragma unroll
+            for (int w = 0; w < F::kKBytes / 4; w++) {
+                uint32_t ra[4], rb[4];
+                dequant8(ka[w], lut_lane, ra);
+                dequant8(kb[w], lut_lane, rb);
+                if constexpr (NT == 1) {       // two chains
+                    mma16816(s_acc[0], ra[0], rb[0], ra[1], rb[1], qf[0][4 * w], qf[0][4 * w + 1]);
+                    mma16816(s_acc2, ra[2], rb[2], ra[3], rb[3], qf[0][4 * w + 2], qf[0][4 * w + 3]);
+                } else {
+                    uint32_t qs[NT][4];
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        if (t < F::kRegTiles) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) qs[t][i] = qf[t][4 * w + i];
+                        } else {
+                            const uint4 v = lds128(frag_at + 1024u * (t * (PD / 32) + w));
+                            qs[t][0] = v.x; qs[t][1] = v.y; qs[t][2] = v.z; qs[t][3] = v.w;
+                        }
+                    }
+#pragma unroll
+                    for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[0], rb[0], ra[1], rb[1], qs[t][0], qs[t][1]);
+#pragma unroll
+                    for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[2], rb[2], ra[3], rb[3], qs[t][2], qs[t][3]);
+                }
+            }
+            if constexpr (NT == 1) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) s_acc[0][i] += s_acc2[i];
+            }
+            // Only the last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
+            // slots contain) and their scores biased to -inf.
+            float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kKPitch) * p.k_scale;
+            vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kVPitch) * p.v_scale;
+            float bias_a = 0.0f, bias_b = 0.0f;
+            if (left < kPageTokens) {
+                if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
+                if (tb >= left) { kfb = 0.0f; vfb = 0.0f; bias_b = -INFINITY; }
+            }
+#pragma unroll
+            for (int t = 0; t < NT; t++) {
+                float (&x)[4] = s_acc[t];
+                x[0] = fmaf(x[0], kfa, bias_a);
+                x[1] = fmaf(x[1], kfa, bias_a);
+                x[2] = fmaf(x[2], kfb, bias_b);
+                x[3] = fmaf(x[3], kfb, bias_b);
+            }
+            if (p.causal && left < kPageTokens + p.nq - 1) {       // a page that some query sees in part, or not at all
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    const int s0 = left + 1 - p.nq + (8 * t + 2 * tg) / p.real_group, s1 = left + 1 - p.nq + (8 * t + 2 * tg + 1) / p.real_group;
+                    if (ta >= s0) s_acc[t][0] = -INFINITY;
+                    if (ta >= s1) s_acc[t][1] = -INFINITY;
+                    if (tb >= s0) s_acc[t][2] = -INFINITY;
+                    if (tb >= s1) s_acc[t][3] = -INFINITY;
+                }
+            }
+        };
+        // ---- online softmax (base 2) with a maximum that is raised only when a score exceeds it by kRaiseThreshold
+        auto exceeds = [&](const float (&s_acc)[NT][4]) {
+            bool over = false;
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+                over |= fmaxf(s_acc[t][0], s_acc[t][2]) > m0[t] + kRaiseThreshold || fmaxf(s_acc[t][1], s_acc[t][3]) > m1[t] + kRaiseThreshold;
+            return __any_sync(0xffffffffu, over) != 0;
+        };
+        auto page_max = [&](const float (&x)[4], float& mx0, float& mx1) {
+            mx0 = fmaxf(x[0], x[2]);
+            mx1 = fmaxf(x[1], x[3]);
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+            }
+        };
+        auto raise_to = [&](int t, float mx0, float mx1) {
+            const bool raise0 = mx0 > m0[t] + kRaiseThreshold, raise1 = mx1 > m1[t] + kRaiseThreshold;
+            const float c0 = raise0 ? fast_exp2(m0[t] - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1[t] - mx1) : 1.0f;
+            if (raise0) m0[t] = mx0;
+            if (raise1) m1[t] = mx1;
+            l0[t] *= c0;
+            l1[t] *= c1;
+#pragma unroll
+            for (int i = 0; i < kAccTiles; i++) {
+                o_acc[t][i][0] *= c0; o_acc[t][i][1] *= c1; o_acc[t][i][2] *= c0; o_acc[t][i][3] *= c1;
+            }
+        };
+        // P = exp2(x - m) times the V norm as B fragments, and its column sums over this lane's two tokens
+        auto probabilities = [&](const float (&s_acc)[NT][4], float vfa, float vfb, uint32_t (&pb0)[NT], uint32_t (&pb1)[NT], float (&a0)[NT], float (&a1)[NT]) {
+#pragma unroll
+            for (int t = 0; t < NT; t++) {
+                const float e0 = fast_exp2(s_acc[t][0] - m0[t]), e1 = fast_exp2(s_acc[t][1] - m1[t]);
+                const float e2 = fast_exp2(s_acc[t][2] - m0[t]), e3 = fast_exp2(s_acc[t][3] - m1[t]);
+                a0[t] = e0 + e2;
+                a1[t] = e1 + e3;
+                pb0[t] = movmatrix_trans(pack_half2(e0 * vfa, e1 * vfa));
+                pb1[t] = movmatrix_trans(pack_half2(e2 * vfb, e3 * vfb));
+            }
+        };
+        // ---- O^T += V^^T P: four code bytes of four tokens, V^ rows g <- odd dim, g + 8 <- even dim of code byte 4 w + j
+        auto accumulate = [&](int w, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const uint32_t (&pb0)[NT], const uint32_t (&pb1)[NT]) {
+            const uint32_t lo01 = (v0 & 0x0F0F0F0Fu) | ((v1 << 4) & 0xF0F0F0F0u);      // odd dims
+            const uint32_t hi01 = ((v0 >> 4) & 0x0F0F0F0Fu) | (v1 & 0xF0F0F0F0u);      // even dims
+            const uint32_t lo23 = (v2 & 0x0F0F0F0Fu) | ((v3 << 4) & 0xF0F0F0F0u);
+            const uint32_t hi23 = ((v2 >> 4) & 0x0F0F0F0Fu) | (v3 & 0xF0F0F0F0u);
+            uint32_t a_lo01[4], a_hi01[4], a_lo23[4], a_hi23[4];
+            dequant8(lo01, lut_lane, a_lo01);
+            dequant8(hi01, lut_lane, a_hi01);
+            dequant8(lo23, lut_lane, a_lo23);
+            dequant8(hi23, lut_lane, a_hi23);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int t = 0; t < NT; t++) mma16816(o_acc[t][4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0[t], pb1[t]);
+        };
         uint32_t st = 0, st_issue = (F::kStages - 1) * F::kStageBytes;      // stage offsets
         int left = len - (fp + p0 + wg) * kPageTokens;                       // tokens from this warp's page on
-        for (int it = 0; it < n; it++, left -= GW * kPageTokens) {
+        auto copy_ahead = [&](int it) {
             const int ahead_i = it + F::kStages - 1;
             if ((ahead_i & 31) == 0) {          // the ids of the next 32 pages, and the load of those after them
                 id_now = id_next;
                 id_next = ahead_i + 32 < n ? fetch_ids(ahead_i + 32) : 0;
             }
             issue(ahead_i, st_issue);
-            split_cp_async_wait<F::kStages - 1>();
-            __syncwarp();
-            {
-                // ---- S = K^ Q^T -----------------------------------------------------------------------------
-                uint32_t ka[F::kKBytes / 4], kb[F::kKBytes / 4];
-                split_lds<F::kKBytes>(k_at + st, ka);
-                split_lds<F::kKBytes>(k_at + st + 8 * F::kKPitch, kb);
+        };
+        auto next_stage = [&] {
+            st_issue = st;
+            st = st + F::kStageBytes == F::kRingBytes ? 0 : st + F::kStageBytes;
+        };
+        const int turns = F::kPair ? (p1 - p0 > (wg & ~1) ? (p1 - p0 - (wg & ~1) + GW - 1) / GW : 0) : n;
+        if constexpr (!F::kPair) {
+            for (int it = 0; it < n; it++, left -= GW * kPageTokens) {
+                copy_ahead(it);
+                split_cp_async_wait<F::kStages - 1>();
+                __syncwarp();
                 // the V codes too, ahead of the vote below
                 uint32_t v0[F::kVBytes / 4], v1[F::kVBytes / 4], v2[F::kVBytes / 4], v3[F::kVBytes / 4];
                 split_lds<F::kVBytes>(v_at + st, v0);
                 split_lds<F::kVBytes>(v_at + st + kVNext, v1);
                 split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch, v2);
                 split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch + kVNext, v3);
-                float s_acc[NT][4], s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int t = 0; t < NT; t++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) s_acc[t][i] = 0.0f;
-#pragma unroll
-                for (int w = 0; w < F::kKBytes / 4; w++) {
-                    uint32_t ra[4], rb[4];
-                    dequant8(ka[w], lut_lane, ra);
-                    dequant8(kb[w], lut_lane, rb);
-                    if constexpr (NT == 1) {       // two chains
-                        mma16816(s_acc[0], ra[0], rb[0], ra[1], rb[1], qf[0][4 * w], qf[0][4 * w + 1]);
-                        mma16816(s_acc2, ra[2], rb[2], ra[3], rb[3], qf[0][4 * w + 2], qf[0][4 * w + 3]);
-                    } else {
-                        uint32_t qs[NT][4];
-#pragma unroll
-                        for (int t = 0; t < NT; t++) {
-                            if (t < F::kRegTiles) {
-#pragma unroll
-                                for (int i = 0; i < 4; i++) qs[t][i] = qf[t][4 * w + i];
-                            } else {
-                                const uint4 v = lds128(frag_at + 1024u * ((t - F::kRegTiles) * (PD / 32) + w));
-                                qs[t][0] = v.x; qs[t][1] = v.y; qs[t][2] = v.z; qs[t][3] = v.w;
-                            }
-                        }
-#pragma unroll
-                        for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[0], rb[0], ra[1], rb[1], qs[t][0], qs[t][1]);
-#pragma unroll
-                        for (int t = 0; t < NT; t++) mma16816(s_acc[t], ra[2], rb[2], ra[3], rb[3], qs[t][2], qs[t][3]);
-                    }
-                }
-                if constexpr (NT == 1) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) s_acc[0][i] += s_acc2[i];
-                }
-                // ---- online softmax (base 2): rows g, g + 8 are tokens ta, tb; columns 2tg, 2tg + 1 query heads.  Only the
-                // last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
-                // slots contain) and their scores biased to -inf.  Row 0 of every page is inside.
-                float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kKPitch) * p.k_scale;
-                float vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kVPitch) * p.v_scale;
-                float bias_a = 0.0f, bias_b = 0.0f;
-                if (left < kPageTokens) {
-                    if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
-                    if (tb >= left) { kfb = 0.0f; vfb = 0.0f; bias_b = -INFINITY; }
-                }
-                bool raise = false;
-#pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    float (&x)[4] = s_acc[t];
-                    x[0] = fmaf(x[0], kfa, bias_a);
-                    x[1] = fmaf(x[1], kfa, bias_a);
-                    x[2] = fmaf(x[2], kfb, bias_b);
-                    x[3] = fmaf(x[3], kfb, bias_b);
-                }
-                if (p.causal && left < kPageTokens + p.nq - 1) {       // a page that some query sees in part, or not at all
-#pragma unroll
-                    for (int t = 0; t < NT; t++) {
-                        const int s0 = left + 1 - p.nq + (8 * t + 2 * tg) / p.real_group, s1 = left + 1 - p.nq + (8 * t + 2 * tg + 1) / p.real_group;
-                        if (ta >= s0) s_acc[t][0] = -INFINITY;
-                        if (ta >= s1) s_acc[t][1] = -INFINITY;
-                        if (tb >= s0) s_acc[t][2] = -INFINITY;
-                        if (tb >= s1) s_acc[t][3] = -INFINITY;
-                    }
-                }
-#pragma unroll
-                for (int t = 0; t < NT; t++)
-                    raise |= fmaxf(s_acc[t][0], s_acc[t][2]) > m0[t] + kRaiseThreshold || fmaxf(s_acc[t][1], s_acc[t][3]) > m1[t] + kRaiseThreshold;
-                if (__any_sync(0xffffffffu, raise)) {
-#pragma unroll
-                    for (int t = 0; t < NT; t++) {
-                        float mx0 = fmaxf(s_acc[t][0], s_acc[t][2]), mx1 = fmaxf(s_acc[t][1], s_acc[t][3]);
-#pragma unroll
-                        for (int o = 4; o < 32; o <<= 1) {
-                            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-                            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-                        }
-                        const bool raise0 = mx0 > m0[t] + kRaiseThreshold, raise1 = mx1 > m1[t] + kRaiseThreshold;
-                        const float c0 = raise0 ? fast_exp2(m0[t] - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1[t] - mx1) : 1.0f;
-                        if (raise0) m0[t] = mx0;
-                        if (raise1) m1[t] = mx1;
-                        l0[t] *= c0;
-                        l1[t] *= c1;
-#pragma unroll
-                        for (int i = 0; i < PD / 16; i++) {
-                            o_acc[t][i][0] *= c0; o_acc[t][i][1] *= c1; o_acc[t][i][2] *= c0; o_acc[t][i][3] *= c1;
-                        }
-                    }
-                }
+                float s_acc[NT][4], vfa, vfb, a0[NT], a1[NT];
                 uint32_t pb0[NT], pb1[NT];
+                scores(st, left, s_acc, vfa, vfb);
+                if (exceeds(s_acc)) {
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        float mx0, mx1;
+                        page_max(s_acc[t], mx0, mx1);
+                        raise_to(t, mx0, mx1);
+                    }
+                }
+                probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
-                    const float e0 = fast_exp2(s_acc[t][0] - m0[t]), e1 = fast_exp2(s_acc[t][1] - m1[t]);
-                    const float e2 = fast_exp2(s_acc[t][2] - m0[t]), e3 = fast_exp2(s_acc[t][3] - m1[t]);
-                    l0[t] += e0 + e2;
-                    l1[t] += e1 + e3;
-                    pb0[t] = movmatrix_trans(pack_half2(e0 * vfa, e1 * vfa));
-                    pb1[t] = movmatrix_trans(pack_half2(e2 * vfb, e3 * vfb));
+                    l0[t] += a0[t];
+                    l1[t] += a1[t];
                 }
-                // ---- O^T += V^^T P ----------------------------------------------------------------------------
 #pragma unroll
-                for (int w = 0; w < F::kVBytes / 4; w++) {
-                    const uint32_t lo01 = (v0[w] & 0x0F0F0F0Fu) | ((v1[w] << 4) & 0xF0F0F0F0u);      // odd dims
-                    const uint32_t hi01 = ((v0[w] >> 4) & 0x0F0F0F0Fu) | (v1[w] & 0xF0F0F0F0u);      // even dims
-                    const uint32_t lo23 = (v2[w] & 0x0F0F0F0Fu) | ((v3[w] << 4) & 0xF0F0F0F0u);
-                    const uint32_t hi23 = ((v2[w] >> 4) & 0x0F0F0F0Fu) | (v3[w] & 0xF0F0F0F0u);
-                    uint32_t a_lo01[4], a_hi01[4], a_lo23[4], a_hi23[4];
-                    dequant8(lo01, lut_lane, a_lo01);
-                    dequant8(hi01, lut_lane, a_hi01);
-                    dequant8(lo23, lut_lane, a_lo23);
-                    dequant8(hi23, lut_lane, a_hi23);
-#pragma unroll
-                    for (int j = 0; j < 4; j++)     // rows: g <- odd dim, g + 8 <- even dim of code byte 4 w + j
-#pragma unroll
-                        for (int t = 0; t < NT; t++) mma16816(o_acc[t][4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0[t], pb1[t]);
-                }
+                for (int w = 0; w < F::kVBytes / 4; w++) accumulate(w, v0[w], v1[w], v2[w], v3[w], pb0, pb1);
+                __syncwarp();      // every lane has read the stage before a later iteration copies into it
+                next_stage();
             }
-            __syncwarp();      // every lane has read the stage before a later iteration copies into it
-            st_issue = st;
-            st = st + F::kStageBytes == F::kRingBytes ? 0 : st + F::kStageBytes;
+        } else {
+            // A pair's turn is two pages, one a warp: scores and probabilities of its own, then half of the dims of both.  One
+            // barrier a turn, at which the probabilities are in shared memory and both pages' copies have landed; it also tells
+            // that the pair is through with the turn before, whose stage and whose hand-over buffer are written next.
+            const uint32_t hand = smem_u32(smem) + (kLutAddr + kLutSpan - smem_base) + F::kHandAt + 16u * lane;
+            const uint32_t mine = split_keep(hand + warp * 2 * F::kHandBytes), other = split_keep(hand + (warp ^ 1) * 2 * F::kHandBytes);
+            const int ow = warp ^ 1;
+            const uint32_t other_ring = smem_base + (ow < F::kRingsBelow ? (uint32_t)ow * F::kRingBytes
+                                                                         : kLutAddr + kLutSpan - smem_base + (uint32_t)(ow - F::kRingsBelow) * F::kRingBytes);
+            const uint32_t v_off = 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + 32 * (wg & 1) + 4 * g;
+            const uint32_t v_own = split_keep(ring_at + v_off), v_other = split_keep(other_ring + v_off);
+            auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + NG + (warp >> 1)) : "memory"); };
+            auto put = [&](uint32_t at, const uint32_t (&pb0)[NT], const uint32_t (&pb1)[NT]) {
+#pragma unroll
+                for (int t = 0; t < NT; t += 2)
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + 256u * t), "r"(pb0[t]), "r"(pb1[t]), "r"(t + 1 < NT ? pb0[(t + 1) % NT] : 0u),
+                                 "r"(t + 1 < NT ? pb1[(t + 1) % NT] : 0u) : "memory");
+            };
+            for (int it = 0; it < turns; it++, left -= GW * kPageTokens) {
+                split_cp_async_wait<F::kStages - 2>();
+                __syncwarp();
+                float s_acc[NT][4], vfa, vfb, a0[NT], a1[NT];
+                uint32_t pb0[NT], pb1[NT];
+                scores(st, it < n ? left : 0, s_acc, vfa, vfb);      // past its last page a warp has no tokens: P = 0
+                const uint32_t turn = (uint32_t)(it & 1) * F::kHandBytes;
+                const bool over = exceeds(s_acc);
+                probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
+                put(mine + turn, pb0, pb1);
+                if (lane == 0) raise_s[it & 1][warp] = over;
+                pair_sync();
+                if (over || raise_s[it & 1][ow]) {      // rare: both warps raise to the maximum of both pages, and the probabilities again
+                    float mx0[NT], mx1[NT];
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        page_max(s_acc[t], mx0[t], mx1[t]);
+                        if (g == 0) {
+                            max_s[warp][8 * t + 2 * tg] = mx0[t];
+                            max_s[warp][8 * t + 2 * tg + 1] = mx1[t];
+                        }
+                    }
+                    pair_sync();
+#pragma unroll
+                    for (int t = 0; t < NT; t++) raise_to(t, fmaxf(mx0[t], max_s[ow][8 * t + 2 * tg]), fmaxf(mx1[t], max_s[ow][8 * t + 2 * tg + 1]));
+                    probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
+                    put(mine + turn, pb0, pb1);
+                    pair_sync();
+                }
+                copy_ahead(it);
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    l0[t] += a0[t];
+                    l1[t] += a1[t];
+                }
+                accumulate(0, lds32(v_own + st), lds32(v_own + st + kVNext), lds32(v_own + st + 8 * F::kVPitch), lds32(v_own + st + 8 * F::kVPitch + kVNext), pb0, pb1);
+#pragma unroll
+                for (int t = 0; t < NT; t += 2) {
+                    const uint4 v = lds128(other + turn + 256u * t);
+                    pb0[t] = v.x;
+                    pb1[t] = v.y;
+                    if (t + 1 < NT) {
+                        pb0[(t + 1) % NT] = v.z;
+                        pb1[(t + 1) % NT] = v.w;
+                    }
+                }
+                accumulate(0, lds32(v_other + st), lds32(v_other + st + kVNext), lds32(v_other + st + 8 * F::kVPitch), lds32(v_other + st + 8 * F::kVPitch + kVNext), pb0, pb1);
+                next_stage();
+            }
         }
         split_cp_async_wait<0>();
+        if constexpr (F::kPair) group_sync();      // the other warp has read this one's last stage
 
         // ---- combine the group's warps ------------------------------------------------------------------------
 #pragma unroll
@@ -718,20 +822,23 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 l_s[gg][wg][8 * t + 2 * tg + 1] = l1[t];
             }
         }
-        // The warp's accumulators as rows of PD floats in its own ring (the copies have landed and been read).  The 16-byte pieces of
-        // a row are swapped by the column, which keeps the four columns a quarter warp stores at a time in different banks.
+        // The warp's accumulators as rows of PD floats (a pair: half rows, half of the dims each) in its own ring (the copies have landed and
+        // been read).  The 16-byte pieces of a row are swapped by the column, which keeps the columns a quarter warp stores at a time in
+        // different banks.
         __syncwarp();
         float* const mine = reinterpret_cast<float*>(ring);
-        if (n > 0) {
+        constexpr int kRowFloats = F::kPair ? PD / 2 : PD;
+        auto swap_of = [](int c) -> int { return F::kPair ? (c & 1) | ((c & 2) << 1) : c; };     // of column pair c
+        if (turns > 0) {
 #pragma unroll
-            for (int w = 0; w < F::kVBytes / 2; w++) {      // bytes 2 w, 2 w + 1 of this lane: dims d ... d + 3
-                const int piece = (g * F::kVBytes + 2 * w) / 2;
+            for (int w = 0; w < kAccTiles / 2; w++) {      // bytes 2 w, 2 w + 1 of this lane: dims d ... d + 3
+                const int piece = (g * kAccTiles + 2 * w) / 2;
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
                     const int c = 8 * t + 2 * tg;
                     const float(&a)[4] = o_acc[t][2 * w], (&b4)[4] = o_acc[t][2 * w + 1];
-                    if (c < G) *reinterpret_cast<float4*>(mine + c * PD + 4 * (piece ^ tg)) = make_float4(a[2], a[0], b4[2], b4[0]);
-                    if (c + 1 < G) *reinterpret_cast<float4*>(mine + (c + 1) * PD + 4 * (piece ^ tg)) = make_float4(a[3], a[1], b4[3], b4[1]);
+                    if (c < G) *reinterpret_cast<float4*>(mine + c * kRowFloats + 4 * (piece ^ swap_of(tg))) = make_float4(a[2], a[0], b4[2], b4[0]);
+                    if (c + 1 < G) *reinterpret_cast<float4*>(mine + (c + 1) * kRowFloats + 4 * (piece ^ swap_of(tg))) = make_float4(a[3], a[1], b4[3], b4[1]);
                 }
             }
         }
@@ -745,23 +852,25 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             float o[E], ll = 0.0f;
 #pragma unroll
             for (int i = 0; i < E; i++) o[i] = 0.0f;
+            constexpr int kStep = F::kPair ? 2 : 1;
 #pragma unroll
-            for (int w = 0; w < GW; w++) {
+            for (int w = 0; w < GW; w += kStep) {
                 const float mw = m_s[gg][w][r];
                 if (mw > kNoMax) {            // a warp without a page has stored nothing
                     const float c = fast_exp2(mw - mm);
-                    ll += c * l_s[gg][w][r];
-                    const int other = gg * GW + w;
+                    ll += c * (F::kPair ? l_s[gg][w][r] + l_s[gg][w + kStep - 1][r] : l_s[gg][w][r]);
+                    const int other = gg * GW + w + (F::kPair ? lane >> 4 : 0);      // a pair: dims 64 ... are the second warp's
                     const float* row = reinterpret_cast<const float*>(
                                            smem + (other < F::kRingsBelow ? (uint32_t)other * F::kRingBytes
-                                                                         : kLutAddr + kLutSpan - smem_base + (uint32_t)(other - F::kRingsBelow) * F::kRingBytes)) + r * PD;
+                                                                         : kLutAddr + kLutSpan - smem_base + (uint32_t)(other - F::kRingsBelow) * F::kRingBytes)) + r * kRowFloats;
+                    const int at = F::kPair ? lane & 15 : lane, swap = swap_of((r & 7) >> 1);
                     if constexpr (E == 2) {
-                        const float2 t = *reinterpret_cast<const float2*>(row + 4 * ((lane >> 1) ^ ((r & 7) >> 1)) + 2 * (lane & 1));
+                        const float2 t = *reinterpret_cast<const float2*>(row + 4 * ((at >> 1) ^ swap) + 2 * (at & 1));
                         o[0] += c * t.x; o[1] += c * t.y;
                     } else {
 #pragma unroll
                         for (int i = 0; i < E / 4; i++) {
-                            const float4 t = *reinterpret_cast<const float4*>(row + 4 * ((lane * (E / 4) + i) ^ ((r & 7) >> 1)));
+                            const float4 t = *reinterpret_cast<const float4*>(row + 4 * ((at * (E / 4) + i) ^ swap));
                             o[4 * i] += c * t.x; o[4 * i + 1] += c * t.y; o[4 * i + 2] += c * t.z; o[4 * i + 3] += c * t.w;
                         }
                     }
