@@ -824,17 +824,28 @@ typedef CUresult (*MqEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, vo
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static MqEncodeFn mq_encode_fn() {
-    static MqEncodeFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
+    static const MqEncodeFn fn = [] {
         void* sym = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<MqEncodeFn>(sym);
-        tried = true;
-    }
+        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<MqEncodeFn>(sym) : nullptr;
+    }();
     return fn;
+}
+
+// The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab.
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes) {
+    MqEncodeFn enc = mq_encode_fn();
+    TQ_REQUIRE(enc != nullptr, TQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)num_blocks * kPageTokens, 2};
+    const cuuint64_t strides[2] = {dims[0], dims[0] * dims[1]};
+    const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, 1u};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(kv_cache), dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    TQ_REQUIRE(rc == CUDA_SUCCESS, TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the cache (%d)", (int)rc);
+    return TQ_OK;
 }
 
 // Is the wide-tile kernel applicable?  Dense cache rows of 2, 4, 8 or 16 KV heads, padded head size 128.
@@ -848,17 +859,8 @@ int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks
     mp.head_pairs = num_kv_heads / 2;
     mp.ncols = d.group;
     mp.causal = causal;
-    MqEncodeFn enc = mq_encode_fn();
-    TQ_REQUIRE(enc != nullptr, TQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t row_bytes = (cuuint64_t)num_kv_heads * kSlotBytes;
-    const cuuint64_t dims[3] = {row_bytes, (cuuint64_t)num_blocks * kPageTokens, 2};
-    const cuuint64_t strides[2] = {row_bytes, (cuuint64_t)d.slab_bytes};
-    const cuuint32_t box[3] = {160u, (cuuint32_t)kPageTokens, 1u};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult rc = enc(&mp.cache_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(d.kv_cache), dims, strides, box,
-                            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    TQ_REQUIRE(rc == CUDA_SUCCESS, TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the cache (%d)", (int)rc);
+    const int rc = encode_cache_map(&mp.cache_map, d.kv_cache, num_blocks, (int64_t)num_kv_heads * kSlotBytes, 160);
+    if (rc != TQ_OK) return rc;
     const int smem = (int)kMqSmemEnd;
     static bool configured[64] = {};
     int dev = 0;

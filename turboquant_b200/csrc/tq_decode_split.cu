@@ -19,6 +19,8 @@
 #include <cmath>
 #include <cstring>
 
+#include <cuda.h>  // CUtensorMap and its enums only: the encoder is looked up at run time
+
 #include "tq_decode_common.cuh"
 
 namespace tq {
@@ -33,18 +35,17 @@ struct SplitShape {
     static constexpr int kE = PD / 32;                       // elements per lane of a row
     static constexpr int kKBytes = PD / 8, kVBytes = PD / 16;  // code bytes per lane and token, K and V
     static constexpr int kRow = ((PD / 2 + 2 * (PD / 64)) + 15) & ~15;   // staged bytes of a slot: 48 / 80 / 144
-    // Pitches of the staged rows and the token of an MMA row, chosen so that the K loads (16 bytes a lane: two
-    // rows at a time; 8 bytes at head 64) and the V loads (four rows, 32 bytes each) meet no bank twice.  128: rows 2i, 2i + 1 are
-    // tokens i, i + 4 (80-byte K rows 64 bytes apart mod 128; 96-byte V rows of tokens 0 ... 3 in four quarters).
-    // 256: 144-byte rows do it as they are.  64: the V loads do, two K loads take three wavefronts for two.
-    static constexpr int kKPitch = kRow, kVPitch = PD == 128 ? 96 : kRow;
-    static constexpr int kStageBytes = 16 * (kKPitch + kVPitch);
+    // A stage is a page's K box, then its V box: 16 dense rows each.  V loads (four rows, 32 bytes each) meet no bank twice at
+    // any of the three pitches; the K loads (16 bytes a lane, two rows at a time) of 80-byte rows take two wavefronts a quarter for
+    // one (8 a page of about 130), those of 144-byte rows one.
+    static constexpr int kHalfBytes = 16 * kRow, kStageBytes = 2 * kHalfBytes;
+    static_assert(kHalfBytes % 128 == 0, "boxes start on 128 bytes");
     // Wide tiles (128-wide heads): 32 accumulators a thread and tile.  Two tiles: 12 warps of 168 registers.  Three or four tiles would
     // leave 8 warps of 255, so two warps go as a pair: each works out the probabilities of its own page and accumulates half of the
     // dims of both (12 warps again).  Batch 8 x 32768 causal, 32 query / 8 KV heads: 8 queries a row 194 -> 181 us, 6: 171 -> 159 us,
     // 32 ragged sequences x 4096, 8 queries: 87 -> 71 us; as a pair two tiles are slower (124 -> 140 us).
     static constexpr bool kPair = NT >= 3;
-    static constexpr int kStages = NT == 2 && !kPair ? 4 : PD == 256 ? 2 : 3;
+    static constexpr int kStages = NT > 1 ? 4 : PD == 256 ? 2 : 3;
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
@@ -53,22 +54,19 @@ struct SplitShape {
     // page's 64 lookups; in registers they spill: 8 queries 181 -> 185 us with one tile, 234 with two)
     static constexpr int kRegTiles = NT == 4 ? 0 : NT == 3 ? 2 : NT;
     static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
-    static constexpr int kRingsBelow = kPair ? (NT == 2 ? 7 : 6) : NT == 2 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
+    static constexpr int kRingsBelow = NT > 1 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
     // What the warps of a pair hand each other: the probabilities of a page as fragments, two pages' worth in turn.
     static constexpr int kHandBytes = kPair ? (NT + 1) / 2 * 512 : 0, kHandAt = (kWarps - kRingsBelow) * kRingBytes;
-    static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)kHandAt + 2 * kWarps * kHandBytes;   // from offset 0: ample
+    static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)kHandAt + 2 * kWarps * kHandBytes - 1024;   // from offset 1024 (the system's part): ample
     static_assert(kRingBytes >= kCols * PD * (kPair ? 2 : 4), "a warp's partial output goes through its ring");
     // in the unused upper halves of the table's rows: rotated queries, the warps' plans
     static constexpr uint32_t kPlanAt = kGroups * kCols * PD * 2;
     static_assert(kPlanAt + kWarps * 512 <= kLutSpan / 2, "the upper halves hold 32 KB");
     static_assert(NT == 1 || PD == 128, "wide tiles are for 128-wide heads");
-    // A page's copies, 16 bytes a lane: rounds of kRoundTokens tokens' code bytes (kPieces lanes a token) for K, the same for V, and one
-    // round for the 16 + 16 pieces with the norms.  Rounds lie a fixed distance apart, so a lane keeps two source pointers.
-    static constexpr int kPieces = PD / 32, kRoundTokens = 32 / kPieces, kRounds = 16 / kRoundTokens;
-    static __device__ __forceinline__ int token(int r) { return PD == 128 ? (r & 8) + ((r & 1) << 2) + ((r & 7) >> 1) : r; }
 };
 
 struct SplitParams {
+    alignas(64) CUtensorMap cache_map;   // uint8 [2][num_blocks * 16][H * slot], boxes of [1][16][kRow]
     const void* q;
     const uint8_t* kv_cache;
     const int32_t* page_indices;
@@ -80,7 +78,7 @@ struct SplitParams {
     float* partial_o;       // [2 x groups of the grid][group columns][PD], normalized, rotated domain
     void* out;
     float* out_lse;
-    int64_t slab_bytes, num_blocks, kv_begin, kv_end, tok_stride;
+    int64_t num_blocks, kv_begin, kv_end;
     int batch, kv_heads, group, max_pages, q_dtype, out_dtype, emit_rotated;
     int nq, real_heads, real_group, head_dim, slot_bytes;
     int causal;             // query i of nq sees the first len - (nq - 1 - i) tokens
@@ -213,8 +211,19 @@ __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, i
     split_load(p, s, 0, 0, true);
 }
 
-__device__ __forceinline__ void split_cp_async16_if(bool on, uint32_t dst, const void* src) {   // predicated: no branch in the loop
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(dst), "l"(src), "r"((uint32_t)on) : "memory");
+// One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V).  No multicast; x is a
+// multiple of the slot, hence of 16.
+__device__ __forceinline__ void split_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void split_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool split_try_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
 // A value the compiler cannot work out again: a lane's constants stay in registers through the page loop instead of being recomputed
 // from the thread index in every iteration.
@@ -222,10 +231,6 @@ __device__ __forceinline__ uint32_t split_keep(uint32_t v) {
     asm volatile("" : "+r"(v));
     return v;
 }
-__device__ __forceinline__ void split_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void split_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // BYTES (4, 8, 16 or 32) of a staged code row into words
 template <int BYTES>
 __device__ __forceinline__ void split_lds(uint32_t addr, uint32_t (&w)[BYTES / 4]) {
@@ -356,6 +361,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     __shared__ float sign_s[PD];
     __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols];      // a pair's maxima of a page that raises them, and whether it does
     __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
+    __shared__ uint64_t full_s[F::kWarps][F::kStages];               // a stage's two boxes have landed
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -390,6 +396,9 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     }
     // the signs are a constant of the context (as in the cache write): read ahead of the wait
     for (int i = tid; i < PD; i += F::kThreads) sign_s[i] = p.signs[i];
+    if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.cache_map) : "memory");
+    if (lane < F::kStages) mbar_init(&full_s[warp][lane], 1);
+    fence_barrier_init();
     // The small inputs into L2 while the kernel before this one drains: a whole KV stream may have passed since they were last
     // touched, and a prefetch hands no value over.
     if (blockIdx.x == 0 && tid * 32 < p.batch) prefetch_l2(p.seq_lens + tid * 32);
@@ -424,18 +433,16 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     int base = 0;
     const uint32_t lut_lane = split_keep(smem_u32(lut) + 4u * lane);
     const int fp = (int)(p.kv_begin / kPageTokens);
-    // this lane's places in a stage: code pieces, norm pieces; fragment rows
-    const int c_tok = lane / F::kPieces, c_piece = lane % F::kPieces;
-    const uint32_t dst_k = split_keep(ring_at + c_tok * F::kKPitch + 16 * c_piece);
-    const uint32_t dst_v = F::kKPitch == F::kVPitch ? dst_k + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + c_tok * F::kVPitch + 16 * c_piece);
-    const uint32_t dst_n = split_keep(ring_at + (lane < 16 ? lane * F::kKPitch : 16 * F::kKPitch + (lane - 16) * F::kVPitch) + PD / 2);
-    const int ta = F::token(g), tb = ta + 8;
-    const uint32_t k_at = split_keep(ring_at + ta * F::kKPitch + tg * F::kKBytes), kn_at = split_keep(ring_at + ta * F::kKPitch + PD / 2);
-    const uint32_t v_at = split_keep(ring_at + 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + g * F::kVBytes);
-    const uint32_t vn_at = F::kKPitch == F::kVPitch ? kn_at + 16 * F::kKPitch : split_keep(ring_at + 16 * F::kKPitch + ta * F::kVPitch + PD / 2);
+    // this lane's places in a stage: fragment rows g, g + 8 of K are tokens ta, tb
+    const int ta = g, tb = g + 8;
+    const uint32_t k_at = split_keep(ring_at + g * F::kRow + tg * F::kKBytes), kn_at = split_keep(ring_at + g * F::kRow + PD / 2);
+    const uint32_t v_at = split_keep(ring_at + F::kHalfBytes + 2 * tg * F::kRow + g * F::kVBytes), vn_at = kn_at + F::kHalfBytes;
+    const uint32_t full_at = split_keep(smem_u32(&full_s[warp][0]));
     const uint32_t frag_at = split_keep(smem_u32(lut) + ((uint32_t)gg * F::kCols * PD * 4) + 128u + ((uint32_t)(lane >> 3) << 8) + 16u * (lane & 7));
-    constexpr int kVNext = (PD == 128 ? 4 : 1) * F::kVPitch;      // from token(2 tg) to token(2 tg + 1)
-    const uint32_t page_bytes = (uint32_t)(kPageTokens * p.tok_stride), round_bytes = (uint32_t)(F::kRoundTokens * p.tok_stride);
+    constexpr int kVNext = F::kRow;      // from token 2 tg to token 2 tg + 1
+    // The ring goes on from segment to segment: a stage's barrier completes once per page, in turn.
+    uint32_t stage = 0, parity = 0;
+    bool lost = false;                    // a wait ran out: nothing is copied or waited for from then on
     bool bad_page = false;
 
     while (pos < hi) {
@@ -508,23 +515,21 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
 #pragma unroll
                 for (int e = 0; e < E; e++) qv[i][e] = 0.0f;
             }
-        const uint8_t* const src_k = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)(c_tok * p.tok_stride) + 16 * c_piece;
-        const uint8_t* const src_n = p.kv_cache + (size_t)head * p.slot_bytes + (uint32_t)((lane & 15) * p.tok_stride) + PD / 2 + (lane < 16 ? 0 : p.slab_bytes);
-        auto issue = [&](int i, uint32_t stage_off) {
-            const uint32_t id = (uint32_t)__shfl_sync(0xffffffffu, id_now, i & 31);
-            const bool on = i < n;
-            const uint8_t* const k = src_k + (uint64_t)id * page_bytes;
-            const uint8_t* const v = k + p.slab_bytes;
-#pragma unroll
-            for (int r = 0; r < F::kRounds; r++) {
-                split_cp_async16_if(on, dst_k + stage_off + r * F::kRoundTokens * F::kKPitch, k + r * round_bytes);
-                split_cp_async16_if(on, dst_v + stage_off + r * F::kRoundTokens * F::kVPitch, v + r * round_bytes);
+        const int turns = F::kPair ? (p1 - p0 > (wg & ~1) ? (p1 - p0 - (wg & ~1) + GW - 1) / GW : 0) : n;      // the pair's
+        const int x = head * p.slot_bytes;
+        auto issue = [&](int i, uint32_t to) {       // page i of this warp into stage `to`
+            const int id = __shfl_sync(0xffffffffu, id_now, i & 31);
+            if (lane == 0 && i < turns && !lost) {
+                const uint32_t bar = full_at + 8 * to, dst = ring_at + to * F::kStageBytes;
+                split_expect(bar, i < n ? F::kStageBytes : 0);      // no page: the warps of a pair stay at the same stage
+                if (i < n) {
+                    split_box(dst, &p.cache_map, x, id * kPageTokens, 0, bar);
+                    split_box(dst + F::kHalfBytes, &p.cache_map, x, id * kPageTokens, 1, bar);
+                }
             }
-            split_cp_async16_if(on, dst_n + stage_off, src_n + (uint64_t)id * page_bytes);
-            split_cp_async_commit();
         };
 #pragma unroll
-        for (int i = 0; i < F::kStages - 1; i++) issue(i, i * F::kStageBytes);
+        for (int i = 0; i < F::kStages - 1; i++) issue(i, stage + i < F::kStages ? stage + i : stage + i - F::kStages);
         auto put_q = [&](int r, float (&v)[E]) {
 #pragma unroll
             for (int i = 0; i < E; i++) v[i] *= sign[i];
@@ -567,7 +572,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
         auto scores = [&](uint32_t st, int left, float (&s_acc)[NT][4], float& vfa, float& vfb) {
             uint32_t ka[F::kKBytes / 4], kb[F::kKBytes / 4];
             split_lds<F::kKBytes>(k_at + st, ka);
-            split_lds<F::kKBytes>(k_at + st + 8 * F::kKPitch, kb);
+            split_lds<F::kKBytes>(k_at + st + 8 * F::kRow, kb);
             float s_acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int t = 0; t < NT; t++)
@@ -605,8 +610,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             }
             // Only the last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
             // slots contain) and their scores biased to -inf.
-            float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kKPitch) * p.k_scale;
-            vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kVPitch) * p.v_scale;
+            float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kRow) * p.k_scale;
+            vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kRow) * p.v_scale;
             float bias_a = 0.0f, bias_b = 0.0f;
             if (left < kPageTokens) {
                 if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
@@ -688,7 +693,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
 #pragma unroll
                 for (int t = 0; t < NT; t++) mma16816(o_acc[t][4 * w + j], a_lo01[j], a_hi01[j], a_lo23[j], a_hi23[j], pb0[t], pb1[t]);
         };
-        uint32_t st = 0, st_issue = (F::kStages - 1) * F::kStageBytes;      // stage offsets
+        uint32_t st = stage * F::kStageBytes;                                // offset of the stage in turn
         int left = len - (fp + p0 + wg) * kPageTokens;                       // tokens from this warp's page on
         auto copy_ahead = [&](int it) {
             const int ahead_i = it + F::kStages - 1;
@@ -696,24 +701,41 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 id_now = id_next;
                 id_next = ahead_i + 32 < n ? fetch_ids(ahead_i + 32) : 0;
             }
-            issue(ahead_i, st_issue);
+            issue(ahead_i, stage == 0 ? F::kStages - 1 : stage - 1);
+        };
+        auto wait_page = [&] {
+            if (!lost) {
+                bool there = false;
+                for (uint32_t i = 0; i < kSpinLimit && !there; i++) there = split_try_wait(full_at + 8 * stage, parity);
+                if (!__all_sync(0xffffffffu, there)) {
+                    lost = true;      // the output is void; what is still in flight gets its time to land
+                    if (lane == 0) atomicExch(&p.header[0], 1);
+                    for (uint32_t k = 1; k < F::kStages; k++) {
+                        const bool wraps = stage + k >= F::kStages;
+                        for (uint32_t i = 0; i < kSpinLimit / 64; i++)
+                            if (split_try_wait(full_at + 8 * (wraps ? stage + k - F::kStages : stage + k), wraps ? parity ^ 1 : parity)) break;
+                    }
+                }
+            }
+            __syncwarp();
         };
         auto next_stage = [&] {
-            st_issue = st;
-            st = st + F::kStageBytes == F::kRingBytes ? 0 : st + F::kStageBytes;
+            if (++stage == F::kStages) {
+                stage = 0;
+                parity ^= 1;
+            }
+            st = stage * F::kStageBytes;
         };
-        const int turns = F::kPair ? (p1 - p0 > (wg & ~1) ? (p1 - p0 - (wg & ~1) + GW - 1) / GW : 0) : n;
         if constexpr (!F::kPair) {
             for (int it = 0; it < n; it++, left -= GW * kPageTokens) {
                 copy_ahead(it);
-                split_cp_async_wait<F::kStages - 1>();
-                __syncwarp();
+                wait_page();
                 // the V codes too, ahead of the vote below
                 uint32_t v0[F::kVBytes / 4], v1[F::kVBytes / 4], v2[F::kVBytes / 4], v3[F::kVBytes / 4];
                 split_lds<F::kVBytes>(v_at + st, v0);
                 split_lds<F::kVBytes>(v_at + st + kVNext, v1);
-                split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch, v2);
-                split_lds<F::kVBytes>(v_at + st + 8 * F::kVPitch + kVNext, v3);
+                split_lds<F::kVBytes>(v_at + st + 8 * F::kRow, v2);
+                split_lds<F::kVBytes>(v_at + st + 8 * F::kRow + kVNext, v3);
                 float s_acc[NT][4], vfa, vfb, a0[NT], a1[NT];
                 uint32_t pb0[NT], pb1[NT];
                 scores(st, left, s_acc, vfa, vfb);
@@ -745,7 +767,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             const int ow = warp ^ 1;
             const uint32_t other_ring = smem_base + (ow < F::kRingsBelow ? (uint32_t)ow * F::kRingBytes
                                                                          : kLutAddr + kLutSpan - smem_base + (uint32_t)(ow - F::kRingsBelow) * F::kRingBytes);
-            const uint32_t v_off = 16 * F::kKPitch + F::token(2 * tg) * F::kVPitch + 32 * (wg & 1) + 4 * g;
+            const uint32_t v_off = F::kHalfBytes + 2 * tg * F::kRow + 32 * (wg & 1) + 4 * g;
             const uint32_t v_own = split_keep(ring_at + v_off), v_other = split_keep(other_ring + v_off);
             auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + NG + (warp >> 1)) : "memory"); };
             auto put = [&](uint32_t at, const uint32_t (&pb0)[NT], const uint32_t (&pb1)[NT]) {
@@ -755,8 +777,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                                  "r"(t + 1 < NT ? pb1[(t + 1) % NT] : 0u) : "memory");
             };
             for (int it = 0; it < turns; it++, left -= GW * kPageTokens) {
-                split_cp_async_wait<F::kStages - 2>();
-                __syncwarp();
+                wait_page();
                 float s_acc[NT][4], vfa, vfb, a0[NT], a1[NT];
                 uint32_t pb0[NT], pb1[NT];
                 scores(st, it < n ? left : 0, s_acc, vfa, vfb);      // past its last page a warp has no tokens: P = 0
@@ -789,7 +810,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                     l0[t] += a0[t];
                     l1[t] += a1[t];
                 }
-                accumulate(0, lds32(v_own + st), lds32(v_own + st + kVNext), lds32(v_own + st + 8 * F::kVPitch), lds32(v_own + st + 8 * F::kVPitch + kVNext), pb0, pb1);
+                accumulate(0, lds32(v_own + st), lds32(v_own + st + kVNext), lds32(v_own + st + 8 * F::kRow), lds32(v_own + st + 8 * F::kRow + kVNext), pb0, pb1);
 #pragma unroll
                 for (int t = 0; t < NT; t += 2) {
                     const uint4 v = lds128(other + turn + 256u * t);
@@ -800,11 +821,10 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                         pb1[(t + 1) % NT] = v.w;
                     }
                 }
-                accumulate(0, lds32(v_other + st), lds32(v_other + st + kVNext), lds32(v_other + st + 8 * F::kVPitch), lds32(v_other + st + 8 * F::kVPitch + kVNext), pb0, pb1);
+                accumulate(0, lds32(v_other + st), lds32(v_other + st + kVNext), lds32(v_other + st + 8 * F::kRow), lds32(v_other + st + 8 * F::kRow + kVNext), pb0, pb1);
                 next_stage();
             }
         }
-        split_cp_async_wait<0>();
         if constexpr (F::kPair) group_sync();      // the other warp has read this one's last stage
 
         // ---- combine the group's warps ------------------------------------------------------------------------
@@ -894,7 +914,10 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 if (lane == 0) p.partial_lse[at] = lse2;
             }
         }
-        if (pos < hi) group_sync();    // rings and query rows are free again
+        if (pos < hi) {
+            fence_proxy_async();       // the ring was written and read as rows
+            group_sync();              // rings and query rows are free again
+        }
     }
     if (bad_page) atomicExch(&p.header[0], kStatusBadPage);
 }
@@ -1020,6 +1043,11 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
 // ---------------------------------------------------------------------------------------------
 int device_sm_count(int* out);
 cudaEvent_t decode_event(int i);
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes);
+
+static int split_box_bytes(int padded) {
+    return padded == 64 ? SplitShape<64, 1>::kRow : padded == 128 ? SplitShape<128, 1>::kRow : SplitShape<256, 1>::kRow;
+}
 
 static size_t split_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -1080,9 +1108,9 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
     p.partial_o = reinterpret_cast<float*>(ws + 256 + split_up((size_t)2 * ctas * 4 * p.group * sizeof(float)));
     p.out = out;
     p.out_lse = out_lse;
-    p.tok_stride = (int64_t)num_kv_heads * slot_bytes;
-    p.slab_bytes = num_blocks * kPageTokens * p.tok_stride;
     p.num_blocks = num_blocks;
+    const int map_rc = encode_cache_map(&p.cache_map, kv_cache, num_blocks, (int64_t)num_kv_heads * slot_bytes, split_box_bytes(padded));
+    if (map_rc != TQ_OK) return map_rc;
     p.kv_begin = kv_begin;
     p.kv_end = kv_end;
     p.batch = batch;
