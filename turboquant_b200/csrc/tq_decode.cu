@@ -913,19 +913,21 @@ static int chunk_heads(int remaining) { return remaining >= 16 ? 16 : remaining 
 static int largest_chunk(int num_kv_heads) { return single_launch(num_kv_heads) ? num_kv_heads : chunk_heads(num_kv_heads); }
 
 // Page-heads (pages x KV heads; the host knows their bound, batch x table width) up to which the kernel that splits by head is
-// the faster one.  It starts sooner and spreads further, the streaming kernel above moves a page in fewer copies.  Measured on uniform
-// batches, split against streaming, us: 32 query / 8 KV heads, 8192 page-heads 15 / 16 - 22, 32768: 32 - 34 / 27 - 37, 65536: 53 - 58 / 43 - 51; eight
-// query heads per KV head (more rows to rotate and merge per block) or four KV heads (four page lanes, four partials) cross at 65536;
-// more than 16 KV heads take several launches of the streaming kernel on strided rows: 163 against 179 at 262144.  A ragged batch
-// holds fewer pages than its bound and crosses later.
-// More than eight columns, against the tcgen05 kernel: up to 24 the split kernel is faster or equal at every size (8 x 32768 tokens, 8
-// KV heads, 12 / 16 / 24 columns: 124 / 124 / 159 against 163 / 165 / 171; 32 ragged sequences: 38 / 40 / 56 against 69 / 73 / 85).
-// With 32 columns it is up to 65536 (71 against 93 at 32 ragged sequences, 103 against 107 at 8 x 32768 and 4 KV heads), not at 131072
-// (181 against 173).
+// the faster one.  Write + decode of a step in a graph, streaming / split, us:
+//   8 KV heads (32 query heads), uniform 1 x 16384 18.6 / 15.3, 8 x 8192 33 / 28, 16 x 8192 45 / 45, 8 x 32768 75.5 / 72.3; ragged
+//   (log-uniform over a factor 256) 8 x 32768 35 / 29, 64 x 16384 73 / 64, 64 x 65536 209 / 204.
+//   4 KV heads: 64 x 16384 ragged 73 / 45, 8 x 32768 57 / 45.  32 (several launches of the streaming kernel on strided rows): 64 x
+//   16384 ragged 269 / 212, 8 x 32768 339 / 270.
+//   16 KV heads fill the streaming kernel's block with one page of all heads (one partial a block, no page lanes to merge): 8 x 4096
+//   28 / 28, 16 x 4096 ragged 24 / 20, 8 x 8192 42 / 45, 8 x 16384 71 / 80, 64 x 16384 ragged 105 / 112.
+// More than eight columns, tcgen05 / split, 8 KV heads: 16 x 8192 with 16 / 24 / 32 columns 114 / 66, 115 / 83, 119 / 93, 64 x 65536
+// ragged 632 / 276, 681 / 382, 710 / 475, one sequence of 1048576 with 32 columns 548 / 535: split at every size.
+// Up to four columns on 8 KV heads the two differ by 5 % either way from 65536 on (N(0, 1) keys and values, eager calls: 8 x 32768 82 / 86,
+// 64 ragged x 131072 560 / 605): streaming.  Five to eight: 40 / 8 heads 8 x 32768 80 / 72, 64 x 65536 ragged 146 / 114: split.
 static int64_t split_limit(int num_kv_heads, int columns) {
-    if (columns > 8) return columns <= 24 ? INT64_MAX : 81920;
-    if (!single_launch(num_kv_heads)) return 262144;
-    return columns > 4 || num_kv_heads <= 4 ? 81920 : 40960;
+    if (columns > 8) return INT64_MAX;
+    if (num_kv_heads == 16) return 32768;
+    return num_kv_heads == 8 && columns <= 4 ? 65536 : INT64_MAX;
 }
 
 struct ExchangeArgs {

@@ -1,7 +1,9 @@
 // Paged decode attention for WIDE query tiles (more than 8 and up to 32 query columns per KV head:
 // several decode queries that share one sequence's KV, times the GQA ratio; causal query chunks),
 // on the 5th-generation tensor cores: tcgen05.mma with the accumulators and one operand in tensor
-// memory.
+// memory.  Taken by calls that set their grid or pass a CSR page table; any other goes to the kernel that splits by KV head
+// (tq_decode_split.cu), which turned out faster at every size: this one is bound by the shared-memory pipe (V^ through shared memory
+// as an operand) and starts late on short contexts.
 //
 // The mma.sync kernel (tq_decode.cu) holds eight query columns in registers; 32 columns would need
 // 128 accumulator registers per thread, so a query tile of 8 queries x GQA 4 made four passes over

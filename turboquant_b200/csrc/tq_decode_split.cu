@@ -1,6 +1,6 @@
 // Paged decode attention split over (sequence, KV head, page range): every padded head size (64, 128, 256).
 //
-// The streaming kernel of tq_decode.cu gives a block all KV heads of a page range, which is what a long context of
+// The streaming kernel of tq_decode.cu gives a block all KV heads of a page range, which is what a long uniform context of
 // 128-wide heads wants (whole page halves in a few bulk copies) and what a short one does not: 1024 cached tokens are
 // eight blocks of four pages per warp, and the merge reads one partial per block, head and page lane.  Here a group of
 // warps takes ONE head of a page range.  Work that fits the chip in one page per warp is spread that wide; anything larger is cut into
@@ -9,9 +9,12 @@
 //   * One block per SM = kGroups groups of kGroupWarps warps around one lookup table.  A group works alone (its own
 //     named barrier); the table, the longest part of a block's prologue, is filled before the dependency wait.
 //   * Plan on the device, by every warp for itself from seq_lens (no barrier): see SplitPlan.
-//   * A warp takes whole pages of its head: 16-byte asynchronous copies into its own ring of stages, codes looked up straight
+//   * A warp takes whole pages of its head: two tiled tensor copies (16 rows of the head's slot each, from K and from V) into its
+//     own ring of stages (eleven 16-byte asynchronous copies a lane filled the load/store queue: 40 / 8 heads, 32 ragged
+//     sequences 34.4 -> 27.5 us a step, head size 64 34 -> 28, 256 37 -> 32), codes looked up straight
 //     into mma.sync.m16n8k16 fragments (the scheme of tq_decode.cu: K bytes are A fragments of S = K^ Q^T, V nibbles of
-//     two tokens zipped into bytes are A fragments of O^T += V^^T P).
+//     two tokens zipped into bytes are A fragments of O^T += V^^T P).  Up to 32 query columns (128-wide heads) are up to four
+//     MMA column tiles over one dequantization; see SplitShape for how registers are found for them.
 //   * The group's warps combine in shared memory.  A head whose whole sequence the group covered is finished there
 //     (inverse rotation, cast, store); only a head that was cut leaves partials for the merge kernel, which replans
 //     while the decode kernel runs (it is launched when every decode block is past its own wait) and has two dependent
@@ -55,6 +58,12 @@ struct SplitShape {
     static constexpr int kRegTiles = NT == 4 ? 0 : NT == 3 ? 2 : NT;
     static constexpr int kWarps = kGroups * kGroupWarps, kThreads = kWarps * 32;
     static constexpr int kRingsBelow = NT > 1 ? 5 : PD == 64 ? 13 : PD == 128 ? 7 : 6;   // rings below the table at 64 KB, the rest above it
+    // What starting an item (a sequence's set of heads) costs a group, in pages of it: page ids, queries to rotate, a ring to fill, a combine.
+    // Too little makes the blocks that hold many short sequences the last ones. 32 / 8 heads, 64 sequences of 64 ... 16384 tokens (log-
+    // uniform): cost 6 / 10 / 14 / 20 / 26 / 32 gives 103 / 83 / 71 / 64 / 66 / 67 us; 16 columns 16 / 26 / 40 / 60 / 80: 140 / 110 /
+    // 99 / 106 / 110; 24 columns 16 / 32 / 40 / 60: 214 / 148 / 130 / 136; 32 columns 32 / 40 / 60 / 80: 184 / 164 / 158 / 170; head size
+    // 64, 6 / 10 / 16: 76 / 61 / 50 (but 16 x 8192 uniform 35 / 35 / 43); 256, 6 / 10 / 16: 127 / 102 / 104.
+    static constexpr int kItemCost = PD != 128 ? 10 : NT == 1 ? 20 : NT < 4 ? 40 : 60;
     // What the warps of a pair hand each other: the probabilities of a page as fragments, two pages' worth in turn.
     static constexpr int kHandBytes = kPair ? (NT + 1) / 2 * 512 : 0, kHandAt = (kWarps - kRingsBelow) * kRingBytes;
     static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)kHandAt + 2 * kWarps * kHandBytes - 1024;   // from offset 1024 (the system's part): ample
@@ -83,6 +92,7 @@ struct SplitParams {
     int nq, real_heads, real_group, head_dim, slot_bytes;
     int causal;             // query i of nq sees the first len - (nq - 1 - i) tokens
     int grid, head_set, head_sets;   // blocks of the decode launch; heads side by side in a block when the work is cut evenly, and kv_heads / head_set
+    int item_cost;          // virtual pages that starting an item is worth (SplitShape::kItemCost)
     float inv_warps;        // 1 / warps of the grid
     int all_or_nothing;     // a sequence longer than its table empties the whole batch (128-wide heads), or only itself
     float k_scale, v_scale, scale;
@@ -95,12 +105,12 @@ struct SplitParams {
 //   pieces: every head is cut into equal pieces of at most kGroupWarps x `tiles` pages, with the smallest number of tiles (pages per
 //           warp) for which all pieces fit the groups of the grid; a worker is a group and takes one piece.  One start and one combine per
 //           group, and a head that fits a piece is not cut at all; but the pieces of a ragged batch are of many sizes.
-//   even:   the list of all pages (sequence, head set, page) is cut into equal ranges, one per worker, with kSplitItemCost virtual
+//   even:   the list of all pages (sequence, head set, page) is cut into equal ranges, one per worker, with item_cost virtual
 //           pages in front of every item for what starting it costs (queries to rotate, a combine).  The head_set groups of a worker
 //           take neighbouring heads of the same pages, so that the slots they read share their DRAM lines.
 // Pieces are taken when their tiles exceed the even share by at most kSplitSlackTiles (about what a second start costs a group).
 // ---------------------------------------------------------------------------------------------
-constexpr int kSplitItemCost = 6, kSplitSlackTiles = 3;
+constexpr int kSplitSlackTiles = 3;
 // The running maximum before any score: finite, so that a column whose tokens are all masked so far has exp2(-inf - m) = 0.
 constexpr float kNoMax = -3.402823466e38f;
 
@@ -156,7 +166,7 @@ __device__ __forceinline__ void split_load(const SplitParams& p, SplitPlan& s, i
     s.base = base;
     s.run = run;
     int v = 0;
-    if (s.np > 0) v = s.piece ? p.kv_heads * split_div_up(s.np, s.piece) : p.head_sets * (s.np + kSplitItemCost);
+    if (s.np > 0) v = s.piece ? p.kv_heads * split_div_up(s.np, s.piece) : p.head_sets * (s.np + p.item_cost);
     int incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -207,7 +217,7 @@ __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, i
     }
     s.head_set = s.piece ? 1 : p.head_set;
     s.workers = p.grid * (s.head_set == 1 ? NG : s.head_set == 2 ? NG / 2 : NG / 4);
-    s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * kSplitItemCost);
+    s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * p.item_cost);
     split_load(p, s, 0, 0, true);
 }
 
@@ -472,13 +482,13 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             p1 = p0 + size + (j < more ? 1 : 0);
             pos = hi;
         } else {
-            const int item = np + kSplitItemCost;
+            const int item = np + p.item_cost;
             hset = split_div(rel, item);
             const int off = rel - hset * item;
             const int left = hi - pos, rest = item - off;      // up to the end of the range or of the item
             const int take = left < rest ? left : rest;
-            p0 = off > kSplitItemCost ? off - kSplitItemCost : 0;
-            p1 = off + take - kSplitItemCost;
+            p0 = off > p.item_cost ? off - p.item_cost : 0;
+            p1 = off + take - p.item_cost;
             pos += take;
             if (p1 <= p0) continue;
         }
@@ -951,7 +961,7 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
             count = split_div_up(np, s.piece);
             first = vstart + hset * count;
         } else {
-            const int64_t at = vstart + (int64_t)hset * (np + kSplitItemCost) + kSplitItemCost, end = at + np;   // its pages in the list
+            const int64_t at = vstart + (int64_t)hset * (np + p.item_cost) + p.item_cost, end = at + np;   // its pages in the list
             first = (int)(((at + 1) * s.workers + s.total - 1) / s.total) - 1;
             count = (int)((end * s.workers + s.total - 1) / s.total) - first;
         }
@@ -1071,6 +1081,7 @@ static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
     p.grid = ctas;
     p.head_set = F::kGroups == 4 && p.kv_heads % 4 == 0 ? 4 : p.kv_heads % 2 == 0 ? 2 : 1;
     p.head_sets = p.kv_heads / p.head_set;
+    p.item_cost = F::kItemCost;
     p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
     TQ_CUDA(launch_serialized(decode_split_kernel<PD, NT>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
     if (cudaEvent_t mid = decode_event(1)) TQ_CUDA(cudaEventRecord(mid, s));
