@@ -58,3 +58,36 @@ def test_every_cut_matches_the_oracle(oracle, name):
         empty = np.array(lens) == 0
         assert (out.cpu().numpy()[empty] == 0).all() and np.isneginf(lse.cpu().numpy()[empty]).all()
         assert torch.isfinite(lse[torch.from_numpy(~empty)]).all()
+
+
+# (query heads, KV heads, head size, queries a row): one to eight columns and the wide tiles
+FEW_LIVE = [(32, 8, 128, 1), (8, 1, 128, 1), (8, 2, 128, 1), (16, 8, 64, 1), (4, 1, 64, 1), (16, 8, 256, 1), (2, 2, 256, 1), (8, 2, 128, 5), (8, 4, 128, 8)]
+
+
+@pytest.mark.parametrize("hq,hkv,d,nq", FEW_LIVE)
+@pytest.mark.parametrize("rows,live,tokens", [(257, 1, 320), (300, 2, 160), (512, 5, 400), (290, 3, 1)])
+def test_many_rows_of_which_few_hold_tokens(oracle, hq, hkv, d, nq, rows, live, tokens):
+    """A mixed step or a padded batch: the plan's list is shorter than the number of workers, on a fresh workspace and on one that a
+    call with more work has filled."""
+    lens = [0] * rows
+    for i in range(live):
+        lens[(7 + 61 * i) % rows] = tokens
+    attn = TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv)
+    case = synthetic.decode_case(seed=rows + live, seq_lens=lens, dtype=torch.float16, heads=(hq, hkv), head_dim=d)
+    cache = torch.zeros(kv_cache_shape(max(case.num_blocks, 1), 16, hkv, d), dtype=torch.uint8, device=DEV)
+    attn.write(case.k.to(DEV), case.v.to(DEV), cache, case.slot_mapping.to(DEV))
+    q = torch.randn(rows, nq, hq, d, generator=torch.Generator().manual_seed(3)).to(torch.float16)
+    at = np.array(lens) > 0
+    want = oracle.decode_paged(q[at].float().numpy().reshape(-1, hq, d), cache.cpu().numpy(), np.repeat(case.block_table.numpy()[at], nq, axis=0),
+                               np.full(live * nq, tokens, np.int32), attn.signs(DEV).cpu().numpy(), attn.scale)
+    q, bt, sl = q.to(DEV), case.block_table.to(DEV), case.seq_lens.to(DEV)
+    full = torch.full_like(sl, tokens)                                  # every row, over the pages of the first (all ids are in range)
+    for turn in range(2):
+        out = torch.full_like(q, float("nan"))
+        attn.decode_shared(q, cache, bt, sl, out)
+        assert attn.status(rows, DEV, nq) == 0
+        got = out.float().cpu().numpy()
+        assert (got[~at] == 0).all()
+        assert_attention_close(got[at].reshape(-1, hq, d), want, f"turn {turn}")
+        if turn == 0:
+            attn.decode_shared(q, cache, bt, full, out)

@@ -105,8 +105,8 @@ struct SplitParams {
 //   pieces: every head is cut into equal pieces of at most kGroupWarps x `tiles` pages, with the smallest number of tiles (pages per
 //           warp) for which all pieces fit the groups of the grid; a worker is a group and takes one piece.  One start and one combine per
 //           group, and a head that fits a piece is not cut at all; but the pieces of a ragged batch are of many sizes.
-//   even:   the list of all pages (sequence, head set, page) is cut into equal ranges, one per worker, with item_cost virtual
-//           pages in front of every item for what starting it costs (queries to rotate, a combine).  The head_set groups of a worker
+//   even:   the list of all pages (sequence, head set, page) is cut into equal ranges, one per worker and none of them empty, with
+//           item_cost virtual pages in front of every item for what starting it costs (queries to rotate, a combine).  The head_set groups of a worker
 //           take neighbouring heads of the same pages, so that the slots they read share their DRAM lines.
 // Pieces are taken when their tiles exceed the even share by at most kSplitSlackTiles (about what a second start costs a group).
 // ---------------------------------------------------------------------------------------------
@@ -218,6 +218,9 @@ __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, i
     s.head_set = s.piece ? 1 : p.head_set;
     s.workers = p.grid * (s.head_set == 1 ? NG : s.head_set == 2 ? NG / 2 : NG / 4);
     s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * p.item_cost);
+    // Every worker of the even cut has a position of the list: one with an empty range would write no partial, and the merge counts
+    // all workers between a head's first and last as its parts.  (A short list is cut too: many sequences of which few hold tokens.)
+    if (!s.piece && s.workers > s.total) s.workers = s.total;
     split_load(p, s, 0, 0, true);
 }
 
@@ -425,11 +428,11 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     const int hs = s.head_set;
     const int sub = hs == 1 ? gg : hs == 2 ? gg >> 1 : gg >> 2, hsub = gg - sub * hs;
     const int worker = sub * p.grid + (int)blockIdx.x;   // neighbouring workers sit on different SMs
-    int pos, hi;
+    int pos = 0, hi = 0;
     if (s.piece) {
         pos = worker;
         hi = worker < s.total ? worker + 1 : worker;
-    } else {
+    } else if (worker < s.workers) {
         pos = split_cut(worker, s.total, s.workers);
         hi = split_cut(worker + 1, s.total, s.workers);
     }
