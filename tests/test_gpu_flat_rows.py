@@ -40,3 +40,19 @@ def test_rows_match_the_oracle(oracle, dim, n, dtype):
             np.testing.assert_array_equal(norms.cpu().numpy(), want_n)
             out = _cabi.dequantize_flat(p, norms, signs.to(DEV), dim, bits, cache_order=cache_order)
             np.testing.assert_array_equal(out.cpu().numpy(), oracle.dequantize_flat(want_p, want_n, signs.numpy(), dim, bits))
+
+
+@pytest.mark.parametrize("dim", [128, 100])                 # the row kernels and the plain ones
+def test_pack_order_takes_any_truth_value(dim):
+    x, signs = _rows(20, dim, torch.float16, 5).to(DEV), synthetic.make_signs(128, 42).to(DEV)
+    want, norms = _cabi.quantize_flat(x, signs, 4, cache_order=True)
+    low_first, _ = _cabi.quantize_flat(x, signs, 4, cache_order=False)
+    assert not torch.equal(want, low_first)
+    back = _cabi.dequantize_flat(want, norms, signs, dim, 4, cache_order=True)
+    for yes, no in ((1, 0), (np.bool_(True), np.bool_(False)), ("cache", None)):
+        assert torch.equal(_cabi.quantize_flat(x, signs, 4, cache_order=yes)[0], want)
+        assert torch.equal(_cabi.quantize_flat(x, signs, 4, cache_order=no)[0], low_first)
+        assert torch.equal(_cabi.dequantize_flat(want, norms, signs, dim, 4, cache_order=yes).nan_to_num(), back.nan_to_num())
+        assert torch.equal(_cabi.dequantize_flat(low_first, norms, signs, dim, 4, cache_order=no).nan_to_num(), back.nan_to_num())
+    with pytest.raises(ValueError):
+        _cabi.quantize_flat(x, signs, 4, cache_order=np.array([True, False]))      # no truth value

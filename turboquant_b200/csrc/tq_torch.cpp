@@ -141,6 +141,7 @@ PyObject* layer_write(PyObject* o, PyObject* const* args, Py_ssize_t n) {
         if (t->dim() != 3 || t->size(0) < T || t->size(1) != H || t->size(2) != D || t->stride(2) != 1 || t->stride(1) != D) Py_RETURN_NONE;
     if (T == 0) Py_RETURN_TRUE;
     const int zero_pad = PyObject_IsTrue(args[4]);
+    if (zero_pad < 0) return nullptr;
     void* stream = stream_of(dev);
     int rc;
     {
@@ -263,6 +264,8 @@ PyObject* quantize_flat(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!x || !signs || x->dim() < 1 || !x->is_contiguous() || x->numel() == 0 || float_code(x->scalar_type()) < 0) Py_RETURN_NONE;
     const long bits = PyLong_AsLong(args[2]);
     if (bits == -1 && PyErr_Occurred()) return nullptr;
+    const int order = PyObject_IsTrue(args[3]);      // any truth value, as the Python layer takes it
+    if (order < 0) return nullptr;
     const int64_t d = x->size(-1), pd = padded_dim(d);
     if (bits < 1 || bits > 4 || signs->get_device() != x->get_device() || signs->scalar_type() != at::kFloat || !signs->is_contiguous() ||
         signs->numel() < pd)
@@ -275,7 +278,6 @@ PyObject* quantize_flat(PyObject*, PyObject* const* args, Py_ssize_t n) {
     shape.pop_back();
     at::Tensor norms = at::empty(shape, options.dtype(at::kFloat));
     void* stream = stream_of(x->get_device());
-    const bool order = args[3] == Py_True;
     int rc;
     {
         Gil gil;
@@ -299,7 +301,8 @@ PyObject* dequantize_flat(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor *packed = cuda_tensor(args[0]), *norms = cuda_tensor(args[1]), *signs = cuda_tensor(args[2]);
     if (!packed || !norms || !signs || packed->dim() < 1) Py_RETURN_NONE;
     const long d = PyLong_AsLong(args[3]), bits = PyLong_AsLong(args[4]);
-    if (PyErr_Occurred()) return nullptr;
+    const int order = PyErr_Occurred() ? -1 : PyObject_IsTrue(args[5]);
+    if (order < 0) return nullptr;
     const int dev = packed->get_device();
     if (norms->get_device() != dev || signs->get_device() != dev || packed->scalar_type() != at::kByte || !packed->is_contiguous() ||
         norms->scalar_type() != at::kFloat || !norms->is_contiguous() || signs->scalar_type() != at::kFloat || !signs->is_contiguous())
@@ -311,7 +314,6 @@ PyObject* dequantize_flat(PyObject*, PyObject* const* args, Py_ssize_t n) {
     shape.push_back(d);
     at::Tensor out = at::empty(shape, at::TensorOptions().device(packed->device()).dtype(at::kFloat));
     void* stream = stream_of(dev);
-    const bool order = args[5] == Py_True;
     int rc;
     {
         Gil gil;
