@@ -56,3 +56,24 @@ def test_pack_order_takes_any_truth_value(dim):
         assert torch.equal(_cabi.dequantize_flat(low_first, norms, signs, dim, 4, cache_order=no).nan_to_num(), back.nan_to_num())
     with pytest.raises(ValueError):
         _cabi.quantize_flat(x, signs, 4, cache_order=np.array([True, False]))      # no truth value
+
+
+@pytest.mark.parametrize("dim", [64, 128, 256])
+def test_signs_beyond_one(oracle, dim):
+    """Any sign vector is taken: the row kernels agree with the plain ones (which rows that start off their alignment take) and, where all
+    values are finite, with the oracle."""
+    g = torch.Generator().manual_seed(dim)
+    x = _rows(50, dim, torch.float16, 4)
+    odd = torch.empty(50 * dim + 1, dtype=torch.float16, device=DEV)[1:].view(50, dim)
+    odd.copy_(x)
+    ones = synthetic.make_signs(dim, 42)
+    for name, signs in (("threes", 3.0 * ones), ("wide", torch.randn(dim, generator=g) * 1e6), ("fractions", 0.5 * ones), ("zeros", 0.0 * ones),
+                        ("infinite", torch.where(torch.arange(dim) % 17 == 3, ones * float("inf"), ones)),
+                        ("nan", torch.where(torch.arange(dim) == 5, ones * float("nan"), ones)), ("largest", ones * 3.4e38)):
+        for bits in (1, 2, 3, 4):
+            p, norms = _cabi.quantize_flat(x.to(DEV), signs.to(DEV), bits)
+            plain, plain_norms = _cabi.quantize_flat(odd, signs.to(DEV), bits)
+            assert torch.equal(p, plain), (name, bits)
+            np.testing.assert_array_equal(norms.cpu().numpy(), plain_norms.cpu().numpy())
+            if bool((signs.abs() < 1e30).all()):
+                np.testing.assert_array_equal(p.cpu().numpy(), oracle.quantize_flat(x.float().numpy(), signs.numpy(), bits)[0], err_msg=f"{name} {bits}")

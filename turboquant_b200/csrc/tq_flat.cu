@@ -233,8 +233,15 @@ __global__ void __launch_bounds__(kRowsThreads, E == 8 ? 4 : E == 16 ? 3 : 2) qu
     grid_launch_dependents();
     for (int i = threadIdx.x; i < kFlatBins * kFlatCols; i += kRowsThreads) bins_s[i] = p.bins[i / kFlatCols];
     grid_dependency_wait();      // only the table is made ahead of it
-    for (int i = threadIdx.x; i < kPd; i += kRowsThreads) sign_s[i] = i < dim ? p.f.signs[i] : 1.0f;
-    __syncthreads();
+    bool beyond = false;
+    for (int i = threadIdx.x; i < kPd; i += kRowsThreads) {
+        const float sg = i < dim ? p.f.signs[i] : 1.0f;
+        sign_s[i] = sg;
+        beyond |= !(fabsf(sg) <= 1.0f);
+    }
+    // A normalized row keeps |y| <= 1, well inside the table, as long as no sign exceeds one.  Any other vector is taken too (infinities and
+    // NaN among them): its values are brought inside the table first, beyond every boundary all the same.
+    const bool wild = __syncthreads_or(beyond);
     // (the bit pattern of 2^23 + k) * 128 = 2^31 + 128 k modulo 2^32: entry k of this lane's column
     const uint32_t table_lane = smem_u32(bins_s) + 8u * (lane & (kFlatCols - 1)) - 0x80000000u;
     const P2 bin_scale2 = pk(p.bin_scale, p.bin_scale), bin_magic2 = pk(p.bin_magic, p.bin_magic), scale2 = pk(p.f.scale, p.f.scale);
@@ -301,6 +308,16 @@ __global__ void __launch_bounds__(kRowsThreads, E == 8 ? 4 : E == 16 ? 3 : 2) qu
             x[j] = mul2(x[j], pk(sg.x, sg.y));
         }
         rows_fwht<E>(x, m);
+        if (wild) {
+            const float most = 1.5f / p.f.scale;
+            auto inside = [most](float v) { return v < most ? fmaxf(v, -most) : most; };      // NaN: the last code
+#pragma unroll
+            for (int j = 0; j < E; j++) {
+                float a, b;
+                up(x[j], a, b);
+                x[j] = pk(inside(a), inside(b));
+            }
+        }
         // codes.  A NaN row is NaN in every element (each output takes every input): torch puts NaN in the last bucket.
         float y0, y1;
         up(mul2(x[0], scale2), y0, y1);
