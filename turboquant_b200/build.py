@@ -21,6 +21,7 @@ LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libturboquant_b200.so"
 NATIVE = PKG / "_native.so"
 NATIVE_SRC = CSRC / "tq_torch.cpp"
+NATIVE_STAMP = PKG / "build" / "native.stamp"      # what NATIVE was built against
 HEADER = PKG.parent / "include" / "turboquant_b200.h"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -57,6 +58,23 @@ def _native_command() -> list[str]:
             "-L", str(root / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
 
 
+def _native_stamp() -> str:
+    import sysconfig
+    import torch
+    return "\n".join([torch.__version__, str(sysconfig.get_config_var("SOABI")), *_native_command()])
+
+
+def _native_stale() -> bool:
+    """Older than its source, or built against another torch or Python: the module is bound to both."""
+    built_against = NATIVE_STAMP.read_text() if NATIVE_STAMP.exists() else ""
+    return _stale(NATIVE, [NATIVE_SRC, HEADER, Path(__file__)]) or built_against != _native_stamp()
+
+
+def _build_native() -> None:
+    subprocess.check_call(_native_command())
+    NATIVE_STAMP.write_text(_native_stamp())
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = PKG / "build"
@@ -76,8 +94,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
     with ThreadPoolExecutor(max_workers=5) as ex:
         native = None
-        if force or _stale(NATIVE, [NATIVE_SRC, HEADER, Path(__file__)]):
-            native = ex.submit(subprocess.check_call, _native_command())
+        if force or _native_stale():
+            native = ex.submit(_build_native)
         objs = list(ex.map(compile_one, UNITS.items()))
         if native:
             native.result()
