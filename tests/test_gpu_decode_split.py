@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from turboquant_b200 import TurboQuantPagedAttention, synthetic
+from turboquant_b200 import TurboQuantPagedAttention, _cabi, synthetic
 from turboquant_b200.paged_attention import kv_cache_shape
 
 from tests.gpu_util import assert_attention_close
@@ -91,3 +91,47 @@ def test_many_rows_of_which_few_hold_tokens(oracle, hq, hkv, d, nq, rows, live, 
         assert_attention_close(got[at].reshape(-1, hq, d), want, f"turn {turn}")
         if turn == 0:
             attn.decode_shared(q, cache, bt, full, out)
+
+
+def _exact(attn, cache, table, lens, q, causal=False):
+    """Attention over the cache's own bytes in 64 bits; q [rows, queries, heads, size]."""
+    H, D, pd = attn.num_kv_heads, attn.head_size, attn.padded_dim
+    rot = torch.ones(1, 1, dtype=torch.float64, device=DEV)
+    while rot.shape[0] < pd:
+        rot = torch.cat([torch.cat([rot, rot], 1), torch.cat([rot, -rot], 1)], 0)
+    rot = rot / math.sqrt(pd) * attn.signs(DEV).double()
+    centroids = _cabi.codebook(pd, 4)[0].double().to(DEV)
+    out = torch.zeros(q.shape, dtype=torch.float64, device=DEV)
+    for b, n in enumerate(lens):
+        slots = cache[:, table[b, : (n + 15) // 16].long()].flatten(1, 2)[:, :n]
+        codes, norms = slots[..., : pd // 2], slots[..., pd // 2: pd // 2 + 2].contiguous().view(torch.float16).double()
+        kv = torch.stack([centroids[(codes >> 4).long()], centroids[(codes & 15).long()]], -1).flatten(-2) @ rot * norms
+        s = torch.einsum("nhgd,thd->nhgt", q[b].double().unflatten(1, (H, -1)), kv[0, ..., :D]) * attn.scale
+        if causal:
+            hidden = torch.arange(n, device=DEV)[None, :] >= n - torch.arange(q.shape[1] - 1, -1, -1, device=DEV)[:, None]
+            s.masked_fill_(hidden[:, None, None], -math.inf)
+        out[b] = torch.einsum("nhgt,thd->nhgd", s.softmax(-1), kv[1, ..., :D]).flatten(1, 2)
+    return out
+
+
+def _error(attn, nq, lens, v_scale, q_scale=1.0, causal=False):
+    """Relative error (2-norm) of a decode call in fp32 against 64 bits, N(0, 1) keys, values and queries times a scale."""
+    H, D = attn.num_kv_heads, attn.head_size
+    g = torch.Generator(DEV).manual_seed(11)
+    case = synthetic.decode_case(seed=4, seq_lens=lens, heads=(H, H), head_dim=D)
+    cache = torch.zeros(kv_cache_shape(case.num_blocks, 16, H, D), dtype=torch.uint8, device=DEV)
+    k, v = (torch.randn(sum(lens), H, D, generator=g, device=DEV) for _ in range(2))
+    attn.write(k, v * v_scale, cache, case.slot_mapping.to(DEV))
+    q = torch.randn(len(lens), nq, attn.num_heads, D, generator=g, device=DEV) * q_scale
+    table = case.block_table.to(DEV)
+    out = (attn.decode_causal if causal else attn.decode_shared)(q, cache, table, case.seq_lens.to(DEV))
+    want = _exact(attn, cache, table, lens, q, causal)
+    return float((out.double() - want).norm() / want.norm())
+
+
+# Bounds: 1.15 times what these sizes show with the head's own fp16 centroids and the V norm as it is (3.6e-4 and 4.7e-4 at every scale; with
+# the N(0, 1) centroids and 1 / sqrt(d) ahead of the rounding 4.7 ... 5.6e-4 at 80 and, at a scale of 1e-4, 6.8e-4 at 64 and 7.0e-4 at 256).
+@pytest.mark.parametrize("hq,hkv,d,bound", [(16, 2, 80, 4.15e-4), (16, 8, 64, 5.4e-4), (16, 8, 256, 5.4e-4)])
+@pytest.mark.parametrize("v_scale", [1e-4, 1e-3, 1.0, 50.0])
+def test_error_of_other_head_sizes_at_any_size_of_v(hq, hkv, d, bound, v_scale):
+    assert _error(TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv), 1, [2000, 700, 4096], v_scale) <= bound

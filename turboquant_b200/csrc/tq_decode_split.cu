@@ -1141,12 +1141,20 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
     p.all_or_nothing = all_or_nothing;
     p.causal = causal;
     const double inv = 1.0 / std::sqrt((double)padded);
-    p.scale = p.v_scale = (float)inv;
-    p.k_scale = (float)(inv * (double)sm_scale * 1.4426950408889634);
+    p.scale = (float)inv;
+    // The table is fp16 and so is P times the V norm.  Heads of 128 / 96 share the N(0, 1) centroids with the streaming kernel and have
+    // 1 / sqrt(d) in the scales; other sizes have it in their own centroids, as the plain kernel does.  Error of the output against 64 bits,
+    // N(0, 1) queries and keys, with the N(0, 1) centroids / with their own: head size 80 4.7 ... 5.6e-4 / 3.6e-4; V rows of norm 1e-3 at head size
+    // 64 6.8e-4 / 4.7e-4, 256 7.0e-4 / 4.7e-4 (the scale brings P times the norm 8 and 16 times nearer to fp16's subnormals).
+    const bool own_table = head_dim != kHeadDim && head_dim != 96;
+    float cen[16], bnd[15];
+    host_codebook(padded, 4, cen, bnd);
     for (int k = 0; k < 16; k++) {
-        const __half h = __float2half_rn((float)kCentroidsN01_4bit[k]);
+        const __half h = __float2half_rn(own_table ? cen[k] : (float)kCentroidsN01_4bit[k]);
         memcpy(&p.centroid_h[k], &h, 2);
     }
+    p.v_scale = own_table ? 1.0f : (float)inv;
+    p.k_scale = (float)((own_table ? 1.0 : inv) * (double)sm_scale * 1.4426950408889634);
     switch (padded) {
         case 64: return launch_split<64, 1>(p, ctas, s);
         case 128:
