@@ -93,28 +93,33 @@ def test_many_rows_of_which_few_hold_tokens(oracle, hq, hkv, d, nq, rows, live, 
             attn.decode_shared(q, cache, bt, full, out)
 
 
-def _exact(attn, cache, table, lens, q, causal=False):
-    """Attention over the cache's own bytes in 64 bits; q [rows, queries, heads, size]."""
+def _exact(attn, cache, table, lens, q, causal=False, fp16_operands=False):
+    """Attention over the cache's own bytes in 64 bits, in the rotated domain; q [rows, queries, heads, size].  ``fp16_operands``: with
+    the queries and centroids rounded as the kernel's, which leaves the rounding of P times the V norm."""
     H, D, pd = attn.num_kv_heads, attn.head_size, attn.padded_dim
     rot = torch.ones(1, 1, dtype=torch.float64, device=DEV)
     while rot.shape[0] < pd:
         rot = torch.cat([torch.cat([rot, rot], 1), torch.cat([rot, -rot], 1)], 0)
     rot = rot / math.sqrt(pd) * attn.signs(DEV).double()
     centroids = _cabi.codebook(pd, 4)[0].double().to(DEV)
+    q = torch.nn.functional.pad(q.double(), (0, pd - D)) @ rot.T
+    if fp16_operands:
+        unit = math.sqrt(pd) if D in (128, 96) else 1.0                 # those share the N(0, 1) table
+        q, centroids = q.half().double(), (centroids * unit).half().double() / unit
     out = torch.zeros(q.shape, dtype=torch.float64, device=DEV)
     for b, n in enumerate(lens):
         slots = cache[:, table[b, : (n + 15) // 16].long()].flatten(1, 2)[:, :n]
         codes, norms = slots[..., : pd // 2], slots[..., pd // 2: pd // 2 + 2].contiguous().view(torch.float16).double()
-        kv = torch.stack([centroids[(codes >> 4).long()], centroids[(codes & 15).long()]], -1).flatten(-2) @ rot * norms
-        s = torch.einsum("nhgd,thd->nhgt", q[b].double().unflatten(1, (H, -1)), kv[0, ..., :D]) * attn.scale
+        kv = torch.stack([centroids[(codes >> 4).long()], centroids[(codes & 15).long()]], -1).flatten(-2) * norms
+        s = torch.einsum("nhgd,thd->nhgt", q[b].unflatten(1, (H, -1)), kv[0]) * attn.scale
         if causal:
             hidden = torch.arange(n, device=DEV)[None, :] >= n - torch.arange(q.shape[1] - 1, -1, -1, device=DEV)[:, None]
             s.masked_fill_(hidden[:, None, None], -math.inf)
-        out[b] = torch.einsum("nhgt,thd->nhgd", s.softmax(-1), kv[1, ..., :D]).flatten(1, 2)
-    return out
+        out[b] = torch.einsum("nhgt,thd->nhgd", s.softmax(-1), kv[1]).flatten(1, 2)
+    return (out @ rot)[..., :D]
 
 
-def _error(attn, nq, lens, v_scale, q_scale=1.0, causal=False):
+def _error(attn, nq, lens, v_scale, q_scale=1.0, causal=False, fp16_operands=False):
     """Relative error (2-norm) of a decode call in fp32 against 64 bits, N(0, 1) keys, values and queries times a scale."""
     H, D = attn.num_kv_heads, attn.head_size
     g = torch.Generator(DEV).manual_seed(11)
@@ -125,7 +130,7 @@ def _error(attn, nq, lens, v_scale, q_scale=1.0, causal=False):
     q = torch.randn(len(lens), nq, attn.num_heads, D, generator=g, device=DEV) * q_scale
     table = case.block_table.to(DEV)
     out = (attn.decode_causal if causal else attn.decode_shared)(q, cache, table, case.seq_lens.to(DEV))
-    want = _exact(attn, cache, table, lens, q, causal)
+    want = _exact(attn, cache, table, lens, q, causal, fp16_operands)
     return float((out.double() - want).norm() / want.norm())
 
 
@@ -135,3 +140,23 @@ def _error(attn, nq, lens, v_scale, q_scale=1.0, causal=False):
 @pytest.mark.parametrize("v_scale", [1e-4, 1e-3, 1.0, 50.0])
 def test_error_of_other_head_sizes_at_any_size_of_v(hq, hkv, d, bound, v_scale):
     assert _error(TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv), 1, [2000, 700, 4096], v_scale) <= bound
+
+
+# Bound: 1.15 times the largest error of these calls at V scale 1 with the tcgen05 kernel (5.7e-4), whose operands are P and V^ apart; with 1 / sqrt(128) in
+# front of the rounding they showed up to 8.7e-4 at a scale of 1e-4, and infinities from norms of 16000 on.
+@pytest.mark.parametrize("hq,hkv,d,nq", [(8, 8, 128, 4), (32, 8, 128, 2), (16, 8, 128, 8), (24, 8, 128, 8), (32, 8, 128, 8), (32, 8, 96, 5)])
+@pytest.mark.parametrize("v_scale", [1e-4, 1.0, 3000.0])
+def test_error_of_causal_queries_at_any_size_of_v(hq, hkv, d, nq, v_scale):
+    assert _error(TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv), nq, [2000, 700, 4096], v_scale, causal=True) <= 6.6e-4
+
+
+@pytest.mark.parametrize("hq,hkv,d,nq", [(16, 8, 64, 1), (16, 8, 256, 1), (16, 4, 128, 1), (16, 8, 128, 8), (24, 8, 128, 8), (32, 8, 128, 8)])
+@pytest.mark.parametrize("order", ["up", "down", "spikes"])
+def test_v_norms_of_many_sizes_in_a_sequence(hq, hkv, d, nq, order):
+    """The warps' scale is lowered again and again, or once, by the first page or by a few tokens.  Bound: what is left after the operands'
+    rounding is that of P times the norm, 2^-11 of each term at most."""
+    lens = [2000, 700, 4096]
+    size = {"up": lambda t: 10.0 ** (-3 + 6 * t), "down": lambda t: 10.0 ** (3 - 6 * t), "spikes": lambda t: 1.0 + 2500.0 * (torch.frac(t * 37.0) < 0.01)}[order]
+    v_scale = torch.cat([size(torch.arange(n, device=DEV) / n) for n in lens])[:, None, None]
+    attn = TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv)
+    assert _error(attn, nq, lens, v_scale, q_scale=3.0, fp16_operands=True) <= 2.0 ** -11

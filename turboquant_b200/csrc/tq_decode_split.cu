@@ -113,6 +113,14 @@ struct SplitParams {
 constexpr int kSplitSlackTiles = 3;
 // The running maximum before any score: finite, so that a column whose tokens are all masked so far has exp2(-inf - m) = 0.
 constexpr float kNoMax = -3.402823466e38f;
+// P times the V norm is rounded to fp16 as the MMA's operand.  Norms are any fp16 value, so each warp scales them by a power of two, the
+// way the maxima are raised: a page whose largest scaled norm exceeds kVNormMost (2^kRaiseThreshold times that is still finite in fp16) lowers the
+// scale until that norm lies in [256, 512), and the accumulators with it; the combine takes the scale out in fp32.  It starts at
+// 16: norms up to 62 never lower it, and those down to fp16's smallest normal number leave P its bits (1 / sqrt(128) in place of
+// it: V rows of norm 1e-3 under 16 ... 32 causal columns had an error of 7 ... 8.7e-4 against 64 bits, now 5.6e-4 as at norm 11, and norms of
+// 16000 and more overflowed).  A lookup in shared memory, a maximum and a comparison a
+// page: 8 x 32768 causal, 8 queries 164.3 -> 165.8 us, 32 ragged sequences 27.9 -> 28.1, head size 64 28.0 -> 28.5.
+constexpr float kVNormMost = 1000.0f, kVScaleStart = 16.0f;
 
 // n / d for 0 <= n < 2^24, d > 0: a reciprocal, then the quotient put right.  (The plan is repeated by every warp, and the compiler's
 // division is three times as long.)
@@ -370,11 +378,11 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     using F = SplitShape<PD, NT>;
     constexpr int E = F::kE, NG = F::kGroups, GW = F::kGroupWarps;
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ float m_s[NG][GW][F::kCols], l_s[NG][GW][F::kCols];
+    __shared__ float m_s[NG][GW][F::kCols], l_s[NG][GW][F::kCols], v_s[NG][GW];
     __shared__ float sign_s[PD];
-    __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols];      // a pair's maxima of a page that raises them, and whether it does
+    __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols + 1];  // a pair's maxima of a page that raises them (and its largest V norm), and whether it does
     __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
-    __shared__ uint64_t full_s[F::kWarps][F::kStages];               // a stage's two boxes have landed
+    __shared__ uint64_t full_s[F::kWarps][F::kStages + 1];           // a stage's two boxes have landed; and a word for the warp's scale of the V norms
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -559,6 +567,12 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             split_load_row<E>(p.q, p.q_dtype, q_row(r), p.head_dim, lane * E, qv[0]);
             put_q(r, qv[0]);
         }
+        // in shared memory: a register more spills
+        auto v_norm_scale = [&]() -> float { return __uint_as_float(lds32(full_at + 8 * F::kStages)); };
+        auto set_v_norm_scale = [&](float v) {
+            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(full_at + 8 * F::kStages), "r"(__float_as_uint(v)) : "memory");
+        };
+        set_v_norm_scale(kVScaleStart);
         group_sync();
         uint32_t qf[F::kRegTiles > 0 ? F::kRegTiles : 1][PD / 8];    // B fragments of Q^T: dims 2 x (code bytes tg PD/8 ...) of query column 8 j + g
 #pragma unroll
@@ -624,7 +638,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             // Only the last page of a sequence holds tokens past the window: their norms are zeroed (whatever the unwritten
             // slots contain) and their scores biased to -inf.
             float kfa = lds_half(kn_at + st) * p.k_scale, kfb = lds_half(kn_at + st + 8 * F::kRow) * p.k_scale;
-            vfa = lds_half(vn_at + st) * p.v_scale, vfb = lds_half(vn_at + st + 8 * F::kRow) * p.v_scale;
+            const float v_norm = v_norm_scale();
+            vfa = lds_half(vn_at + st) * v_norm, vfb = lds_half(vn_at + st + 8 * F::kRow) * v_norm;
             float bias_a = 0.0f, bias_b = 0.0f;
             if (left < kPageTokens) {
                 if (ta >= left) { kfa = 0.0f; vfa = 0.0f; bias_a = -INFINITY; }
@@ -650,8 +665,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             }
         };
         // ---- online softmax (base 2) with a maximum that is raised only when a score exceeds it by kRaiseThreshold
-        auto exceeds = [&](const float (&s_acc)[NT][4]) {
-            bool over = false;
+        auto exceeds = [&](const float (&s_acc)[NT][4], float vfa, float vfb) {
+            bool over = fmaxf(fabsf(vfa), fabsf(vfb)) > kVNormMost;
 #pragma unroll
             for (int t = 0; t < NT; t++)
                 over |= fmaxf(s_acc[t][0], s_acc[t][2]) > m0[t] + kRaiseThreshold || fmaxf(s_acc[t][1], s_acc[t][3]) > m1[t] + kRaiseThreshold;
@@ -666,16 +681,26 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
             }
         };
-        auto raise_to = [&](int t, float mx0, float mx1) {
+        // the largest V norm of the page if it is beyond the limit, else zero; and the power of two that brings it to [256, 512)
+        auto norm_max = [&](float vfa, float vfb) {
+            float v = fmaxf(fabsf(vfa), fabsf(vfb));
+            if (!__any_sync(0xffffffffu, v > kVNormMost)) return 0.0f;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+            return v;
+        };
+        auto norm_factor = [](float v) { return v > kVNormMost ? __uint_as_float((127 + 8 + 127 - (__float_as_uint(v) >> 23)) << 23) : 1.0f; };
+        auto raise_to = [&](int t, float mx0, float mx1, float f) {
             const bool raise0 = mx0 > m0[t] + kRaiseThreshold, raise1 = mx1 > m1[t] + kRaiseThreshold;
             const float c0 = raise0 ? fast_exp2(m0[t] - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1[t] - mx1) : 1.0f;
             if (raise0) m0[t] = mx0;
             if (raise1) m1[t] = mx1;
             l0[t] *= c0;
             l1[t] *= c1;
+            const float f0 = c0 * f, f1 = c1 * f;
 #pragma unroll
             for (int i = 0; i < kAccTiles; i++) {
-                o_acc[t][i][0] *= c0; o_acc[t][i][1] *= c1; o_acc[t][i][2] *= c0; o_acc[t][i][3] *= c1;
+                o_acc[t][i][0] *= f0; o_acc[t][i][1] *= f1; o_acc[t][i][2] *= f0; o_acc[t][i][3] *= f1;
             }
         };
         // P = exp2(x - m) times the V norm as B fragments, and its column sums over this lane's two tokens
@@ -752,12 +777,18 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 float s_acc[NT][4], vfa, vfb, a0[NT], a1[NT];
                 uint32_t pb0[NT], pb1[NT];
                 scores(st, left, s_acc, vfa, vfb);
-                if (exceeds(s_acc)) {
+                if (exceeds(s_acc, vfa, vfb)) {
+                    const float f = norm_factor(norm_max(vfa, vfb));
 #pragma unroll
                     for (int t = 0; t < NT; t++) {
                         float mx0, mx1;
                         page_max(s_acc[t], mx0, mx1);
-                        raise_to(t, mx0, mx1);
+                        raise_to(t, mx0, mx1, f);
+                    }
+                    if (f < 1.0f) {
+                        vfa *= f;
+                        vfb *= f;
+                        set_v_norm_scale(v_norm_scale() * f);
                     }
                 }
                 probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
@@ -795,7 +826,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 uint32_t pb0[NT], pb1[NT];
                 scores(st, it < n ? left : 0, s_acc, vfa, vfb);      // past its last page a warp has no tokens: P = 0
                 const uint32_t turn = (uint32_t)(it & 1) * F::kHandBytes;
-                const bool over = exceeds(s_acc);
+                const bool over = exceeds(s_acc, vfa, vfb);
                 probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
                 put(mine + turn, pb0, pb1);
                 if (lane == 0) raise_s[it & 1][warp] = over;
@@ -810,9 +841,17 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                             max_s[warp][8 * t + 2 * tg + 1] = mx1[t];
                         }
                     }
+                    const float v_max = norm_max(vfa, vfb);
+                    if (lane == 0) max_s[warp][F::kCols] = v_max;
                     pair_sync();
+                    const float f = norm_factor(fmaxf(v_max, max_s[ow][F::kCols]));
 #pragma unroll
-                    for (int t = 0; t < NT; t++) raise_to(t, fmaxf(mx0[t], max_s[ow][8 * t + 2 * tg]), fmaxf(mx1[t], max_s[ow][8 * t + 2 * tg + 1]));
+                    for (int t = 0; t < NT; t++) raise_to(t, fmaxf(mx0[t], max_s[ow][8 * t + 2 * tg]), fmaxf(mx1[t], max_s[ow][8 * t + 2 * tg + 1]), f);
+                    if (f < 1.0f) {
+                        vfa *= f;
+                        vfb *= f;
+                        set_v_norm_scale(v_norm_scale() * f);
+                    }
                     probabilities(s_acc, vfa, vfb, pb0, pb1, a0, a1);
                     put(mine + turn, pb0, pb1);
                     pair_sync();
@@ -855,6 +894,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 l_s[gg][wg][8 * t + 2 * tg + 1] = l1[t];
             }
         }
+        if (lane == 0) v_s[gg][wg] = p.v_scale * __frcp_rn(v_norm_scale());      // the reciprocal of a power of two
         // The warp's accumulators as rows of PD floats (a pair: half rows, half of the dims each) in its own ring (the copies have landed and
         // been read).  The 16-byte pieces of a row are swapped by the column, which keeps the columns a quarter warp stores at a time in
         // different banks.
@@ -890,8 +930,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             for (int w = 0; w < GW; w += kStep) {
                 const float mw = m_s[gg][w][r];
                 if (mw > kNoMax) {            // a warp without a page has stored nothing
-                    const float c = fast_exp2(mw - mm);
-                    ll += c * (F::kPair ? l_s[gg][w][r] + l_s[gg][w + kStep - 1][r] : l_s[gg][w][r]);
+                    const float cl = fast_exp2(mw - mm), c = cl * v_s[gg][w];
+                    ll += cl * (F::kPair ? l_s[gg][w][r] + l_s[gg][w + kStep - 1][r] : l_s[gg][w][r]);
                     const int other = gg * GW + w + (F::kPair ? lane >> 4 : 0);      // a pair: dims 64 ... are the second warp's
                     const float* row = reinterpret_cast<const float*>(
                                            smem + (other < F::kRingsBelow ? (uint32_t)other * F::kRingBytes
