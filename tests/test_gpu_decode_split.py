@@ -93,6 +93,29 @@ def test_many_rows_of_which_few_hold_tokens(oracle, hq, hkv, d, nq, rows, live, 
             attn.decode_shared(q, cache, bt, full, out)
 
 
+@pytest.mark.parametrize("hq,hkv,d,nq", [(8, 4, 128, 1), (4, 1, 64, 1), (4, 2, 256, 1), (8, 2, 128, 5)])
+@pytest.mark.parametrize("rows", [33, 64, 255, 256, 257, 1023, 1025, 2100])
+def test_batches_around_the_plans_groups(oracle, hq, hkv, d, nq, rows):
+    """Groups of 32 sequences, eight of them loaded at a time, 32 of them remembered; empty groups among them and a long sequence at each end."""
+    rng = np.random.default_rng(rows)
+    lens = rng.integers(0, 60, rows)
+    lens[32 * (rows // 64): 32 * (rows // 64) + 32] = 0
+    lens[0], lens[-1] = 600, 777
+    attn = TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv)
+    case = synthetic.decode_case(seed=rows, seq_lens=lens.tolist(), dtype=torch.float16, heads=(hq, hkv), head_dim=d)
+    cache = torch.zeros(kv_cache_shape(case.num_blocks, 16, hkv, d), dtype=torch.uint8, device=DEV)
+    attn.write(case.k.to(DEV), case.v.to(DEV), cache, case.slot_mapping.to(DEV))
+    q = torch.randn(rows, nq, hq, d, generator=torch.Generator().manual_seed(1)).to(torch.float16)
+    want = oracle.decode_paged(q.float().numpy().reshape(-1, hq, d), cache.cpu().numpy(), np.repeat(case.block_table.numpy(), nq, axis=0),
+                               np.repeat(case.seq_lens.numpy(), nq), attn.signs(DEV).cpu().numpy(), attn.scale)
+    out = torch.full_like(q, float("nan"), device=DEV)
+    attn.decode_shared(q.to(DEV), cache, case.block_table.to(DEV), case.seq_lens.to(DEV), out)
+    assert attn.status(rows, DEV, nq) == 0
+    got = out.float().cpu().numpy()
+    assert (got[lens == 0] == 0).all()
+    assert_attention_close(got.reshape(-1, hq, d), want, f"{rows} rows")
+
+
 def _exact(attn, cache, table, lens, q, causal=False, fp16_operands=False):
     """Attention over the cache's own bytes in 64 bits, in the rotated domain; q [rows, queries, heads, size].  ``fp16_operands``: with
     the queries and centroids rounded as the kernel's, which leaves the rounding of P times the V norm."""

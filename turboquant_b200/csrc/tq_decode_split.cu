@@ -117,9 +117,8 @@ constexpr float kNoMax = -3.402823466e38f;
 // way the maxima are raised: a page whose largest scaled norm exceeds kVNormMost (2^kRaiseThreshold times that is still finite in fp16) lowers the
 // scale until that norm lies in [256, 512), and the accumulators with it; the combine takes the scale out in fp32.  It starts at
 // 16: norms up to 62 never lower it, and those down to fp16's smallest normal number leave P its bits (1 / sqrt(128) in place of
-// it: V rows of norm 1e-3 under 16 ... 32 causal columns had an error of 7 ... 8.7e-4 against 64 bits, now 5.6e-4 as at norm 11, and norms of
-// 16000 and more overflowed).  A lookup in shared memory, a maximum and a comparison a
-// page: 8 x 32768 causal, 8 queries 164.3 -> 165.8 us, 32 ragged sequences 27.9 -> 28.1, head size 64 28.0 -> 28.5.
+// it: V rows of norm 1e-3 under 16 ... 32 causal columns had an error of 7 ... 8.7e-4 against 64 bits, now 4.9e-4 at any norm, and those of 16000
+// and more overflowed).  A lookup in shared memory, a maximum and a comparison a page: 8 x 32768 causal, 8 queries 164.3 -> 165.8 us, 32 ragged sequences 27.9 -> 28.1, head size 64 28.0 -> 28.5.
 constexpr float kVNormMost = 1000.0f, kVScaleStart = 16.0f;
 
 // n / d for 0 <= n < 2^24, d > 0: a reciprocal, then the quotient put right.  (The plan is repeated by every warp, and the compiler's
@@ -144,6 +143,7 @@ struct SplitPlan {
     int np, len;             // the lane's sequence: pages inside the window, tokens up to the window's end
     int vstart, vend;        // its span in the list, in units of pieces or of virtual pages (even)
     int run;                 // end of the span of the last sequence before this batch
+    int ends;                // of many sequences: the list position where the lane's bin of them ends
     int total, workers, head_set;
     int piece;               // pages of a piece at most, 0: the even cut
     bool too_long;           // some sequence is longer than its page table
@@ -185,6 +185,18 @@ __device__ __forceinline__ void split_load(const SplitParams& p, SplitPlan& s, i
     s.vend = run + incl;
 }
 
+// The cut of a work list of `pages` pages in `nonempty` sequences (and, in pieces, the piece and their number).
+template <int NG>
+__device__ __forceinline__ void split_cut_list(const SplitParams& p, SplitPlan& s, int pages, int nonempty, int pieces) {
+    s.head_set = s.piece ? 1 : p.head_set;
+    s.workers = p.grid * (s.head_set == 1 ? NG : s.head_set == 2 ? NG / 2 : NG / 4);
+    s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * p.item_cost);
+    // Every worker of the even cut has a position of the list: one with an empty range would write no partial, and the merge counts
+    // all workers between a head's first and last as its parts.  (A short list is cut too: many sequences of which few hold tokens.)
+    if (!s.piece && s.workers > s.total) s.workers = s.total;
+}
+// Up to kSplitSelf sequences: every warp of both kernels plans for itself, and walks the list a batch of 32 at a time.
+constexpr int kSplitSelf = 64;
 template <int GW, int NG>
 __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, int lane) {
     s.lane = lane;
@@ -209,7 +221,7 @@ __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, i
     const int share = (int)even + (even > (float)(int)even ? 1 : 0);
     s.piece = 0;
     int pieces = 0;
-    for (int t = share < 1 ? 1 : share; t <= share + kSplitSlackTiles && p.batch <= 256; t++) {
+    for (int t = share < 1 ? 1 : share; t <= share + kSplitSlackTiles; t++) {
         const int size = t * GW;
         pieces = __reduce_add_sync(0xffffffffu, split_div_up(np_first, size));
         for (int base = 32; base < p.batch && !s.void_batch; base += 32) {
@@ -223,13 +235,102 @@ __device__ __forceinline__ void split_plan(const SplitParams& p, SplitPlan& s, i
             break;
         }
     }
-    s.head_set = s.piece ? 1 : p.head_set;
-    s.workers = p.grid * (s.head_set == 1 ? NG : s.head_set == 2 ? NG / 2 : NG / 4);
-    s.total = s.piece ? pieces * p.kv_heads : p.head_sets * (pages + nonempty * p.item_cost);
-    // Every worker of the even cut has a position of the list: one with an empty range would write no partial, and the merge counts
-    // all workers between a head's first and last as its parts.  (A short list is cut too: many sequences of which few hold tokens.)
-    if (!s.piece && s.workers > s.total) s.workers = s.total;
+    split_cut_list<NG>(p, s, pages, nonempty, pieces);
     split_load(p, s, 0, 0, true);
+}
+
+// More sequences: the decode kernel's warps load the lengths of 256 at a time and remember where each of up to 32 bins of sequences ends in the list (a
+// bin is one batch of 32, or as many as make 32 bins do), to find their place in one step.  Up to 256 may be cut in pieces (beyond that it measured slower: 512 of 2048
+// tokens, ragged, 8 heads on one 29 -> 41 us).  The merge,
+// whose blocks are more than fit the chip at once, reads this plan from the workspace (words 1 ... 4 and 8 ... 39) after its wait.
+// The plan above costs a warp two trips over the lengths and half of a third one, in every block of the merge too: 8 heads on one, head size 64, 1000
+// sequences of 500 tokens 75 -> 42 us with this one, 2000 of 64 157 -> 52; 64 / 8 heads, 256 ragged ones x 1024 98 -> 56.  At 64
+// sequences and fewer the one above is faster by up to 8 %.
+__device__ __forceinline__ int split_bin(const SplitParams& p) { return (p.batch + 1023) >> 10; }     // batches of 32 in a bin
+
+template <int GW, int NG>
+__device__ __forceinline__ void split_plan_many(const SplitParams& p, SplitPlan& s, int lane) {
+    constexpr int kAhead = 8;
+    s.lane = lane;
+    s.too_long = s.void_batch = false;
+    s.np = s.len = 0;
+    const int span = split_bin(p);
+    int np[kAhead], pages = 0, nonempty = 0, bin_pages = 0, bin_live = 0, bin = 0, in_bin = 0;
+    for (int g0 = 0; 32 * g0 < p.batch; g0 += kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            const int b = 32 * (g0 + u) + lane;
+            int len = 0;
+            np[u] = b < p.batch ? split_pages(p, b, len, s.too_long) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            if (32 * (g0 + u) >= p.batch) break;
+            const int sum = __reduce_add_sync(0xffffffffu, np[u]), live = __popc(__ballot_sync(0xffffffffu, np[u] > 0));
+            if (lane == bin) { bin_pages += sum; bin_live += live; }
+            if (++in_bin == span) { in_bin = 0; bin++; }
+            pages += sum;
+            nonempty += live;
+        }
+    }
+    s.too_long = __any_sync(0xffffffffu, s.too_long);
+    s.void_batch = s.too_long && p.all_or_nothing;
+    if (s.void_batch) {
+        pages = nonempty = bin_pages = bin_live = 0;
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) np[u] = 0;
+    }
+    const int groups = p.grid * NG;
+    const float even = (float)pages * (float)p.kv_heads * p.inv_warps;
+    const int share = (int)even + (even > (float)(int)even ? 1 : 0);
+    s.piece = 0;
+    int pieces = 0, bin_pieces = 0;
+    for (int t = share < 1 ? 1 : share; t <= share + kSplitSlackTiles && p.batch <= 32 * kAhead; t++) {      // np has them all
+        const int size = t * GW;
+        pieces = 0;
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            if (32 * u >= p.batch) break;
+            const int sum = __reduce_add_sync(0xffffffffu, split_div_up(np[u], size));
+            if (lane == u) bin_pieces = sum;
+            pieces += sum;
+        }
+        if (pieces * p.kv_heads <= groups) {
+            s.piece = size;
+            break;
+        }
+    }
+    split_cut_list<NG>(p, s, pages, nonempty, pieces);
+    s.ends = s.piece ? p.kv_heads * bin_pieces : p.head_sets * (bin_pages + bin_live * p.item_cost);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, s.ends, o);
+        if (lane >= o) s.ends += t;
+    }
+}
+// to the first sequences of bin i
+__device__ __forceinline__ void split_jump(const SplitParams& p, SplitPlan& s, int i) {
+    const int before = __shfl_sync(0xffffffffu, s.ends, (i - 1) & 31);
+    split_load(p, s, 32 * split_bin(p) * i, i > 0 ? before : 0, false);
+}
+__device__ __forceinline__ void split_keep_plan(const SplitParams& p, const SplitPlan& s) {
+    if (s.lane == 0) {
+        p.header[1] = s.total;
+        p.header[2] = s.workers;
+        p.header[3] = s.piece;
+        p.header[4] = s.void_batch;
+    }
+    p.header[8 + s.lane] = s.ends;
+}
+__device__ __forceinline__ void split_kept_plan(const SplitParams& p, SplitPlan& s, int lane) {
+    s.lane = lane;
+    s.total = p.header[1];
+    s.workers = p.header[2];
+    s.piece = p.header[3];
+    s.void_batch = p.header[4] != 0;
+    s.ends = p.header[8 + lane];
+    s.head_set = s.piece ? 1 : p.head_set;
+    s.len = 0;
 }
 
 // One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V).  No multicast; x is a
@@ -373,7 +474,8 @@ __device__ __forceinline__ void split_finish(const SplitParams& p, const float* 
     if (p.out_lse && lane == 0) p.out_lse[orow] = lse2 * 0.6931471805599453f;
 }
 
-template <int PD, int NT>
+// MANY: more than kSplitSelf sequences (the plan's registers would spill in the page loop of a kernel that has both)
+template <int PD, int NT, bool MANY>
 __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_kernel(const __grid_constant__ SplitParams p) {
     using F = SplitShape<PD, NT>;
     constexpr int E = F::kE, NG = F::kGroups, GW = F::kGroupWarps;
@@ -390,7 +492,10 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     const int G = p.group;
     if (smem_base + F::kRingsBelow * F::kRingBytes > kLutAddr) {   // the map does not fit
         grid_dependency_wait();
-        if (tid == 0) atomicExch(&p.header[0], 3);
+        if (tid == 0) {
+            p.header[1] = 0;      // no plan for the merge
+            atomicExch(&p.header[0], 3);
+        }
         return;
     }
     uint8_t* const ring = smem + (warp < F::kRingsBelow ? (uint32_t)warp * F::kRingBytes
@@ -431,7 +536,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     grid_launch_dependents();    // the merge may now be scheduled: it reads seq_lens ahead of its own wait
 
     SplitPlan s;
-    split_plan<GW, NG>(p, s, lane);
+    if constexpr (MANY) split_plan_many<GW, NG>(p, s, lane);
+    else split_plan<GW, NG>(p, s, lane);
     if (s.too_long && blockIdx.x == 0 && tid == 0) atomicExch(&p.header[0], kStatusSeqTooLong);
     const int hs = s.head_set;
     const int sub = hs == 1 ? gg : hs == 2 ? gg >> 1 : gg >> 2, hsub = gg - sub * hs;
@@ -444,6 +550,10 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
         pos = split_cut(worker, s.total, s.workers);
         hi = split_cut(worker + 1, s.total, s.workers);
     }
+    if constexpr (MANY) {
+        if (blockIdx.x == 0 && warp == 0) split_keep_plan(p, s);
+        split_jump(p, s, pos < hi ? __ffs(__ballot_sync(0xffffffffu, s.ends > pos)) - 1 : 0);      // a range lies inside the list
+    }
     // the lane's sequence of the plan waits in shared memory while pages are worked on (registers are what the loop is short of)
     auto plan_at = [&]() -> uint8_t* {
         const uint32_t at = F::kPlanAt + (uint32_t)warp * 512u + (uint32_t)lane * 16u;
@@ -451,7 +561,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     };
     *reinterpret_cast<int4*>(plan_at()) = make_int4(s.np, s.len, s.vstart, s.vend);
     const int piece = s.piece;
-    int base = 0;
+    int base = MANY ? s.base : 0;
     const uint32_t lut_lane = split_keep(smem_u32(lut) + 4u * lane);
     const int fp = (int)(p.kv_begin / kPageTokens);
     // this lane's places in a stage: fragment rows g, g + 8 of K are tokens ta, tb
@@ -994,12 +1104,19 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
     for (int i = threadIdx.x; i < PD; i += RW == 16 ? 512 : 128) sign_s[i] = p.signs[i];
     if (RW == 1) __syncthreads();
     SplitPlan s;
-    split_plan<GW, NG>(p, s, lane);     // every decode block is past its wait: the lengths are final
+    const bool many = p.batch > kSplitSelf;
+    if (many) {
+        grid_dependency_wait();
+        split_kept_plan(p, s, lane);
+        split_jump(p, s, b < p.batch ? b / (32 * split_bin(p)) : 0);
+    } else {
+        split_plan<GW, NG>(p, s, lane);     // every decode block is past its wait: the lengths are final
+    }
     while (s.base + 32 <= b && b < p.batch) split_load(p, s, s.base + 32, __shfl_sync(0xffffffffu, s.vend, 31), false);
     const int np = __shfl_sync(0xffffffffu, s.np, (b - s.base) & 31), vstart = __shfl_sync(0xffffffffu, s.vstart, (b - s.base) & 31);
     const int hs = s.head_set, hset = head / hs, hsub = head - hset * hs;
     int first = 0, count = 0;           // workers of this head's parts
-    if (np > 0) {
+    if (np > 0 && s.total > 0) {
         if (s.piece) {
             count = split_div_up(np, s.piece);
             first = vstart + hset * count;
@@ -1009,7 +1126,7 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
             count = (int)((end * s.workers + s.total - 1) / s.total) - first;
         }
     }
-    grid_dependency_wait();
+    if (!many) grid_dependency_wait();
     if (count == 1 || b >= p.batch) return;
     // part i: worker first + i; the first part starts its sequence (odd slot of the worker), the others continue it
     auto slot_row = [&](int i) -> int64_t { return ((int64_t)((first + i) * 2 + (i == 0 ? 1 : 0)) * hs + hsub) * G + r; };
@@ -1110,23 +1227,31 @@ size_t split_workspace_bytes(int columns, int padded, int ctas) {
     return 256 + split_up(rows * sizeof(float)) + split_up(rows * padded * sizeof(float));
 }
 
-template <int PD, int NT>
-static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
+template <int PD, int NT, bool MANY>
+static int launch_split_kernel(const SplitParams& p, cudaStream_t s) {
     using F = SplitShape<PD, NT>;
-    static_assert(F::kGroups <= 4, "split_workspace_bytes counts four groups a block");
     static bool configured[64] = {};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(decode_split_kernel<PD, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::kSmem));
+        TQ_CUDA(cudaFuncSetAttribute(decode_split_kernel<PD, NT, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::kSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
+    TQ_CUDA(launch_serialized(decode_split_kernel<PD, NT, MANY>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
+    return TQ_OK;
+}
+
+template <int PD, int NT>
+static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
+    using F = SplitShape<PD, NT>;
+    static_assert(F::kGroups <= 4, "split_workspace_bytes counts four groups a block");
     p.grid = ctas;
     p.head_set = F::kGroups == 4 && p.kv_heads % 4 == 0 ? 4 : p.kv_heads % 2 == 0 ? 2 : 1;
     p.head_sets = p.kv_heads / p.head_set;
     p.item_cost = F::kItemCost;
     p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
-    TQ_CUDA(launch_serialized(decode_split_kernel<PD, NT>, dim3((unsigned)p.grid), dim3(F::kThreads), F::kSmem, s, p));
+    const int rc = p.batch > kSplitSelf ? launch_split_kernel<PD, NT, true>(p, s) : launch_split_kernel<PD, NT, false>(p, s);
+    if (rc != TQ_OK) return rc;
     if (cudaEvent_t mid = decode_event(1)) TQ_CUDA(cudaEventRecord(mid, s));
     // A head has about groups / (sequences x heads) parts at most: a warp fetches eight at a time, so up to eight go to one warp
     // (a block takes four rows), more to four or sixteen warps.
