@@ -183,3 +183,23 @@ def test_v_norms_of_many_sizes_in_a_sequence(hq, hkv, d, nq, order):
     v_scale = torch.cat([size(torch.arange(n, device=DEV) / n) for n in lens])[:, None, None]
     attn = TurboQuantPagedAttention(hq, d, 1.0 / math.sqrt(d), hkv)
     assert _error(attn, nq, lens, v_scale, q_scale=3.0, fp16_operands=True) <= 2.0 ** -11
+
+
+@pytest.mark.parametrize("heads,rows", [(16, 47), (16, 48), (32, 511), (32, 512), (48, 512)])
+def test_one_column_on_either_side_of_its_route(oracle, heads, rows):
+    """One query head per KV head on 16 KV heads or launches of 16: many rows go to the streaming kernel.  Bounds: 1.15 times the error of fp16
+    operands and products (4.9e-4, see above) and of the fp16 output (2^-11 / sqrt(3)) over all rows; five times that for the worst head of a row."""
+    lens = (np.arange(rows) * 7 % 40).tolist()
+    attn = TurboQuantPagedAttention(heads, 128, 1.0 / math.sqrt(128), heads)
+    case = synthetic.decode_case(seed=rows, seq_lens=lens, dtype=torch.float16, heads=(heads, heads), head_dim=128)
+    cache = torch.zeros(kv_cache_shape(case.num_blocks, 16, heads, 128), dtype=torch.uint8, device=DEV)
+    attn.write(case.k.to(DEV), case.v.to(DEV), cache, case.slot_mapping.to(DEV))
+    want = oracle.decode_paged(case.q.float().numpy(), cache.cpu().numpy(), case.block_table.numpy(), case.seq_lens.numpy(), attn.signs(DEV).cpu().numpy(),
+                               attn.scale)
+    out = attn.decode(case.q.to(DEV), cache, case.block_table.to(DEV), case.seq_lens.to(DEV))
+    assert attn.status(rows, DEV) == 0
+    err = np.linalg.norm(out.float().cpu().numpy() - want, axis=-1)
+    size = np.linalg.norm(want, axis=-1)
+    assert np.linalg.norm(err) <= 6.5e-4 * np.linalg.norm(size)
+    assert (err <= 5 * 6.5e-4 * size).all()
+    assert (out.cpu().numpy()[np.array(lens) == 0] == 0).all()

@@ -924,8 +924,13 @@ static int largest_chunk(int num_kv_heads) { return single_launch(num_kv_heads) 
 // ragged 632 / 276, 681 / 382, 710 / 475, one sequence of 1048576 with 32 columns 548 / 535: split at every size.
 // Up to four columns on 8 KV heads the two differ by 5 % either way from 65536 on (N(0, 1) keys and values, eager calls: 8 x 32768 82 / 86,
 // 64 ragged x 131072 560 / 605): streaming.  Five to eight: 40 / 8 heads 8 x 32768 80 / 72, 64 x 65536 ragged 146 / 114: split.
-static int64_t split_limit(int num_kv_heads, int columns) {
+// One column on 16 KV heads (or launches of 16): a page of all heads fills the streaming kernel's block, and the split kernel starts each head of many
+// short sequences by itself.  16 / 16 heads 64 x 200 23 / 25, 128 x 200 33 / 40, 512 x 64 73 / 79, but 32 x 200 18 / 13; 32 / 32 heads 512 x 16 117 / 131,
+// 2000 x 64 511 / 566, but 256 x 64 82 / 77.  Four columns: split (64 / 16 heads 128 x 200 59 / 44, 512 x 64 166 / 92).  8192 pages are at most 57
+// sequences a block: the streaming kernel's list holds 96.
+static int64_t split_limit(int num_kv_heads, int columns, int64_t batch, int64_t max_pages) {
     if (columns > 8) return INT64_MAX;
+    if (columns == 1 && num_kv_heads % 16 == 0 && batch >= (num_kv_heads == 16 ? 48 : 512) && batch * max_pages <= 8192) return 0;
     if (num_kv_heads == 16) return 32768;
     return num_kv_heads == 8 && columns <= 4 ? 65536 : INT64_MAX;
 }
@@ -1029,7 +1034,7 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
     TQ_REQUIRE(workspace_bytes >= w.total, TQ_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, w.total);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    if (num_ctas == 0 && !page_indptr && ((wide && cols <= 8) || (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, cols))) {
+    if (num_ctas == 0 && !page_indptr && ((wide && cols <= 8) || (int64_t)batch * max_pages * num_kv_heads <= split_limit(num_kv_heads, cols, batch, max_pages))) {
         auto split = [&](void* o, int o_dtype, float* lse, int rotated) {
             return split_decode(q, q_dtype, batch, nq, real_q_heads, num_kv_heads, head_dim, kHeadDim, kv_cache, num_blocks, slot_bytes,
                                 page_indices, page_indptr, max_pages, seq_lens, kv_begin, kv_end, signs, sm_scale, workspace, workspace_bytes,
