@@ -45,7 +45,8 @@ enum {
     TQ_WRITE_ZERO_PAD = 1, /* also store zeros to the pad bytes after the norms (the reference leaves them alone) */
     TQ_WRITE_EXACT_PATH = 2, /* always run the kernel that evaluates the reference's arithmetic for every element
                                 (default: large writes of 16-bit rows take the tensor-core kernel, which produces
-                                the same bytes and re-derives only the codes next to a boundary that way) */
+                                the same bytes and re-derives only the codes next to a boundary that way, and
+                                writes of up to 2048 rows a kernel with a warp per row) */
     TQ_WRITE_TENSOR_PATH = 4 /* always run the tensor-core kernel (fp16 / bf16 rows of 128 elements only) */
 };
 

@@ -144,3 +144,33 @@ def test_fwht_api(golden):
     np.testing.assert_array_equal(_cabi.fwht(x, 128, 128).cpu().numpy(), golden["fwht_out"])
     kat = _cabi.fwht(torch.tensor([1.0, 0, 0, 0], device=DEV), 4, 4)
     np.testing.assert_array_equal(kat.cpu().numpy(), np.full(4, 0.5, np.float32))
+
+
+@pytest.mark.parametrize("path", ["auto", "exact"])                     # a warp per row (small writes), and the kernel of large fp32 / 96-wide ones
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,H", [(1, 1), (7, 8), (33, 3), (95, 8), (64, 16)])
+def test_special_rows_on_either_small_write(oracle, golden, path, dtype, T, H):
+    """Zero, one-hot, tie, huge, tiny, inf and NaN rows, strided tokens, skipped slots, pad bytes kept or zeroed, and row counts that leave
+    a part of a tile: both kernels write the oracle's bytes and no others."""
+    gen = torch.Generator().manual_seed(T + H)
+    rows = torch.from_numpy(golden["q_rows"])
+    pick = torch.cat([torch.randperm(len(rows), generator=gen) for _ in range(1 + 2 * T * H // len(rows))])[: 2 * T * H]
+    both = rows[pick].reshape(T, 2 * H, 128).to(dtype)                  # K and V of a token side by side: strided tokens
+    k, v = both[:, :H], both[:, H:]
+    nb = T // 16 + 2
+    slots = torch.randperm(nb * 16, generator=gen)[:T]
+    slots[::9] = -1
+    signs = synthetic.make_signs(128, 7)
+    want = np.full((2, nb, 16, H, 80), 0xEE, np.uint8)
+    oracle.write_kv_cache(want, k.float().contiguous().numpy(), v.float().contiguous().numpy(), signs.numpy(), slots.numpy(), 128)
+    both = both.to(DEV)
+    for zero_pad in (False, True):
+        cache = torch.full((2, nb, 16, H, 80), 0xEE, dtype=torch.uint8, device=DEV)
+        _cabi.write_kv_cache(cache, both[:, :H], both[:, H:], signs.to(DEV), slots.to(DEV), 128, zero_pad=zero_pad, path=path)
+        got = cache.cpu().numpy()
+        np.testing.assert_array_equal(got[..., :64], want[..., :64])
+        np.testing.assert_array_equal(got[..., 64:68].copy().view(np.float16), want[..., 64:68].copy().view(np.float16))      # any NaN is one
+        pad = got.reshape(2, -1, H, 80)[..., 68:]
+        written = np.zeros(nb * 16, bool)
+        written[slots[slots >= 0].numpy()] = True
+        assert (pad[:, written] == (0 if zero_pad else 0xEE)).all() and (pad[:, ~written] == 0xEE).all()

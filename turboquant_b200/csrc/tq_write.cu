@@ -1009,7 +1009,7 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
     TQ_REQUIRE(((uintptr_t)kv_cache % 16) == 0, TQ_ERR_INVALID, "kv_cache must be 16-byte aligned");
 
     // A decode step's new tokens (a few rows per SM at most): a warp per row.  The limit is where it stops being the faster one.
-    if ((flags & TQ_WRITE_TENSOR_PATH) == 0 && 2 * num_tokens * num_kv_heads <= 2048)
+    if ((flags & (TQ_WRITE_EXACT_PATH | TQ_WRITE_TENSOR_PATH)) == 0 && 2 * num_tokens * num_kv_heads <= 2048)
         return generic_write(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, key, value, in_dtype, num_tokens, k_token_stride,
                              v_token_stride, signs, slot_mapping, slot_dtype, head_dim, flags, stream);
 
