@@ -159,10 +159,10 @@ int tq_decode_paged(const void* q, int q_dtype, int batch, int num_q_heads, int 
  * rows): q and out are [batch][queries_per_seq][num_q_heads][head_dim], out_lse
  * [batch][queries_per_seq][num_q_heads]; seq_lens and the page table are per sequence.  The
  * queries ride in the columns of one query tile, so the KV is streamed and dequantized once for
- * all of them.  queries_per_seq x (num_q_heads / num_kv_heads) <= 8 takes the 8-wide tile of the
- * mma.sync kernel; 9 ... 32 columns take the wide-tile kernel (tcgen05.mma, accumulators in tensor
- * memory), which needs head_dim 128 or 96 and 2, 4, 8 or 16 KV heads and ignores num_ctas below the
- * number of KV-head pairs.  Other head sizes (33 ... 256) take up to 8 columns.
+ * all of them.  queries_per_seq x (num_q_heads / num_kv_heads) columns: up to 8 on any geometry, up
+ * to 32 with head_dim 128 or 96 and 2, 4, 8 or 16 KV heads.  With num_ctas = 0 and a dense page table the kernel
+ * split by KV head takes more than 8; with a grid or a CSR table the tcgen05 kernel does (accumulators in
+ * tensor memory), which ignores num_ctas below the number of KV-head pairs.
  * The workspace is sized with tq_decode_workspace_bytes(batch, queries_per_seq * num_q_heads, ...).
  * kv_begin / kv_end restrict the tokens as in tq_decode_paged_partial (0, -1: all of them);
  * rotated_partial != 0 makes out (fp32) and out_lse (required) the rotated-domain partial and
@@ -183,7 +183,7 @@ int tq_decode_paged_multi(const void* q, int q_dtype, int batch, int queries_per
  * seq_len - (queries_per_seq - 1 - i) tokens.  This is a chunk of a prefill that continues over the
  * quantized cache, or the verification step of speculative decoding, in one pass over the KV for
  * up to 32 / (num_q_heads / num_kv_heads) query tokens; a longer chunk is several batch rows that
- * share the page table and differ in seq_lens.  Always the wide-tile kernel: head_dim 128 or 96,
+ * share the page table and differ in seq_lens.  head_dim 128 or 96,
  * 2, 4, 8 or 16 KV heads, whole sequences.  A query without a visible token gets zeros and LSE -inf.
  * The reference's prefill does not read the cache at all (turboquant/vllm_backend_fused.py:336-369:
  * FlashAttention over the fresh K / V only), so a chunk after the first one is wrong there; its

@@ -285,7 +285,7 @@ def test_vllm_backend_pure_first_chunks_use_fresh_kv(oracle, golden):
 @pytest.mark.parametrize("with_builder_facts", [False, True])
 def test_vllm_backend_short_chunks_attend_the_quantized_cache(oracle, golden, with_builder_facts):
     """Rows with two to eight new tokens over cached context (short continuation chunks, speculative
-    verification) go through the causal wide-tile kernel, next to decode rows, a longer chunk and a
+    verification) go through the causal kernel, next to decode rows, a longer chunk and a
     first chunk; one of them has fewer cached tokens than pad queries."""
     _backend_step(oracle, golden, [500, 3, 37, 1200, 0, 64], [1, 6, 3, 12, 2, 8], with_builder_facts)
 
@@ -293,7 +293,7 @@ def test_vllm_backend_short_chunks_attend_the_quantized_cache(oracle, golden, wi
 @pytest.mark.parametrize("heads,d", [((64, 8), 128), ((16, 8), 64), ((8, 1), 128)])
 @pytest.mark.parametrize("with_builder_facts", [False, True])
 def test_vllm_backend_short_chunks_without_the_causal_kernel(oracle, golden, with_builder_facts, heads, d):
-    """Geometries the causal wide-tile kernel does not take (eight query heads per KV head, head size 64, one KV
+    """Geometries the causal kernel does not take (eight query heads per KV head, head size 64, one KV
     head): rows with two to eight new tokens go the dense way, decode rows still ride the paged kernel, and the
     dense buffer is sized for them."""
     _backend_step(oracle, golden, [500, 3, 37, 300, 0, 64], [1, 6, 3, 12, 2, 8], with_builder_facts, heads=heads, d=d)

@@ -260,7 +260,7 @@ def test_config4_full_size_vs_oracle(oracle, golden):
     print(f"config 4 full size: max-abs {max_abs:.3e}, relative {rel:.3e}")
 
 
-# the last five go through the wide-tile (tensor-memory) kernel: 9 to 32 query columns per KV head
+# the last five are wide: 9 to 32 query columns per KV head.  At the default grid they take the kernel split by KV head, with a grid the tensor-memory one.
 @pytest.mark.parametrize("nq,hq,hkv", [(2, 32, 8), (8, 8, 8), (3, 8, 4), (4, 4, 2), (1, 32, 8),
                                        (8, 32, 8), (3, 32, 8), (5, 8, 4), (16, 4, 2), (9, 16, 16)])
 def test_shared_kv_queries_match_repeated_rows(oracle, golden, nq, hq, hkv):
@@ -352,8 +352,8 @@ def test_causal_chunk_as_rows_sharing_a_page_table(oracle, golden):
 
 
 def test_wide_tile_csr_table_and_kv_windows(oracle, golden):
-    """The wide-tile kernel (8 queries x GQA 4 = 32 columns) with a CSR page table, and as
-    rotated partials over KV windows merged by tq_merge_rotated (the multi-GPU contract)."""
+    """8 queries x GQA 4 = 32 columns with a CSR page table (the tensor-memory kernel), and as rotated partials over KV
+    windows of a dense one (the kernel split by KV head) merged by tq_merge_rotated (the multi-GPU contract)."""
     lens = [1500, 90, 0, 300]
     B, nq, hq = len(lens), 8, 32
     case = synthetic.decode_case(seed=61, seq_lens=lens, dtype=torch.bfloat16)
@@ -395,7 +395,7 @@ def test_wide_tile_csr_table_and_kv_windows(oracle, golden):
 
 def test_wide_tile_many_short_sequences(oracle, golden):
     """120 short sequences (empty ones among them) with 8 shared-KV queries each: many segments per
-    thread block in the wide-tile kernel, plain and causal."""
+    thread block, plain and causal, in both kernels that take wide queries."""
     rng = np.random.default_rng(11)
     lens = [int(x) for x in rng.integers(0, 150, size=120)]
     B, nq, hq = len(lens), 8, 32

@@ -27,7 +27,7 @@ CASES = {
     "odd_heads": (12, 6, 128, [700, 80, 5]),                            # head sets of two (padded head size 128 of another slot is below)
     "three_heads": (6, 3, 64, [700, 80, 5]),
     "many_heads": (32, 32, 128, [333, 90]),
-    "many_sequences": (8, 4, 128, [20] * 300),                          # beyond what the piece search looks at
+    "many_sequences": (8, 4, 128, [20] * 300),                          # always cut evenly
     "head_96": (32, 8, 96, [100, 777]),
     "head_64": (16, 8, 64, [1500, 31, 0, 640]),
     "head_64_even": (16, 8, 64, [4000, 100, 100, 2000] * 8),

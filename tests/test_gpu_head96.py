@@ -80,7 +80,7 @@ def test_decode_and_dequant_head96(oracle, golden, heads):
 
 
 def test_wide_tile_and_causal_queries_head96(oracle, golden):
-    """Head size 96 through the wide-tile kernel: 8 shared-KV queries and 5 causal ones."""
+    """Wide queries at head size 96: 8 shared-KV queries and 5 causal ones."""
     lens = [700, 0, 33, 2049]
     heads = (32, 8)
     case = _case(8, lens, heads)

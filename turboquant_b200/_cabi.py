@@ -265,7 +265,7 @@ def _decode_args(q, kv_cache, page_indices, page_indptr, max_pages, seq_lens, si
 
 def decode_max_queries_per_seq(num_q_heads: int, num_kv_heads: int, head_size: int = 128) -> int:
     """How many decode queries that share one sequence's KV fit one pass of ``decode_paged_multi``:
-    the wide-tile kernel (up to ``tq_decode_max_query_columns()`` columns) takes 2, 4, 8 or 16 KV heads at head
+    wide queries (up to ``tq_decode_max_query_columns()`` columns) take 2, 4, 8 or 16 KV heads at head
     size 128 / 96; any other KV-head count or head size keeps the 8 columns of the mma.sync kernels."""
     wide = num_kv_heads in (2, 4, 8, 16) and head_size in (128, 96)
     cols = int(lib().tq_decode_max_query_columns()) if wide else 8
@@ -321,7 +321,7 @@ def decode_paged_multi(q, kv_cache, page_indices, seq_lens, signs, sm_scale: flo
                        page_indptr=None, max_pages: int | None = None, out_lse=None, num_ctas: int = 0,
                        kv_begin: int = 0, kv_end: int = -1, rotated_partial: bool = False):
     """One decode step for sequences that carry several queries sharing their KV: ``q`` and ``out``
-    are [batch, queries, Hq, D], ``out_lse`` fp32 [batch, queries, Hq]; queries x (Hq / H) <= 32 (more than 8: the wide-tile kernel).
+    are [batch, queries, Hq, D], ``out_lse`` fp32 [batch, queries, Hq]; queries x (Hq / H) <= 32.
     The workspace is sized for queries x Hq heads.  ``rotated_partial``: fp32 rotated-domain
     partial + base-2 LSE over tokens [kv_begin, kv_end), as ``decode_paged_partial``."""
     if max_pages is None:

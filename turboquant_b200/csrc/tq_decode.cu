@@ -1007,9 +1007,10 @@ static int decode_common(const void* q, int q_dtype, int batch, int nq, int real
                "the kernel-side exchange takes at most 16 KV heads per GPU, got %d", num_kv_heads);
     TQ_REQUIRE(nq >= 1 && real_q_heads >= 1 && real_q_heads % num_kv_heads == 0, TQ_ERR_INVALID,
                "query heads must be a positive multiple of the KV heads, queries_per_seq >= 1");
-    // up to 8 query columns per KV head: the mma.sync kernel; up to 32: the tcgen05 kernel
+    // Calls that set their grid or pass a CSR table: up to 8 query columns per KV head the streaming kernel, up to 32 the tcgen05 kernel; the others
+    // as split_limit says.
     const int cols = nq * (real_q_heads / num_kv_heads);
-    // (causal queries always take the wide-tile kernel: it masks per column)
+    // (causal queries count as wide: the streaming kernel has no mask per column)
     const bool wide = cols > 8 || causal;
     TQ_REQUIRE(!causal || (mq_applicable(num_kv_heads, cols < 9 ? 9 : cols) && !x && kv_begin == 0 && kv_end < 0 && !emit_rotated),
                TQ_ERR_UNSUPPORTED, "causal queries: queries_per_seq x query heads per KV head up to 32, 2, 4, 8 or 16 KV heads, "

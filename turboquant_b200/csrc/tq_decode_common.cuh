@@ -1,5 +1,4 @@
-// Pieces shared by the decode kernels (the mma.sync kernel for up to 8 query columns per KV head
-// and the tcgen05 kernel for wider query tiles): geometry constants, the launch parameters, the
+// Pieces shared by the decode kernels (streaming, split by KV head, tcgen05): geometry constants, the launch parameters, the
 // device-side helpers for the page window of a sequence and for the lookup-table dequantizer.
 #pragma once
 

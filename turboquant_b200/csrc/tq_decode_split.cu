@@ -52,7 +52,7 @@ struct SplitShape {
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
-    static constexpr int kGroups = kPair ? (NT == 2 ? 4 : 2) : 4, kGroupWarps = kPair ? (NT == 2 ? 4 : 6) : NT == 2 ? 3 : PD == 64 ? 5 : PD == 128 ? 4 : 3;
+    static constexpr int kGroups = kPair ? 2 : 4, kGroupWarps = kPair ? 6 : NT == 2 ? 3 : PD == 64 ? 5 : PD == 128 ? 4 : 3;
     // query fragments kept in registers; the other tiles' are read from shared memory on every page (16 wavefronts a tile beside the
     // page's 64 lookups; in registers they spill: 8 queries 181 -> 185 us with one tile, 234 with two)
     static constexpr int kRegTiles = NT == 4 ? 0 : NT == 3 ? 2 : NT;
@@ -1262,8 +1262,7 @@ static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
     return TQ_OK;
 }
 
-// The caller has checked pointers, types and geometry: 16-byte slots, padded head size 64 / 128 / 256, up to 8 query
-// columns per KV head.
+// The caller has checked pointers, types and geometry: slots a multiple of 16 bytes, padded head size 64 / 128 / 256.
 int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads, int num_kv_heads, int head_dim, int padded,
                  const void* kv_cache, int64_t num_blocks, int slot_bytes, const int32_t* page_indices, const int32_t* page_indptr,
                  int max_pages, const int32_t* seq_lens, int64_t kv_begin, int64_t kv_end, const float* signs, float sm_scale,

@@ -97,7 +97,7 @@ class TurboQuantMetadataBuilder(FlashAttentionMetadataBuilder):
 
 # Rows with cached context and at most this many new tokens (a short continuation chunk, the
 # verification step of speculative decoding) attend over the quantized cache in one pass of the
-# causal wide-tile decode kernel instead of a dequantized dense copy of their whole context.
+# causal decode kernel instead of a dequantized dense copy of their whole context.
 FUSED_CHUNK_MAX = 8
 
 
@@ -131,7 +131,7 @@ def step_shape(common):
 
 
 def causal_chunk_supported(num_heads: int, num_kv_heads: int, head_size: int) -> bool:
-    """Whether FUSED_CHUNK_MAX causal queries of a row fit one pass of the wide-tile decode kernel: head size
+    """Whether FUSED_CHUNK_MAX causal queries of a row fit one pass of the causal decode kernel: head size
     128 or 96, 2 / 4 / 8 / 16 KV heads, and FUSED_CHUNK_MAX x (query heads per KV head) within its 32 columns."""
     from . import _cabi
     if head_size not in (128, 96) or num_kv_heads not in (2, 4, 8, 16):
@@ -220,11 +220,11 @@ class TurboQuantFusedImpl(FlashAttentionImpl):
           the quantized cache: all rows are handed to it with the length of every other row set
           to zero, and their outputs are dropped.
         * Rows with cached context and 2 ... FUSED_CHUNK_MAX new tokens run through the causal
-          wide-tile decode kernel: their tokens are already in the cache, the row's queries are
+          decode kernel: their tokens are already in the cache, the row's queries are
           padded at the front to FUSED_CHUNK_MAX (a pad query sees fewer tokens than the first real
           one and its output is dropped), every other row has length zero there.  Geometries without that
           kernel (``causal_chunk_supported``: other head sizes, more than four query heads per KV head, KV
-          head counts the wide tile does not take) send these rows the dense way below.
+          head counts wide queries do not take) send these rows the dense way below.
         * Every other row b contributes ``seq_lens[b]`` keys to a dense varlen K/V: its cached
           tokens, dequantized from the cache, then the chunk's own fresh K/V (the chunk is already
           in the cache as well, quantized; its fresh values are used, as a first chunk would).  The
