@@ -64,6 +64,7 @@ struct SplitShape {
     // 99 / 106 / 110; 24 columns 16 / 32 / 40 / 60: 214 / 148 / 130 / 136; 32 columns 32 / 40 / 60 / 80: 184 / 164 / 158 / 170; head size
     // 64, 6 / 10 / 16: 76 / 61 / 50 (but 16 x 8192 uniform 35 / 35 / 43); 256, 6 / 10 / 16: 127 / 102 / 104.
     static constexpr int kItemCost = PD != 128 ? 10 : NT == 1 ? 20 : NT < 4 ? 40 : 60;
+    static constexpr bool kNormScale = NT > 1 || PD == 256;      // see kVNormMost
     // What the warps of a pair hand each other: the probabilities of a page as fragments, two pages' worth in turn.
     static constexpr int kHandBytes = kPair ? (NT + 1) / 2 * 512 : 0, kHandAt = (kWarps - kRingsBelow) * kRingBytes;
     static constexpr size_t kSmem = kLutAddr + kLutSpan + (size_t)kHandAt + 2 * kWarps * kHandBytes - 1024;   // from offset 1024 (the system's part): ample
@@ -113,12 +114,14 @@ struct SplitParams {
 constexpr int kSplitSlackTiles = 3;
 // The running maximum before any score: finite, so that a column whose tokens are all masked so far has exp2(-inf - m) = 0.
 constexpr float kNoMax = -3.402823466e38f;
-// P times the V norm is rounded to fp16 as the MMA's operand.  Norms are any fp16 value, so each warp scales them by a power of two, the
-// way the maxima are raised: a page whose largest scaled norm exceeds kVNormMost (2^kRaiseThreshold times that is still finite in fp16) lowers the
-// scale until that norm lies in [256, 512), and the accumulators with it; the combine takes the scale out in fp32.  It starts at
-// 16: norms up to 62 never lower it, and those down to fp16's smallest normal number leave P its bits (1 / sqrt(128) in place of
-// it: V rows of norm 1e-3 under 16 ... 32 causal columns had an error of 7 ... 8.7e-4 against 64 bits, now 4.9e-4 at any norm, and those of 16000
-// and more overflowed).  A lookup in shared memory, a maximum and a comparison a page: 8 x 32768 causal, 8 queries 164.3 -> 165.8 us, 32 ragged sequences 27.9 -> 28.1, head size 64 28.0 -> 28.5.
+// P times the V norm is rounded to fp16 as the MMA's operand; 1 / sqrt(128) is taken out in fp32 at the combine (ahead of the rounding it cost V rows of
+// norm 1e-3 under 16 ... 32 causal columns 7 ... 8.7e-4 of error against 64 bits, now 4.9e-4 at any norm).  Norms are any fp16 value; a
+// page whose largest exceeds kVNormMost (2^kRaiseThreshold times that is still finite in fp16) would overflow.
+//   One column tile of padded size 64 / 128: that page's norms are brought to [256, 512) and the accumulators scaled down and up again around
+//   it, so that other pages pay a maximum and a comparison (head size 64, 22 x 14327: 67 us as with a fixed scale, 75 with the one below).
+//   Else: the warp keeps a power of two for the norms, 16 at first, and lowers it with the accumulators; a word in shared memory, for a register
+//   more spills, and so does the code of the other form (8 x 32768 causal, 8 queries 162.6 us with a fixed scale, 163.2 so, 166 the other
+//   way; one sequence of 1048576 567 / 577 / 587; head size 256, 1 x 1917 13.0 / 13.3 / 13.4).
 constexpr float kVNormMost = 1000.0f, kVScaleStart = 16.0f;
 
 // n / d for 0 <= n < 2^24, d > 0: a reciprocal, then the quotient put right.  (The plan is repeated by every warp, and the compiler's
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     __shared__ float sign_s[PD];
     __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols + 1];  // a pair's maxima of a page that raises them (and its largest V norm), and whether it does
     __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
-    __shared__ uint64_t full_s[F::kWarps][F::kStages + 1];           // a stage's two boxes have landed; and a word for the warp's scale of the V norms
+    __shared__ uint64_t full_s[F::kWarps][F::kStages + F::kNormScale];   // a stage's two boxes have landed; and a word for the warp's scale of the V norms
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -677,10 +680,12 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             split_load_row<E>(p.q, p.q_dtype, q_row(r), p.head_dim, lane * E, qv[0]);
             put_q(r, qv[0]);
         }
-        // in shared memory: a register more spills
-        auto v_norm_scale = [&]() -> float { return __uint_as_float(lds32(full_at + 8 * F::kStages)); };
+        auto v_norm_scale = [&]() -> float {
+            if constexpr (F::kNormScale) return __uint_as_float(lds32(full_at + 8 * F::kStages));
+            else return 1.0f;
+        };
         auto set_v_norm_scale = [&](float v) {
-            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(full_at + 8 * F::kStages), "r"(__float_as_uint(v)) : "memory");
+            if (F::kNormScale && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(full_at + 8 * F::kStages), "r"(__float_as_uint(v)) : "memory");
         };
         set_v_norm_scale(kVScaleStart);
         group_sync();
@@ -800,6 +805,15 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
             return v;
         };
         auto norm_factor = [](float v) { return v > kVNormMost ? __uint_as_float((127 + 8 + 127 - (__float_as_uint(v) >> 23)) << 23) : 1.0f; };
+        auto power_inverse = [](float f) { return __uint_as_float(0x7f000000u - __float_as_uint(f)); };      // of a power of two
+        auto scale_sums = [&](float f) {
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int i = 0; i < kAccTiles; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) o_acc[t][i][j] *= f;
+        };
         auto raise_to = [&](int t, float mx0, float mx1, float f) {
             const bool raise0 = mx0 > m0[t] + kRaiseThreshold, raise1 = mx1 > m1[t] + kRaiseThreshold;
             const float c0 = raise0 ? fast_exp2(m0[t] - mx0) : 1.0f, c1 = raise1 ? fast_exp2(m1[t] - mx1) : 1.0f;
@@ -893,9 +907,22 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                     for (int t = 0; t < NT; t++) {
                         float mx0, mx1;
                         page_max(s_acc[t], mx0, mx1);
-                        raise_to(t, mx0, mx1, f);
+                        raise_to(t, mx0, mx1, F::kNormScale ? f : 1.0f);
                     }
-                    if (f < 1.0f) {
+                    if constexpr (!F::kNormScale) {
+                        if (f < 1.0f) {
+                            probabilities(s_acc, vfa * f, vfb * f, pb0, pb1, a0, a1);
+                            scale_sums(f);
+#pragma unroll
+                            for (int w = 0; w < F::kVBytes / 4; w++) accumulate(w, v0[w], v1[w], v2[w], v3[w], pb0, pb1);
+                            scale_sums(power_inverse(f));
+                            l0[0] += a0[0];
+                            l1[0] += a1[0];
+                            __syncwarp();
+                            next_stage();
+                            continue;
+                        }
+                    } else if (f < 1.0f) {
                         vfa *= f;
                         vfb *= f;
                         set_v_norm_scale(v_norm_scale() * f);
@@ -1004,7 +1031,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 l_s[gg][wg][8 * t + 2 * tg + 1] = l1[t];
             }
         }
-        if (lane == 0) v_s[gg][wg] = p.v_scale * __frcp_rn(v_norm_scale());      // the reciprocal of a power of two
+        if (lane == 0) v_s[gg][wg] = p.v_scale * power_inverse(v_norm_scale());
         // The warp's accumulators as rows of PD floats (a pair: half rows, half of the dims each) in its own ring (the copies have landed and
         // been read).  The 16-byte pieces of a row are swapped by the column, which keeps the columns a quarter warp stores at a time in
         // different banks.
