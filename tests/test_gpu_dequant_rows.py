@@ -1,0 +1,97 @@
+"""Bulk dequantization at the edges of its units of work: 16 or 32 rows of a page, K rows before V rows, in the kernel of small jobs and (behind a
+wide page table) in that of large ones.  fp32 output equals the oracle bit for bit, 16-bit output is its rounding."""
+import numpy as np
+import pytest
+import torch
+
+from turboquant_b200 import _cabi, synthetic
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+LENS = [0, 1, 15, 16, 17, 33, 160, 0, 97]
+SLOT = {64: 48, 96: 80, 128: 80, 256: 144}
+
+
+def _cache(rng, pages, block, heads, dim, slot):
+    """Random codes, finite fp16 norms."""
+    cache = rng.integers(0, 256, (2, pages, block, heads, slot), dtype=np.uint8)
+    padded = 1 << (dim - 1).bit_length()
+    norms = rng.uniform(0.0, 20.0, cache.shape[:-1]).astype(np.float16)
+    cache[..., padded // 2:padded // 2 + 2] = norms[..., None].view(np.uint8)
+    return cache
+
+
+def _want(oracle, cache, table, lens, signs, dim):
+    block = cache.shape[2]
+    slot = SLOT[dim]
+    rows = []
+    for which in range(2):
+        parts = []
+        for b, n in enumerate(lens):
+            t = np.arange(n)
+            got = np.ascontiguousarray(cache[which, table[b, t // block], t % block][..., :slot])
+            parts.append(oracle.dequant_cache_rows(got, signs, dim).reshape(n, cache.shape[3], dim))
+        rows.append(np.concatenate(parts))
+    return rows
+
+
+def _check(oracle, dim, heads, *, wide, block=16, slot=None, strided=False, listed=False, lens=LENS):
+    rng = np.random.default_rng(dim + heads + block)
+    slot = slot or SLOT[dim]
+    signs = synthetic.make_signs(1 << (dim - 1).bit_length(), 42)
+    need = max((n + block - 1) // block for n in lens)
+    pages = sum((n + block - 1) // block for n in lens) + 2
+    cache = _cache(rng, pages, block, heads, dim, slot)
+    order, at = rng.permutation(pages), 0
+    units = 2 * heads * block // 32 + 1
+    width = need if not wide else max(need, 24 * 160 // (len(lens) * units) * units + 4000 // units)      # beyond the small jobs' bound
+    table = np.zeros((len(lens), width), np.int32)
+    for b, n in enumerate(lens):
+        k = (n + block - 1) // block
+        table[b, :k] = order[at:at + k]
+        at += k
+    want = _want(oracle, cache, table, lens, signs.numpy(), dim)
+    total = sum(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=DEV)
+    extra = {}
+    pages_arg = torch.from_numpy(table).to(DEV)
+    if listed:
+        per = [(n + block - 1) // block for n in lens]
+        pages_arg = torch.from_numpy(np.concatenate([table[b, :k] for b, k in enumerate(per)])).to(DEV)
+        extra = dict(page_indptr=torch.tensor(np.concatenate([[0], np.cumsum(per)]), dtype=torch.int32, device=DEV), max_pages=width)
+    for dtype in (torch.float32, torch.bfloat16, torch.float16):
+        if strided:
+            both = torch.full((total + 1, 2, heads, dim), 7.0, dtype=dtype, device=DEV)
+            k, v = both[:total, 0], both[:total, 1]
+        else:
+            both = torch.full((2, total + 1, heads, dim), 7.0, dtype=dtype, device=DEV)
+            k, v = both[0, :total], both[1, :total]
+        _cabi.dequant_paged(torch.from_numpy(cache).to(DEV), pages_arg, torch.tensor(lens, dtype=torch.int32, device=DEV), cu, signs.to(DEV), k, v, **extra)
+        for got, ref in ((k, want[0]), (v, want[1])):
+            assert torch.equal(got.cpu(), torch.from_numpy(ref).to(dtype)), (dtype, dim, heads)
+        rest = both[total] if strided else both[:, total]
+        assert bool((rest == 7.0).all())      # nothing past the last row
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("dim,heads", [(128, 1), (128, 3), (128, 8), (96, 2), (96, 5), (64, 1), (64, 8), (64, 5), (256, 1), (256, 4), (256, 3)])
+def test_edges_of_units(oracle, dim, heads, wide):
+    _check(oracle, dim, heads, wide=wide)
+    _check(oracle, dim, heads, wide=wide, strided=True)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("dim,heads,block,slot,listed", [(128, 3, 5, None, False), (96, 4, 1, None, True), (128, 8, 16, 96, True), (64, 2, 16, 64, False),
+                                                         (256, 2, 16, 160, True)])
+def test_other_pages_and_slots(oracle, dim, heads, block, slot, listed, wide):
+    """Page sizes that leave part units, slots with bytes behind them (copied row by row), lists of pages."""
+    _check(oracle, dim, heads, wide=wide, block=block, slot=slot, listed=listed)
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_many_sequences(oracle, dim):
+    """More sequences than a warp has lanes, most of them short or empty; more units a warp than it looks up at a time."""
+    rng = np.random.default_rng(dim)
+    _check(oracle, dim, 1, wide=False, lens=[int(n) for n in rng.integers(0, 40, 100)])
+    _check(oracle, dim, 8, wide=True, lens=[int(n) for n in rng.integers(0, 70, 70)])
+    _check(oracle, dim, 16, wide=False, lens=[3, 0, 60000 if dim == 64 else 66000, 20])

@@ -14,19 +14,24 @@
 // With fp32 output the result equals the CPU restatement bit for bit; fp16/bf16 outputs are its
 // correctly rounded values.
 //
-// Mapping: two lanes own one row (lane m: dims 64m .. 64m+63, i.e. code bytes 32m .. 32m+31), a
-// warp works on 16 rows; stages h = 1..32 are register-local (packed f32x2 arithmetic from h = 2
-// on), h = 64 is one shuffle per element.  Persistent blocks walk the (sequence, page, K / V) items
-// and fetch each item's codes one item ahead.
+// Mapping: a lane owns a row (two lanes a row of 256), a warp 32 / lanes-per-row consecutive rows of a page (its K rows, then its V rows).
+// The butterflies are then register-local and packed in pairs (f32x2): stage h = 1 comes out of the lookup table, h = 2 .. 64 are
+// whole-register adds.  Rows reach and leave the registers through shared memory: each warp copies the slots of unit n + 2 there while it works
+// on unit n, and stages its output so that a store instruction covers whole rows.
+//   8 ragged sequences of 5000 .. 13000 tokens x 8 heads of 128 -> bf16 (336 MB): 100 us with two lanes a row (a shuffle per element for
+//   h = 64, on the pipe of the lookups and stores; 4 warps a scheduler, work found row by row) -> 71.6 us = 72 % of the copy rate.  Heads of 64, 8 x 1000 .. 8000 tokens: 41.4 -> 17.3 us, of
+//   256, 8 x 1000 .. 4000: 73.7 -> 44.2, of 96, 3 x 1000 .. 16000 x 32 heads: 144 -> 87 (eight and two lanes a row before).  What bounds
+//   it now is that pipe (74 % busy: 128 wavefronts of lookups, 192 of output, 32 of signs in about 430 a unit) at three warps a scheduler.
+//   Output by tensor copies of 16 rows x 128 bytes in place of the read-back: 123 us.
 #include <cmath>
 
 #include "tq_common.cuh"
 
 namespace tq {
 
-constexpr int kDqThreads = 256;
+int device_sm_count(int* out);
+
 constexpr int kDqDim = 128;
-constexpr int kDqSlotCodes = 64;
 
 struct DequantParams {
     const uint8_t* kv_cache;
@@ -37,281 +42,337 @@ struct DequantParams {
     const int32_t* seq_lens;
     const int32_t* cu_seqlens;    // [batch + 1]: first output row of every sequence
     const float* signs;
-    void* out[2];                 // K, V: [total_tokens][H][128]
+    void* out[2];                 // K, V: [total_tokens][H][head_dim]
     int64_t out_token_stride;     // elements between tokens
-    int max_pages, H, head_shift, block_size, slot_bytes, out_dtype, batch;  // head_shift: log2(H) or -1
-    int head_dim;                 // elements per output row: 128, or 96 (the padded dims are dropped)
-    float cen[16];                // (float)(C[i] / sqrt(128))
-    float scale;                  // (float)(1 / sqrt(128))
+    int max_pages, H, head_shift, block_size, slot_bytes, batch;  // head_shift: log2(H) or -1
+    float cen[16];                // (float)(C[i] / sqrt(padded))
+    float scale;                  // (float)(1 / sqrt(padded))
 };
 
-struct Q2 { unsigned long long v; };
-__device__ __forceinline__ Q2 qpk(float lo, float hi) {
-    Q2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void qup(Q2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
-__device__ __forceinline__ Q2 qadd(Q2 a, Q2 b) { Q2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ Q2 qsub(Q2 a, Q2 b) { Q2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ Q2 qmul(Q2 a, Q2 b) { Q2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ Q2 qfma(Q2 a, Q2 b, Q2 c) {
-    Q2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-
-// 16-byte piece i of a lane's 64 output elements in the output type.
-template <int DT>
-__device__ __forceinline__ uint4 out_piece(const Q2 (&x)[32], int i);
-
-template <>
-__device__ __forceinline__ uint4 out_piece<TQ_F32>(const Q2 (&x)[32], int i) {  // 16 pieces of 4 floats
-    float a, b, c, e;
-    qup(x[2 * i], a, b);
-    qup(x[2 * i + 1], c, e);
-    return make_uint4(__float_as_uint(a), __float_as_uint(b), __float_as_uint(c), __float_as_uint(e));
-}
-template <>
-__device__ __forceinline__ uint4 out_piece<TQ_F16>(const Q2 (&x)[32], int i) {  // 8 pieces of 8 halves
-    uint32_t w[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        float a, b;
-        qup(x[4 * i + k], a, b);
-        const __half2 h = __floats2half2_rn(a, b);
-        w[k] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
-template <>
-__device__ __forceinline__ uint4 out_piece<TQ_BF16>(const Q2 (&x)[32], int i) {
-    uint32_t w[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        float a, b;
-        qup(x[4 * i + k], a, b);
-        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        w[k] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// Output staging of one warp pass: 16 rows in the output type, 16-byte pieces.  Piece j of the half
-// row (row, m) sits at position j ^ ((2 row + m) & 7) of that half row: the eight lanes served
-// together hit eight different bank groups both when the lanes write their own half rows and when
-// they read the pass back in linear order for the global stores.
-template <int DT>
-struct DqStage {
-    static constexpr int kEsz = DT == TQ_F32 ? 4 : 2;
-    static constexpr int kRowBytes = kDqDim * kEsz;
-    static constexpr int kHalfPieces = kRowBytes / 32;     // 16-byte pieces per lane: 8 or 16
-    static constexpr int kRowPieces = 2 * kHalfPieces;
-    static constexpr int kWarpBytes = 16 * kRowBytes;      // 4 KB or 8 KB
-    static constexpr int kTableBytes = 256 * 16 * 8;
-    static constexpr int kSmem = kTableBytes + (kDqThreads / 32) * kWarpBytes;
-};
-
-// What one warp needs of one work item (the K or V half of one page): its rows' codes and norm
-// are fetched one item ahead, so that the loads of the next page are in flight during the
-// arithmetic of the current one.
 // Page halves skipped because the page id lay outside the cache or the sequence was longer than
 // its page list; read back by tq_fault_counts.
 static __device__ int32_t g_dequant_skipped = 0;
 
-struct DqItem {
-    uint4 c0, c1;
-    float norm;
-    int64_t out_row0;  // first output row (token) of the page
-    int rows;          // (token, head) rows in the page half; 0: nothing to do
-    int which;
+// HD: elements of an output row; PD: of the rotated row (HD rounded up to a power of two).  SMALL: jobs of a few units a scheduler.  With
+// rows of 128 over two lanes a unit takes half as long, and the blocks leave room for the next kernel's beside them.
+template <int DT, int PD, int HD, bool SMALL>
+struct DqShape {
+    static constexpr int kEsz = DT == TQ_F32 ? 4 : 2;
+    static constexpr int kLanes = PD == 256 || (SMALL && PD == 128) ? 2 : 1, kRows = 32 / kLanes;    // lanes of a row, rows of a unit
+    static constexpr int kPairs = PD / kLanes / 2;                           // packed pairs of values a lane
+    static constexpr int kWarps = SMALL ? 8 : PD == 64 ? 20 : 12, kThreads = 32 * kWarps;      // 128 values a lane: 168 registers, 64: 96
+    static constexpr int kCodes = PD / 2, kRow = (kCodes + 2 * (PD / 64) + 15) & ~15;   // staged bytes of a slot: 48, 80, 144
+    static constexpr int kStage = kRows * kRow;
+    // Output leaves in passes of 32 to 128 dims of every row.  A lane holds kLaneDims of them.
+    static constexpr int kPassDims = kLanes == 2 ? PD / 2 : PD == 64 ? 128 / kEsz : 256 / kEsz, kLaneDims = kPassDims / kLanes;
+    static constexpr int kPasses = (HD + kPassDims - 1) / kPassDims;
+    static constexpr int kPitch = kPassDims * kEsz, kOut = kRows * kPitch;
+    // Shared memory: rings, barriers, signs; the table, 16 columns of 8 bytes a code byte (served half a warp at a time: no two lanes meet in a
+    // bank); the output staging.  Large jobs have the table at 64 KB with a 256-byte row a code byte, so that one byte permute makes an entry's address.
+    static constexpr uint32_t kSignBytes = PD * 4 + 64;                     // blocks of a pass's dims 16 bytes apart: two lanes of a row meet no bank
+    static constexpr uint32_t kBelow = 2 * kWarps * kStage + ((2 * kWarps * 8 + kSignBytes + 127) & ~127);
+    static constexpr uint32_t kEntry = SMALL ? 128 : 256, kTable = 65536;
+    static constexpr uint32_t kSmem = SMALL ? 128 + kBelow + 256 * kEntry + kWarps * kOut : 2 * kTable + kWarps * kOut - 1024;   // from offset 1024 (the system's part)
+    static_assert(SMALL || (kBelow + 1024 + 128 <= kTable && kSmem <= 232448), "shared memory");
 };
 
-template <int DT>
-__device__ __forceinline__ void fetch_item(const DequantParams& p, int64_t item, int64_t num_items, int warp, int lane,
-                                           DqItem& it) {
-    it.rows = 0;
-    it.which = 0;
-    it.out_row0 = 0;
-    if (item >= num_items) return;
-    const int which = (int)(item & 1);
-    const int64_t pb = item >> 1;
-    const int b = (int)(pb / p.max_pages), page_in_seq = (int)(pb - (int64_t)b * p.max_pages);
-    const int len = p.seq_lens[b];
-    const int tok0 = page_in_seq * p.block_size;
-    if (tok0 >= len) return;
-    const int64_t tbl = p.page_indptr ? (int64_t)p.page_indptr[b] : (int64_t)b * p.max_pages;
-    const bool listed = !p.page_indptr || tbl + page_in_seq < (int64_t)p.page_indptr[b + 1];
-    const int64_t page = listed ? (int64_t)p.page_indices[tbl + page_in_seq] : -1;
-    if ((uint64_t)page >= (uint64_t)p.num_blocks) {  // never form an address from it: the rows stay unwritten
-        if (warp == 0 && lane == 0 && which == 0) atomicAdd(&g_dequant_skipped, 1);
+template <int DT, int PD, int HD, bool SMALL>
+__global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL && PD != 256 ? 2 : 1) dequant_paged_kernel(const __grid_constant__ DequantParams p) {
+    using S = DqShape<DT, PD, HD, SMALL>;
+    constexpr uint32_t kAll = 0xffffffffu;
+    extern __shared__ __align__(128) uint8_t dq_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t smem0 = (smem_u32(dq_smem) + 127u) & ~127u;
+    const uint32_t bars = smem0 + 2 * S::kWarps * S::kStage, sgn = bars + 2 * S::kWarps * 8;
+    const uint32_t table = SMALL ? smem0 + S::kBelow : S::kTable, stagings = table + 256 * S::kEntry;
+    if (!SMALL && (smem0 + S::kBelow > S::kTable || smem0 < 1024)) {      // the shared window starts elsewhere than on any driver known
+        if (tid == 0 && blockIdx.x == 0) atomicAdd(&g_dequant_skipped, 1);
         return;
     }
-    const int ntok = len - tok0 < p.block_size ? len - tok0 : p.block_size;
-    it.rows = ntok * p.H;
-    it.which = which;
-    it.out_row0 = (int64_t)p.cu_seqlens[b] + tok0;
-    // rows beyond a warp's first pass (more than 128 rows per page half) are fetched in place
-    const int r = warp * 16 + (lane >> 1);
-    const uint8_t* slot = p.kv_cache + (size_t)which * p.slab_bytes +
-                          ((size_t)page * p.block_size * p.H + (size_t)(r < it.rows ? r : 0)) * p.slot_bytes;
-    it.c0 = *reinterpret_cast<const uint4*>(slot + 32 * (lane & 1));
-    it.c1 = *reinterpret_cast<const uint4*>(slot + 32 * (lane & 1) + 16);
-    it.norm = __half2float(*reinterpret_cast<const __half*>(slot + kDqSlotCodes));
-}
-
-// Persistent blocks over the work items (sequence, page, K / V), item = 2 * (b * max_pages + page) + which.
-template <int DT>
-__global__ void __launch_bounds__(kDqThreads) dequant_paged_kernel(const __grid_constant__ DequantParams p) {
-    // byte -> {centroid(high nibble), centroid(low nibble)}, 16 columns: an 8-byte load is served
-    // half a warp at a time, so the lookups of a warp never conflict
-    extern __shared__ __align__(128) uint8_t dq_smem[];
-    float2* table_s = reinterpret_cast<float2*>(dq_smem);
-    // scale * sign of dims 0..63 and 64..127 in different banks: a half warp reads both halves
-    __shared__ __align__(16) float sgn_s[2][kDqDim / 2 + 2];
-    using St = DqStage<DT>;
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint8_t* const ring = dq_smem + (smem0 - smem_u32(dq_smem)) + warp * 2 * S::kStage;
+    uint64_t* const bar = reinterpret_cast<uint64_t*>(dq_smem + (bars - smem_u32(dq_smem))) + 2 * warp;
     grid_launch_dependents();
-    for (int i = tid; i < 256 * 16; i += kDqThreads) {
-        const int v = i >> 4;
-        table_s[i] = make_float2(p.cen[v >> 4], p.cen[v & 15]);
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    // byte -> {high + low, high - low}: butterfly stage h = 1 of the two centroids
+    for (int i = tid; i < 256 * 8; i += S::kThreads) {
+        const int v = i >> 3;
+        const float hi = p.cen[v >> 4], lo = p.cen[v & 15];
+        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%1,%2};" ::"r"(table + S::kEntry * v + 16u * (i & 7)), "f"(__fadd_rn(hi, lo)), "f"(__fsub_rn(hi, lo)) : "memory");
     }
     grid_dependency_wait();  // the cache, the page table and the lengths belong to earlier kernels
-    if (tid < kDqDim) sgn_s[tid >> 6][tid & 63] = __fmul_rn(p.signs[tid], p.scale);  // exact: the sign is +-1
+    for (int d = tid; d < PD; d += S::kThreads) {
+        float v = d < HD ? __fmul_rn(p.signs[d], p.scale) : 0.0f;  // exact: the sign is +-1, or the scale a power of two
+        if (S::kLanes == 2 && d >= PD * 3 / 4) v = -v;                     // see the last stage
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(sgn + 4u * d + (S::kLanes == 2 ? 16u * (d / (PD / 4)) : 0u)), "f"(v) : "memory");
+    }
     __syncthreads();
 
-    constexpr int kEsz = St::kEsz;
-    uint8_t* stage = dq_smem + St::kTableBytes + (size_t)warp * St::kWarpBytes;
-    // Linear read-back of a staged pass: iteration i of lane l takes piece lin_pin of row
-    // lin_row + i * kLinRows, stored at position piece ^ ((2 row + half) & 7) of its half row.
-    constexpr int kLinRows = 32 / St::kRowPieces;            // rows covered by one warp-wide access: 2 or 1
-    constexpr int kLinIters = 16 / kLinRows;
-    const int lin_row = lane / St::kRowPieces, lin_pin = lane % St::kRowPieces;
-    const int lin_half = lin_pin / St::kHalfPieces, lin_pp = lin_pin % St::kHalfPieces;
-    const int lin_key = 2 * lin_row + lin_half;
-    const int lin_base = lin_row * St::kRowBytes + lin_half * (St::kRowBytes / 2);
-    const bool dense = p.head_dim == kDqDim && p.out_token_stride == (int64_t)p.H * kDqDim;
-    const int m = lane & 1;
-    const uint32_t table_lane = smem_u32(table_s) + 8u * (lane & 15);
-    const float hsgn = m ? -1.0f : 1.0f;
-    const int64_t num_items = 2 * (int64_t)p.batch * p.max_pages;
-
-    DqItem cur, nxt;
-    fetch_item<DT>(p, blockIdx.x, num_items, warp, lane, cur);
-    for (int64_t item = blockIdx.x; item < num_items; item += gridDim.x) {
-        fetch_item<DT>(p, item + gridDim.x, num_items, warp, lane, nxt);
-        uint8_t* out_base = static_cast<uint8_t*>(p.out[cur.which]);
-        for (int r0 = warp * 16; r0 < cur.rows; r0 += (kDqThreads / 32) * 16) {
-            const int r = r0 + (lane >> 1);
-            const bool ok = r < cur.rows;
-            uint4 c0 = cur.c0, c1 = cur.c1;
-            float norm = cur.norm;
-            if (r0 != warp * 16) {  // later passes of a page half with more than 128 rows: fetch now
-                const int64_t pb = item >> 1;
-                const int b = (int)(pb / p.max_pages), page_in_seq = (int)(pb - (int64_t)b * p.max_pages);
+    // The work list: the pages of all sequences, each cut into units of 32 or 16 rows (the page's K rows, then its V rows).  A warp takes every
+    // workers-th unit; its lanes look 32 of them up at a time, which costs a unit less than a tenth of what one by one does.
+    const int half_rows = p.block_size * p.H, units = (2 * half_rows + S::kRows - 1) / S::kRows;
+    const int workers = (int)gridDim.x * S::kWarps;
+    int64_t first = (int64_t)warp * gridDim.x + blockIdx.x;      // lane 0's unit; neighbouring units go to different SMs
+    uint64_t src;       // this lane's unit: where its slots begin (0: nothing to do, 1: the end of the work; else a multiple of 16) ...
+    int unit, ntok;     // ... which of the page's units, tokens in the page ...
+    int row0;           // ... and the output row (token) of the page's first token
+    auto look_up = [&]() {
+        const int64_t k = first + (int64_t)lane * workers, at = k / units;
+        src = 1;
+        unit = (int)(k - at * units);
+        int64_t run = 0;
+        for (int base = 0; base < p.batch; base += 32) {
+            int len = 0, np = 0, cu = 0;
+            if (base + lane < p.batch) {
+                len = p.seq_lens[base + lane];
+                cu = p.cu_seqlens[base + lane];
+                np = len > 0 ? (int)(((int64_t)len + p.block_size - 1) / p.block_size) : 0;
+                if (np > p.max_pages) np = p.max_pages;
+            }
+            int64_t end = np;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t t = __shfl_up_sync(kAll, end, o);
+                if (lane >= o) end += t;
+            }
+            end += run;
+            const int64_t start = end - np;
+            run = __shfl_sync(kAll, end, 31);
+            int j = 0;      // this lane's unit lies in sequence base + j
+            const int live = p.batch - base < 32 ? p.batch - base : 32;
+#pragma unroll 4
+            for (int i = 0; i < live; i++) j += __shfl_sync(kAll, end, i) <= at ? 1 : 0;
+            const bool here = j < live && src == 1;
+            const int pg = (int)(at - __shfl_sync(kAll, start, j & 31));
+            const int left = __shfl_sync(kAll, len, j & 31) - pg * p.block_size, row = __shfl_sync(kAll, cu, j & 31) + pg * p.block_size;
+            if (here) {
+                const int b = base + j;
                 const int64_t tbl = p.page_indptr ? (int64_t)p.page_indptr[b] : (int64_t)b * p.max_pages;
-                const int64_t page = p.page_indices[tbl + page_in_seq];
-                const uint8_t* slot = p.kv_cache + (size_t)cur.which * p.slab_bytes +
-                                      ((size_t)page * p.block_size * p.H + (size_t)(ok ? r : 0)) * p.slot_bytes;
-                c0 = *reinterpret_cast<const uint4*>(slot + 32 * m);
-                c1 = *reinterpret_cast<const uint4*>(slot + 32 * m + 16);
-                norm = __half2float(*reinterpret_cast<const __half*>(slot + kDqSlotCodes));
-            }
-            const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            Q2 x[32];  // x[i] = dims (64m + 2i, 64m + 2i + 1) = code byte 32m + i
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                uint32_t byte;  // byte i & 3 of the word, zero extended, by one byte permute
-                asm("prmt.b32 %0, %1, 0, %2;" : "=r"(byte) : "r"(w[i >> 2]), "r"(0x4440u | (uint32_t)(i & 3)));
-                float hi, lo;
-                asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(hi), "=f"(lo) : "r"(byte * 128u + table_lane));
-                // stage h = 1 inside the pair
-                x[i] = qpk(__fadd_rn(hi, lo), __fsub_rn(hi, lo));
-            }
-            // stages h = 2 .. 32: pairs i and i + h/2
-#pragma unroll
-            for (int hp = 1; hp < 32; hp <<= 1)
-#pragma unroll
-                for (int i = 0; i < 32; i++)
-                    if (!(i & hp)) {
-                        const Q2 a = x[i], c = x[i + hp];
-                        x[i] = qadd(a, c);
-                        x[i + hp] = qsub(a, c);
-                    }
-            // stage h = 64 between the two lanes: lower half mine + other, upper half other - mine
-            {
-                const Q2 s2 = qpk(hsgn, hsgn);
-#pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    float a, c;
-                    qup(x[i], a, c);
-                    const float oa = __shfl_xor_sync(0xffffffffu, a, 1), oc = __shfl_xor_sync(0xffffffffu, c, 1);
-                    x[i] = qfma(x[i], s2, qpk(oa, oc));
+                const int64_t page = !p.page_indptr || tbl + pg < (int64_t)p.page_indptr[b + 1] ? (int64_t)p.page_indices[tbl + pg] : -1;
+                ntok = left < p.block_size ? left : p.block_size;
+                row0 = row;
+                if ((uint64_t)page >= (uint64_t)p.num_blocks) {  // never form an address from it: the rows stay unwritten
+                    if (unit == 0) atomicAdd(&g_dequant_skipped, 1);
+                    src = 0;
+                } else {
+                    src = reinterpret_cast<uint64_t>(p.kv_cache) + (uint64_t)page * half_rows * p.slot_bytes;
                 }
             }
-            // (w * scale) * sign == w * (scale * sign) exactly; then the norm
-            const Q2 n2 = qpk(norm, norm);
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const float2 sg = *reinterpret_cast<const float2*>(&sgn_s[m][2 * i]);
-                x[i] = qmul(qmul(x[i], qpk(sg.x, sg.y)), n2);
-            }
-            // stage the 16 rows, then store them in linear order: every store instruction of the warp
-            // covers whole rows (512 contiguous bytes when the heads of a token are contiguous)
-            {
-                uint8_t* half_row = stage + (lane >> 1) * St::kRowBytes + m * (St::kRowBytes / 2);
-                const int key = lane & 7;  // (2 row + m) & 7
-#pragma unroll
-                for (int i = 0; i < St::kHalfPieces; i++)
-                    *reinterpret_cast<uint4*>(half_row + ((i ^ key) << 4)) = out_piece<DT>(x, i);
-            }
-            __syncwarp();
-            if (dense) {
-                // heads of a token contiguous: the rows of the page half are one contiguous range
-                uint8_t* dst = out_base + ((cur.out_row0 * p.H + r0 + lin_row) * (int64_t)St::kRowBytes) + lin_pin * 16;
-#pragma unroll
-                for (int i = 0; i < kLinIters; i++) {
-                    const uint4 piece = *reinterpret_cast<const uint4*>(stage + lin_base + i * kLinRows * St::kRowBytes +
-                                                                        ((lin_pp ^ ((lin_key + 2 * i * kLinRows) & 7)) << 4));
-                    if (r0 + lin_row + i * kLinRows < cur.rows)
-                        *reinterpret_cast<uint4*>(dst + (size_t)i * kLinRows * St::kRowBytes) = piece;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < kLinIters; i++) {
-                    const uint4 piece = *reinterpret_cast<const uint4*>(stage + lin_base + i * kLinRows * St::kRowBytes +
-                                                                        ((lin_pp ^ ((lin_key + 2 * i * kLinRows) & 7)) << 4));
-                    const int rr = r0 + lin_row + i * kLinRows;
-                    if (rr < cur.rows && lin_pin * 16 < p.head_dim * kEsz) {
-                        int t, h;
-                        if (p.head_shift >= 0) { t = rr >> p.head_shift; h = rr & (p.H - 1); }
-                        else { t = rr / p.H; h = rr - t * p.H; }
-                        uint8_t* dst = out_base + ((cur.out_row0 + t) * p.out_token_stride + (int64_t)h * p.head_dim) * kEsz;
-                        *reinterpret_cast<uint4*>(dst + lin_pin * 16) = piece;
-                    }
-                }
-            }
-            __syncwarp();
+            if (__all_sync(kAll, src != 1)) break;
         }
-        cur = nxt;
+    };
+    // The slots of unit i into stage s: neighbouring rows are neighbours in the cache, so one copy for the K and one for the V rows.
+    auto issue = [&](int i, int s) {
+        const uint64_t k0 = __shfl_sync(kAll, src, i);
+        if (k0 <= 1) return;
+        const int r0 = S::kRows * __shfl_sync(kAll, unit, i);
+        const int rows = 2 * half_rows - r0 < S::kRows ? 2 * half_rows - r0 : S::kRows;
+        uint8_t* dst = ring + s * S::kStage;
+        __syncwarp();
+        fence_proxy_async();   // the stage has been read out by ordinary loads
+        if (p.slot_bytes == S::kRow) {
+            if (lane == 0) {
+                const int nk = half_rows - r0 < 0 ? 0 : half_rows - r0 < rows ? half_rows - r0 : rows;
+                const uint8_t* from = reinterpret_cast<const uint8_t*>(k0) + (int64_t)r0 * S::kRow;
+                mbar_arrive_expect_tx(&bar[s], (uint32_t)(rows * S::kRow));
+                if (nk > 0) bulk_g2s(dst, from, (uint32_t)(nk * S::kRow), &bar[s]);
+                if (nk < rows) bulk_g2s(dst + nk * S::kRow, from + p.slab_bytes + (int64_t)(nk - half_rows) * S::kRow, (uint32_t)((rows - nk) * S::kRow), &bar[s]);
+            }
+        } else {      // slots with more behind them: row by row
+            if (lane == 0) mbar_arrive_expect_tx(&bar[s], (uint32_t)(rows * S::kRow));
+            __syncwarp();
+            const int r = r0 + lane;
+            if (lane < rows)
+                bulk_g2s(dst + lane * S::kRow, reinterpret_cast<const uint8_t*>(k0) + (r < half_rows ? (int64_t)r * p.slot_bytes : p.slab_bytes + (int64_t)(r - half_rows) * p.slot_bytes),
+                         S::kRow, &bar[s]);
+        }
+    };
+
+    // Of a pass, 16-byte piece i of a row (a lane's part of it is lane_pieces) is staged with the low three bits of i changed by the part's number, or
+    // the row's where a part is half of 128 bytes: the eight lanes served together meet no bank twice, writing and reading.
+    const int m = lane & (S::kLanes - 1);
+    constexpr int kPer = 16 / S::kEsz, lane_pieces = S::kLaneDims / kPer;      // dims of a piece
+    const uint32_t staging = stagings + (uint32_t)warp * S::kOut;
+    auto staged = [&](int row, int pc) {
+        const int key = lane_pieces >= 8 ? row * S::kLanes + pc / lane_pieces : row;
+        return staging + row * S::kPitch + (pc >> 3) * 128 + (((pc ^ key) & 7) << 4);
+    };
+    const uint32_t my_part = staged(lane / S::kLanes, m * lane_pieces);
+    const uint32_t table_lane = table + 8u * (lane & 15);
+    const bool dense = p.out_token_stride == (int64_t)p.H * HD;
+
+    look_up();
+    issue(0, 0);
+    issue(1, 1);
+    uint32_t phases = 0;
+    for (int i = 0, s = 0;; i++, s ^= 1) {
+        if (i == 30) {      // the next units: this one becomes the first
+            first += 30 * (int64_t)workers;
+            look_up();
+            i = 0;
+        }
+        const uint64_t k0 = __shfl_sync(kAll, src, i);
+        if (k0 == 1) break;
+        if (k0 != 0) {
+            if (!mbar_wait(&bar[s], (phases >> s) & 1)) return;  // the copy never landed: nothing more is written
+            phases ^= 1u << s;
+            const uint32_t slot = smem_u32(ring) + s * S::kStage + (uint32_t)(lane / S::kLanes) * S::kRow;
+            P2 x[S::kPairs];   // x[i] = dims 2 i, 2 i + 1 = code byte i (two lanes: of the row's half m)
+#pragma unroll
+            for (int j = 0; j < S::kPairs / 16; j++) {
+                uint32_t w[4];
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(slot + (PD / 4) * m + 16 * j));
+                if (S::kLanes == 2 && j >= S::kPairs / 32) {      // see the last stage
+#pragma unroll
+                    for (int e = 0; e < 4; e++) w[e] ^= 0u - m;
+                }
+#pragma unroll
+                for (int e = 0; e < 16; e++) {
+                    uint32_t at;      // byte e & 3 of the word becomes byte 1 of the address: row of the table
+                    if constexpr (!SMALL) asm("prmt.b32 %0, %1, %2, %3;" : "=r"(at) : "r"(w[e >> 2]), "r"(table_lane), "r"(0x7604u | (uint32_t)((e & 3) << 4)));
+                    else at = __byte_perm(w[e >> 2], 0, 0x4440 | (e & 3)) * S::kEntry + table_lane;
+                    asm("ld.shared.b64 %0, [%1];" : "=l"(x[16 * j + e].v) : "r"(at));
+                }
+            }
+            uint32_t nh;
+            asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(nh) : "r"(slot + S::kCodes));
+            const float norm = __half2float(__ushort_as_half((unsigned short)nh));
+#pragma unroll
+            for (int h = 1; h < S::kPairs; h <<= 1)
+#pragma unroll
+                for (int e = 0; e < S::kPairs; e++)
+                    if (!(e & h)) {
+                        const P2 a = x[e], c = x[e + h];
+                        x[e] = add2(a, c);
+                        x[e + h] = sub2(a, c);
+                    }
+            if constexpr (S::kLanes == 2) {
+                // The last stage is between the lanes: each keeps its first half of values and sends the other, half the shuffles of sending all.  For that
+                // the upper lane has to hold its values with the halves exchanged, which it does when the inputs of the second half change sign (the transform
+                // of (-1)^[e >= n / 2] x is that of x at e ^ (n / 2), bit for bit); the codebook is symmetric, so the complement of a code is its
+                // negative.  Lower outputs are mine + other, upper ones mine - other, negated in the upper lane (in its signs).
+                constexpr int kHalf = S::kPairs / 2;
+#pragma unroll
+                for (int e = 0; e < kHalf; e++) {
+                    float a, c;
+                    up(x[kHalf + e], a, c);
+                    const P2 mine = x[e], other = pk(__shfl_xor_sync(kAll, a, 1), __shfl_xor_sync(kAll, c, 1));
+                    x[e] = add2(mine, other);
+                    x[kHalf + e] = sub2(mine, other);
+                }
+            }
+            const P2 n2 = pk(norm, norm);
+            const int r0 = S::kRows * __shfl_sync(kAll, unit, i), left = __shfl_sync(kAll, ntok, i);
+            const int64_t out0 = __shfl_sync(kAll, row0, i);
+            const bool in_v = r0 >= half_rows;
+            // All rows are K rows or all V rows, and neighbours in the output.
+            const bool whole = dense && (in_v ? r0 - half_rows : r0) + S::kRows <= left * p.H;
+#pragma unroll
+            for (int pass = 0; pass < S::kPasses; pass++) {
+                // pieces of a row that are kept
+                const int d0 = pass * S::kPassDims, dims = HD - d0 < S::kPassDims ? HD - d0 : S::kPassDims, pieces = dims / kPer;
+                const uint32_t sgn_part = sgn + (S::kLanes == 2 ? (2 * pass + m) * (PD + 16) : 0);
+#pragma unroll
+                for (int c = 0; c < lane_pieces; c++) {
+                    if (S::kLanes == 1 && c >= pieces) break;
+                    uint32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < kPer / 4; q++) {
+                        const int d = pass * S::kLaneDims + c * kPer + 4 * q;      // of the lane's values
+                        const int sd = S::kLanes == 2 ? c * kPer + 4 * q : d;
+                        float4 sg;
+                        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(sg.x), "=f"(sg.y), "=f"(sg.z), "=f"(sg.w) : "r"(sgn_part + 4u * sd));
+                        // (w * scale) * sign == w * (scale * sign) exactly; then the norm
+                        float a, b, f, g;
+                        up(mul2(mul2(x[d / 2], pk(sg.x, sg.y)), n2), a, b);
+                        up(mul2(mul2(x[d / 2 + 1], pk(sg.z, sg.w)), n2), f, g);
+                        if constexpr (DT == TQ_F32) {
+                            w[0] = __float_as_uint(a); w[1] = __float_as_uint(b); w[2] = __float_as_uint(f); w[3] = __float_as_uint(g);
+                        } else if constexpr (DT == TQ_F16) {
+                            const __half2 u = __floats2half2_rn(a, b), v = __floats2half2_rn(f, g);
+                            w[2 * q] = *reinterpret_cast<const uint32_t*>(&u); w[2 * q + 1] = *reinterpret_cast<const uint32_t*>(&v);
+                        } else {
+                            const __nv_bfloat162 u = __floats2bfloat162_rn(a, b), v = __floats2bfloat162_rn(f, g);
+                            w[2 * q] = *reinterpret_cast<const uint32_t*>(&u); w[2 * q + 1] = *reinterpret_cast<const uint32_t*>(&v);
+                        }
+                    }
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"((my_part ^ ((c & 7) << 4)) + (c >> 3) * 128), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+                }
+                __syncwarp();
+                // piece lane + 32 e of the pass in row order, from where it was staged
+                int row = lane / pieces, pc = lane - row * pieces;
+                if (whole) {
+                    const uint32_t first_piece = staged(row, pc);
+                    uint8_t* dst = static_cast<uint8_t*>(p.out[in_v]) + ((out0 * p.H + r0 - (in_v ? half_rows : 0)) * HD + d0) * S::kEsz +
+                                   row * (HD * S::kEsz) + pc * 16;
+#pragma unroll
+                    for (int e = 0; e < pieces / S::kLanes; e++) {
+                        // 32 is a multiple of the pieces, or (96-wide rows, 12 pieces) they wrap within it
+                        const int q_row = 32 % pieces ? (lane + 32 * e) / pieces : row + e * (32 / pieces), q_pc = 32 % pieces ? (lane + 32 * e) % pieces : pc;
+                        const uint32_t at = 32 % pieces ? staged(q_row, q_pc) : (first_piece ^ ((e * (32 / pieces) * (lane_pieces >= 8 ? S::kLanes : 1) & 7) << 4)) + e * (32 / pieces) * S::kPitch;
+                        uint4 v;
+                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+                        *reinterpret_cast<uint4*>(dst + ((q_row - row) * (HD * S::kEsz) + (q_pc - pc) * 16)) = v;
+                    }
+                } else {
+#pragma unroll 1
+                    for (int e = 0; e < pieces / S::kLanes; e++) {
+                        const int r = r0 + row, v_row = r >= half_rows, rr = v_row ? r - half_rows : r;
+                        const int t = p.head_shift >= 0 ? rr >> p.head_shift : rr / p.H;
+                        uint4 v;
+                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                     : "r"(staged(row, pc)) : "memory");
+                        if (r < 2 * half_rows && t < left)
+                            *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out[v_row]) + ((out0 + t) * p.out_token_stride + (rr - t * p.H) * HD + d0) * S::kEsz + pc * 16) = v;
+                        row += 32 / pieces;
+                        pc += 32 % pieces;
+                        if (pc >= pieces) { pc -= pieces; row++; }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        issue(i + 2, s);
     }
 }
 
-int device_sm_count(int* out);
-
-template <int DT>
-static int launch_dequant(const DequantParams& p, dim3 grid, cudaStream_t stream) {
+template <int DT, int PD, int HD, bool SMALL>
+static int launch_dequant(const DequantParams& p, int64_t grid, cudaStream_t stream) {
+    using S = DqShape<DT, PD, HD, SMALL>;
     static bool configured[64] = {};  // per template instance and device
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(dequant_paged_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     DqStage<DT>::kSmem));
+        TQ_CUDA(cudaFuncSetAttribute(dequant_paged_kernel<DT, PD, HD, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    TQ_CUDA(launch_serialized(dequant_paged_kernel<DT>, grid, dim3(kDqThreads), DqStage<DT>::kSmem, stream, p));
+    TQ_CUDA(launch_serialized(dequant_paged_kernel<DT, PD, HD, SMALL>, dim3((unsigned)grid), dim3(S::kThreads), S::kSmem, stream, p));
     return TQ_OK;
+}
+// Up to this many units of 32 rows an SM (two a warp of the large kernel) the small blocks are faster: 8 heads of 128, 4800 tokens (16 units an
+// SM) 8.2 us against 8.9; 16 ragged rows x 600, 4 heads 5.3 / 6.1; at 2400 tokens both 5.8; heads of 256, 3600 tokens 12.8 / 13.2.
+constexpr int kDqSmallUnits = 24;
+
+template <int DT, int PD, int HD>
+static int launch_dequant(const DequantParams& p, int sms, cudaStream_t stream) {
+    // The lengths are on the device: the table's width bounds the units of 32 rows.
+    const int64_t units = (int64_t)p.batch * p.max_pages * ((2 * (int64_t)p.block_size * p.H + 31) / 32);
+    if (units <= (int64_t)kDqSmallUnits * sms) {
+        const int64_t most = (int64_t)sms * (PD == 256 ? 1 : 2), count = units * DqShape<DT, PD, HD, true>::kLanes;
+        return launch_dequant<DT, PD, HD, true>(p, count < most ? count : most, stream);
+    }
+    return launch_dequant<DT, PD, HD, false>(p, units < sms ? units : sms, stream);
+}
+template <int PD, int HD>
+static int launch_dequant(const DequantParams& p, int out_dtype, int sms, cudaStream_t stream) {
+    switch (out_dtype) {
+        case TQ_F32: return launch_dequant<TQ_F32, PD, HD>(p, sms, stream);
+        case TQ_F16: return launch_dequant<TQ_F16, PD, HD>(p, sms, stream);
+        default: return launch_dequant<TQ_BF16, PD, HD>(p, sms, stream);
+    }
 }
 void host_codebook(int dim, int bits, float* centroids, float* boundaries);
 
@@ -341,16 +402,21 @@ extern "C" int tq_dequant_paged(const void* kv_cache, int64_t num_blocks, int bl
     TQ_REQUIRE(batch >= 0 && num_blocks >= 0, TQ_ERR_INVALID, "negative size");
     if (batch == 0 || max_pages == 0) return TQ_OK;
     TQ_REQUIRE(kv_cache && page_indices && seq_lens && cu_seqlens && signs && k_out && v_out, TQ_ERR_INVALID, "null pointer");
-    if (head_dim != kDqDim && head_dim != 96) {  // other head sizes (64, 256, ...): the plain kernel
+    const bool wide = head_dim == kDqDim || head_dim == 96;      // the sizes that take nothing but aligned slots and rows
+    const int esz = out_dtype == TQ_F32 ? 4 : 2;
+    const bool aligned = slot_bytes % 16 == 0 && (uintptr_t)kv_cache % 16 == 0 && (uintptr_t)k_out % 16 == 0 && (uintptr_t)v_out % 16 == 0 &&
+                         out_token_stride * esz % 16 == 0;
+    const bool second = (head_dim == 64 || head_dim == 256) && aligned && block_size == 16 && slot_bytes >= (head_dim == 64 ? 48 : 144);
+    if (!wide && !second) {  // other head sizes, slots that are no multiple of 16 bytes: the plain kernel
         TQ_REQUIRE(num_kv_heads >= 1 && out_dtype >= TQ_F32 && out_dtype <= TQ_BF16 &&
                        out_token_stride >= (int64_t)num_kv_heads * head_dim, TQ_ERR_INVALID, "bad geometry");
         return generic_dequant(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, page_indices, page_indptr, max_pages,
                                seq_lens, cu_seqlens, batch, signs, head_dim, k_out, v_out, out_dtype, out_token_stride, stream);
     }
-    TQ_REQUIRE(slot_bytes >= 80 && slot_bytes % 16 == 0, TQ_ERR_INVALID, "slot_bytes must be a multiple of 16 and >= 80");
+    TQ_REQUIRE(!wide || (slot_bytes >= 80 && slot_bytes % 16 == 0), TQ_ERR_INVALID, "slot_bytes must be a multiple of 16 and >= 80");
     TQ_REQUIRE(block_size >= 1 && num_kv_heads >= 1 && max_pages >= 1 && batch >= 1, TQ_ERR_INVALID, "bad geometry");
     TQ_REQUIRE(out_dtype >= TQ_F32 && out_dtype <= TQ_BF16, TQ_ERR_INVALID, "bad out_dtype");
-    TQ_REQUIRE(out_token_stride >= (int64_t)num_kv_heads * head_dim && out_token_stride % 8 == 0, TQ_ERR_INVALID,
+    TQ_REQUIRE(out_token_stride >= (int64_t)num_kv_heads * head_dim && (!wide || out_token_stride % 8 == 0), TQ_ERR_INVALID,
                "out_token_stride must cover one token and keep rows 16-byte aligned");
     TQ_REQUIRE(((uintptr_t)kv_cache % 16) == 0 && ((uintptr_t)k_out % 16) == 0 && ((uintptr_t)v_out % 16) == 0,
                TQ_ERR_INVALID, "kv_cache, k_out and v_out must be 16-byte aligned");
@@ -373,21 +439,19 @@ extern "C" int tq_dequant_paged(const void* kv_cache, int64_t num_blocks, int bl
         if ((1 << sft) == num_kv_heads) p.head_shift = sft;
     p.block_size = block_size;
     p.slot_bytes = slot_bytes;
-    p.out_dtype = out_dtype;
     p.batch = batch;
-    p.head_dim = head_dim;
     float bnd[15];
-    host_codebook(kDqDim, 4, p.cen, bnd);
-    p.scale = (float)(1.0 / std::sqrt((double)kDqDim));
+    const int padded = wide ? kDqDim : head_dim;
+    host_codebook(padded, 4, p.cen, bnd);
+    p.scale = (float)(1.0 / std::sqrt((double)padded));
     int sms = 0;
     int rc = device_sm_count(&sms);
     if (rc != TQ_OK) return rc;
-    const int64_t items = 2 * (int64_t)batch * max_pages;
-    const dim3 grid((unsigned)(items < 2 * (int64_t)sms ? items : 2 * (int64_t)sms));  // two resident blocks per SM
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (out_dtype) {
-        case TQ_F32: return launch_dequant<TQ_F32>(p, grid, s);
-        case TQ_F16: return launch_dequant<TQ_F16>(p, grid, s);
-        default: return launch_dequant<TQ_BF16>(p, grid, s);
+    switch (head_dim) {
+        case 64: return launch_dequant<64, 64>(p, out_dtype, sms, s);
+        case 96: return launch_dequant<128, 96>(p, out_dtype, sms, s);
+        case 256: return launch_dequant<256, 256>(p, out_dtype, sms, s);
+        default: return launch_dequant<128, 128>(p, out_dtype, sms, s);
     }
 }
