@@ -29,6 +29,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relax
 UNITS = {
     "tq_api.cu": [],
     "tq_write.cu": ["-fmad=false"],
+    "tq_write_rows.cu": ["-fmad=false"],
     "tq_flat.cu": ["-fmad=false"],
     "tq_decode.cu": [],
     "tq_decode_mq.cu": [],

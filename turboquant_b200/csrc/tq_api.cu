@@ -1,4 +1,6 @@
 // Host-side pieces shared by the C ABI: error text, codebook constants, device queries.
+#include <cuda.h>  // CUtensorMap and its enums only
+
 #include <cmath>
 #include <cstring>
 
@@ -53,6 +55,22 @@ int device_sm_count(int* out) {
     }
     *out = cached;
     return TQ_OK;
+}
+
+// cuTensorMapEncodeTiled, looked up through the runtime (no link-time dependency on the driver library)
+bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                       const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+    typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                           const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Fn fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Fn>(sym) : nullptr;
+    }();
+    const cuuint32_t ones[5] = {1u, 1u, 1u, 1u, 1u};
+    return fn && fn(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 int write_fault_count(int32_t* out);

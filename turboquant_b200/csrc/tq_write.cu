@@ -865,36 +865,15 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
     }
 }
 
-// cuTensorMapEncodeTiled, looked up through the runtime (no link-time dependency on the driver library)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-        tried = true;
-    }
-    return fn;
-}
+bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                       const cuuint32_t* box, CUtensorMapSwizzle swizzle);
 
 // [rows][128] 16-bit elements, row pitch 256 bytes, boxes of 16 rows x 64 elements with the 128-byte swizzle
 static bool encode_rows_map(CUtensorMap* map, const void* base, int64_t rows, bool is_bf16) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)kD * 2};
     const cuuint32_t box[2] = {64u, (cuuint32_t)MmaShape::kRows};
-    const cuuint32_t estr[2] = {1u, 1u};
-    return fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-              const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode_tensor_map(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <typename T>
@@ -964,13 +943,20 @@ int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv
                   const void* value, int in_dtype, int64_t num_tokens, int64_t k_token_stride, int64_t v_token_stride,
                   const float* signs, const void* slot_mapping, int slot_dtype, int head_dim, int flags, void* stream);
 int generic_fault_counts(int32_t* write_dropped, int32_t* dequant_skipped);
+int generic_slot_bytes(int head_dim);
+bool write_rows(void* kv_cache, int64_t num_blocks, int block_size, int num_kv_heads, int slot_bytes, const void* key, const void* value, int in_dtype,
+                int64_t num_tokens, int64_t k_token_stride, int64_t v_token_stride, const float* signs, const void* slot_mapping, int slot_dtype,
+                int head_dim, int flags, void* stream, int* rc);
+int write_rows_fault_count(int32_t* out);
 
 int write_fault_count(int32_t* out) {
-    int32_t a = 0, b = 0, c = 0;
+    int32_t a = 0, b = 0, c = 0, d = 0;
     TQ_CUDA(cudaMemcpyFromSymbol(&a, g_write_dropped, sizeof(int32_t)));
     int rc = generic_fault_counts(&b, &c);
     if (rc != TQ_OK) return rc;
-    *out = a + b;
+    rc = write_rows_fault_count(&d);
+    if (rc != TQ_OK) return rc;
+    *out = a + b + d;
     return TQ_OK;
 }
 
@@ -989,11 +975,16 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
     TQ_REQUIRE(num_kv_heads >= 1 && block_size >= 1, TQ_ERR_INVALID, "bad geometry");
     TQ_REQUIRE(in_dtype == TQ_F32 || in_dtype == TQ_F16 || in_dtype == TQ_BF16, TQ_ERR_INVALID, "bad in_dtype");
     TQ_REQUIRE(slot_dtype == TQ_I32 || slot_dtype == TQ_I64, TQ_ERR_INVALID, "bad slot_dtype");
-    if (head_dim != 128 && head_dim != 96) {  // other head sizes (64, 256, ...): the plain kernels
+    if (head_dim != 128 && head_dim != 96) {  // other head sizes (64, 256, ...)
         TQ_REQUIRE(k_token_stride >= (int64_t)num_kv_heads * head_dim && v_token_stride >= (int64_t)num_kv_heads * head_dim,
                    TQ_ERR_INVALID, "token stride smaller than one token");
         TQ_REQUIRE((flags & TQ_WRITE_TENSOR_PATH) == 0, TQ_ERR_UNSUPPORTED,
                    "the tensor-core write kernel takes fp16 / bf16 rows of 128 elements");
+        int rc = TQ_OK;
+        if ((flags & TQ_WRITE_EXACT_PATH) == 0 && slot_bytes >= generic_slot_bytes(head_dim) &&
+            write_rows(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, key, value, in_dtype, num_tokens, k_token_stride, v_token_stride, signs,
+                       slot_mapping, slot_dtype, head_dim, flags, stream, &rc))
+            return rc;
         return generic_write(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, key, value, in_dtype, num_tokens,
                              k_token_stride, v_token_stride, signs, slot_mapping, slot_dtype, head_dim, flags, stream);
     }
