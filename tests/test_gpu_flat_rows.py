@@ -77,3 +77,27 @@ def test_signs_beyond_one(oracle, dim):
             np.testing.assert_array_equal(norms.cpu().numpy(), plain_norms.cpu().numpy())
             if bool((signs.abs() < 1e30).all()):
                 np.testing.assert_array_equal(p.cpu().numpy(), oracle.quantize_flat(x.float().numpy(), signs.numpy(), bits)[0], err_msg=f"{name} {bits}")
+
+
+@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8200 + 17), (96, 8192 + 31), (72, 8195), (64, 49152), (64, 49152 + 33), (256, 2048), (256, 2048 + 15), (192, 2051)])
+def test_dequantization_of_many_rows(oracle, dim, n):
+    """A lane (two lanes) a row: the fewest rows that go this way, part units, short rows, both pack orders, any sign vector."""
+    padded = 1 << (dim - 1).bit_length()
+    rng = np.random.default_rng(dim + n)
+    norms = rng.uniform(0.0, 30.0, n).astype(np.float32)
+    norms[:3] = np.inf, np.nan, 0.0
+    signs = synthetic.make_signs(padded, 42)
+    for bits in (2, 3, 4):
+        per = 8 // bits
+        codes = rng.integers(0, 1 << bits, (n, padded // per, per), dtype=np.uint8)
+        low = (codes << (bits * np.arange(per, dtype=np.uint8))).sum(axis=2).astype(np.uint8)
+        high = (codes << (bits * np.arange(per - 1, -1, -1, dtype=np.uint8))).sum(axis=2).astype(np.uint8)
+        want = oracle.dequantize_flat(low, norms, signs.numpy(), dim, bits)
+        for packed, order in ((low, False), (high, True)):
+            out = _cabi.dequantize_flat(torch.from_numpy(packed).to(DEV), torch.from_numpy(norms).to(DEV), signs.to(DEV), dim, bits, cache_order=order)
+            np.testing.assert_array_equal(out.cpu().numpy(), want, err_msg=f"bits {bits} cache order {order}")
+    # factors other than +-1, against the four-lane kernel (the same rows in short calls)
+    signs = torch.from_numpy(rng.normal(size=padded).astype(np.float32)).to(DEV)
+    packed, norms = torch.from_numpy(low).to(DEV), torch.from_numpy(norms).to(DEV)
+    parts = [_cabi.dequantize_flat(packed[i:i + 2000], norms[i:i + 2000], signs, dim, 4) for i in range(0, n, 2000)]
+    assert torch.equal(_cabi.dequantize_flat(packed, norms, signs, dim, 4).nan_to_num(), torch.cat(parts).nan_to_num())
