@@ -1,4 +1,4 @@
-"""The cache write of more than 8192 16-bit rows padded to 64 or 256, a lane (two lanes) a row.  Every byte equals the oracle's, and over many random
+"""The cache write of many 16-bit rows of 96, or padded to 64 or 256, a lane (two lanes) a row.  Every byte equals the oracle's, and over many random
 rows that of the kernel that divides and searches for every element."""
 import numpy as np
 import pytest
@@ -60,7 +60,7 @@ def _codes(cache):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d,heads,tokens", [(64, 8, 523), (64, 1, 4129), (64, 20, 211), (64, 3, 1400), (56, 6, 701), (256, 8, 521), (256, 1, 4111), (256, 5, 833),
-                                            (192, 16, 259), (136, 2, 2051)])
+                                            (192, 16, 259), (136, 2, 2051), (96, 8, 1030), (96, 40, 207), (96, 3, 2735)])
 def test_large_writes_vs_oracle(oracle, d, heads, tokens, dtype):
     gen = torch.Generator().manual_seed(d + heads)
     k = _special(torch.randn(tokens, heads, d, generator=gen), dtype).to(dtype)
@@ -93,7 +93,7 @@ def test_large_writes_vs_oracle(oracle, d, heads, tokens, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("d,slot", [(64, None), (64, 64), (256, None), (256, 160)])
+@pytest.mark.parametrize("d,slot", [(64, None), (64, 64), (256, None), (256, 160), (96, None)])
 def test_volume_vs_the_dividing_kernel(d, slot, dtype):
     gen = torch.Generator(device=DEV)
     gen.manual_seed(d)
@@ -112,7 +112,7 @@ def test_volume_vs_the_dividing_kernel(d, slot, dtype):
     np.testing.assert_array_equal(got, want)
 
 
-@pytest.mark.parametrize("d", [64, 256])
+@pytest.mark.parametrize("d", [64, 96, 256])
 def test_norms_whose_significand_is_all_ones(oracle, d):
     """There the refined reciprocal may miss the IEEE quotient."""
     gen = torch.Generator().manual_seed(5)
@@ -132,7 +132,7 @@ def test_norms_whose_significand_is_all_ones(oracle, d):
     flips = torch.randint(0, 2, (9600, 4), generator=gen) * 2.0 - 1.0
     x.view(-1, d)[:, :4] = four * flips * torch.exp2(torch.randint(-10, 11, (9600, 1), generator=gen).float())
     x = x.to(torch.bfloat16)
-    signs = synthetic.make_signs(d, 42)
+    signs = synthetic.make_signs(1 << (d - 1).bit_length(), 42)
     slots = torch.arange(1200)
     want = np.full((2, 75, 16, 8, _slot(d)), 0xEE, np.uint8)
     oracle.write_kv_cache(want, x.float().numpy(), x.float().numpy(), signs.numpy(), slots.numpy(), d)

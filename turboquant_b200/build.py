@@ -81,7 +81,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = PKG / "build"
     obj_dir.mkdir(exist_ok=True)
-    deps = [CSRC / "tq_common.cuh", CSRC / "tq_decode_common.cuh", HEADER, Path(__file__)]
+    deps = [CSRC / "tq_common.cuh", CSRC / "tq_rows.cuh", CSRC / "tq_decode_common.cuh", HEADER, Path(__file__)]
 
     def compile_one(item):
         name, extra = item

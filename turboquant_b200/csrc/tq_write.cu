@@ -999,6 +999,11 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
                TQ_ERR_INVALID, "token stride smaller than one token");
     TQ_REQUIRE(((uintptr_t)kv_cache % 16) == 0, TQ_ERR_INVALID, "kv_cache must be 16-byte aligned");
 
+    int rows_rc = TQ_OK;
+    if (head_dim == 96 && (flags & (TQ_WRITE_EXACT_PATH | TQ_WRITE_TENSOR_PATH)) == 0 &&
+        write_rows(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, key, value, in_dtype, num_tokens, k_token_stride, v_token_stride, signs,
+                   slot_mapping, slot_dtype, head_dim, flags, stream, &rows_rc))
+        return rows_rc;
     // A decode step's new tokens (a few rows per SM at most): a warp per row.  The limit is where it stops being the faster one.
     if ((flags & (TQ_WRITE_EXACT_PATH | TQ_WRITE_TENSOR_PATH)) == 0 && 2 * num_tokens * num_kv_heads <= 2048)
         return generic_write(kv_cache, num_blocks, block_size, num_kv_heads, slot_bytes, key, value, in_dtype, num_tokens, k_token_stride,
@@ -1033,7 +1038,7 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
     if (rc != TQ_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Large writes of 16-bit rows go to the tensor-core kernel; small ones (a decode step's new
-    // tokens), fp32 rows and padded heads keep the kernel that needs no tables beyond one.
+    // tokens), fp32 rows and smaller writes of 96-wide ones keep the kernel that needs no tables beyond one.
     const bool exact_only = (flags & TQ_WRITE_EXACT_PATH) != 0, tensor_only = (flags & TQ_WRITE_TENSOR_PATH) != 0;
     TQ_REQUIRE(!(exact_only && tensor_only), TQ_ERR_INVALID, "TQ_WRITE_EXACT_PATH and TQ_WRITE_TENSOR_PATH exclude each other");
     TQ_REQUIRE(!tensor_only || (head_dim == 128 && in_dtype != TQ_F32), TQ_ERR_UNSUPPORTED,
