@@ -101,3 +101,32 @@ def test_dequantization_of_many_rows(oracle, dim, n):
     packed, norms = torch.from_numpy(low).to(DEV), torch.from_numpy(norms).to(DEV)
     parts = [_cabi.dequantize_flat(packed[i:i + 2000], norms[i:i + 2000], signs, dim, 4) for i in range(0, n, 2000)]
     assert torch.equal(_cabi.dequantize_flat(packed, norms, signs, dim, 4).nan_to_num(), torch.cat(parts).nan_to_num())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8192 + 17), (96, 8192 + 31), (72, 8195), (64, 16384), (64, 16384 + 33), (256, 4096), (256, 4096 + 15), (192, 4099)])
+def test_quantization_of_many_rows(oracle, dim, n, dtype):
+    """A lane (two lanes) a row: the fewest rows that go this way, part units, short rows, special rows, every width and both pack orders."""
+    signs = synthetic.make_signs(1 << (dim - 1).bit_length(), 42)
+    x = _rows(n, dim, dtype, 7 + dim + n)
+    if dtype == torch.bfloat16:
+        x[20, 5], x[21] = 1e-30, 0.0                       # a tiny value among ordinary ones; a zero row
+        x[22] *= 1e-35
+    for bits in (1, 2, 3, 4):
+        per = 8 // bits
+        want_p, want_n = oracle.quantize_flat(x.float().numpy(), signs.numpy(), bits)
+        codes = (want_p[:, :, None] >> (bits * np.arange(per, dtype=np.uint8))) & ((1 << bits) - 1)
+        want_c = (codes << (bits * np.arange(per - 1, -1, -1, dtype=np.uint8))).sum(axis=2).astype(np.uint8)
+        for cache_order, want in ((False, want_p), (True, want_c)):
+            p, norms = _cabi.quantize_flat(x.to(DEV), signs.to(DEV), bits, cache_order=cache_order)
+            np.testing.assert_array_equal(p.cpu().numpy(), want, err_msg=f"bits {bits} cache order {cache_order}")
+            np.testing.assert_array_equal(norms.cpu().numpy(), want_n)
+    # factors other than +-1, against the four-lane kernel (the same rows in short calls)
+    g = torch.Generator().manual_seed(n)
+    for factors in (torch.randn(signs.numel(), generator=g), 3e30 * signs, torch.where(torch.arange(signs.numel()) == 5, float("nan"), signs)):
+        factors = factors.to(DEV)
+        for bits in (2, 4):
+            p, norms = _cabi.quantize_flat(x.to(DEV), factors, bits)
+            parts = [_cabi.quantize_flat(x[i:i + 2000].to(DEV), factors, bits) for i in range(0, n, 2000)]
+            assert torch.equal(p, torch.cat([a for a, _ in parts]))
+            np.testing.assert_array_equal(norms.cpu().numpy(), torch.cat([b for _, b in parts]).cpu().numpy())

@@ -32,6 +32,7 @@ UNITS = {
     "tq_write_rows.cu": ["-fmad=false"],
     "tq_flat.cu": ["-fmad=false"],
     "tq_flat_rows.cu": ["-fmad=false"],
+    "tq_flat_quant.cu": ["-fmad=false"],
     "tq_decode.cu": [],
     "tq_decode_mq.cu": [],
     "tq_decode_split.cu": [],

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32) fwht_kernel(const __grid_cons
 // of the cache write, with bins scaled to the row's length).
 // 65536 rows of 128 fp16 values, 4 bits: quantize 107 us with the plain kernel (a warp a row, butterflies in shared memory, a
 // compare per boundary: 20 times the memory floor) -> 15 us here (dequantize 77 -> 13 us); the limits are instruction issue and the shuffles of stages 2 and 4.
-// Dequantization of many rows goes a lane a row (tq_flat_rows.cu).
+// Many rows go a lane a row: 16-bit ones to codes by tq_flat_quant.cu, codes to rows by tq_flat_rows.cu.
 // ---------------------------------------------------------------------------------------------
 constexpr int kRowsWarps = 8, kRowsThreads = kRowsWarps * 32;
 constexpr int kFlatBinZero = 144, kFlatBins = 2 * kFlatBinZero + 1;      // |y| <= 1.5 in bins of sqrt(128 / padded) / 64: 136 at 256
@@ -422,6 +422,9 @@ __global__ void __launch_bounds__(kRowsThreads, E == 8 ? 5 : E == 16 ? 4 : 2) de
 bool dequantize_lanes(const uint8_t* packed, const float* norms, int64_t n, int dim, int padded, const float* signs, int bits, bool cache_order, float* out,
                       void* stream, int* rc);
 
+bool quantize_lanes(const void* x, int x_dtype, int64_t n, int dim, int padded, const float* signs, int bits, bool cache_order, uint8_t* packed, float* norms,
+                    void* stream, int* rc);
+
 static int next_pow2(int n) {
     int p = 1;
     while (p < n) p <<= 1;
@@ -534,6 +537,8 @@ extern "C" int tq_quantize_flat(const void* x, int x_dtype, int64_t n, int dim, 
     p.padded = next_pow2(dim); p.bits = bits; p.cache_order = pack_order == TQ_PACK_CACHE;
     p.scale = (float)(1.0 / std::sqrt((double)p.padded));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int rc = TQ_OK;
+    if (quantize_lanes(x, x_dtype, n, dim, p.padded, signs, bits, p.cache_order, packed, norms, stream, &rc)) return rc;
     if (rows_kernel_takes(dim, p.padded, x, x_dtype == TQ_F32 ? 8 : 4, packed, 4) && x_dtype >= TQ_F32 && x_dtype <= TQ_BF16) {
         const FlatBinTable& t = flat_bins(p.padded, bits);
         if (t.ok) {
