@@ -171,3 +171,20 @@ def test_volume_random_rows(dtype):
     share = flagged / total
     print(f"{dtype}: {total} rows, {flagged} re-derived exactly ({100 * share:.2f} %)")
     assert 0.005 < share < 0.08
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,tokens", [(1, 33), (3, 17), (5, 40), (6, 9), (8, 3), (16, 5), (40, 7), (48, 2)])
+def test_strided_tiles_of_heads_and_tokens(oracle, golden, heads, tokens, dtype):
+    """Inputs that are not dense go a box of heads and tokens a tile: head counts that make boxes of 1 ... 16 heads, part boxes, and K dense beside a strided V."""
+    gen = torch.Generator().manual_seed(heads)
+    both = (torch.randn(tokens, 2 * heads + 1, 128, generator=gen) * 2.0).to(dtype)
+    k, v = both[:, :heads], both[:, heads:2 * heads]
+    nb = (tokens + 15) // 16 + 1
+    slots = torch.randperm(nb * 16, generator=gen)[:tokens]
+    slots[tokens // 2] = -1
+    want = np.full((2, nb, 16, heads, 80), 0xEE, np.uint8)
+    oracle.write_kv_cache(want, k.float().contiguous().numpy(), v.float().contiguous().numpy(), golden["signs_seed42_d128"], slots.numpy(), 128)
+    d = both.to(DEV)
+    for kd, vd in ((d[:, :heads], d[:, heads:2 * heads]), (d[:, :heads].contiguous(), d[:, heads:2 * heads])):
+        np.testing.assert_array_equal(write(kd, vd, slots.to(DEV), nb, "tensor", H=heads, fill=0xEE).cpu().numpy(), want)

@@ -57,7 +57,9 @@ struct WriteParams {
     const float* signs;       // [128] +-1, device
     float2 bin_table[kBins];  // per bin of y: {boundary inside the bin or +inf, number of boundaries in lower bins}
     float fwht_scale;         // (float)(1/sqrt(128))
-    // tensor-core kernel, dense inputs: key / value as [rows][128] tensors, boxes of 16 rows x 64 elements
+    // tensor-core kernel: dense key / value as [rows][128] tensors, boxes of 64 elements x 16 rows; else as [tokens][heads][128], boxes of 64 elements x
+    // box_heads (a power of two) x 16 / box_heads tokens
+    int box_heads, box_shift, head_boxes;   // box_shift: log2(box_heads); head_boxes: boxes that make up the heads
     alignas(64) CUtensorMap tmap[2];
 };
 
@@ -439,19 +441,21 @@ static int launch_write(const WriteParams& p, int sm_count, cudaStream_t stream)
 //     least 24 bits, so each addend loses less than 2^-23 of that largest one -- times 8 chunks,
 //     50 u * norm from the three fp32 stages, 1.5 u relative from the rounded scale factor.
 //     Together |y_fast - y_ref| < 55 u = 3.3e-6.  A code is taken from y_fast only when y_fast is
-//     farther than 2^-18 = 3.8e-6 from the boundary of its bin: z = (y_fast - b) * 2^17 + 1/2,
-//     s = saturate(z) is exactly 0 or 1 then, and code = (boundaries in lower bins) + s.  Any
-//     s strictly between 0 and 1 makes sum s (1 - s) positive for the row (non-negative terms, so
-//     nothing cancels), and such a row is done again by the exact path below, 32 lanes on one row,
+//     farther than 2^-18 (1 - 2^-8) = 3.80e-6 from the boundary of its bin: z = (y_fast - b) * 2^17 + 1/2,
+//     s = saturate(z) is within 2^-9 of 0 or 1 then, and code = (boundaries in lower bins) + s, whose sum is
+//     formed at a scale that keeps eight bits of the fraction.  Any of them set in the bits of a row's sums (or'ed together)
+//     and the row is done again by the exact path below, 32 lanes on one row,
 //     from the staged input.  About 3.6 % of N(0,1) rows take it.  Rows whose norm is not a
 //     moderate finite number (zero rows, overflowing or non-finite rows) always take it.
 //   * The bins of y_fast are formed from Y * (64 * f) rather than from the rounded y, so next to a
 //     bin edge the two paths may pick neighbouring bins; the host checks that no boundary lies
 //     within 2^-13 of a bin edge, which makes both bins give the same code there.
-//   * Staging.  Dense inputs (token stride = heads x 128) are fetched by tiled tensor copies
+//   * Staging.  A tile is 16 rows: consecutive ones of dense inputs, a box of neighbouring heads and tokens of others (K / V as column slices of a fused
+//     projection; as boxes dense inputs take 3 - 6 % longer), fetched by tiled tensor copies
 //     (cp.async.bulk.tensor, two boxes of 16 rows x 128 bytes per tile, 128-byte swizzle, issued
-//     by one lane); the swizzle makes the ldmatrix reads conflict free.  Strided inputs (K / V as
-//     column slices of a fused projection) use one bulk copy per row into rows of 272 bytes.
+//     by one lane); the swizzle makes the ldmatrix reads conflict free.
+//   * Latency bounds it, not issue: 7 % fewer instructions (fused squares, flags and codes in integers) at 16 warps a block of 128 registers
+//     changed nothing, the 20 warps of 96 that they leave room for did: 32768 x 8 bf16 58.4 -> 55.8 us, 2000 x 40 23.0 -> 22.0, 600 x 8 5.2 -> 4.8.
 // =============================================================================================
 constexpr float kGuardBig = 131072.0f;  // 2^17
 
@@ -488,13 +492,11 @@ struct MmaOps<__half> {
     }
 };
 
-// Shared-memory map of the tensor-core kernel.  A warp's stage buffer holds its 16-row tile either
-// as two swizzled halves of 16 rows x 128 bytes (tensor copies) or as rows of 272 bytes (per-row
-// copies; 272 = 16 mod 128, so the eight rows of an ldmatrix hit different banks).
+// Shared-memory map of the tensor-core kernel.  A warp's stage buffer holds its 16-row tile as two swizzled halves of 16 rows x 128 bytes.
 struct MmaShape {
-    static constexpr int kThreads = 512, kWarps = 16, kRows = 16;
-    static constexpr int kRowBytes = 256, kPitch = 272;
-    static constexpr int kWarpStage = 5120;                        // >= 16 x 272, a multiple of 1024 (swizzle atom)
+    static constexpr int kThreads = 640, kWarps = kThreads / 32, kRows = 16;      // 96 registers a thread
+    static constexpr int kRowBytes = 256;
+    static constexpr int kWarpStage = kRows * kRowBytes;           // a multiple of 1024 (swizzle atom)
     static constexpr size_t kStageBytes = (size_t)2 * kWarps * kWarpStage;
     static constexpr size_t kTableBytes = (size_t)kBins * 16 * 8 + 1024;  // 16 columns of 8-byte entries + the boundaries
     static constexpr size_t kBfragBytes = (size_t)8 * 32 * 16;     // B fragments of the 8 chunks, per lane
@@ -512,37 +514,43 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& a0, uint32_
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(addr));
 }
-// Tiled tensor copy global -> shared of one box at element coordinates (x, y), completing on an
-// mbarrier.  x times the element size is a multiple of 16 bytes at both call sites (0 and 128).
+// Tiled tensor copies global -> shared of one box at element x of row y, or of head y of token z, completing on an
+// mbarrier.  x times the element size is a multiple of 16 bytes at all call sites (0 and 128).
 __device__ __forceinline__ void tensor_g2s_2d(void* dst_smem, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tensor_g2s_3d(void* dst_smem, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
 
-// One code byte (even dim in the high nibble) of the pair (Y0, Y1) of one row, as a float, and the
-// row's ambiguity sum.  Table entry of a bin (8 bytes, 16 columns: an 8-byte load is served half a
-// warp at a time, so lookups never conflict): {1/2 - b * 2^17 (or -inf), boundaries in lower bins}.
-__device__ __forceinline__ float guarded_byte(P2 Y2, P2 kf2, float zf, uint32_t table_lane, P2& amb) {
+// The code byte (even dim in the high nibble) of the pair (Y0, Y1) of one row, in bits 8 ... 15 of the result, and what flags the row.  Table entry of a bin
+// (8 bytes, 16 columns: an 8-byte load is served half a warp at a time, so lookups never conflict): {1/2 - b * 2^17 (or -inf), kCodeMagic + boundaries in
+// lower bins}.  The sum of that and s has the code in bits 8 ... 11 and the fraction of s, to 2^-8, below them: zero exactly when s is within 2^-9 of 0 or 1.
+constexpr float kCodeMagic = 32768.0f;
+__device__ __forceinline__ uint32_t guarded_byte(P2 Y2, P2 kf2, float zf, uint32_t table_lane, uint32_t& amb) {
     float Y0, Y1, k0, k1;
     up(Y2, Y0, Y1);
     up(fma2(Y2, kf2, pk(kBinMagic, kBinMagic)), k0, k1);
     float c0, below0, c1, below1;
     asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c0), "=f"(below0) : "r"(__float_as_uint(k0) * 128u + table_lane));
     asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c1), "=f"(below1) : "r"(__float_as_uint(k1) * 128u + table_lane));
-    const float s0 = fma_sat(Y0, zf, c0), s1 = fma_sat(Y1, zf, c1);
-    const P2 s2 = pk(s0, s1);
-    amb = fma2(s2, sub2(pk(1.0f, 1.0f), s2), amb);  // s (1 - s): zero exactly when s is 0 or 1
-    return __fmaf_rn(__fadd_rn(s0, below0), 16.0f, __fadd_rn(s1, below1));
+    const uint32_t n0 = __float_as_uint(__fadd_rn(fma_sat(Y0, zf, c0), below0)), n1 = __float_as_uint(__fadd_rn(fma_sat(Y1, zf, c1), below1));
+    amb |= n0 | n1;
+    return (n0 << 4) + n1;
 }
 
-template <typename T, bool TMA>
+template <typename T, bool DENSE>
 __global__ void __launch_bounds__(MmaShape::kThreads, 1)
 write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
     using O = MmaOps<T>;
     using W = MmaShape;
-    constexpr int kPitch = W::kPitch, kRows = W::kRows;
+    constexpr int kRows = W::kRows;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[W::kWarps][2];
     __shared__ __align__(16) float signs_s[kD];
@@ -556,7 +564,9 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
     const int row_in_warp = lane >> 1;
     const int H = p.num_kv_heads;
     const int64_t rows = p.num_tokens * H;
-    const int64_t num_tiles = 2 * ((rows + kRows - 1) / kRows);  // K and V tiles alternate
+    const int box_tokens = DENSE ? 0 : kRows >> p.box_shift;
+    // K and V tiles alternate
+    const int64_t num_tiles = 2 * (DENSE ? (rows + kRows - 1) / kRows : (p.num_tokens + box_tokens - 1) / box_tokens * p.head_boxes);
 
     grid_launch_dependents();
     if (lane == 0) {
@@ -568,7 +578,7 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
     float* bnd_s = reinterpret_cast<float*>(smem + W::kStageBytes + (size_t)kBins * 16 * 8);  // exact path only
     for (int i = tid; i < kBins * 16; i += W::kThreads) {
         const float2 e = p.bin_table[i >> 4];  // {boundary inside the bin or +inf, boundaries in lower bins}
-        tab_s[i] = make_float2(e.x < INFINITY ? __fmaf_rn(-e.x, kGuardBig, 0.5f) : -INFINITY, e.y);
+        tab_s[i] = make_float2(e.x < INFINITY ? __fmaf_rn(-e.x, kGuardBig, 0.5f) : -INFINITY, __fadd_rn(e.y, kCodeMagic));
         if ((i & 15) == 0) bnd_s[i >> 4] = e.x;
     }
     const uint32_t table_lane = smem_u32(tab_s) + 8u * (lane & 15) - 0x80000000u;
@@ -594,31 +604,33 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
     grid_dependency_wait();  // K, V, the slots and the cache belong to earlier kernels
     __syncthreads();
 
+    // first token and head of a tile
+    auto place = [&](int64_t tile, int& t0, int& h0) {
+        const int64_t k = tile >> 1;
+        int64_t tb = k;
+        h0 = 0;
+        if (p.head_boxes > 1) {
+            tb = k < 0x7fffffff ? (int64_t)((uint32_t)k / (uint32_t)p.head_boxes) : k / p.head_boxes;
+            h0 = (int)(k - tb * p.head_boxes) << p.box_shift;
+        }
+        t0 = (int)(tb * box_tokens);      // num_tokens fits the copy's 32-bit coordinate
+    };
     auto issue = [&](int64_t tile, int buf) {
         const int which = (int)(tile & 1);
-        const int64_t row0 = (tile >> 1) * kRows;
         uint8_t* dst0 = smem + ((size_t)buf * W::kWarps + warp) * W::kWarpStage;
+        int t0 = 0, h0 = 0;
+        if (!DENSE) place(tile, t0, h0);
         fence_proxy_async();  // earlier shared-memory reads of this buffer precede the copy engine's writes
-        if (TMA) {
-            // two boxes of 16 rows x 64 elements; rows past the end of the tensor arrive as zeros
-            if (lane == 0) {
-                mbar_arrive_expect_tx(&full_bar[warp][buf], (uint32_t)(kRows * W::kRowBytes));
-                tensor_g2s_2d(dst0, &p.tmap[which], 0, (int)row0, &full_bar[warp][buf]);
-                tensor_g2s_2d(dst0 + 2048, &p.tmap[which], 64, (int)row0, &full_bar[warp][buf]);
-            }
-        } else {
-            const int64_t left = rows - row0;
-            const int64_t nrows = left < kRows ? left : (int64_t)kRows;
-            if (lane == 0) mbar_arrive_expect_tx(&full_bar[warp][buf], (uint32_t)(nrows * W::kRowBytes));
-            __syncwarp();
-            if (lane < nrows) {
-                const int64_t r = row0 + lane;
-                int64_t t;
-                int h;
-                split_row(r, H, p.head_shift, t, h);
-                const T* src = reinterpret_cast<const T*>(p.src[which]) + t * p.token_stride[which] + (int64_t)h * kD;
-                bulk_g2s(dst0 + (size_t)lane * kPitch, src, W::kRowBytes, &full_bar[warp][buf]);
-            }
+        // two boxes of 16 rows x 64 elements; rows past the end arrive as zeros
+        if (DENSE && lane == 0) {
+            const int row0 = (int)((tile >> 1) * kRows);
+            mbar_arrive_expect_tx(&full_bar[warp][buf], (uint32_t)(kRows * W::kRowBytes));
+            tensor_g2s_2d(dst0, &p.tmap[which], 0, row0, &full_bar[warp][buf]);
+            tensor_g2s_2d(dst0 + 2048, &p.tmap[which], 64, row0, &full_bar[warp][buf]);
+        } else if (!DENSE && lane == 0) {
+            mbar_arrive_expect_tx(&full_bar[warp][buf], (uint32_t)(kRows * W::kRowBytes));
+            tensor_g2s_3d(dst0, &p.tmap[which], 0, h0, t0, &full_bar[warp][buf]);
+            tensor_g2s_3d(dst0 + 2048, &p.tmap[which], 64, h0, t0, &full_bar[warp][buf]);
         }
     };
 
@@ -636,24 +648,32 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
         if (next < num_tiles) issue(next, buf ^ 1);
 
         const int which = (int)(tile & 1);
-        const int64_t r = (tile >> 1) * kRows + row_in_warp;  // the row this lane stores
-        const bool row_ok = r < rows;
-        int64_t slot = -1;
+        // the row this lane stores
+        int64_t t = 0;
         int h = 0;
+        bool row_ok;
+        if (DENSE) {
+            const int64_t r = (tile >> 1) * kRows + row_in_warp;
+            row_ok = r < rows;
+            if (row_ok) split_row(r, H, p.head_shift, t, h);
+        } else {
+            int t0, h0;
+            place(tile, t0, h0);
+            t = t0 + (row_in_warp >> p.box_shift);
+            h = h0 + (row_in_warp & (p.box_heads - 1));
+            row_ok = t < p.num_tokens;
+        }
+        int64_t slot = -1;
         if (row_ok) {
-            int64_t t;
-            split_row(r, H, p.head_shift, t, h);
             slot = p.slot_is_i64 ? reinterpret_cast<const int64_t*>(p.slot_mapping)[t]
                                  : (int64_t) reinterpret_cast<const int32_t*>(p.slot_mapping)[t];
         }
         if (!mbar_wait(&full_bar[warp][buf], (it >> 1) & 1)) return;
         const uint8_t* stage = smem + ((size_t)buf * W::kWarps + warp) * W::kWarpStage;
-        // Rows past the end of the tensor hold zeros or stale bytes: they are computed like any
-        // others (whatever they contain ends in a finite code or in the exact path) and never stored.
+        // Rows past the end of the tensor hold zeros: they are computed like any others and never stored.
         // byte address of 16-byte piece `piece` (0..15) of row `row` of the staged tile
         auto piece_addr = [&](int row, int piece) -> uint32_t {
-            if (TMA) return smem_u32(stage) + (piece >> 3) * 2048 + row * 128 + (((piece & 7) ^ (row & 7)) << 4);
-            return smem_u32(stage) + row * kPitch + piece * 16;
+            return smem_u32(stage) + (piece >> 3) * 2048 + row * 128 + (((piece & 7) ^ (row & 7)) << 4);
         };
 
         // ---- chunk products (stages h = 1..8) and the exact sums of squares -----------------------
@@ -673,10 +693,11 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
             // elements 8 (2c) + 2tg, +1; e1 = elements 8 (2c + 1) + 2tg, +1.
             O::mma(e0, a0, a1, a2, a3, ident, 0u);
             O::mma(e1, a0, a1, a2, a3, 0u, ident);
-            P2 x2 = pk(e0[0], e0[1]); n_lo = add2(n_lo, mul2(x2, x2));
-            x2 = pk(e0[2], e0[3]); n_hi = add2(n_hi, mul2(x2, x2));
-            x2 = pk(e1[0], e1[1]); n_lo = add2(n_lo, mul2(x2, x2));
-            x2 = pk(e1[2], e1[3]); n_hi = add2(n_hi, mul2(x2, x2));
+            // squares of 16-bit values are exact: one rounding, that of the sum
+            P2 x2 = pk(e0[0], e0[1]); n_lo = fma2(x2, x2, n_lo);
+            x2 = pk(e0[2], e0[3]); n_hi = fma2(x2, x2, n_hi);
+            x2 = pk(e1[0], e1[1]); n_lo = fma2(x2, x2, n_lo);
+            x2 = pk(e1[2], e1[3]); n_hi = fma2(x2, x2, n_hi);
         }
         // the eight accumulators of a row sit in its quad, two per lane: combine them left to right
         float norm_lo, norm_hi;
@@ -722,7 +743,7 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
         // ---- guarded codes: bytes 8c + 2tg and 8c + 2tg + 1 of rows g and g + 8 ---------------------
         uint8_t* orow_lo = out_s + (size_t)(warp * kRows + g) * W::kOutPitch + 2 * tg;
         uint8_t* orow_hi = orow_lo + 8 * W::kOutPitch;
-        P2 amb_lo = pk(0.0f, 0.0f), amb_hi = pk(0.0f, 0.0f);
+        uint32_t amb_lo = 0, amb_hi = 0;
         const float zf_lo = f_lo * kGuardBig, zf_hi = f_hi * kGuardBig;
         const P2 kf_lo = pk(f_lo * 64.0f, f_lo * 64.0f), kf_hi = pk(f_hi * 64.0f, f_hi * 64.0f);
         // A row off the fast path (norm zero, huge or not finite) may hold values whose bin is not a
@@ -731,41 +752,36 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
         if (__all_sync(0xffffffffu, fast_lo && fast_hi)) {
 #pragma unroll
             for (int c = 0; c < 8; c++) {
-                const float b0 = guarded_byte(v[c][0][0], kf_lo, zf_lo, table_lane, amb_lo);
-                const float b1 = guarded_byte(v[c][1][0], kf_lo, zf_lo, table_lane, amb_lo);
+                const uint32_t b0 = guarded_byte(v[c][0][0], kf_lo, zf_lo, table_lane, amb_lo);
+                const uint32_t b1 = guarded_byte(v[c][1][0], kf_lo, zf_lo, table_lane, amb_lo);
                 *reinterpret_cast<uint16_t*>(orow_lo + 8 * c) =
-                    (uint16_t)__float_as_uint(__fadd_rn(__fmaf_rn(b1, 256.0f, b0), 8388608.0f));
-                const float b2 = guarded_byte(v[c][0][1], kf_hi, zf_hi, table_lane, amb_hi);
-                const float b3 = guarded_byte(v[c][1][1], kf_hi, zf_hi, table_lane, amb_hi);
+                    (uint16_t)__byte_perm(b0, b1, 0x4451);
+                const uint32_t b2 = guarded_byte(v[c][0][1], kf_hi, zf_hi, table_lane, amb_hi);
+                const uint32_t b3 = guarded_byte(v[c][1][1], kf_hi, zf_hi, table_lane, amb_hi);
                 *reinterpret_cast<uint16_t*>(orow_hi + 8 * c) =
-                    (uint16_t)__float_as_uint(__fadd_rn(__fmaf_rn(b3, 256.0f, b2), 8388608.0f));
+                    (uint16_t)__byte_perm(b2, b3, 0x4451);
             }
         } else {
             if (fast_lo) {
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
-                    const float b0 = guarded_byte(v[c][0][0], kf_lo, zf_lo, table_lane, amb_lo);
-                    const float b1 = guarded_byte(v[c][1][0], kf_lo, zf_lo, table_lane, amb_lo);
+                    const uint32_t b0 = guarded_byte(v[c][0][0], kf_lo, zf_lo, table_lane, amb_lo);
+                    const uint32_t b1 = guarded_byte(v[c][1][0], kf_lo, zf_lo, table_lane, amb_lo);
                     *reinterpret_cast<uint16_t*>(orow_lo + 8 * c) =
-                        (uint16_t)__float_as_uint(__fadd_rn(__fmaf_rn(b1, 256.0f, b0), 8388608.0f));
+                        (uint16_t)__byte_perm(b0, b1, 0x4451);
                 }
             }
             if (fast_hi) {
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
-                    const float b2 = guarded_byte(v[c][0][1], kf_hi, zf_hi, table_lane, amb_hi);
-                    const float b3 = guarded_byte(v[c][1][1], kf_hi, zf_hi, table_lane, amb_hi);
+                    const uint32_t b2 = guarded_byte(v[c][0][1], kf_hi, zf_hi, table_lane, amb_hi);
+                    const uint32_t b3 = guarded_byte(v[c][1][1], kf_hi, zf_hi, table_lane, amb_hi);
                     *reinterpret_cast<uint16_t*>(orow_hi + 8 * c) =
-                        (uint16_t)__float_as_uint(__fadd_rn(__fmaf_rn(b3, 256.0f, b2), 8388608.0f));
+                        (uint16_t)__byte_perm(b2, b3, 0x4451);
                 }
             }
         }
-        float al0, al1, ah0, ah1;
-        up(amb_lo, al0, al1);
-        up(amb_hi, ah0, ah1);
-        // NaN compares false on "== 0": a row that produced NaNs is flagged as well
-        const bool flag_lo = !fast_lo || !(__fadd_rn(al0, al1) == 0.0f);
-        const bool flag_hi = !fast_hi || !(__fadd_rn(ah0, ah1) == 0.0f);
+        const bool flag_lo = !fast_lo || (amb_lo & 0xffu) != 0, flag_hi = !fast_hi || (amb_hi & 0xffu) != 0;
         uint32_t m_lo = __ballot_sync(0xffffffffu, flag_lo), m_hi = __ballot_sync(0xffffffffu, flag_hi);
         m_lo = (m_lo | (m_lo >> 1) | (m_lo >> 2) | (m_lo >> 3)) & 0x11111111u;  // bit 4g: row g flagged
         m_hi = (m_hi | (m_hi >> 1) | (m_hi >> 2) | (m_hi >> 3)) & 0x11111111u;
@@ -823,7 +839,7 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
                     } else {
                         const float kf = __fmaf_rn(yy, 64.0f, kBinMagic);
                         const uint32_t bin = __float_as_uint(kf) - 0x4B000000u;
-                        const float below = tab_s[bin * 16 + (lane & 15)].y;
+                        const float below = __fsub_rn(tab_s[bin * 16 + (lane & 15)].y, kCodeMagic);
                         code[i] = yy > bnd_s[bin] ? __fadd_rn(below, 1.0f) : below;
                     }
                 }
@@ -868,35 +884,45 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
 bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
                        const cuuint32_t* box, CUtensorMapSwizzle swizzle);
 
-// [rows][128] 16-bit elements, row pitch 256 bytes, boxes of 16 rows x 64 elements with the 128-byte swizzle
-static bool encode_rows_map(CUtensorMap* map, const void* base, int64_t rows, bool is_bf16) {
-    const cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)kD * 2};
-    const cuuint32_t box[2] = {64u, (cuuint32_t)MmaShape::kRows};
-    return encode_tensor_map(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-}
-
-template <typename T>
-static int launch_write_mma(WriteParams& p, int sm_count, cudaStream_t stream) {
+template <typename T, bool DENSE>
+static int launch_write_mma_kernel(const WriteParams& p, int64_t tiles, int sm_count, cudaStream_t stream) {
     using W = MmaShape;
-    const int64_t rows = p.num_tokens * p.num_kv_heads;
-    // tensor copies need dense [rows][128] tensors whose row index fits the copy's 32-bit coordinate
-    const bool dense = p.token_stride[0] == (int64_t)p.num_kv_heads * kD && p.token_stride[1] == (int64_t)p.num_kv_heads * kD &&
-                       rows < (int64_t)0x7fffffff;
-    const bool tma = dense && encode_rows_map(&p.tmap[0], p.src[0], rows, sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value) &&
-                     encode_rows_map(&p.tmap[1], p.src[1], rows, std::is_same<T, __nv_bfloat16>::value);
-    auto kernel = tma ? write_kv_cache_mma_kernel<T, true> : write_kv_cache_mma_kernel<T, false>;
-    static bool configured[2][64] = {};
+    static bool configured[64] = {};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[tma][dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::kSmem));
-        if (dev >= 0 && dev < 64) configured[tma][dev] = true;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        TQ_CUDA(cudaFuncSetAttribute(write_kv_cache_mma_kernel<T, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::kSmem));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const int64_t tiles = 2 * ((rows + W::kRows - 1) / W::kRows);
-    const int64_t grid = tiles < (int64_t)sm_count ? tiles : (int64_t)sm_count;
-    TQ_CUDA(launch_serialized(kernel, dim3((unsigned)grid), dim3(W::kThreads), W::kSmem, stream, p));
+    TQ_CUDA(launch_serialized(write_kv_cache_mma_kernel<T, DENSE>, dim3((unsigned)(tiles < sm_count ? tiles : sm_count)), dim3(W::kThreads), W::kSmem, stream, p));
     return TQ_OK;
+}
+// Returns false, having done nothing, where no map can be made of the tensors.
+template <typename T>
+static bool launch_write_mma(WriteParams& p, int sm_count, cudaStream_t stream, int* rc) {
+    using W = MmaShape;
+    const int64_t rows = p.num_tokens * p.num_kv_heads;
+    const bool dense = p.token_stride[0] == (int64_t)p.num_kv_heads * kD && p.token_stride[1] == p.token_stride[0] && rows < 0x7fffff00;      // 32-bit coordinates
+    if (p.num_tokens >= 0x7fffff00) return false;
+    p.box_heads = 1;
+    p.box_shift = 0;
+    while (!dense && p.box_heads < W::kRows && p.num_kv_heads % (2 * p.box_heads) == 0) {
+        p.box_heads *= 2;
+        p.box_shift++;
+    }
+    p.head_boxes = p.num_kv_heads / p.box_heads;
+    const CUtensorMapDataType type = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    for (int i = 0; i < 2; i++) {
+        const cuuint64_t flat[2] = {(cuuint64_t)kD, (cuuint64_t)rows}, dims[3] = {(cuuint64_t)kD, (cuuint64_t)p.num_kv_heads, (cuuint64_t)p.num_tokens};
+        const cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)p.token_stride[i] * 2};
+        const cuuint32_t flat_box[2] = {64u, (cuuint32_t)W::kRows}, box[3] = {64u, (cuuint32_t)p.box_heads, (cuuint32_t)(W::kRows / p.box_heads)};
+        if (!encode_tensor_map(&p.tmap[i], type, dense ? 2 : 3, p.src[i], dense ? flat : dims, strides, dense ? flat_box : box, CU_TENSOR_MAP_SWIZZLE_128B))
+            return false;
+    }
+    const int tokens = W::kRows >> p.box_shift;
+    *rc = dense ? launch_write_mma_kernel<T, true>(p, 2 * ((rows + W::kRows - 1) / W::kRows), sm_count, stream)
+                : launch_write_mma_kernel<T, false>(p, 2 * ((p.num_tokens + tokens - 1) / tokens) * p.head_boxes, sm_count, stream);
+    return true;
 }
 
 int write_guard_stats(unsigned long long* out2) {
@@ -1043,8 +1069,10 @@ extern "C" int tq_write_kv_cache(void* kv_cache, int64_t num_blocks, int block_s
     TQ_REQUIRE(!(exact_only && tensor_only), TQ_ERR_INVALID, "TQ_WRITE_EXACT_PATH and TQ_WRITE_TENSOR_PATH exclude each other");
     TQ_REQUIRE(!tensor_only || (head_dim == 128 && in_dtype != TQ_F32), TQ_ERR_UNSUPPORTED,
                "the tensor-core write kernel takes fp16 / bf16 rows of 128 elements");
-    if (!exact_only && head_dim == 128 && in_dtype != TQ_F32 && (tensor_only || num_tokens * num_kv_heads >= 4096))
-        return in_dtype == TQ_F16 ? launch_write_mma<__half>(p, sms, s) : launch_write_mma<__nv_bfloat16>(p, sms, s);
+    if (!exact_only && head_dim == 128 && in_dtype != TQ_F32 && (tensor_only || num_tokens * num_kv_heads >= 4096)) {
+        if (in_dtype == TQ_F16 ? launch_write_mma<__half>(p, sms, s, &rc) : launch_write_mma<__nv_bfloat16>(p, sms, s, &rc)) return rc;
+        TQ_REQUIRE(!tensor_only, TQ_ERR_CUDA, "no tensor map of the key / value tensors");
+    }
     if (head_dim == 96) {
         switch (in_dtype) {
             case TQ_F32: return launch_write<float, 96>(p, sms, s);
