@@ -71,7 +71,8 @@ int tq_codebook(int dim, int bits, float* centroids, float* boundaries);
  * head_dim 128, or 96 (rows of 96 elements, zero-padded to 128 by the rotation; signs has 128
  * entries either way).  Any other head size from 33 to 256 (64 with 48-byte slots, 256 with
  * 144-byte slots: turboquant/vllm_backend_fused.py:64-72, turboquant/kernel_config.py:75-109)
- * goes through plain, untuned kernels with the same arithmetic; signs then has next_pow2(head_dim)
+ * goes through kernels of its own with the same arithmetic (large fp16 / bf16 writes a lane or two a row,
+ * the others plain ones); signs then has next_pow2(head_dim)
  * entries.  signs is a constant of the context, as in the reference (one seeded
  * vector per process): the kernel reads it ahead of its wait on the preceding kernel, so it must
  * be complete before that kernel is launched.
