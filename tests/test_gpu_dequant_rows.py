@@ -95,3 +95,29 @@ def test_many_sequences(oracle, dim):
     _check(oracle, dim, 1, wide=False, lens=[int(n) for n in rng.integers(0, 40, 100)])
     _check(oracle, dim, 8, wide=True, lens=[int(n) for n in rng.integers(0, 70, 70)])
     _check(oracle, dim, 16, wide=False, lens=[3, 0, 60000 if dim == 64 else 66000, 20])
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("dim,heads", [(64, 3), (96, 2), (128, 3), (256, 2)])
+def test_zeros_keep_their_sign(oracle, dim, heads, wide):
+    """Rows of repeated codes, whose sums cancel: the outputs' bits, which tell -0 from +0, with norms of zero among them."""
+    rng = np.random.default_rng(dim)
+    padded, tokens = 1 << (dim - 1).bit_length(), 96
+    cache = _cache(rng, tokens // 16, 16, heads, dim, SLOT[dim])
+    rows = cache.reshape(-1, SLOT[dim])
+    rows[:, :padded // 2] = np.repeat(rng.integers(0, 256, (len(rows), padded // 16), dtype=np.uint8), 8, axis=1)
+    rows[::3, :padded // 2] = rows[::3, :1]
+    rows[::5, :padded // 4], rows[::5, padded // 4:padded // 2] = rows[::5, :1], ~rows[::5, :1]
+    rows[::7, padded // 2:padded // 2 + 2] = 0
+    signs = synthetic.make_signs(padded, 42)
+    table = np.zeros((1, 60000 if wide else tokens // 16), np.int32)      # a wide table: beyond the small jobs' bound
+    table[0, :tokens // 16] = rng.permutation(tokens // 16)
+    want = _want(oracle, cache, table, [tokens], signs.numpy(), dim)
+    assert any((w == 0).any() for w in want)
+    for dtype in (torch.float32, torch.bfloat16):
+        k, v = (torch.empty(tokens, heads, dim, dtype=dtype, device=DEV) for _ in range(2))
+        _cabi.dequant_paged(torch.from_numpy(cache).to(DEV), torch.from_numpy(table).to(DEV), torch.tensor([tokens], dtype=torch.int32, device=DEV),
+                            torch.tensor([0, tokens], dtype=torch.int32, device=DEV), signs.to(DEV), k, v)
+        for got, ref in ((k, want[0]), (v, want[1])):
+            as_int = torch.int32 if dtype == torch.float32 else torch.int16
+            assert torch.equal(got.cpu().view(as_int), torch.from_numpy(ref).to(dtype).view(as_int)), (dtype, dim)

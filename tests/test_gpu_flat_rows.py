@@ -130,3 +130,23 @@ def test_quantization_of_many_rows(oracle, dim, n, dtype):
             parts = [_cabi.quantize_flat(x[i:i + 2000].to(DEV), factors, bits) for i in range(0, n, 2000)]
             assert torch.equal(p, torch.cat([a for a, _ in parts]))
             np.testing.assert_array_equal(norms.cpu().numpy(), torch.cat([b for _, b in parts]).cpu().numpy())
+
+
+@pytest.mark.parametrize("dim,n", [(64, 49152), (128, 8192), (256, 2048), (192, 2051)])
+def test_zeros_keep_their_sign_in_many_rows(oracle, dim, n):
+    """Rows of repeated codes, whose sums cancel: the outputs' bits, which tell -0 from +0, with norms of zero among them."""
+    padded = 1 << (dim - 1).bit_length()
+    rng = np.random.default_rng(dim)
+    signs = synthetic.make_signs(padded, 42)
+    norms = rng.uniform(0.5, 30.0, n).astype(np.float32)
+    norms[::7] = 0.0
+    for bits in (2, 3, 4):
+        per = 8 // bits
+        codes = np.repeat(rng.integers(0, 1 << bits, (n, padded // 8), dtype=np.uint8), 8, axis=1)
+        codes[::3] = codes[::3, :1]
+        codes[::5, :padded // 2], codes[::5, padded // 2:] = codes[::5, :1], (1 << bits) - 1 - codes[::5, :1]
+        packed = (codes.reshape(n, padded // per, per) << (bits * np.arange(per, dtype=np.uint8))).sum(axis=2).astype(np.uint8)
+        want = oracle.dequantize_flat(packed, norms, signs.numpy(), dim, bits)
+        assert (want == 0).any()
+        got = _cabi.dequantize_flat(torch.from_numpy(packed).to(DEV), torch.from_numpy(norms).to(DEV), signs.to(DEV), dim, bits)
+        np.testing.assert_array_equal(got.cpu().numpy().view(np.int32), want.view(np.int32), err_msg=f"bits {bits}")

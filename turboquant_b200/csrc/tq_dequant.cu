@@ -105,8 +105,7 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
     }
     grid_dependency_wait();  // the cache, the page table and the lengths belong to earlier kernels
     for (int d = tid; d < PD; d += S::kThreads) {
-        float v = d < HD ? __fmul_rn(p.signs[d], p.scale) : 0.0f;  // exact: the sign is +-1, or the scale a power of two
-        if (S::kLanes == 2 && d >= PD * 3 / 4) v = -v;                     // see the last stage
+        const float v = d < HD ? __fmul_rn(p.signs[d], p.scale) : 0.0f;  // exact: the sign is +-1, or the scale a power of two
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(sgn + 4u * d + (S::kLanes == 2 ? 16u * (d / (PD / 4)) : 0u)), "f"(v) : "memory");
     }
     __syncthreads();
@@ -252,16 +251,18 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
             if constexpr (S::kLanes == 2) {
                 // The last stage is between the lanes: each keeps its first half of values and sends the other, half the shuffles of sending all.  For that
                 // the upper lane has to hold its values with the halves exchanged, which it does when the inputs of the second half change sign (the transform
-                // of (-1)^[e >= n / 2] x is that of x at e ^ (n / 2), bit for bit); the codebook is symmetric, so the complement of a code is its
-                // negative.  Lower outputs are mine + other, upper ones mine - other, negated in the upper lane (in its signs).
+                // of (-1)^[e >= n / 2] x is that of x at e ^ (n / 2)); the codebook is symmetric, so the complement of a code is its
+                // negative.  Bit for bit: sums that cancel are +0 either way, and no input is a zero.  Lower outputs are mine + other, upper ones mine - other
+                // or, in the upper lane, other - mine (not its negative, which is -0 where the two are equal).
                 constexpr int kHalf = S::kPairs / 2;
+                const P2 mine_sign = m ? pk(-1.0f, -1.0f) : pk(1.0f, 1.0f), other_sign = m ? pk(1.0f, 1.0f) : pk(-1.0f, -1.0f);
 #pragma unroll
                 for (int e = 0; e < kHalf; e++) {
                     float a, c;
                     up(x[kHalf + e], a, c);
                     const P2 mine = x[e], other = pk(__shfl_xor_sync(kAll, a, 1), __shfl_xor_sync(kAll, c, 1));
                     x[e] = add2(mine, other);
-                    x[kHalf + e] = sub2(mine, other);
+                    x[kHalf + e] = fma2(other, other_sign, mul2(mine, mine_sign));      // exact products: one rounding, that of the difference
                 }
             }
             const P2 n2 = pk(norm, norm);

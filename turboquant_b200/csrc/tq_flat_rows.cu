@@ -77,8 +77,7 @@ __global__ void __launch_bounds__(DequantRowsShape<PD, BITS>::kThreads, 1) dequa
     }
     grid_dependency_wait();      // only the table is made ahead of it
     for (int d = tid; d < PD; d += S::kThreads) {
-        float v = d < p.dim ? p.signs[d] : 0.0f;
-        if (S::kLanes == 2 && d >= PD * 3 / 4) v = -v;                     // see the last stage
+        const float v = d < p.dim ? p.signs[d] : 0.0f;
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(sgn + 4u * d + (S::kLanes == 2 ? 16u * (d / (PD / 4)) : 0u)), "f"(v) : "memory");
     }
     __syncthreads();
@@ -148,16 +147,18 @@ __global__ void __launch_bounds__(DequantRowsShape<PD, BITS>::kThreads, 1) dequa
                 }
         if constexpr (S::kLanes == 2) {
             // The last stage is between the lanes: each keeps its first half of values and sends the other.  For that the second lane holds its values
-            // with the halves exchanged, as it does when the inputs of the second half change sign (bit for bit).  Upper outputs come out negated in
-            // that lane (in its signs).
+            // with the halves exchanged, as it does when the inputs of the second half change sign; bit for bit: a sum with an unchanged first half that
+            // cancels is +0 whatever the second's zero.  Upper outputs are mine - other or, in that lane, other - mine (not its negative, which is
+            // -0 where the two are equal).
             constexpr int kHalf = S::kPairs / 2;
+            const P2 mine_sign = m ? pk(-1.0f, -1.0f) : pk(1.0f, 1.0f), other_sign = m ? pk(1.0f, 1.0f) : pk(-1.0f, -1.0f);
 #pragma unroll
             for (int e = 0; e < kHalf; e++) {
                 float a, c;
                 up(x[kHalf + e], a, c);
                 const P2 mine = x[e], other = pk(__shfl_xor_sync(kAll, a, 1), __shfl_xor_sync(kAll, c, 1));
                 x[e] = add2(mine, other);
-                x[kHalf + e] = sub2(mine, other);
+                x[kHalf + e] = fma2(other, other_sign, mul2(mine, mine_sign));      // exact products: one rounding, that of the difference
             }
         }
         const P2 norm2 = pk(norm, norm);

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(LaneRowsShape<PD>::kThreads, 1) lane_rows_kern
                 }
         if constexpr (S::kLanes == 2) {
             // The last stage is between the lanes: each keeps its first half of values and sends the other.  For that the second lane holds its values
-            // with the halves exchanged, as it does when the inputs of the second half change sign (bit for bit).
+            // with the halves exchanged, as it does when the inputs of the second half change sign (equal values; zeros may change sign, which no code depends on).
             const P2 flip = m ? pk(-1.0f, -1.0f) : pk(1.0f, 1.0f);
             constexpr int kHalf = S::kPairs / 2;
 #pragma unroll
