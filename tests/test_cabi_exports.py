@@ -73,3 +73,14 @@ def test_cpu_tensors_rejected():
     from turboquant_b200 import _cabi
     with pytest.raises(_cabi.TurboQuantError, match="CUDA tensor"):
         _cabi.quantize_flat(torch.zeros(2, 128), torch.ones(128), 4)
+
+
+def test_dequantizers_take_the_table_at_64k_only_where_it_fits(lib):
+    """The rule by which the host picks the dequantization kernels whose lookup table has a fixed place in shared memory: the system's part of it, as
+    the device states it (1024 bytes on the drivers known), and the kernel's own bytes have to end below that place."""
+    fits = getattr(lib, "_ZN2tq18shared_window_fitsEij")
+    fits.argtypes, fits.restype = [ctypes.c_int, ctypes.c_uint32], ctypes.c_bool
+    assert fits(1024, 65536 - 1024) and not fits(1024, 65536 - 1023)
+    assert fits(2048, 62208) and not fits(1025, 65536 - 1024)        # the kernels round up to 128 bytes
+    assert not fits(0, 1000) and not fits(1023, 1000)                 # the request counts on 1024
+    assert fits(65536, 0) and not fits(65537, 0) and not fits(2**31 - 1, 0) and not fits(-1, 0)

@@ -57,6 +57,23 @@ int device_sm_count(int* out) {
     return TQ_OK;
 }
 
+// Kernels that have a lookup table at address 64 KB of the block's shared window (so that one byte permute makes an entry's address) need the system's
+// part at the window's start to leave room for their `below` bytes under it, and count on 1024 of it in what they ask for.
+bool shared_window_fits(int reserved, uint32_t below) {
+    return reserved >= 1024 && reserved <= 65536 && (((uint32_t)reserved + 127u) & ~127u) + below <= 65536u;
+}
+int device_shared_window_fits(uint32_t below, bool* fits) {
+    static thread_local int cached_dev = -1, cached = 0;
+    int dev = 0;
+    TQ_CUDA(cudaGetDevice(&dev));
+    if (dev != cached_dev) {
+        TQ_CUDA(cudaDeviceGetAttribute(&cached, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+        cached_dev = dev;
+    }
+    *fits = shared_window_fits(cached, below);
+    return TQ_OK;
+}
+
 // cuTensorMapEncodeTiled, looked up through the runtime (no link-time dependency on the driver library)
 bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
                        const cuuint32_t* box, CUtensorMapSwizzle swizzle) {

@@ -30,6 +30,7 @@
 namespace tq {
 
 int device_sm_count(int* out);
+int device_shared_window_fits(uint32_t below, bool* fits);
 
 constexpr int kDqDim = 128;
 
@@ -50,7 +51,7 @@ struct DequantParams {
 };
 
 // Page halves skipped because the page id lay outside the cache or the sequence was longer than
-// its page list; read back by tq_fault_counts.
+// its page list, and launches that did nothing; read back by tq_fault_counts.
 static __device__ int32_t g_dequant_skipped = 0;
 
 // HD: elements of an output row; PD: of the rotated row (HD rounded up to a power of two).  SMALL: jobs of a few units a scheduler.  With
@@ -85,7 +86,8 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
     const uint32_t smem0 = (smem_u32(dq_smem) + 127u) & ~127u;
     const uint32_t bars = smem0 + 2 * S::kWarps * S::kStage, sgn = bars + 2 * S::kWarps * 8;
     const uint32_t table = SMALL ? smem0 + S::kBelow : S::kTable, stagings = table + 256 * S::kEntry;
-    if (!SMALL && (smem0 + S::kBelow > S::kTable || smem0 < 1024)) {      // the shared window starts elsewhere than on any driver known
+    if (!SMALL && (smem0 + S::kBelow > S::kTable || smem0 < 1024)) {      // the shared window starts elsewhere than the device said
+        grid_dependency_wait();
         if (tid == 0 && blockIdx.x == 0) atomicAdd(&g_dequant_skipped, 1);
         return;
     }
@@ -361,7 +363,11 @@ template <int DT, int PD, int HD>
 static int launch_dequant(const DequantParams& p, int sms, cudaStream_t stream) {
     // The lengths are on the device: the table's width bounds the units of 32 rows.
     const int64_t units = (int64_t)p.batch * p.max_pages * ((2 * (int64_t)p.block_size * p.H + 31) / 32);
-    if (units <= (int64_t)kDqSmallUnits * sms) {
+    // A device whose shared window leaves no room under the large blocks' table has the small blocks do all.
+    bool fits = false;
+    const int rc = device_shared_window_fits(DqShape<DT, PD, HD, false>::kBelow, &fits);
+    if (rc != TQ_OK) return rc;
+    if (!fits || units <= (int64_t)kDqSmallUnits * sms) {
         const int64_t most = (int64_t)sms * (PD == 256 ? 1 : 2), count = units * DqShape<DT, PD, HD, true>::kLanes;
         return launch_dequant<DT, PD, HD, true>(p, count < most ? count : most, stream);
     }
@@ -382,13 +388,16 @@ int generic_dequant(const void* kv_cache, int64_t num_blocks, int block_size, in
                     const int32_t* cu_seqlens, int batch, const float* signs, int head_dim, void* k_out, void* v_out,
                     int out_dtype, int64_t out_token_stride, void* stream);
 int generic_fault_counts(int32_t* write_dropped, int32_t* dequant_skipped);
+int flat_rows_fault_count(int32_t* out);
 
 int dequant_fault_count(int32_t* out) {
-    int32_t a = 0, b = 0, c = 0;
+    int32_t a = 0, b = 0, c = 0, d = 0;
     TQ_CUDA(cudaMemcpyFromSymbol(&a, g_dequant_skipped, sizeof(int32_t)));
     int rc = generic_fault_counts(&b, &c);
     if (rc != TQ_OK) return rc;
-    *out = a + c;
+    rc = flat_rows_fault_count(&d);
+    if (rc != TQ_OK) return rc;
+    *out = a + c + d;
     return TQ_OK;
 }
 

@@ -12,6 +12,7 @@
 namespace tq {
 
 int device_sm_count(int* out);
+int device_shared_window_fits(uint32_t below, bool* fits);
 
 struct DequantRowsParams {
     const uint8_t* packed;
@@ -42,8 +43,12 @@ struct DequantRowsShape {
     static_assert(kBelow + 1024 + 128 <= kTable && kSmem <= 232448, "shared memory");
 };
 
-// Blocks that found the shared window elsewhere than at 1024 did nothing.
+// Launches that did nothing (their blocks' shared window started elsewhere than the device said); read back by tq_fault_counts.
 static __device__ int32_t g_flat_rows_unfit = 0;
+int flat_rows_fault_count(int32_t* out) {
+    TQ_CUDA(cudaMemcpyFromSymbol(out, g_flat_rows_unfit, sizeof(int32_t)));
+    return TQ_OK;
+}
 
 template <int PD, int BITS>
 __global__ void __launch_bounds__(DequantRowsShape<PD, BITS>::kThreads, 1) dequantize_lanes_kernel(const __grid_constant__ DequantRowsParams p) {
@@ -54,7 +59,8 @@ __global__ void __launch_bounds__(DequantRowsShape<PD, BITS>::kThreads, 1) dequa
     const int m = lane & (S::kLanes - 1), row = lane / S::kLanes;
     const uint32_t smem0 = (smem_u32(fr_smem) + 127u) & ~127u;
     if (smem0 + S::kBelow > S::kTable || smem0 < 1024) {
-        if (tid == 0) atomicAdd(&g_flat_rows_unfit, 1);
+        grid_dependency_wait();
+        if (tid == 0 && blockIdx.x == 0) atomicAdd(&g_flat_rows_unfit, 1);
         return;
     }
     const uint32_t ring = smem0 + (uint32_t)warp * 2 * S::kStage, norms = smem0 + 2 * S::kWarps * S::kStage + (uint32_t)warp * 256 + 4 * lane;
@@ -230,12 +236,21 @@ static int launch_dequantize_lanes(const DequantRowsParams& p, int bits, int sms
 // 13.3 / 12.3, 48000 25.9 / 19.4, 131072 53.8 / 44.5, 3000 9.1 / 9.1; 256 wide 3000 rows 17.2 / 13.7, 60000 56.8 / 49.9; 64 wide 40000 rows
 // 12.0 / 13.6, 64000 18.2 / 15.2, 120000 28.1 / 25.7).
 static int64_t lanes_from(int padded) { return padded == 64 ? 49152 : padded == 128 ? 8192 : 2048; }
-// Calls that this kernel takes: many rows of a multiple of 8 elements padded to 64, 128 or 256, 2 to 4 bits, codes and output on 16 bytes.  Returns false,
-// having done nothing, for others.
+static uint32_t lanes_below(int padded, int bits) {
+    return padded == 64 ? (bits == 2 ? DequantRowsShape<64, 2>::kBelow : DequantRowsShape<64, 4>::kBelow)
+         : padded == 128 ? (bits == 2 ? DequantRowsShape<128, 2>::kBelow : DequantRowsShape<128, 4>::kBelow)
+                         : (bits == 2 ? DequantRowsShape<256, 2>::kBelow : DequantRowsShape<256, 4>::kBelow);
+}
+// Calls that this kernel takes: many rows of a multiple of 8 elements padded to 64, 128 or 256, 2 to 4 bits, codes and output on 16 bytes, on a device
+// whose shared window has room for the table's place.  Returns false, having done nothing, for others.
 bool dequantize_lanes(const uint8_t* packed, const float* norms, int64_t n, int dim, int padded, const float* signs, int bits, bool cache_order, float* out,
                       void* stream, int* rc) {
     if (padded < 64 || n < lanes_from(padded) || dim % 8 != 0 || bits < 2 || (uintptr_t)packed % 16 != 0 || (uintptr_t)out % 16 != 0 || (uintptr_t)norms % 4 != 0)
         return false;
+    bool fits = false;
+    *rc = device_shared_window_fits(lanes_below(padded, bits), &fits);
+    if (*rc != TQ_OK) return true;
+    if (!fits) return false;
     DequantRowsParams p{};
     p.packed = packed;
     p.norms = norms;
