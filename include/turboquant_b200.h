@@ -321,12 +321,14 @@ int tq_decode_static_status(int32_t* status_out, void* stream);
  * does not need to bind these.
  * --------------------------------------------------------------------------------------- */
 
-/* Index faults that the kernels without a workspace caught instead of dereferencing, since the
- * library was loaded on the current device: counts3[0] tokens whose slot was at or beyond
- * num_blocks * block_size in tq_write_kv_cache (dropped like a negative slot), counts3[1] page
- * halves tq_dequant_paged skipped (page id outside the cache, or a sequence longer than its page
- * list; their output rows stay unwritten) and launches of it or of tq_dequantize_flat that wrote nothing
- * (a block's shared memory was not laid out as the device had said), counts3[2] pages tq_pages_gather / _scatter skipped.
+/* Faults that the kernels without a workspace caught, since the library was loaded on the current
+ * device: counts3[0] tokens whose slot was at or beyond num_blocks * block_size in tq_write_kv_cache
+ * (dropped like a negative slot), and copies of rows that never arrived, there or in
+ * tq_quantize_flat (what those rows make stays unwritten); counts3[1] page halves tq_dequant_paged
+ * skipped (page id outside the cache, or a sequence longer than its page list; their output rows
+ * stay unwritten), copies of slots that never arrived there, and launches of it or of
+ * tq_dequantize_flat that wrote nothing (a block's shared memory was not laid out as the device had
+ * said); counts3[2] pages tq_pages_gather / _scatter skipped.
  * Host array of three; synchronises the device.  The reference only checks shapes
  * (csrc/src/quantize_write_binding.cu:216-227). */
 int tq_fault_counts(int32_t* counts3);

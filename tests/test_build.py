@@ -1,5 +1,6 @@
 """What the build leaves behind: an installed package holds every built file, and a module built against another torch or Python is
 built anew."""
+import re
 import tomllib
 from pathlib import Path
 
@@ -24,3 +25,17 @@ def test_the_native_module_is_bound_to_torch_and_python(monkeypatch, tmp_path):
     monkeypatch.undo()
     monkeypatch.setattr(build, "NATIVE_STAMP", tmp_path / "none")      # a module of before the stamp
     assert build._native_stale()
+
+
+def test_no_kernel_gives_up_on_a_copy_in_silence():
+    """Every bounded wait for a copy, where it runs out, raises a status or counts a fault before its warp returns; a copy that is lost cannot be made on
+    purpose, so this reads the source."""
+    csrc = Path(build.__file__).parent / "csrc"
+    seen = 0
+    for path in sorted(csrc.glob("*.cu*")):
+        text = path.read_text()
+        for at in re.finditer(r"\bmbar_wait\(&", text):
+            seen += 1
+            handler = text[at.start():at.start() + 400]
+            assert "copy_lost(" in handler or "abort_flag = 1" in handler, f"{path.name}: {handler[:120]}"
+    assert seen >= 6

@@ -274,8 +274,8 @@ def decode_max_queries_per_seq(num_q_heads: int, num_kv_heads: int, head_size: i
 
 def fault_counts():
     """(dropped cache-write tokens, skipped dequant page halves, skipped offload pages) that the
-    kernels caught as out-of-range indices since the library was loaded (the second also counts launches of a
-    dequantization that wrote nothing); synchronises."""
+    kernels caught as out-of-range indices since the library was loaded; synchronises.  The first two also count
+    copies that never arrived, the second launches of a dequantization that wrote nothing."""
     c = (ctypes.c_int32 * 3)()
     _check(lib().tq_fault_counts(c))
     return tuple(int(x) for x in c)

@@ -102,6 +102,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
+// What a whole warp does that gave up on its copy (`if (!__all_sync(...mbar_wait...))`), before it returns with nothing more written: count the fault, and
+// wait, a shorter while, for the copies it has in flight, that and the next (`other`), so that none lands in memory that has been given on.
+__device__ __forceinline__ void copy_lost(int32_t* faults, int lane, uint64_t* bar, uint32_t parity, bool other, uint64_t* other_bar, uint32_t other_parity) {
+    if (lane == 0) atomicAdd(faults, 1);
+    for (uint32_t i = 0; i < kSpinLimit / 64; i++)
+        if (mbar_try_wait(bar, parity) && (!other || mbar_try_wait(other_bar, other_parity))) break;
+}
 
 // Brings one line into L2 without handing a value to the kernel (L2 is the point of coherence, so a
 // line fetched early still shows later writes of other kernels).

@@ -51,7 +51,7 @@ struct DequantParams {
 };
 
 // Page halves skipped because the page id lay outside the cache or the sequence was longer than
-// its page list, and launches that did nothing; read back by tq_fault_counts.
+// its page list, copies of slots that never landed, and launches that did nothing; read back by tq_fault_counts.
 static __device__ int32_t g_dequant_skipped = 0;
 
 // HD: elements of an output row; PD: of the rotated row (HD rounded up to a power of two).  SMALL: jobs of a few units a scheduler.  With
@@ -218,7 +218,10 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
         const uint64_t k0 = __shfl_sync(kAll, src, i);
         if (k0 == 1) break;
         if (k0 != 0) {
-            if (!mbar_wait(&bar[s], (phases >> s) & 1)) return;  // the copy never landed: nothing more is written
+            if (!__all_sync(kAll, mbar_wait(&bar[s], (phases >> s) & 1))) {
+                copy_lost(&g_dequant_skipped, lane, &bar[s], (phases >> s) & 1, __shfl_sync(kAll, src, i + 1) > 1, &bar[s ^ 1], (phases >> (s ^ 1)) & 1);
+                return;
+            }
             phases ^= 1u << s;
             const uint32_t slot = smem_u32(ring) + s * S::kStage + (uint32_t)(lane / S::kLanes) * S::kRow;
             P2 x[S::kPairs];   // x[i] = dims 2 i, 2 i + 1 = code byte i (two lanes: of the row's half m)

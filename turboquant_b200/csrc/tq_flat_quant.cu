@@ -56,4 +56,9 @@ bool quantize_lanes(const void* x, int x_dtype, int64_t n, int dim, int padded, 
     return true;
 }
 
+int flat_quant_fault_count(int32_t* out) {
+    TQ_CUDA(cudaMemcpyFromSymbol(out, g_rows_dropped, sizeof(int32_t)));
+    return TQ_OK;
+}
+
 }  // namespace tq

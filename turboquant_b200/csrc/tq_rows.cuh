@@ -60,7 +60,8 @@ struct LaneRowsShape {
     static_assert(kSmem <= 232448, "shared memory");
 };
 
-static __device__ int32_t g_rows_dropped = 0;      // of the cache write
+// Tokens that the cache write dropped (slot outside the cache), and copies of rows that never landed; read back by tq_fault_counts.
+static __device__ int32_t g_rows_dropped = 0;
 
 template <typename T>
 struct RowWord;
@@ -268,7 +269,10 @@ __global__ void __launch_bounds__(LaneRowsShape<PD>::kThreads, 1) lane_rows_kern
     fetch(unit + step, 1);
     uint32_t phases = 0;
     for (int s = 0; unit < units; unit += step, s ^= 1) {
-        if (!mbar_wait(&bar[s], (phases >> s) & 1)) return;  // the copy never landed: nothing more is written
+        if (!__all_sync(kAll, mbar_wait(&bar[s], (phases >> s) & 1))) {
+            copy_lost(&g_rows_dropped, lane, &bar[s], (phases >> s) & 1, unit + step < units, &bar[s ^ 1], (phases >> (s ^ 1)) & 1);
+            return;
+        }
         phases ^= 1u << s;
         const uint32_t stage = ring + s * S::kStage;
         // 16-byte piece c (8 elements) of this lane's values

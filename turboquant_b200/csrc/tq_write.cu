@@ -105,7 +105,7 @@ __device__ __forceinline__ void split_row(int64_t r, int H, int head_shift, int6
 }
 
 // Rows dropped because their slot lay outside the cache (a stale or garbage slot id must never
-// become a store address); read back by tq_fault_counts.
+// become a store address), and copies of rows that never landed; read back by tq_fault_counts.
 static __device__ int32_t g_write_dropped = 0;
 // Rows the tensor-core kernel handled, and how many of them it re-derived with the exact path
 // (read back by tq_write_guard_stats).
@@ -246,7 +246,10 @@ write_kv_cache_kernel(const __grid_constant__ WriteParams p) {
                                  : (int64_t) reinterpret_cast<const int32_t*>(p.slot_mapping)[t];
         }
 
-        if (!mbar_wait(&full_bar[warp][buf], (it >> 1) & 1)) return;  // copy never landed: touch nothing
+        if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[warp][buf], (it >> 1) & 1))) {
+            copy_lost(&g_write_dropped, lane, &full_bar[warp][buf], (it >> 1) & 1, next < num_tiles, &full_bar[warp][buf ^ 1], ((it + 1) >> 1) & 1);
+            return;
+        }
         // All lanes run the arithmetic (the shuffles need whole pairs).  Rows past the end compute
         // on whatever the buffer holds, take neither the divisions (a decode step of an odd batch spent 10 us in the division
         // routine on what the kernel before had left there: 13 us against 3 for the write) nor a lookup, and store nothing.
@@ -668,7 +671,10 @@ write_kv_cache_mma_kernel(const __grid_constant__ WriteParams p) {
             slot = p.slot_is_i64 ? reinterpret_cast<const int64_t*>(p.slot_mapping)[t]
                                  : (int64_t) reinterpret_cast<const int32_t*>(p.slot_mapping)[t];
         }
-        if (!mbar_wait(&full_bar[warp][buf], (it >> 1) & 1)) return;
+        if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[warp][buf], (it >> 1) & 1))) {
+            copy_lost(&g_write_dropped, lane, &full_bar[warp][buf], (it >> 1) & 1, next < num_tiles, &full_bar[warp][buf ^ 1], ((it + 1) >> 1) & 1);
+            return;
+        }
         const uint8_t* stage = smem + ((size_t)buf * W::kWarps + warp) * W::kWarpStage;
         // Rows past the end of the tensor hold zeros: they are computed like any others and never stored.
         // byte address of 16-byte piece `piece` (0..15) of row `row` of the staged tile
@@ -974,15 +980,17 @@ bool write_rows(void* kv_cache, int64_t num_blocks, int block_size, int num_kv_h
                 int64_t num_tokens, int64_t k_token_stride, int64_t v_token_stride, const float* signs, const void* slot_mapping, int slot_dtype,
                 int head_dim, int flags, void* stream, int* rc);
 int write_rows_fault_count(int32_t* out);
+int flat_quant_fault_count(int32_t* out);
 
 int write_fault_count(int32_t* out) {
-    int32_t a = 0, b = 0, c = 0, d = 0;
+    int32_t a = 0, b = 0, c = 0, d = 0, e = 0;
     TQ_CUDA(cudaMemcpyFromSymbol(&a, g_write_dropped, sizeof(int32_t)));
     int rc = generic_fault_counts(&b, &c);
     if (rc != TQ_OK) return rc;
     rc = write_rows_fault_count(&d);
+    if (rc == TQ_OK) rc = flat_quant_fault_count(&e);
     if (rc != TQ_OK) return rc;
-    *out = a + b + d;
+    *out = a + b + d + e;
     return TQ_OK;
 }
 

@@ -65,7 +65,6 @@ bool write_rows(void* kv_cache, int64_t num_blocks, int block_size, int num_kv_h
     return true;
 }
 
-
 int write_rows_fault_count(int32_t* out) {
     TQ_CUDA(cudaMemcpyFromSymbol(out, g_rows_dropped, sizeof(int32_t)));
     return TQ_OK;
