@@ -121,3 +121,20 @@ def test_zeros_keep_their_sign(oracle, dim, heads, wide):
         for got, ref in ((k, want[0]), (v, want[1])):
             as_int = torch.int32 if dtype == torch.float32 else torch.int16
             assert torch.equal(got.cpu().view(as_int), torch.from_numpy(ref).to(dtype).view(as_int)), (dtype, dim)
+
+
+@pytest.mark.parametrize("dim,heads", [(128, 1), (64, 1), (256, 1)])
+def test_every_bad_page_is_counted_once(dim, heads):
+    """A job of more units a warp than are looked up at a time, all of its pages outside the cache: as many faults as pages, and nothing written."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = 16 if dim == 256 else 32                                    # of a unit: a page of one head has 32
+    pages = 33 * sms * (20 if dim == 64 else 12) * rows // 32 + 7       # warps of a block
+    table = torch.full((1, pages), 5, dtype=torch.int32, device=DEV)
+    table[0, ::3] = -1
+    cache = torch.zeros((2, 5, 16, heads, SLOT[dim]), dtype=torch.uint8, device=DEV)
+    k, v = (torch.full((pages * 16, heads, dim), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    before = _cabi.fault_counts()
+    _cabi.dequant_paged(cache, table, torch.tensor([pages * 16], dtype=torch.int32, device=DEV), torch.tensor([0, pages * 16], dtype=torch.int32, device=DEV),
+                        synthetic.make_signs(dim, 42).to(DEV), k, v)
+    assert _cabi.fault_counts()[1] - before[1] == pages
+    assert bool((k == 7.0).all()) and bool((v == 7.0).all())

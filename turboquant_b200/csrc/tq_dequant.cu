@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
                 ntok = left < p.block_size ? left : p.block_size;
                 row0 = row;
                 if ((uint64_t)page >= (uint64_t)p.num_blocks) {  // never form an address from it: the rows stay unwritten
-                    if (unit == 0) atomicAdd(&g_dequant_skipped, 1);
+                    if (unit == 0 && lane < 30) atomicAdd(&g_dequant_skipped, 1);      // the last two units are looked up again
                     src = 0;
                 } else {
                     src = reinterpret_cast<uint64_t>(p.kv_cache) + (uint64_t)page * half_rows * p.slot_bytes;
