@@ -835,13 +835,13 @@ static MqEncodeFn mq_encode_fn() {
     return fn;
 }
 
-// The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab, or of both.
-int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes, int slabs) {
+// The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab.
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes) {
     MqEncodeFn enc = mq_encode_fn();
     TQ_REQUIRE(enc != nullptr, TQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)num_blocks * kPageTokens, 2};
     const cuuint64_t strides[2] = {dims[0], dims[0] * dims[1]};
-    const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, (cuuint32_t)slabs};
+    const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, 1u};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(kv_cache), dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -861,7 +861,7 @@ int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks
     mp.head_pairs = num_kv_heads / 2;
     mp.ncols = d.group;
     mp.causal = causal;
-    const int rc = encode_cache_map(&mp.cache_map, d.kv_cache, num_blocks, (int64_t)num_kv_heads * kSlotBytes, 160, 1);
+    const int rc = encode_cache_map(&mp.cache_map, d.kv_cache, num_blocks, (int64_t)num_kv_heads * kSlotBytes, 160);
     if (rc != TQ_OK) return rc;
     const int smem = (int)kMqSmemEnd;
     static bool configured[64] = {};

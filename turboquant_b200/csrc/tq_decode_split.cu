@@ -9,7 +9,7 @@
 //   * One block per SM = kGroups groups of kGroupWarps warps around one lookup table.  A group works alone (its own
 //     named barrier); the table, the longest part of a block's prologue, is filled before the dependency wait.
 //   * Plan on the device, by every warp for itself from seq_lens (no barrier): see SplitPlan.
-//   * A warp takes whole pages of its head: one tiled tensor copy (16 rows of the head's slot from K and 16 from V) into its
+//   * A warp takes whole pages of its head: two tiled tensor copies (16 rows of the head's slot each, from K and from V) into its
 //     own ring of stages (eleven 16-byte asynchronous copies a lane filled the load/store queue: 40 / 8 heads, 32 ragged
 //     sequences 34.4 -> 27.5 us a step, head size 64 34 -> 28, 256 37 -> 32), codes looked up straight
 //     into mma.sync.m16n8k16 fragments (the scheme of tq_decode.cu: K bytes are A fragments of S = K^ Q^T, V nibbles of
@@ -76,7 +76,7 @@ struct SplitShape {
 };
 
 struct SplitParams {
-    alignas(64) CUtensorMap cache_map;   // uint8 [2][num_blocks * 16][H * slot], boxes of [2][16][kRow], pairs of warps: [1][16][kRow]
+    alignas(64) CUtensorMap cache_map;   // uint8 [2][num_blocks * 16][H * slot], boxes of [1][16][kRow]
     const void* q;
     const uint8_t* kv_cache;
     const int32_t* page_indices;
@@ -336,7 +336,7 @@ __device__ __forceinline__ void split_kept_plan(const SplitParams& p, SplitPlan&
     s.len = 0;
 }
 
-// One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V), or of both.  No multicast; x is a
+// One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V).  No multicast; x is a
 // multiple of the slot, hence of 16.
 __device__ __forceinline__ void split_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     __shared__ float sign_s[PD];
     __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols + 1];  // a pair's maxima of a page that raises them (and its largest V norm), and whether it does
     __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
-    __shared__ uint64_t full_s[F::kWarps][F::kStages + F::kNormScale];   // a stage's page has landed; and a word for the warp's scale of the V norms
+    __shared__ uint64_t full_s[F::kWarps][F::kStages + F::kNormScale];   // a stage's two boxes have landed; and a word for the warp's scale of the V norms
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 split_expect(bar, i < n ? F::kStageBytes : 0);      // no page: the warps of a pair stay at the same stage
                 if (i < n) {
                     split_box(dst, &p.cache_map, x, id * kPageTokens, 0, bar);
-                    if (F::kPair) split_box(dst + F::kHalfBytes, &p.cache_map, x, id * kPageTokens, 1, bar);
+                    split_box(dst + F::kHalfBytes, &p.cache_map, x, id * kPageTokens, 1, bar);
                 }
             }
         };
@@ -1240,7 +1240,7 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
 // ---------------------------------------------------------------------------------------------
 int device_sm_count(int* out);
 cudaEvent_t decode_event(int i);
-int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes, int slabs);
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes);
 
 static int split_box_bytes(int padded) {
     return padded == 64 ? SplitShape<64, 1>::kRow : padded == 128 ? SplitShape<128, 1>::kRow : SplitShape<256, 1>::kRow;
@@ -1314,7 +1314,7 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
     p.out = out;
     p.out_lse = out_lse;
     p.num_blocks = num_blocks;
-    const int map_rc = encode_cache_map(&p.cache_map, kv_cache, num_blocks, (int64_t)num_kv_heads * slot_bytes, split_box_bytes(padded), padded == 128 && p.group > 16 ? 1 : 2);
+    const int map_rc = encode_cache_map(&p.cache_map, kv_cache, num_blocks, (int64_t)num_kv_heads * slot_bytes, split_box_bytes(padded));
     if (map_rc != TQ_OK) return map_rc;
     p.kv_begin = kv_begin;
     p.kv_end = kv_end;
