@@ -138,3 +138,15 @@ def test_every_bad_page_is_counted_once(dim, heads):
                         synthetic.make_signs(dim, 42).to(DEV), k, v)
     assert _cabi.fault_counts()[1] - before[1] == pages
     assert bool((k == 7.0).all()) and bool((v == 7.0).all())
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("dim,heads,batch,listed", [(128, 8, 257, False), (128, 3, 1000, True), (96, 1, 600, False), (64, 5, 511, True), (256, 2, 513, False)])
+def test_more_sequences_than_parts_of_the_work_list(oracle, dim, heads, batch, listed, wide):
+    """A block's list of work has 256 parts: one and more sequences each, the last ones without any, empty sequences alone and in runs; sequences of one
+    token, whose pages hold units of nothing but free slots."""
+    rng = np.random.default_rng(batch)
+    lens = rng.choice([0, 1, 1, 3, 16, 17, 40], batch)
+    lens[:9], lens[100:180], lens[-5:] = 0, 0, 0
+    lens[200:230] = 1
+    _check(oracle, dim, heads, wide=wide, lens=[int(n) for n in lens], listed=listed)

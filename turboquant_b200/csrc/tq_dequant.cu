@@ -33,6 +33,7 @@ int device_sm_count(int* out);
 int device_shared_window_fits(uint32_t below, bool* fits);
 
 constexpr int kDqDim = 128;
+constexpr int kDqChunks = 256;      // parts of the sequences in a block's table of pages (a power of two; no more than a block's threads)
 
 struct DequantParams {
     const uint8_t* kv_cache;
@@ -68,10 +69,11 @@ struct DqShape {
     static constexpr int kPassDims = kLanes == 2 ? PD / 2 : PD == 64 ? 128 / kEsz : 256 / kEsz, kLaneDims = kPassDims / kLanes;
     static constexpr int kPasses = (HD + kPassDims - 1) / kPassDims;
     static constexpr int kPitch = kPassDims * kEsz, kOut = kRows * kPitch;
-    // Shared memory: rings, barriers, signs; the table, 16 columns of 8 bytes a code byte (served half a warp at a time: no two lanes meet in a
+    // Shared memory: rings, barriers, signs, the work list's table; the lookup table, 16 columns of 8 bytes a code byte (served half a warp at a time: no two lanes meet in a
     // bank); the output staging.  Large jobs have the table at 64 KB with a 256-byte row a code byte, so that one byte permute makes an entry's address.
     static constexpr uint32_t kSignBytes = PD * 4 + 64;                     // blocks of a pass's dims 16 bytes apart: two lanes of a row meet no bank
-    static constexpr uint32_t kBelow = 2 * kWarps * kStage + ((2 * kWarps * 8 + kSignBytes + 127) & ~127);
+    static constexpr uint32_t kListBytes = (kDqChunks + 1 + kDqChunks / 32) * 8;
+    static constexpr uint32_t kBelow = 2 * kWarps * kStage + ((2 * kWarps * 8 + kSignBytes + kListBytes + 127) & ~127);
     static constexpr uint32_t kEntry = SMALL ? 128 : 256, kTable = 65536;
     static constexpr uint32_t kSmem = SMALL ? 128 + kBelow + 256 * kEntry + kWarps * kOut : 2 * kTable + kWarps * kOut - 1024;   // from offset 1024 (the system's part)
     static_assert(SMALL || (kBelow + 1024 + 128 <= kTable && kSmem <= 232448), "shared memory");
@@ -110,60 +112,97 @@ __global__ void __launch_bounds__(DqShape<DT, PD, HD, SMALL>::kThreads, SMALL &&
         const float v = d < HD ? __fmul_rn(p.signs[d], p.scale) : 0.0f;  // exact: the sign is +-1, or the scale a power of two
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(sgn + 4u * d + (S::kLanes == 2 ? 16u * (d / (PD / 4)) : 0u)), "f"(v) : "memory");
     }
-    __syncthreads();
-
-    // The work list: the pages of all sequences, each cut into units of 32 or 16 rows (the page's K rows, then its V rows).  A warp takes every
-    // workers-th unit; its lanes look 32 of them up at a time, which costs a unit less than a tenth of what one by one does.
+    // The work list: units of 32 or 16 rows (a page's K rows, then its V rows) that hold a row of a token, all of a sequence's pages but its last and what
+    // is live of that.  A warp takes every workers-th unit; its lanes look 32 of them up at a time, each its own: in a table of the units ahead of every
+    // 256th part of the sequences, made here by the block, then sequence by sequence.  (With every warp going through all sequences for each 32 units of
+    // whole pages 1024 x 20 tokens x 8 heads of 128 took 78 us and 4096 x 100 1053, against 49 and 622 item by item of a dense table; now 27 and 376.)
     const int half_rows = p.block_size * p.H, units = (2 * half_rows + S::kRows - 1) / S::kRows;
+    const int chunk = (p.batch + kDqChunks - 1) / kDqChunks;
+    int64_t* const starts = reinterpret_cast<int64_t*>(dq_smem + (sgn + S::kSignBytes - smem_u32(dq_smem)));
+    // The live units of a page's first n tokens: k_units from the page's first, v_units from v_first.
+    auto live = [&](int n, int& k_units, int& v_first) {
+        k_units = (n * p.H + S::kRows - 1) / S::kRows;
+        v_first = half_rows / S::kRows;
+        if (v_first < k_units) v_first = k_units;      // a unit of K and V rows counts once
+        return (half_rows + n * p.H + S::kRows - 1) / S::kRows - v_first;
+    };
+    // Pages of sequence b but its last live one, and that one's tokens; the count of its units.
+    auto units_of = [&](int b, int& whole_pages, int& rest) -> int64_t {
+        const int len = b < p.batch ? p.seq_lens[b] : 0;
+        whole_pages = rest = 0;
+        if (len <= 0 || p.max_pages <= 0) return 0;
+        whole_pages = (len - 1) / p.block_size;
+        rest = len - whole_pages * p.block_size;
+        if (whole_pages >= p.max_pages) {      // longer than its page list
+            whole_pages = p.max_pages - 1;
+            rest = p.block_size;
+        }
+        int k_units, v_first;
+        const int v_units = live(rest, k_units, v_first);
+        return (int64_t)whole_pages * units + k_units + v_units;
+    };
+    {
+        int64_t* const totals = starts + kDqChunks + 1;      // of the 32 chunks of a warp
+        int64_t sum = 0;
+        if (tid < kDqChunks) {
+            int whole_pages, rest;
+            for (int j = 0; j < chunk; j++) sum += units_of(tid * chunk + j, whole_pages, rest);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t t = __shfl_up_sync(kAll, sum, o);
+                if (lane >= o) sum += t;
+            }
+            if (lane == 31) totals[warp] = sum;
+        }
+        __syncthreads();
+        if (tid < kDqChunks) {
+            for (int i = 0; i < warp; i++) sum += totals[i];
+            starts[tid + 1] = sum;
+            if (tid == 0) starts[0] = 0;
+        }
+        __syncthreads();
+    }
     const int workers = (int)gridDim.x * S::kWarps;
     int64_t first = (int64_t)warp * gridDim.x + blockIdx.x;      // lane 0's unit; neighbouring units go to different SMs
     uint64_t src;       // this lane's unit: where its slots begin (0: nothing to do, 1: the end of the work; else a multiple of 16) ...
     int unit, ntok;     // ... which of the page's units, tokens in the page ...
     int row0;           // ... and the output row (token) of the page's first token
     auto look_up = [&]() {
-        const int64_t k = first + (int64_t)lane * workers, at = k / units;
+        const int64_t at = first + (int64_t)lane * workers;
         src = 1;
-        unit = (int)(k - at * units);
-        int64_t run = 0;
-        for (int base = 0; base < p.batch; base += 32) {
-            int len = 0, np = 0, cu = 0;
-            if (base + lane < p.batch) {
-                len = p.seq_lens[base + lane];
-                cu = p.cu_seqlens[base + lane];
-                np = len > 0 ? (int)(((int64_t)len + p.block_size - 1) / p.block_size) : 0;
-                if (np > p.max_pages) np = p.max_pages;
-            }
-            int64_t end = np;
+        unit = 0;
+        if (at < starts[kDqChunks]) {
+            int c = 0;      // the part of the sequences that unit `at` lies in: the last that starts at or ahead of it
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t t = __shfl_up_sync(kAll, end, o);
-                if (lane >= o) end += t;
+            for (int step = kDqChunks / 2; step > 0; step >>= 1)
+                if (starts[c + step] <= at) c += step;
+            int64_t rem = at - starts[c];
+            int b = c * chunk, whole_pages, rest;
+            int64_t n = units_of(b, whole_pages, rest);
+            for (int j = 1; j < chunk && rem >= n; j++) {
+                rem -= n;
+                n = units_of(++b, whole_pages, rest);
             }
-            end += run;
-            const int64_t start = end - np;
-            run = __shfl_sync(kAll, end, 31);
-            int j = 0;      // this lane's unit lies in sequence base + j
-            const int live = p.batch - base < 32 ? p.batch - base : 32;
-#pragma unroll 4
-            for (int i = 0; i < live; i++) j += __shfl_sync(kAll, end, i) <= at ? 1 : 0;
-            const bool here = j < live && src == 1;
-            const int pg = (int)(at - __shfl_sync(kAll, start, j & 31));
-            const int left = __shfl_sync(kAll, len, j & 31) - pg * p.block_size, row = __shfl_sync(kAll, cu, j & 31) + pg * p.block_size;
-            if (here) {
-                const int b = base + j;
+            src = 0;
+            if (rem < n) {
+                const int64_t pg = rem / units < whole_pages ? rem / units : whole_pages;
+                unit = (int)(rem - pg * units);
+                ntok = p.block_size;
+                if (pg == whole_pages) {
+                    int k_units, v_first;
+                    live(rest, k_units, v_first);
+                    if (unit >= k_units) unit += v_first - k_units;
+                    ntok = rest;
+                }
+                row0 = p.cu_seqlens[b] + (int)pg * p.block_size;
                 const int64_t tbl = p.page_indptr ? (int64_t)p.page_indptr[b] : (int64_t)b * p.max_pages;
                 const int64_t page = !p.page_indptr || tbl + pg < (int64_t)p.page_indptr[b + 1] ? (int64_t)p.page_indices[tbl + pg] : -1;
-                ntok = left < p.block_size ? left : p.block_size;
-                row0 = row;
-                if ((uint64_t)page >= (uint64_t)p.num_blocks) {  // never form an address from it: the rows stay unwritten
-                    if (unit == 0 && lane < 30) atomicAdd(&g_dequant_skipped, 1);      // the last two units are looked up again
-                    src = 0;
-                } else {
-                    src = reinterpret_cast<uint64_t>(p.kv_cache) + (uint64_t)page * half_rows * p.slot_bytes;
-                }
+                if ((uint64_t)page < (uint64_t)p.num_blocks) src = reinterpret_cast<uint64_t>(p.kv_cache) + (uint64_t)page * half_rows * p.slot_bytes;
+                // else never form an address from it: the rows stay unwritten (the last two units are looked up again)
+                else if (unit == 0 && lane < 30) atomicAdd(&g_dequant_skipped, 1);
             }
-            if (__all_sync(kAll, src != 1)) break;
         }
+        __syncwarp();
     };
     // The slots of unit i into stage s: neighbouring rows are neighbours in the cache, so one copy for the K and one for the V rows.
     auto issue = [&](int i, int s) {
