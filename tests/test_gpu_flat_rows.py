@@ -150,3 +150,40 @@ def test_zeros_keep_their_sign_in_many_rows(oracle, dim, n):
         assert (want == 0).any()
         got = _cabi.dequantize_flat(torch.from_numpy(packed).to(DEV), torch.from_numpy(norms).to(DEV), signs.to(DEV), dim, bits)
         np.testing.assert_array_equal(got.cpu().numpy().view(np.int32), want.view(np.int32), err_msg=f"bits {bits}")
+
+
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _same_as_short_calls(oracle, dim, n, dtype, widths=(1, 2, 3, 4)):
+    """One call of n rows, there and back, against the same rows in calls short enough for the four-lane kernels, and the first and last against the oracle."""
+    padded = 1 << (dim - 1).bit_length()
+    short = {64: 16000, 128: 9000, 256: 1900}[padded]
+    signs = synthetic.make_signs(padded, 42)
+    x, on_gpu = _rows(n, dim, dtype, dim + n).to(DEV), signs.to(DEV)
+    for bits in widths:
+        for cache_order in (False, True):
+            p, norms = _cabi.quantize_flat(x, on_gpu, bits, cache_order=cache_order)
+            out = _cabi.dequantize_flat(p, norms, on_gpu, dim, bits, cache_order=cache_order)
+            for i in range(0, n, short):
+                few_p, few_norms = _cabi.quantize_flat(x[i:i + short], on_gpu, bits, cache_order=cache_order)
+                assert torch.equal(p[i:i + short], few_p), (bits, cache_order, i)
+                assert torch.equal(norms[i:i + short].nan_to_num(7.0), few_norms.nan_to_num(7.0))
+                few = _cabi.dequantize_flat(few_p, few_norms, on_gpu, dim, bits, cache_order=cache_order)
+                nan = few.isnan()
+                assert torch.equal(out[i:i + short].isnan(), nan)
+                assert torch.equal(out[i:i + short].masked_fill(nan, 0).view(torch.int32), few.masked_fill(nan, 0).view(torch.int32)), (bits, cache_order, i)
+            if not cache_order:
+                for part in (slice(0, 40), slice(n - 40, n)):
+                    want_p, want_n = oracle.quantize_flat(x[part].float().cpu().numpy(), signs.numpy(), bits)
+                    np.testing.assert_array_equal(p[part].cpu().numpy(), want_p)
+                    np.testing.assert_array_equal(norms[part].cpu().numpy(), want_n)
+                    np.testing.assert_array_equal(out[part].cpu().numpy(), oracle.dequantize_flat(want_p, want_n, signs.numpy(), dim, bits))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim,per_sm", [(64, 110), (64, 332), (128, 64), (128, 96), (96, 64), (72, 64), (256, 13), (256, 27), (136, 13), (136, 32)])
+def test_rows_an_sm_where_the_kernels_change(oracle, dim, per_sm, dtype):
+    for n in (per_sm * _sms(), per_sm * _sms() + 1):
+        _same_as_short_calls(oracle, dim, n, dtype)

@@ -3,17 +3,21 @@
 
 namespace tq {
 
-// From how many rows on this kernel is the faster one (quantize and dequantize, 4 bits, in us, four lanes a row first: 128 wide 65536 rows 31.4 / 22.8,
-// 131072 53.4 / 37.9, 10000 13.8 / 11.4, 5000 9.3 / 13.7; 96 wide 60000 rows 28.1 / 19.8; 64 wide 120000 28.2 / 19.8, 20000 10.5 / 9.4, 8000
-// 9.5 / 9.4; 256 wide 60000 56.7 / 43.0, 5000 17.4 / 11.6): the time of one unit bounds fewer.
-static int64_t quantize_lanes_from(int padded) { return padded == 64 ? 16384 : padded == 128 ? 8192 : 4096; }
+// Rows an SM above which this kernel is the faster one (us on 148 SMs, 4 bits, the four-lane kernel first).  128 wide: up to 64 an SM the blocks of 64 rows of that
+// one are a wave (9472 rows 5.4 / 4.8, at 2 bits 4.7 / 5.8, bf16 4.5 / 5.8; 10000 6.8 / 4.8, 2 bits 6.9 / 5.8, bf16 6.7 / 6.2; 56832 13.4 / 8.4).  64 wide:
+// 16384 rows 5.1 / 3.4, 49152 8.1 / 5.0.  256 wide: 4096 rows 7.1 / 6.0, 20000 12.2 / 9.1 (136 wide).  The time of one unit bounds fewer.
+static int quantize_lanes_from(int padded) { return padded == 64 ? 110 : padded == 128 ? 64 : 27; }
 // Calls that this kernel takes: many 16-bit rows of a multiple of 8 elements padded to 64, 128 or 256, input and codes on 16 bytes, and a map that can be made.
 // Returns false, having done nothing, for others.
 bool quantize_lanes(const void* x, int x_dtype, int64_t n, int dim, int padded, const float* signs, int bits, bool cache_order, uint8_t* packed, float* norms,
                     void* stream, int* rc) {
-    if (padded < 64 || n < quantize_lanes_from(padded) || n >= 0x7fffff00 || (x_dtype != TQ_F16 && x_dtype != TQ_BF16) || dim % 8 != 0 || (uintptr_t)x % 16 != 0 ||
+    if (padded < 64 || n >= 0x7fffff00 || (x_dtype != TQ_F16 && x_dtype != TQ_BF16) || dim % 8 != 0 || (uintptr_t)x % 16 != 0 ||
         (uintptr_t)packed % 16 != 0 || (uintptr_t)norms % 4 != 0)
         return false;
+    int sms = 0;
+    *rc = device_sm_count(&sms);
+    if (*rc != TQ_OK) return true;
+    if (n <= (int64_t)quantize_lanes_from(padded) * sms) return false;
     struct Tables {
         RowBins t[3][4];
         Tables() {
@@ -44,9 +48,6 @@ bool quantize_lanes(const void* x, int x_dtype, int64_t n, int dim, int padded, 
     p.scale = t.scale;
     memcpy(p.bins, t.bins, sizeof(p.bins));
     memcpy(p.bounds, t.bounds, sizeof(p.bounds));
-    int sms = 0;
-    *rc = device_sm_count(&sms);
-    if (*rc != TQ_OK) return true;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool bf = x_dtype == TQ_BF16;
     if (padded == 64) *rc = bf ? launch_lane_rows<__nv_bfloat16, 64, 0, true>(p, sms, s) : launch_lane_rows<__half, 64, 0, true>(p, sms, s);

@@ -232,10 +232,16 @@ static int launch_dequantize_lanes(const DequantRowsParams& p, int bits, int sms
     return bits == 4 ? launch_dequantize_lanes<PD, 4>(p, sms, stream) : bits == 3 ? launch_dequantize_lanes<PD, 3>(p, sms, stream) : launch_dequantize_lanes<PD, 2>(p, sms, stream);
 }
 
-// From how many rows on this kernel is the faster one (quantize and dequantize of bf16, 4 bits, in us, the four-lane kernel first: 128 wide 10000 rows
-// 13.3 / 12.3, 48000 25.9 / 19.4, 131072 53.8 / 44.5, 3000 9.1 / 9.1; 256 wide 3000 rows 17.2 / 13.7, 60000 56.8 / 49.9; 64 wide 40000 rows
-// 12.0 / 13.6, 64000 18.2 / 15.2, 120000 28.1 / 25.7).
-static int64_t lanes_from(int padded) { return padded == 64 ? 49152 : padded == 128 ? 8192 : 2048; }
+// Rows an SM above which this kernel is the faster one (us on 148 SMs, the four-lane kernel first).  128 wide: up to 64 an SM the blocks of 64 rows of that one
+// are a wave (4 bits, 9472 rows 3.1 / 4.1; 10000 5.9 / 4.1, 60000 13.7 / 10.7; 72 wide 9472 2.8 / 3.8, 10000 4.6 / 3.8).  At 2 bits its output
+// is what counts there, so only whole rows (9472 3.3 / 4.8, 12500 3.9 / 4.9, 16000 5.7 / 5.0, 48000 9.9 / 7.2; 72 wide 60000 7.8 / 9.5, 96 wide
+// 10.0 / 10.7).  256 wide: 2048 rows 5.1 / 3.5, 60000 25 / 16; 136 ... 192 wide at 2 bits 4736 rows 4.1 / 4.4, 7200 5.8 / 4.6.  64 wide: 49152
+// 5.5 / 4.1, 131072 12.5 / 8.6.
+static int lanes_from(int dim, int padded, int bits) {
+    if (padded == 64) return 332;
+    if (padded == 128) return bits > 2 ? 64 : dim == 128 ? 96 : -1;
+    return bits > 2 || dim == 256 ? 13 : 32;
+}
 static uint32_t lanes_below(int padded, int bits) {
     return padded == 64 ? (bits == 2 ? DequantRowsShape<64, 2>::kBelow : DequantRowsShape<64, 4>::kBelow)
          : padded == 128 ? (bits == 2 ? DequantRowsShape<128, 2>::kBelow : DequantRowsShape<128, 4>::kBelow)
@@ -245,8 +251,13 @@ static uint32_t lanes_below(int padded, int bits) {
 // whose shared window has room for the table's place.  Returns false, having done nothing, for others.
 bool dequantize_lanes(const uint8_t* packed, const float* norms, int64_t n, int dim, int padded, const float* signs, int bits, bool cache_order, float* out,
                       void* stream, int* rc) {
-    if (padded < 64 || n < lanes_from(padded) || dim % 8 != 0 || bits < 2 || (uintptr_t)packed % 16 != 0 || (uintptr_t)out % 16 != 0 || (uintptr_t)norms % 4 != 0)
+    if (padded < 64 || dim % 8 != 0 || bits < 2 || (uintptr_t)packed % 16 != 0 || (uintptr_t)out % 16 != 0 || (uintptr_t)norms % 4 != 0)
         return false;
+    int sms = 0;
+    *rc = device_sm_count(&sms);
+    if (*rc != TQ_OK) return true;
+    const int from = lanes_from(dim, padded, bits);
+    if (from < 0 || n <= (int64_t)from * sms) return false;
     bool fits = false;
     *rc = device_shared_window_fits(lanes_below(padded, bits), &fits);
     if (*rc != TQ_OK) return true;
@@ -262,9 +273,6 @@ bool dequantize_lanes(const uint8_t* packed, const float* norms, int64_t n, int 
     p.scale = (float)(1.0 / std::sqrt((double)padded));
     float bnd[15];
     host_codebook(padded, bits, p.cen, bnd);
-    int sms = 0;
-    *rc = device_sm_count(&sms);
-    if (*rc != TQ_OK) return true;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     *rc = padded == 64 ? launch_dequantize_lanes<64>(p, bits, sms, s) : padded == 128 ? launch_dequantize_lanes<128>(p, bits, sms, s) : launch_dequantize_lanes<256>(p, bits, sms, s);
     return true;
