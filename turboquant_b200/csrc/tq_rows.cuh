@@ -47,7 +47,7 @@ struct LaneRowsParams {
     int bits, cache_order, count;     // flat: bits of a code, first value of a byte in its high bits; count of boundaries
     float bin_scale, scale;
     float2 bins[kRowBins];            // {the largest w not above the bin's boundary (or +inf), the bits of: boundaries in lower bins}
-    float bounds[15];
+    float bounds[15];                 // +inf from count on
 };
 
 template <int PD>
@@ -103,7 +103,8 @@ __device__ __forceinline__ void code_into(uint32_t& word, float w, uint32_t entr
     asm("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %1, %2;\n\t@q add.u32 %0, %0, %3;\n\t}" : "+r"(word) : "f"(w), "f"(most), "r"(1u << at));
 }
 
-// One row by the whole warp, lane l on elements E l .. E l + E - 1, with divisions and with the signs as factors; the codes, four bits each in the order of
+// One row by the whole warp, for what the common path leaves out (a row at a time: where all rows are such ones the call takes two to four times what
+// the kernels take that divide for every element, 8000 x 8 rows of 96 with an infinity 179 us against 46, 60000 x 128 with signs of 1.5 82 against 15).  Lane l on elements E l .. E l + E - 1, with divisions and with the signs as factors; the codes, four bits each in the order of
 // code_into, replace the row's first PD / 2 bytes in `row`.  elem(i): shared-memory address of element i.
 template <typename T, int PD, bool FLAT, typename F>
 __device__ __noinline__ void slow_row(const LaneRowsParams& p, F elem, uint32_t row, float norm, int lane) {
@@ -140,8 +141,8 @@ __device__ __noinline__ void slow_row(const LaneRowsParams& p, F elem, uint32_t 
     for (int i = 0; i < E; i++) {
         const float y = __fmul_rn(x[i], p.scale);
         uint32_t c = 0;
-#pragma unroll 1
-        for (int k = 0; k < (FLAT ? p.count : 15); k++) c += p.bounds[k] < y ? 1u : 0u;
+#pragma unroll
+        for (int k = 0; k < 15; k++) c += p.bounds[k] < y ? 1u : 0u;      // fewer bits: the rest are +inf
         if (y != y) c = FLAT ? p.count : 15;      // torch's bucketize sends NaN to the last bucket
         codes |= c << (4 * (FLAT ? i : i ^ 1));
     }
@@ -535,6 +536,7 @@ static RowBins make_row_bins(int padded, int bits) {
         memcpy(&bits, &below, 4);
         r.bins[k] = make_float2(inside, bits);
     }
+    for (int i = count; i < 15; i++) r.bounds[i] = INFINITY;
     return r;
 }
 template <typename T, int PD, int HD, bool FLAT>
