@@ -90,7 +90,7 @@ def test_other_pages_and_slots(oracle, dim, heads, block, slot, listed, wide):
 
 @pytest.mark.parametrize("dim", [64, 128])
 def test_many_sequences(oracle, dim):
-    """More sequences than a warp has lanes, most of them short or empty; more units a warp than it looks up at a time."""
+    """More sequences than a warp has lanes, most of them short or empty; a job of many units a warp against the oracle."""
     rng = np.random.default_rng(dim)
     _check(oracle, dim, 1, wide=False, lens=[int(n) for n in rng.integers(0, 40, 100)])
     _check(oracle, dim, 8, wide=True, lens=[int(n) for n in rng.integers(0, 70, 70)])
@@ -150,3 +150,37 @@ def test_more_sequences_than_parts_of_the_work_list(oracle, dim, heads, batch, l
     lens[:9], lens[100:180], lens[-5:] = 0, 0, 0
     lens[200:230] = 1
     _check(oracle, dim, heads, wide=wide, lens=[int(n) for n in lens], listed=listed)
+
+
+@pytest.mark.parametrize("dim,dtype", [(64, torch.bfloat16), (96, torch.float16), (128, torch.bfloat16), (128, torch.float32), (256, torch.bfloat16)])
+def test_more_units_a_warp_than_are_looked_up_at_a_time(dim, dtype):
+    """Over sixty units a warp (32 are looked up at a time, twice over), three sequences with part pages: one call of the large blocks against calls of the small ones."""
+    heads, padded = 16, 1 << (dim - 1).bit_length()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = 62 * sms * (20 if dim == 64 else 12) * (16 if dim == 256 else 32)
+    pages = rows // (2 * 16 * heads) + 1
+    lens = [pages * 10 - 3, 37, pages * 6 + 40]
+    per = [(n + 15) // 16 for n in lens]
+    g = torch.Generator(device=DEV)
+    g.manual_seed(dim)
+    cache = torch.randint(0, 256, (2, sum(per), 16, heads, SLOT[dim]), dtype=torch.uint8, device=DEV, generator=g)
+    norms = torch.rand(cache.shape[:-1] + (1,), device=DEV, generator=g).to(torch.float16) * 20
+    cache[..., padded // 2:padded // 2 + 2] = norms.view(torch.uint8)
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(dim)).to(torch.int32).to(DEV)
+    signs = synthetic.make_signs(padded, 42).to(DEV)
+    table = torch.zeros(3, max(per), dtype=torch.int32, device=DEV)
+    for b, at in enumerate((0, per[0], per[0] + per[1])):
+        table[b, :per[b]] = order[at:at + per[b]]
+    cu = [0, lens[0], lens[0] + lens[1], sum(lens)]
+    k, v = (torch.full((sum(lens) + 1, heads, dim), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+    _cabi.dequant_paged(cache, table, torch.tensor(lens, dtype=torch.int32, device=DEV), torch.tensor(cu, dtype=torch.int32, device=DEV), signs, k, v)
+    assert bool((k[-1] == 7.0).all()) and bool((v[-1] == 7.0).all())
+    step = 100                                                         # pages of a small call
+    for b in range(3):
+        for first in range(0, per[b], step):
+            n = min(lens[b] - first * 16, step * 16)
+            few_k, few_v = (torch.empty(n, heads, dim, dtype=dtype, device=DEV) for _ in range(2))
+            _cabi.dequant_paged(cache, table[b:b + 1, first:first + step].contiguous(), torch.tensor([n], dtype=torch.int32, device=DEV),
+                                torch.tensor([0, n], dtype=torch.int32, device=DEV), signs, few_k, few_v)
+            at = cu[b] + first * 16
+            assert torch.equal(k[at:at + n], few_k) and torch.equal(v[at:at + n], few_v), (b, first)

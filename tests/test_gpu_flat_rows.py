@@ -79,9 +79,10 @@ def test_signs_beyond_one(oracle, dim):
                 np.testing.assert_array_equal(p.cpu().numpy(), oracle.quantize_flat(x.float().numpy(), signs.numpy(), bits)[0], err_msg=f"{name} {bits}")
 
 
-@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8200 + 17), (96, 8192 + 31), (72, 8195), (64, 49152), (64, 49152 + 33), (256, 2048), (256, 2048 + 15), (192, 2051)])
+@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8200 + 17), (96, 8192 + 31), (72, 8195), (64, 49152), (64, 49152 + 33), (256, 2048), (256, 2048 + 15), (192, 2051),
+                                   (128, 14300), (96, 9600 + 31), (72, 9603), (192, 4803)])
 def test_dequantization_of_many_rows(oracle, dim, n):
-    """A lane (two lanes) a row: the fewest rows that go this way, part units, short rows, both pack orders, any sign vector."""
+    """Many rows, around the counts from which a lane (two lanes) takes a row: part units, short rows, both pack orders, any sign vector."""
     padded = 1 << (dim - 1).bit_length()
     rng = np.random.default_rng(dim + n)
     norms = rng.uniform(0.0, 30.0, n).astype(np.float32)
@@ -104,9 +105,10 @@ def test_dequantization_of_many_rows(oracle, dim, n):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8192 + 17), (96, 8192 + 31), (72, 8195), (64, 16384), (64, 16384 + 33), (256, 4096), (256, 4096 + 15), (192, 4099)])
+@pytest.mark.parametrize("dim,n", [(128, 8192), (128, 8192 + 17), (96, 8192 + 31), (72, 8195), (64, 16384), (64, 16384 + 33), (256, 4096), (256, 4096 + 15), (192, 4099),
+                                   (128, 9600 + 17), (96, 9600 + 31), (72, 9603)])
 def test_quantization_of_many_rows(oracle, dim, n, dtype):
-    """A lane (two lanes) a row: the fewest rows that go this way, part units, short rows, special rows, every width and both pack orders."""
+    """Many rows, around the counts from which a lane (two lanes) takes a row: part units, short rows, special rows, every width and both pack orders."""
     signs = synthetic.make_signs(1 << (dim - 1).bit_length(), 42)
     x = _rows(n, dim, dtype, 7 + dim + n)
     if dtype == torch.bfloat16:
@@ -132,7 +134,7 @@ def test_quantization_of_many_rows(oracle, dim, n, dtype):
             np.testing.assert_array_equal(norms.cpu().numpy(), torch.cat([b for _, b in parts]).cpu().numpy())
 
 
-@pytest.mark.parametrize("dim,n", [(64, 49152), (128, 8192), (256, 2048), (192, 2051)])
+@pytest.mark.parametrize("dim,n", [(64, 49152), (128, 14300), (256, 2048), (192, 4803)])
 def test_zeros_keep_their_sign_in_many_rows(oracle, dim, n):
     """Rows of repeated codes, whose sums cancel: the outputs' bits, which tell -0 from +0, with norms of zero among them."""
     padded = 1 << (dim - 1).bit_length()
@@ -187,3 +189,12 @@ def _same_as_short_calls(oracle, dim, n, dtype, widths=(1, 2, 3, 4)):
 def test_rows_an_sm_where_the_kernels_change(oracle, dim, per_sm, dtype):
     for n in (per_sm * _sms(), per_sm * _sms() + 1):
         _same_as_short_calls(oracle, dim, n, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim", [40, 64, 72, 96, 128, 136, 256])
+def test_several_units_a_warp(oracle, dim, dtype):
+    """Three units of every warp and a part of one: each stage of a warp's ring is filled again after it has been read out."""
+    padded = 1 << (dim - 1).bit_length()
+    a_round = _sms() * (20 if padded == 64 else 12) * (16 if padded == 256 else 32)
+    _same_as_short_calls(oracle, dim, 3 * a_round + 5, dtype)

@@ -148,3 +148,30 @@ def test_signs_other_than_one_are_factors(oracle, d):
         want = np.full((2, 44, 16, 8, _slot(d)), 0xEE, np.uint8)
         oracle.write_kv_cache(want, x.float().numpy(), x.float().numpy(), signs.numpy(), slots.numpy(), d)
         _same(_write(x.to(DEV), x.to(DEV), slots.to(DEV), 44, 8, d, signs), want)
+
+
+@pytest.mark.parametrize("d,heads,tokens", [(64, 8, 600), (256, 3, 1500), (96, 5, 1700)])
+def test_token_strides_that_are_no_multiple_of_a_row(d, heads, tokens):
+    """K and V side by side with eight elements behind them, against the same rows dense."""
+    gen = torch.Generator().manual_seed(d)
+    both = torch.randn(tokens, 2 * heads * d + 8, generator=gen).to(torch.bfloat16).to(DEV)
+    k, v = (t.unflatten(1, (heads, d)) for t in (both[:, :heads * d], both[:, heads * d:2 * heads * d]))
+    signs = synthetic.make_signs(1 << (d - 1).bit_length(), 42)
+    nb = (tokens + 15) // 16
+    slots = torch.randperm(nb * 16, generator=gen)[:tokens].to(DEV)
+    np.testing.assert_array_equal(_write(k, v, slots, nb, heads, d, signs), _write(k.contiguous(), v.contiguous(), slots, nb, heads, d, signs, path="exact"))
+
+
+@pytest.mark.parametrize("d,heads", [(64, 8), (64, 3), (96, 8), (256, 5)])
+def test_several_units_a_warp(d, heads):
+    """Three units of every warp and a part of one, against the kernel that divides and searches for every element."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = 3 * sms * (20 if d == 64 else 12) * (16 if d == 256 else 32)
+    tokens = rows // (2 * heads) + 37
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(d + heads)
+    k, v = ((torch.randn(tokens, heads, d, generator=gen, device=DEV) * 2.0).to(torch.float16) for _ in range(2))
+    signs = synthetic.make_signs(1 << (d - 1).bit_length(), 42)
+    nb = (tokens + 15) // 16
+    slots = torch.randperm(nb * 16, generator=torch.Generator().manual_seed(2))[:tokens].to(DEV)
+    np.testing.assert_array_equal(_write(k, v, slots, nb, heads, d, signs), _write(k, v, slots, nb, heads, d, signs, path="exact"))

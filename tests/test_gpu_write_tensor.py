@@ -188,3 +188,18 @@ def test_strided_tiles_of_heads_and_tokens(oracle, golden, heads, tokens, dtype)
     d = both.to(DEV)
     for kd, vd in ((d[:, :heads], d[:, heads:2 * heads]), (d[:, :heads].contiguous(), d[:, heads:2 * heads])):
         np.testing.assert_array_equal(write(kd, vd, slots.to(DEV), nb, "tensor", H=heads, fill=0xEE).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("heads,tokens", [(1, 40), (8, 67), (3, 50)])
+def test_token_strides_that_are_no_multiple_of_a_row(oracle, golden, heads, tokens):
+    """K and V side by side with eight elements behind them."""
+    gen = torch.Generator().manual_seed(heads)
+    both = (torch.randn(tokens, 2 * heads * 128 + 8, generator=gen) * 2.0).to(torch.bfloat16)
+    k, v = (t.unflatten(1, (heads, 128)) for t in (both[:, :heads * 128], both[:, heads * 128:2 * heads * 128]))
+    nb = (tokens + 15) // 16
+    slots = torch.randperm(nb * 16, generator=gen)[:tokens]
+    want = np.full((2, nb, 16, heads, 80), 0xEE, np.uint8)
+    oracle.write_kv_cache(want, k.float().contiguous().numpy(), v.float().contiguous().numpy(), golden["signs_seed42_d128"], slots.numpy(), 128)
+    d = both.to(DEV)
+    kd, vd = (t.unflatten(1, (heads, 128)) for t in (d[:, :heads * 128], d[:, heads * 128:2 * heads * 128]))
+    np.testing.assert_array_equal(write(kd, vd, slots.to(DEV), nb, "tensor", H=heads, fill=0xEE).cpu().numpy(), want)
