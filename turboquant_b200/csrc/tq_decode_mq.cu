@@ -821,32 +821,16 @@ __global__ void __launch_bounds__(kMqThreads, 1) decode_mq_kernel(const __grid_c
     }
 }
 
-// cuTensorMapEncodeTiled through the runtime (no link-time dependency on the driver library)
-typedef CUresult (*MqEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static MqEncodeFn mq_encode_fn() {
-    static const MqEncodeFn fn = [] {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
-        return ok ? reinterpret_cast<MqEncodeFn>(sym) : nullptr;
-    }();
-    return fn;
-}
+bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                       const cuuint32_t* box, CUtensorMapSwizzle swizzle);
 
 // The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab.
 int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes) {
-    MqEncodeFn enc = mq_encode_fn();
-    TQ_REQUIRE(enc != nullptr, TQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)num_blocks * kPageTokens, 2};
     const cuuint64_t strides[2] = {dims[0], dims[0] * dims[1]};
     const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, 1u};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(kv_cache), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    TQ_REQUIRE(rc == CUDA_SUCCESS, TQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the cache (%d)", (int)rc);
+    TQ_REQUIRE(encode_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, kv_cache, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE), TQ_ERR_CUDA,
+               "cuTensorMapEncodeTiled failed for the cache, or is not available from this driver");
     return TQ_OK;
 }
 
