@@ -824,11 +824,11 @@ __global__ void __launch_bounds__(kMqThreads, 1) decode_mq_kernel(const __grid_c
 bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
                        const cuuint32_t* box, CUtensorMapSwizzle swizzle);
 
-// The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab.
-int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes) {
+// The cache as uint8 [2][num_blocks * 16][row_bytes] in boxes of box_bytes x 16 rows of one slab, or of both.
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes, int slabs) {
     const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)num_blocks * kPageTokens, 2};
     const cuuint64_t strides[2] = {dims[0], dims[0] * dims[1]};
-    const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kPageTokens, (cuuint32_t)slabs};
     TQ_REQUIRE(encode_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, kv_cache, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE), TQ_ERR_CUDA,
                "cuTensorMapEncodeTiled failed for the cache, or is not available from this driver");
     return TQ_OK;
@@ -845,7 +845,7 @@ int launch_decode_mq(const DecodeParams& d, int num_kv_heads, int64_t num_blocks
     mp.head_pairs = num_kv_heads / 2;
     mp.ncols = d.group;
     mp.causal = causal;
-    const int rc = encode_cache_map(&mp.cache_map, d.kv_cache, num_blocks, (int64_t)num_kv_heads * kSlotBytes, 160);
+    const int rc = encode_cache_map(&mp.cache_map, d.kv_cache, num_blocks, (int64_t)num_kv_heads * kSlotBytes, 160, 1);
     if (rc != TQ_OK) return rc;
     const int smem = (int)kMqSmemEnd;
     static bool configured[64] = {};

@@ -9,7 +9,7 @@
 //   * One block per SM = kGroups groups of kGroupWarps warps around one lookup table.  A group works alone (its own
 //     named barrier); the table, the longest part of a block's prologue, is filled before the dependency wait.
 //   * Plan on the device, by every warp for itself from seq_lens (no barrier): see SplitPlan.
-//   * A warp takes whole pages of its head: two tiled tensor copies (16 rows of the head's slot each, from K and from V) into its
+//   * A warp takes whole pages of its head: one tiled tensor copy (16 rows of the head's slot from K and 16 from V; see kSlabs) into its
 //     own ring of stages (eleven 16-byte asynchronous copies a lane filled the load/store queue: 40 / 8 heads, 32 ragged
 //     sequences 34.4 -> 27.5 us a step, head size 64 34 -> 28, 256 37 -> 32), codes looked up straight
 //     into mma.sync.m16n8k16 fragments (the scheme of tq_decode.cu: K bytes are A fragments of S = K^ Q^T, V nibbles of
@@ -49,6 +49,10 @@ struct SplitShape {
     // 32 ragged sequences x 4096, 8 queries: 87 -> 71 us; as a pair two tiles are slower (124 -> 140 us).
     static constexpr bool kPair = NT >= 3;
     static constexpr int kStages = NT > 1 ? 4 : PD == 256 ? 2 : 3;
+    // Slabs of a tensor copy's box: K and V of a page in one is up to 3 % faster (us, two boxes first: 10 x 2199 tokens, 32 / 8 heads of 96 18.1 / 17.6; 3 x 101 ...
+    // 406, 40 heads 12.34 / 12.12; 18 x 1156 ... 37010, 2 causal queries 74.6 / 73.7).  For pairs of warps it is neither (8 x 32768, 8 queries 167.3 / 169.3; 18 x
+    // 1156 ... 37010, 6 queries 117.8 / 115.6; 32 x 100 ... 4096, 8 queries 58.3 / 58.7): they keep two.
+    static constexpr int kSlabs = kPair ? 1 : 2;
     static constexpr int kRingBytes = kStages * kStageBytes;
     // registers decide the warps per SM: 16 accumulator + 8 query registers at head 64 (80 a thread), 32 + 16 at 128
     // (128), 64 + 32 at 256 (168)
@@ -76,7 +80,7 @@ struct SplitShape {
 };
 
 struct SplitParams {
-    alignas(64) CUtensorMap cache_map;   // uint8 [2][num_blocks * 16][H * slot], boxes of [1][16][kRow]
+    alignas(64) CUtensorMap cache_map;   // uint8 [2][num_blocks * 16][H * slot], boxes of [kSlabs][16][kRow]
     const void* q;
     const uint8_t* kv_cache;
     const int32_t* page_indices;
@@ -336,7 +340,7 @@ __device__ __forceinline__ void split_kept_plan(const SplitParams& p, SplitPlan&
     s.len = 0;
 }
 
-// One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V).  No multicast; x is a
+// One box of the cache into shared memory: bytes x ... of 16 token rows from row y of slab z (0: K, 1: V), or of both.  No multicast; x is a
 // multiple of the slot, hence of 16.
 __device__ __forceinline__ void split_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -487,7 +491,7 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
     __shared__ float sign_s[PD];
     __shared__ float max_s[F::kPair ? F::kWarps : 1][F::kCols + 1];  // a pair's maxima of a page that raises them (and its largest V norm), and whether it does
     __shared__ int raise_s[2][F::kPair ? F::kWarps : 1];
-    __shared__ uint64_t full_s[F::kWarps][F::kStages + F::kNormScale];   // a stage's two boxes have landed; and a word for the warp's scale of the V norms
+    __shared__ uint64_t full_s[F::kWarps][F::kStages + F::kNormScale];   // a stage's page has landed; and a word for the warp's scale of the V norms
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gg = warp / GW, wg = warp % GW;      // group of the block, warp of the group
     const int g = lane >> 2, tg = lane & 3;
@@ -657,8 +661,8 @@ __global__ void __launch_bounds__(SplitShape<PD, NT>::kThreads, 1) decode_split_
                 const uint32_t bar = full_at + 8 * to, dst = ring_at + to * F::kStageBytes;
                 split_expect(bar, i < n ? F::kStageBytes : 0);      // no page: the warps of a pair stay at the same stage
                 if (i < n) {
-                    split_box(dst, &p.cache_map, x, id * kPageTokens, 0, bar);
-                    split_box(dst + F::kHalfBytes, &p.cache_map, x, id * kPageTokens, 1, bar);
+#pragma unroll
+                    for (int z = 0; z < 2; z += F::kSlabs) split_box(dst + z * F::kHalfBytes, &p.cache_map, x, id * kPageTokens, z, bar);
                 }
             }
         };
@@ -1240,11 +1244,7 @@ __global__ void __launch_bounds__(RW == 16 ? 512 : 128) merge_split_kernel(const
 // ---------------------------------------------------------------------------------------------
 int device_sm_count(int* out);
 cudaEvent_t decode_event(int i);
-int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes);
-
-static int split_box_bytes(int padded) {
-    return padded == 64 ? SplitShape<64, 1>::kRow : padded == 128 ? SplitShape<128, 1>::kRow : SplitShape<256, 1>::kRow;
-}
+int encode_cache_map(CUtensorMap* map, const void* kv_cache, int64_t num_blocks, int64_t row_bytes, int box_bytes, int slabs);
 
 static size_t split_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -1277,7 +1277,9 @@ static int launch_split(SplitParams& p, int ctas, cudaStream_t s) {
     p.head_sets = p.kv_heads / p.head_set;
     p.item_cost = F::kItemCost;
     p.inv_warps = 1.0f / (float)(ctas * F::kWarps);
-    const int rc = p.batch > kSplitSelf ? launch_split_kernel<PD, NT, true>(p, s) : launch_split_kernel<PD, NT, false>(p, s);
+    int rc = encode_cache_map(&p.cache_map, p.kv_cache, p.num_blocks, (int64_t)p.kv_heads * p.slot_bytes, F::kRow, F::kSlabs);
+    if (rc != TQ_OK) return rc;
+    rc = p.batch > kSplitSelf ? launch_split_kernel<PD, NT, true>(p, s) : launch_split_kernel<PD, NT, false>(p, s);
     if (rc != TQ_OK) return rc;
     if (cudaEvent_t mid = decode_event(1)) TQ_CUDA(cudaEventRecord(mid, s));
     // A head has about groups / (sequences x heads) parts at most: a warp fetches eight at a time, so up to eight go to one warp
@@ -1314,8 +1316,6 @@ int split_decode(const void* q, int q_dtype, int batch, int nq, int real_q_heads
     p.out = out;
     p.out_lse = out_lse;
     p.num_blocks = num_blocks;
-    const int map_rc = encode_cache_map(&p.cache_map, kv_cache, num_blocks, (int64_t)num_kv_heads * slot_bytes, split_box_bytes(padded));
-    if (map_rc != TQ_OK) return map_rc;
     p.kv_begin = kv_begin;
     p.kv_end = kv_end;
     p.batch = batch;
