@@ -335,7 +335,7 @@ int tq_fault_counts(int32_t* counts3);
 
 /* Rows (K and V rows of every token and head, tile padding included) the tensor-core write kernel
  * has processed on the current device since the library was loaded, and how many of them it
- * re-derived with the exact path because a value lay within 2^-18 of a code boundary or the
+ * re-derived with the exact path because a value lay within 3.8e-6 (2^-18 (1 - 2^-8)) of a code boundary or the
  * row's norm was zero, huge or not finite.  Synchronises the device. */
 int tq_write_guard_stats(int64_t* rows_total, int64_t* rows_exact);
 

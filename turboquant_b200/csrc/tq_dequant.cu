@@ -19,8 +19,8 @@
 // whole-register adds.  Rows reach and leave the registers through shared memory: each warp copies the slots of unit n + 2 there while it works
 // on unit n, and stages its output so that a store instruction covers whole rows.
 //   8 ragged sequences of 5000 .. 13000 tokens x 8 heads of 128 -> bf16 (336 MB): 100 us with two lanes a row (a shuffle per element for
-//   h = 64, on the pipe of the lookups and stores; 4 warps a scheduler, work found row by row) -> 71.6 us = 72 % of the copy rate.  Heads of 64, 8 x 1000 .. 8000 tokens: 41.4 -> 17.3 us, of
-//   256, 8 x 1000 .. 4000: 73.7 -> 44.2, of 96, 3 x 1000 .. 16000 x 32 heads: 144 -> 87 (eight and two lanes a row before).  What bounds
+//   h = 64, on the pipe of the lookups and stores; 4 warps a scheduler, work found row by row) -> 70.4 us = 73 % of the copy rate.  Heads of 64, 8 x 1000 .. 8000 tokens (28300): 40.1 -> 18.0 us,
+//   of 256, 8 x 1000 .. 4000 (20100): 89.0 -> 47.4, of 96, 3 x 1000 .. 16000 (31400) x 32 heads: 191 -> 104 (eight and two lanes a row before).  What bounds
 //   it now is that pipe (74 % busy: 128 wavefronts of lookups, 192 of output, 32 of signs in about 430 a unit) at three warps a scheduler.
 //   Output by tensor copies of 16 rows x 128 bytes in place of the read-back: 123 us.
 #include <cmath>

@@ -150,9 +150,9 @@ __global__ void __launch_bounds__(kFlatWarps * 32) fwht_kernel(const __grid_cons
 // plain kernels below, which stay for other lengths; the quotient is the FMA-refined reciprocal with their division as the
 // exception (see tq_write.cu).  The code of a value comes from a table over bins that hold at most one boundary each (the search
 // of the cache write, with bins scaled to the row's length).
-// 65536 rows of 128 fp16 values, 4 bits: quantize 107 us with the plain kernel (a warp a row, butterflies in shared memory, a
-// compare per boundary: 20 times the memory floor) -> 15 us here (dequantize 77 -> 13 us); the limits are instruction issue and the shuffles of stages 2 and 4.
-// Many rows go a lane a row: 16-bit ones to codes by tq_flat_quant.cu, codes to rows by tq_flat_rows.cu.
+// 65536 rows of 128, 4 bits: quantize 107 us with the plain kernel (a warp a row, butterflies in shared memory, a
+// compare per boundary: 20 times the memory floor) -> 16 us here (dequantize 77 -> 14 us); the limits are instruction issue and the shuffles of stages 2 and 4.
+// That many rows come here from fp32 only: many 16-bit ones go to codes a lane a row by tq_flat_quant.cu (10 - 12 us), codes to rows by tq_flat_rows.cu (11).
 // ---------------------------------------------------------------------------------------------
 constexpr int kRowsWarps = 8, kRowsThreads = kRowsWarps * 32;
 constexpr int kFlatBinZero = 144, kFlatBins = 2 * kFlatBinZero + 1;      // |y| <= 1.5 in bins of sqrt(128 / padded) / 64: 136 at 256

@@ -944,8 +944,9 @@ int generic_write(void* kv_cache, int64_t num_blocks, int block_size, int num_kv
                                                                                             : launch_write_row_warp<__nv_bfloat16>(p, s));
         return TQ_OK;
     }
-    // large jobs of the smallest head: a lane group walks all rows of its token (96 us against 101 for 32768 tokens x
-    // 8 heads); small jobs (a decode step's new tokens) and the larger heads, where the index arithmetic is a smaller
+    // (large 16-bit writes with aligned rows and slots go a lane a row: tq_write_rows.cu)
+    // large jobs of the smallest head: a lane group walks all rows of its token (measured with bf16 rows, 32768 tokens x
+    // 8 heads: 96 us against 101); smaller jobs and the larger heads, where the index arithmetic is a smaller
     // share and fewer groups in flight cost more than it saves (347 us against 337 at head 256): a row per group
     p.walk = num_tokens >= 8192 && p.g.padded == 64 ? 2 * num_kv_heads : 1;
     const int64_t items = num_tokens * (2 * num_kv_heads / p.walk);

@@ -1,5 +1,5 @@
 // Quantization of 16-bit rows padded to 64, 128 or 256, a lane (two lanes of one of 256) a row: the cache write of large 16-bit writes at head sizes other than
-// 128 (tq_write_rows.cu) and the flat quantizer of many rows (tq_flat_rows.cu).
+// 128 (tq_write_rows.cu) and the flat quantizer of many rows (tq_flat_quant.cu).
 //
 // The arithmetic is the torch quantizer's (turboquant/quantizer.py:77-91 in the reference) for every element, as in tq_write.cu: eight
 // interleaved sum-of-squares accumulators without FMA, IEEE sqrt and division, signs, butterflies h = 1 .. PD / 2 in order, code = number of
@@ -15,9 +15,10 @@
 //   * The search: bins of w (whose standard deviation is about 1) hold at most one boundary each; {that boundary, boundaries in lower bins}
 //     is one 8-byte lookup, 16 columns (served half a warp at a time: no two lanes meet in a bank).
 //   * Rows of 96: the stages below 64 leave the 32 zeros of the padding alone.
-// What bounds it is instruction issue and the FMA pipe's heavy half (each about 60 % busy) at five (64) and three warps a scheduler; with copies and
-// stores alone a write of 32768 x 8 rows of 128 takes 34 us of its 61.  Rows by 16-byte asynchronous copies in place of the tensor copies cost 2 - 6 % more, two
-// lanes a row of 128 (five warps a scheduler) 17 %.
+// What bounds it is instruction issue (54 - 62 % of the active cycles in writes of 96, 256 and 64) and the FMA pipe's heavy half (49 - 57 %) at five (64) and
+// three warps a scheduler; the flat quantizer of 65536 rows, two units a warp at most, waits for its first copies.  An instance for the cache write of
+// 128, not kept (61 us for 32768 x 8), took 34 us with copies and stores alone, 2 - 6 % more with rows by 16-byte asynchronous copies in place of the
+// tensor copies, and 17 % more with two lanes a row (five warps a scheduler).
 #pragma once
 
 #include <cuda.h>  // CUtensorMap and its enums only

@@ -1,7 +1,8 @@
 // Cache write of large 16-bit K / V at head sizes 96, and padded 64 and 256 (kernel and mapping: tq_rows.cuh).
-//   32768 tokens x 8 heads of 64, bf16: 93.5 us with eight lanes a row (a shuffle per element for each of stages 1, 2, 4, a four-step search) -> 32.8;
-//   16384 x 8 of 256: 166 -> 77.5 (floors 14 and 26).  Heads of 96: 2048 x 32 fp16 19.0 -> 13.8, 16384 x 8 bf16 33.9 -> 25.9 (two lanes
-//   a row of 128 before; the tensor-core kernel of tq_write.cu, padded, 38.7).  Heads of 128 this way take 61 us, the tensor-core kernel 58.
+//   32768 tokens x 8 heads of 64, bf16: 91 us with eight lanes a row (a shuffle per element for each of stages 1, 2, 4, a four-step search) -> 32.4;
+//   16384 x 8 of 256: 167 -> 65.8 (floors 14 and 26).  Heads of 96: 2048 x 32 fp16 19.0 -> 13.7, 16384 x 8 bf16 33.0 -> 25.3 (two lanes
+//   a row of 128 before; the tensor-core kernel of tq_write.cu, padded, 38.7).  Heads of 128 this way, in an instance that was not kept, took 61 us (32768 x 8);
+//   the tensor-core kernel takes 55.8.
 #include "tq_rows.cuh"
 
 namespace tq {
